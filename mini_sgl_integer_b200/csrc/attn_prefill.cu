@@ -1,22 +1,27 @@
 // Prefill / extend attention over the int8 paged pool: many new tokens per sequence, causal inside the new
 // tokens, a cached prefix in front of them.  Same arithmetic as the decode kernel (attn.cu), bit for bit.
 //
-// A CTA owns one (sequence, KV head, tile of 128 / G consecutive new tokens): 128 query rows = tokens x the G
-// query heads of the KV head, 16 rows per warp.  The integer MMA runs with the QUERY rows on M:
+// A CTA owns one (sequence, KV head, tile of 64 / G consecutive new tokens): 64 query rows = tokens x the G query
+// heads of the KV head, 16 rows per PAIR of warps.  The integer MMA runs with the QUERY rows on M:
 //   scores [16 rows x 8 keys]  = Q [16 x 128] . K^T [128 x 8]        (4 k-steps of 32 d; Q stays in registers)
 //   out    [16 rows x 8 d]     = W [16 x 32 keys] . V [32 x 8]       (one k-step per pair of pages, 16 d-tiles)
 // The 8 columns of a score tile are mapped to the keys {4c, 4c+1} (first tile of a page) and {4c+2, 4c+3} (second
 // tile) for column pair c, so a lane ends up with the scores of the keys 4c .. 4c+3 of a page for its two rows:
-// exactly the bytes its A operand of the PV product needs (the probability limbs never leave registers), and the
-// V page is read as the B operand straight from the pool's operand order (v_chunk_offset).
+// exactly the bytes its A operand of the PV product needs, and the V page is read as the B operand straight from the
+// pool's operand order (v_chunk_offset).  Of every 64 keys the two warps of a pair score 32 each; their probability
+// limbs meet in shared memory, and each warp multiplies all 64 with its half of d.  (One warp per 16 rows needs 128
+// accumulator registers: two CTAs per SM then spill.)
 //
 // The softmax is exact (LUT exponential with truncation), so nothing can be rescaled on the fly: the keys are
 // walked three times per tile - row maxima, sums of exponentials, then probabilities and PV - and the scores
-// are recomputed each time (16 MMAs per 32 keys, negligible beside the per-score fixed-point work).  Keeping
-// them instead would take 4 B x 128 rows per key: 2 MB for 4096 keys, beyond shared and tensor memory.  K is
-// therefore read three times and V once per tile, from L2 after the first touch (a sequence's K and V for one
-// head are 256 B per key); HBM sees every K and V page about once per (sequence, KV head).
-// All CTAs of a launch stream the pages through a shared-memory ring filled by 16-byte asynchronous copies.
+// are recomputed each time.  K is therefore read three times and V once per tile, from L2 after the first touch.
+//
+// What bounds it is integer issue: about 35 instructions per score over the three walks.  The general steps (64-bit
+// rounding shifts with saturation, clamps, a table in global memory) took 194, at a quarter of the issue slots; they
+// remain for scales whose scores could saturate.  Otherwise a score is one wide multiply, one shift and a rounding
+// step, and its exponential one wide multiply-add: with nx = max - score, P = 94548 nx - 1 + 2^32 has the shift in
+// its high word and, read backwards, the table index on top of its low word (tests/test_kernel_identities.py).
+// 15 prompts of 100 .. 1000 tokens, 32 / 8 heads: 0.78 ms a layer, 1.77 ms with the general steps and one warp per 16 rows.
 #include "attn_common.cuh"
 #include "luts.cuh"
 
@@ -44,10 +49,25 @@ struct PrefillParams {
 
 constexpr int kPfWarps = 8;
 constexpr int kPfThreads = kPfWarps * 32;
-constexpr int kPfRows = kPfWarps * 16;             // query rows per CTA
+constexpr int kPfGroups = kPfWarps / 2;            // pairs of warps
+constexpr int kPfRows = kPfGroups * 16;            // query rows per CTA
+constexpr int kPfKeys = 64;                        // keys per stage: four pages, two for either warp of a pair
 constexpr int kPfStages = 4;
-constexpr int kPfStageBytes = 4096 + 4096 + 384;   // K pair (swizzled rows), V pair (operand order), two scale blocks
+constexpr int kPfV = 8192, kPfMeta = 16384;        // in a stage: K pages (swizzled rows), V pages (operand order), scale blocks
+constexpr int kPfStageBytes = kPfMeta + 4 * 192;
 constexpr int kPfNeg = (int)(-2147483647 - 1);
+constexpr int kPfListPages = 8192;                 // page ids kept in shared memory; those of longer contexts are read where they are
+constexpr int kPfMaxPages = 42624;                 // of a sequence
+
+// Shared memory behind the ring.
+struct PfShared {
+  int exp_lut[1024];                               // entry 1023 - j of the table, shifted right by 13
+  uint4 limbs[kPfWarps][32][2];                    // probability limbs of a warp's 32 keys as A operands: high, low
+  int red[kPfGroups][2][16];
+  int rel[2][kPfKeys];                             // relative V scales of this stage's and the next one's keys
+  unsigned long long vref;
+  int ks_min, ks_max;
+};
 
 __device__ __forceinline__ void mma_u8s8(int (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
   asm volatile(
@@ -56,21 +76,40 @@ __device__ __forceinline__ void mma_u8s8(int (&c)[4], unsigned a0, unsigned a1, 
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// exp of the decode kernel: LUT[(y & 0xffff) >> 6] >> min(31, 13 - (y >> 16)), y = (x * 94548) >> 16, x <= 0
-__device__ __forceinline__ int pf_exp(int score, int row_max) {
-  const int x = max(sub_sat(score, row_max), -(1 << 30));
-  const long long prod = (long long)x * 94548LL;
-  return __ldg(&g_exp2_attn_lut[((unsigned)prod) >> 22]) >> min(31, 13 - (int)(prod >> 32));
+__device__ __forceinline__ unsigned shr_clamp(unsigned v, unsigned n) {   // 0 from 32 on
+  unsigned r;
+  asm("shr.u32 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(n));
+  return r;
 }
 
-// kMinBlocks: CTAs per SM the register budget is cut for.
-template <int G, int kMinBlocks = 1>
-__global__ void __launch_bounds__(kPfThreads, kMinBlocks)
+// exp of the decode kernel, LUT[(y & 0xffff) >> 6] >> min(31, 13 - (y >> 16)) with y = (x * 94548) >> 16 and x = max(score -
+// row_max, -2^30); `c` = 94548 row_max - 1 + 2^32.
+__device__ __forceinline__ unsigned pf_exp(int score, long long c, const int* lut) {
+  const long long v = (long long)score * -94548LL + c;
+  return shr_clamp((unsigned)lut[(unsigned)v >> 22], (unsigned)(v >> 32));
+}
+
+template <int G>
+__global__ void __launch_bounds__(kPfThreads, 2)
 attn_prefill_kernel(const PrefillParams p) {
   constexpr int TQ = kPfRows / G;                    // new tokens per tile
   const int b = blockIdx.z, kh = blockIdx.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int group = warp >> 1, side = warp & 1;
   const int fr = lane >> 2, fc = lane & 3;
+
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  unsigned char* ring = smem_raw;                                                    // [stages][kPfStageBytes]
+  PfShared& sh = *reinterpret_cast<PfShared*>(smem_raw + kPfStages * kPfStageBytes);
+  int32_t* pages = reinterpret_cast<int32_t*>(smem_raw + kPfStages * kPfStageBytes + sizeof(PfShared));
+  pdl_launch_dependents();
+  for (int i = tid; i < 1024; i += kPfThreads) sh.exp_lut[i] = g_exp2_attn_lut[1023 - i] >> 13;
+  if (tid == 0) {
+    sh.vref = ~0ull;
+    sh.ks_min = 127;
+    sh.ks_max = -128;
+  }
+  pdl_wait();
 
   const int L_all = max(0, min(p.kv_lens[b], p.max_kv_len));
   const int n_q = max(0, min(p.q_lens[b], L_all));
@@ -81,106 +120,117 @@ attn_prefill_kernel(const PrefillParams p) {
   const int64_t q_row0 = p.q_start[b];
   const int prefix = L_all - n_q;                    // keys in front of the new tokens
   const int Lt = min(L_all, prefix + min(n_q, t0 + TQ));   // keys the last row of the tile sees
-  const int n_pairs = (Lt + 31) >> 5;
+  const int n_stages = (Lt + kPfKeys - 1) / kPfKeys;
   const int n_pages = (Lt + kPage - 1) / kPage;
-
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  unsigned char* ring = smem_raw;                                                    // [stages][kPfStageBytes]
-  int32_t* pages = reinterpret_cast<int32_t*>(smem_raw + kPfStages * kPfStageBytes);   // [max pages]
-  __shared__ unsigned long long vref_s;
-
-  // ---- page ids of the keys this tile sees; the reference V scale over ALL keys of the sequence
-  for (int i = tid; i < n_pages; i += kPfThreads) {
-    int64_t pid = p.page_table[(int64_t)b * p.table_pitch + i];
-    pages[i] = (int)(pid < 0 ? 0 : (pid >= p.num_pages ? p.num_pages - 1 : pid));
-  }
-  if (tid == 0) vref_s = ~0ull;
+  const int32_t* table = p.page_table + (int64_t)b * p.table_pitch;
+  auto read_page = [&](int i) {
+    const int64_t pid = __ldg(table + i);
+    return (int)(pid < 0 ? 0 : (pid >= p.num_pages ? p.num_pages - 1 : pid));
+  };
+  const bool listed = n_pages <= kPfListPages;
+  auto page_id = [&](int i) { return listed ? pages[i] : read_page(i); };
+  if (listed)
+    for (int i = tid; i < n_pages; i += kPfThreads) pages[i] = read_page(i);
   __syncthreads();
+
+  // ---- the ring: one stage = four pages.  Thread t copies 16-byte chunk t & 127 of two pages' K (and V) bytes.
+  const unsigned ring_base = (unsigned)__cvta_generic_to_shared(ring);
+  const int c_page = tid >> 7, c_chunk = tid & 127;
+  const unsigned k_dst = ((c_chunk >> 3) << 7) + ((((c_chunk & 7) ^ ((c_chunk >> 3) & 1))) << 4);   // row-parity swizzle
+  const int64_t chunk_off = (int64_t)kh * (kPage * kD) + (c_chunk << 4);
+  const int64_t page_stride = (int64_t)p.kv_heads * (kPage * kD);
+  auto issue = [&](int stage, bool with_v) {
+    if (stage < n_stages) {
+      const unsigned st = ring_base + (stage % kPfStages) * kPfStageBytes;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int pi = c_page + 2 * i, pg = 4 * stage + pi;
+        if (pg < n_pages) {
+          const int64_t off = page_id(pg) * page_stride + chunk_off;
+          cp_async16(st + pi * 2048 + k_dst, reinterpret_cast<const unsigned char*>(p.k_codes) + off);
+          if (with_v) cp_async16(st + kPfV + pi * 2048 + (c_chunk << 4), reinterpret_cast<const unsigned char*>(p.v_codes) + off);
+        }
+      }
+      if (tid < 40) {
+        const int pi = tid / 10, c16 = tid - 10 * pi;
+        if (4 * stage + pi < n_pages)
+          cp_async16(st + kPfMeta + pi * 192 + c16 * 16,
+                     reinterpret_cast<const unsigned char*>(p.meta + ((int64_t)page_id(4 * stage + pi) * p.kv_heads + kh) * kMetaWords) + c16 * 16);
+      }
+    }
+    cp_async_commit();
+  };
+  for (int j = 0; j < kPfStages - 1; ++j) issue(j, false);
+
+  // ---- over ALL keys of the sequence: the reference V scale, and the range of the K shifts
   {
     unsigned long long lv = ~0ull;
+    int lo = 127, hi = -128;
     for (int key = tid; key < L_all; key += kPfThreads) {
-      int64_t pid = p.page_table[(int64_t)b * p.table_pitch + (key >> 4)];
-      pid = pid < 0 ? 0 : (pid >= p.num_pages ? p.num_pages - 1 : pid);
-      const int32_t* mt = p.meta + (pid * p.kv_heads + kh) * kMetaWords;
+      const int32_t* mt = p.meta + ((int64_t)read_page(key >> 4) * p.kv_heads + kh) * kMetaWords;
       const unsigned vm = (unsigned)__ldg(mt + 16 + (key & 15));
-      const int vs = reinterpret_cast<const int8_t*>(mt + 36)[key & 15];
+      const int ks = __ldg(reinterpret_cast<const int8_t*>(mt + 32) + (key & 15)), vs = __ldg(reinterpret_cast<const int8_t*>(mt + 36) + (key & 15));
       const unsigned long long vkey = ((unsigned long long)(unsigned)(vs + 128) << 32) | (unsigned long long)(0xFFFFFFFFu - vm);
       lv = vkey < lv ? vkey : lv;
+      lo = min(lo, ks);
+      hi = max(hi, ks);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const unsigned long long other = __shfl_xor_sync(FULL_MASK, lv, o);
       lv = other < lv ? other : lv;
     }
-    if (lane == 0) atomicMin(&vref_s, lv);
+    lo = __reduce_min_sync(FULL_MASK, lo);
+    hi = __reduce_max_sync(FULL_MASK, hi);
+    if (lane == 0) {
+      atomicMin(&sh.vref, lv);
+      atomicMin(&sh.ks_min, lo);
+      atomicMax(&sh.ks_max, hi);
+    }
   }
-  __syncthreads();
-  const int v_shift_ref = (int)(vref_s >> 32) - 128;
-  const int v_mul_ref = (int)(0xFFFFFFFFu - (unsigned)(vref_s & 0xFFFFFFFFull));
 
   // ---- this lane's two query rows: row r of the CTA is new token t0 + r / G, query head kh * G + r % G
   int lim[2], qm[2], qs[2];
+  bool valid[2];
   int64_t orow[2];                                   // element offset of the row in q / out
   unsigned qa[2][8];                                 // Q bytes [32 fc, 32 fc + 32) of the row: A operand words
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    const int r = warp * 16 + fr + 8 * h;
+    const int r = group * 16 + fr + 8 * h;
     const int tok = t0 + r / G, g = r % G;
-    const bool valid = tok < n_q;
-    lim[h] = valid ? prefix + tok + 1 : 0;           // keys the row sees (0: a row past the sequence's last token)
-    const int64_t hrow = (q_row0 + (valid ? tok : 0)) * p.q_heads + kh * G + g;
+    valid[h] = tok < n_q;                            // a row past the sequence's last token stands for that one and is not stored
+    const int t = min(tok, n_q - 1);
+    lim[h] = prefix + t + 1;                         // keys the row sees
+    const int64_t hrow = (q_row0 + t) * p.q_heads + kh * G + g;
     orow[h] = hrow * kD;
-    qm[h] = valid ? p.q_mul[hrow] : 0;
-    qs[h] = valid ? p.q_shift[hrow] - 48 : 0;
+    qm[h] = p.q_mul[hrow];
+    qs[h] = p.q_shift[hrow] - 48;
     const uint4* qp = reinterpret_cast<const uint4*>(p.q + hrow * kD + fc * 32);
-    const uint4 x0 = valid ? __ldg(qp) : make_uint4(0, 0, 0, 0), x1 = valid ? __ldg(qp + 1) : make_uint4(0, 0, 0, 0);
+    const uint4 x0 = __ldg(qp), x1 = __ldg(qp + 1);
     qa[h][0] = x0.x; qa[h][1] = x0.y; qa[h][2] = x0.z; qa[h][3] = x0.w;
     qa[h][4] = x1.x; qa[h][5] = x1.y; qa[h][6] = x1.z; qa[h][7] = x1.w;
   }
-  // keys this warp needs at all: the largest limit of its 16 rows (uniform over the warp)
-  int warp_lim = max(lim[0], lim[1]);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) warp_lim = max(warp_lim, __shfl_xor_sync(FULL_MASK, warp_lim, o));
+  // the fewest and the most keys that a row of this pair of warps sees (rows are in the order of their tokens)
+  const int lim_all = __reduce_min_sync(FULL_MASK, lim[0]), lim_any = __reduce_max_sync(FULL_MASK, lim[1]);
+  __syncthreads();
+  const int v_shift_ref = (int)(sh.vref >> 32) - 128;
+  const int v_mul_ref = (int)(0xFFFFFFFFu - (unsigned)(sh.vref & 0xFFFFFFFFull));
+  // |dot| <= 2^21 and |(q_mul k_mul) >> 32| <= 2^30: from a shift of 22 on nothing saturates and a shift by one less fits 32 bits
+  const int qs_min = __reduce_min_sync(FULL_MASK, min(qs[0], qs[1])), qs_max = __reduce_max_sync(FULL_MASK, max(qs[0], qs[1]));
+  const bool plain = qs_min > -1024 && qs_max < 1024 && qs_min + sh.ks_min >= 22 && qs_max + sh.ks_max <= 62;
 
-  // ---- the ring: one stage = a pair of pages.  Thread t copies 16-byte chunk t of the pair's K (and V) bytes.
-  const unsigned ring_base = (unsigned)__cvta_generic_to_shared(ring);
-  const int c_page = tid >> 7, c_chunk = tid & 127;                       // which page of the pair, which 16-byte chunk
-  const unsigned k_dst = c_page * 2048 + ((c_chunk >> 3) << 7) + ((((c_chunk & 7) ^ ((c_chunk >> 3) & 1))) << 4);   // row-parity swizzle
-  const unsigned v_dst = 4096 + c_page * 2048 + (c_chunk << 4);
-  const int64_t chunk_off = (int64_t)kh * (kPage * kD) + (c_chunk << 4);
-  const int64_t page_stride = (int64_t)p.kv_heads * (kPage * kD);
-  auto issue = [&](int pair, bool with_v) {
-    if (pair < n_pairs) {
-      const unsigned st = ring_base + (pair % kPfStages) * kPfStageBytes;
-      const int pg = 2 * pair + c_page;
-      if (pg < n_pages) {
-        const int64_t off = pages[pg] * page_stride + chunk_off;
-        cp_async16(st + k_dst, reinterpret_cast<const unsigned char*>(p.k_codes) + off);
-        if (with_v) cp_async16(st + v_dst, reinterpret_cast<const unsigned char*>(p.v_codes) + off);
-      }
-      if (tid < 20) {
-        const int h = tid >= 10, c16 = tid - 10 * h;
-        if (2 * pair + h < n_pages)
-          cp_async16(st + 8192 + h * 192 + c16 * 16,
-                     reinterpret_cast<const unsigned char*>(p.meta + ((int64_t)pages[2 * pair + h] * p.kv_heads + kh) * kMetaWords) + c16 * 16);
-      }
-    }
-    cp_async_commit();
-  };
-
-  // Scores of one pair for this lane: sc[h][pg][e] = row h, key pair * 32 + pg * 16 + 4 fc + e (kPfNeg = not visible)
-  auto scores = [&](const unsigned char* st, int pair, int (&sc)[2][2][4]) {
+  // Scores of this warp's pair of pages for this lane: sc[h][pg][e] = row h, key stage * 64 + side * 32 + pg * 16 + 4 fc + e
+  auto scores = [&](const unsigned char* st, int (&sc)[2][2][4]) {
 #pragma unroll
     for (int pg = 0; pg < 2; ++pg) {
-      const int32_t* mt = reinterpret_cast<const int32_t*>(st + 8192 + pg * 192);
+      const int32_t* mt = reinterpret_cast<const int32_t*>(st + kPfMeta + (2 * side + pg) * 192);
       const int4 km = *reinterpret_cast<const int4*>(mt + 4 * fc);
       const unsigned ksw = reinterpret_cast<const unsigned*>(mt + 32)[fc];
       const int kmv[4] = {km.x, km.y, km.z, km.w};
-      const int key0 = pair * 32 + pg * 16 + 4 * fc;
 #pragma unroll
       for (int jj = 0; jj < 2; ++jj) {
         const int tok = 4 * (fr >> 1) + 2 * jj + (fr & 1);                   // the key row this lane feeds as column fr
-        const unsigned char* kr = st + pg * 2048 + tok * 128;
+        const unsigned char* kr = st + (2 * side + pg) * 2048 + tok * 128;
         const uint4 k0 = *reinterpret_cast<const uint4*>(kr + (((2 * fc) ^ (tok & 1)) << 4));
         const uint4 k1 = *reinterpret_cast<const uint4*>(kr + (((2 * fc + 1) ^ (tok & 1)) << 4));
         int c[4] = {0, 0, 0, 0};
@@ -194,160 +244,207 @@ attn_prefill_kernel(const PrefillParams p) {
           const int e = 2 * jj + e2;
           const int ks = (int)(signed char)((ksw >> (8 * e)) & 0xff);
 #pragma unroll
-          for (int h = 0; h < 2; ++h)
-            sc[h][pg][e] = key0 + e < lim[h] ? mul_shift_sat32(c[2 * h + e2], __mulhi(qm[h], kmv[e]), qs[h] + ks) : kPfNeg;
+          for (int h = 0; h < 2; ++h) sc[h][pg][e] = c[2 * h + e2];
+          if (plain) {                                 // floor((x + 2^(s-1)) / 2^s) = floor((floor(x / 2^(s-1)) + 1) / 2)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+              sc[h][pg][e] = ((int)(((long long)sc[h][pg][e] * (long long)__mulhi(qm[h], kmv[e])) >> (qs[h] + ks - 1)) + 1) >> 1;
+          } else {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) sc[h][pg][e] = mul_shift_sat32(sc[h][pg][e], __mulhi(qm[h], kmv[e]), qs[h] + ks);
+          }
         }
       }
     }
   };
+  // Walks the stages; body(stage's shared memory, first key of this warp's pair of pages).
+  auto walk = [&](bool with_v, auto&& ahead, auto&& body) {
+    for (int stage = 0; stage < n_stages; ++stage) {
+      cp_async_wait<kPfStages - 3>();                    // this stage and the next one
+      __syncthreads();                                   // ... have landed for everybody; the stage before is free
+      issue(stage + kPfStages - 1, with_v);
+      ahead(stage);
+      if (stage * kPfKeys < lim_any) body(ring + (stage % kPfStages) * kPfStageBytes, stage * kPfKeys + side * 32, stage);
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+  };
 
   // ---- pass 1: row maxima
   int row_max[2] = {kPfNeg, kPfNeg};
-  for (int j = 0; j < kPfStages - 1; ++j) issue(j, false);
-  for (int pair = 0; pair < n_pairs; ++pair) {
-    cp_async_wait<kPfStages - 2>();
-    __syncthreads();                                   // the pair has landed for everybody; the stage of pair - 1 is free
-    issue(pair + kPfStages - 1, false);
-    if (pair * 32 >= warp_lim) continue;
+  walk(false, [](int) {}, [&](const unsigned char* st, int key0, int) {
+    if (key0 >= lim_any) return;
     int sc[2][2][4];
-    scores(ring + (pair % kPfStages) * kPfStageBytes, pair, sc);
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-      for (int pg = 0; pg < 2; ++pg)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) row_max[h] = max(row_max[h], sc[h][pg][e]);   // kPfNeg for keys out of sight
-  }
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    row_max[h] = max(row_max[h], __shfl_xor_sync(FULL_MASK, row_max[h], 1));
-    row_max[h] = max(row_max[h], __shfl_xor_sync(FULL_MASK, row_max[h], 2));
-    // keys behind the causal limit take part in the reference's maximum as -2^30
-    if (lim[h] < L_all) row_max[h] = max(row_max[h], -(1 << 30));
-  }
-  cp_async_wait<0>();
-  __syncthreads();
-
-  // ---- pass 2: sums of exponentials
-  unsigned row_sum[2] = {0u, 0u};
-  for (int j = 0; j < kPfStages - 1; ++j) issue(j, false);
-  for (int pair = 0; pair < n_pairs; ++pair) {
-    cp_async_wait<kPfStages - 2>();
-    __syncthreads();
-    issue(pair + kPfStages - 1, false);
-    if (pair * 32 >= warp_lim) continue;
-    int sc[2][2][4];
-    scores(ring + (pair % kPfStages) * kPfStageBytes, pair, sc);
+    scores(st, sc);
+    const bool all = key0 + 32 <= lim_all;
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
       for (int pg = 0; pg < 2; ++pg)
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          if (pair * 32 + pg * 16 + 4 * fc + e < lim[h]) row_sum[h] += (unsigned)pf_exp(sc[h][pg][e], row_max[h]);
+          if (all || key0 + pg * 16 + 4 * fc + e < lim[h]) row_max[h] = max(row_max[h], sc[h][pg][e]);
+  });
+  for (int j = 0; j < kPfStages - 1; ++j) issue(j, false);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    row_max[h] = max(row_max[h], __shfl_xor_sync(FULL_MASK, row_max[h], 1));
+    row_max[h] = max(row_max[h], __shfl_xor_sync(FULL_MASK, row_max[h], 2));
+    if (fc == 0) sh.red[group][side][fr + 8 * h] = row_max[h];
   }
+  __syncthreads();
+  long long exp_c[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    row_max[h] = max(row_max[h], sh.red[group][side ^ 1][fr + 8 * h]);
+    // keys behind the causal limit take part in the reference's maximum as -2^30
+    if (lim[h] < L_all) row_max[h] = max(row_max[h], -(1 << 30));
+    exp_c[h] = (long long)row_max[h] * 94548LL - 1LL + (1LL << 32);
+  }
+
+  // ---- pass 2: sums of exponentials
+  unsigned row_sum[2] = {0u, 0u};
+  walk(false, [](int) {}, [&](const unsigned char* st, int key0, int) {
+    if (key0 >= lim_any) return;
+    int sc[2][2][4];
+    scores(st, sc);
+    const bool all = key0 + 32 <= lim_all;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int pg = 0; pg < 2; ++pg)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const unsigned v = pf_exp(sc[h][pg][e], exp_c[h], sh.exp_lut);
+          if (all || key0 + pg * 16 + 4 * fc + e < lim[h]) row_sum[h] += v;
+        }
+  });
+  for (int j = 0; j < kPfStages - 1; ++j) issue(j, true);
   unsigned inv[2];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
+    // (a lane adds at most 2^16 for each eighth key: 32 bits last for half a million equal keys)
     unsigned long long tot = row_sum[h];
     tot += __shfl_xor_sync(FULL_MASK, tot, 1);
     tot += __shfl_xor_sync(FULL_MASK, tot, 2);
+    if (fc == 0) *reinterpret_cast<unsigned long long*>(&sh.limbs[warp][fr + 8 * h][0]) = tot;
+    row_sum[h] = 0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    unsigned long long tot = *reinterpret_cast<unsigned long long*>(&sh.limbs[warp][fr + 8 * h][0]) +
+                             *reinterpret_cast<unsigned long long*>(&sh.limbs[warp ^ 1][fr + 8 * h][0]);
     if (tot < 1ull) tot = 1ull;
     inv[h] = (unsigned)(2147483647ull / tot);
   }
-  cp_async_wait<0>();
-  __syncthreads();
 
   // ---- pass 3: probabilities (Q0.15) folded with the relative V scale, as two byte limbs, times V
-  int acc_hi[16][4], acc_lo[16][4];
+  int acc_hi[8][4], acc_lo[8][4];
 #pragma unroll
-  for (int nt = 0; nt < 16; ++nt)
+  for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc_hi[nt][j] = acc_lo[nt][j] = 0;
-  for (int j = 0; j < kPfStages - 1; ++j) issue(j, true);
-  for (int pair = 0; pair < n_pairs; ++pair) {
-    cp_async_wait<kPfStages - 2>();
-    __syncthreads();
-    issue(pair + kPfStages - 1, true);
-    if (pair * 32 >= warp_lim) continue;
-    const unsigned char* st = ring + (pair % kPfStages) * kPfStageBytes;
-    int sc[2][2][4];
-    scores(st, pair, sc);
-    unsigned ah[2][2], al[2][2];                        // [row h][page]: four limb bytes = keys 4 fc .. 4 fc + 3
+  // two warps work out the relative V scales of a stage while the one before is multiplied
+  auto rel_scales = [&](int stage, int i) {
+    const int32_t* mt = reinterpret_cast<const int32_t*>(ring + (stage % kPfStages) * kPfStageBytes + kPfMeta + (i >> 4) * 192);
+    const int vs = reinterpret_cast<const int8_t*>(mt + 36)[i & 15];
+    if (stage * kPfKeys + i < Lt) sh.rel[stage & 1][i] = (int)rel_scale_q15((unsigned)mt[16 + (i & 15)], (unsigned)v_mul_ref, vs - v_shift_ref);
+  };
+  cp_async_wait<kPfStages - 2>();
+  __syncthreads();                                       // the first stage; and the sums have been read
+  if (tid < kPfKeys) rel_scales(0, tid);
+  walk(true, [&](int stage) {
+    if (stage + 1 < n_stages && group == (stage & (kPfGroups - 1))) rel_scales(stage + 1, tid & (kPfKeys - 1));
+  }, [&](const unsigned char* st, int key0, int stage) {
+    uint4 own_hi = make_uint4(0, 0, 0, 0), own_lo = make_uint4(0, 0, 0, 0);      // [row h, page]: keys 4 fc .. 4 fc + 3 as bytes
+    if (key0 < lim_any) {
+      int sc[2][2][4];
+      scores(st, sc);
+      const bool all = key0 + 32 <= lim_all;
+      unsigned ah[2][2], al[2][2];
 #pragma unroll
-    for (int pg = 0; pg < 2; ++pg) {
-      const int32_t* mt = reinterpret_cast<const int32_t*>(st + 8192 + pg * 192);
-      const int4 vm = *reinterpret_cast<const int4*>(mt + 16 + 4 * fc);
-      const unsigned vsw = reinterpret_cast<const unsigned*>(mt + 36)[fc];
-      const unsigned vmv[4] = {(unsigned)vm.x, (unsigned)vm.y, (unsigned)vm.z, (unsigned)vm.w};
-      unsigned hi[2] = {0u, 0u}, lo[2] = {0u, 0u};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int key = pair * 32 + pg * 16 + 4 * fc + e;
-        const int vs = (int)(signed char)((vsw >> (8 * e)) & 0xff);
-        const unsigned r = key < warp_lim ? rel_scale_q15(vmv[e], (unsigned)v_mul_ref, vs - v_shift_ref) : 0u;
+      for (int pg = 0; pg < 2; ++pg) {
+        const int4 rv = *reinterpret_cast<const int4*>(&sh.rel[stage & 1][side * 32 + pg * 16 + 4 * fc]);
+        const unsigned r[4] = {(unsigned)rv.x, (unsigned)rv.y, (unsigned)rv.z, (unsigned)rv.w};
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          unsigned w = 0u;
-          if (key < lim[h]) {
-            const unsigned pr = ((unsigned)pf_exp(sc[h][pg][e], row_max[h]) * inv[h]) >> 16;
-            w = (pr * r + 16384u) >> 15;
+          unsigned w[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const unsigned pr = (pf_exp(sc[h][pg][e], exp_c[h], sh.exp_lut) * inv[h]) >> 16;
+            w[e] = (pr * r[e] + 16384u) >> 15;
+            if (!(all || key0 + pg * 16 + 4 * fc + e < lim[h])) w[e] = 0u;
           }
-          hi[h] |= (w >> 8) << (8 * e);
-          lo[h] |= (w & 0xffu) << (8 * e);
+          const unsigned w01 = __byte_perm(w[0], w[1], 0x5410), w23 = __byte_perm(w[2], w[3], 0x5410);
+          ah[h][pg] = __byte_perm(w01, w23, 0x7531);
+          al[h][pg] = __byte_perm(w01, w23, 0x6420);
         }
       }
-      ah[0][pg] = hi[0]; ah[1][pg] = hi[1]; al[0][pg] = lo[0]; al[1][pg] = lo[1];
+      own_hi = make_uint4(ah[0][0], ah[1][0], ah[0][1], ah[1][1]);
+      own_lo = make_uint4(al[0][0], al[1][0], al[0][1], al[1][1]);
     }
-    const bool has_b = 2 * pair + 1 < n_pages;
-    const unsigned char* vp = st + 4096 + lane * 16;
+    sh.limbs[warp][lane][0] = own_hi;
+    sh.limbs[warp][lane][1] = own_lo;
+    asm volatile("bar.sync %0, 64;" ::"r"(group + 1) : "memory");
 #pragma unroll
-    for (int qd = 0; qd < 4; ++qd) {
-      const uint4 va = *reinterpret_cast<const uint4*>(vp + qd * 512);
-      const uint4 vb = has_b ? *reinterpret_cast<const uint4*>(vp + 2048 + qd * 512) : make_uint4(0, 0, 0, 0);
-      const unsigned wa[4] = {va.x, va.y, va.z, va.w}, wb[4] = {vb.x, vb.y, vb.z, vb.w};
+    for (int pp = 0; pp < 2; ++pp) {
+      if (stage * kPfKeys + pp * 32 >= lim_any) break;
+      const uint4 wh = sh.limbs[(warp & ~1) + pp][lane][0], wl = sh.limbs[(warp & ~1) + pp][lane][1];
+      const unsigned char* vp = st + kPfV + pp * 4096 + side * 1024 + lane * 16;      // d-tiles 8 side .. 8 side + 7
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int nt = 4 * qd + i;
-        mma_u8s8(acc_hi[nt], ah[0][0], ah[1][0], ah[0][1], ah[1][1], wa[i], wb[i]);
-        mma_u8s8(acc_lo[nt], al[0][0], al[1][0], al[0][1], al[1][1], wa[i], wb[i]);
+      for (int qd = 0; qd < 2; ++qd) {
+        // (pages past the last one hold leftovers: their limbs are zero)
+        const uint4 va = *reinterpret_cast<const uint4*>(vp + qd * 512), vb = *reinterpret_cast<const uint4*>(vp + 2048 + qd * 512);
+        const unsigned wa[4] = {va.x, va.y, va.z, va.w}, wb[4] = {vb.x, vb.y, vb.z, vb.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          mma_u8s8(acc_hi[4 * qd + i], wh.x, wh.y, wh.z, wh.w, wa[i], wb[i]);
+          mma_u8s8(acc_lo[4 * qd + i], wl.x, wl.y, wl.z, wl.w, wa[i], wb[i]);
+        }
       }
     }
-  }
-  cp_async_wait<0>();
+  });
 
-  // ---- output: acc -> Q15.16, optionally the per-row int8 codes.  C tile: [0] (row fr, d = 8 nt + 2 fc)  [1] (row fr, d + 1)
-  // [2] (row fr + 8, d)  [3] (row fr + 8, d + 1)
+  // ---- output: acc -> Q15.16, optionally the per-row int8 codes.  C tile: [0] (row fr, d = 64 side + 8 nt + 2 fc)  [1] (row fr,
+  // d + 1)  [2] (row fr + 8, d)  [3] (row fr + 8, d + 1)
+  int o[2][16], m[2] = {0, 0};
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    const bool valid = lim[h] > 0;
-    int o[32];
-    int m = 0;
 #pragma unroll
-    for (int nt = 0; nt < 16; ++nt)
+    for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const int a = acc_hi[nt][2 * h + j] * 256 + acc_lo[nt][2 * h + j];
         const int v = mul_shift_sat32_wide((long long)a, v_mul_ref, v_shift_ref - 1);
-        o[2 * nt + j] = v;
-        m = max(m, abs_wrap(v));
+        o[h][2 * nt + j] = v;
+        m[h] = max(m[h], abs_wrap(v));
       }
-    if (p.out_q15 && valid) {
+    if (p.out_q15 && valid[h]) {
 #pragma unroll
-      for (int nt = 0; nt < 16; ++nt)
-        *reinterpret_cast<int2*>(p.out_q15 + orow[h] + 8 * nt + 2 * fc) = make_int2(o[2 * nt], o[2 * nt + 1]);
+      for (int nt = 0; nt < 8; ++nt)
+        *reinterpret_cast<int2*>(p.out_q15 + orow[h] + 64 * side + 8 * nt + 2 * fc) = make_int2(o[h][2 * nt], o[h][2 * nt + 1]);
     }
-    if (p.out_codes) {
-      m = max(m, __shfl_xor_sync(FULL_MASK, m, 1));
-      m = max(1, max(m, __shfl_xor_sync(FULL_MASK, m, 2)));
-      if (valid) {
-        const float mf = __int2float_rn(m);
+  }
+  if (p.out_codes) {                                     // (the same for the whole launch)
 #pragma unroll
-        for (int nt = 0; nt < 16; ++nt) {
-          const unsigned short c2 = (unsigned short)((quant_code(o[2 * nt], mf) & 0xff) | ((quant_code(o[2 * nt + 1], mf) & 0xff) << 8));
-          *reinterpret_cast<unsigned short*>(p.out_codes + orow[h] + 8 * nt + 2 * fc) = c2;
+    for (int h = 0; h < 2; ++h) {
+      m[h] = max(m[h], __shfl_xor_sync(FULL_MASK, m[h], 1));
+      m[h] = max(m[h], __shfl_xor_sync(FULL_MASK, m[h], 2));
+      if (fc == 0) sh.red[group][side][fr + 8 * h] = m[h];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int am = max(1, max(m[h], sh.red[group][side ^ 1][fr + 8 * h]));
+      if (valid[h]) {
+        const float mf = __int2float_rn(am);
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) {
+          const unsigned short c2 = (unsigned short)((quant_code(o[h][2 * nt], mf) & 0xff) | ((quant_code(o[h][2 * nt + 1], mf) & 0xff) << 8));
+          *reinterpret_cast<unsigned short*>(p.out_codes + orow[h] + 64 * side + 8 * nt + 2 * fc) = c2;
         }
-        if (fc == 0) p.out_absmax[orow[h] / kD] = m;
+        if (fc == 0 && side == 0) p.out_absmax[orow[h] / kD] = am;
       }
     }
   }
@@ -356,35 +453,19 @@ attn_prefill_kernel(const PrefillParams p) {
 template <int G>
 static int launch_prefill(const PrefillParams& p, int batch, int max_q_len, cudaStream_t st) {
   constexpr int TQ = kPfRows / G;
-  const size_t smem = (size_t)kPfStages * kPfStageBytes + (size_t)((p.max_kv_len + kPage - 1) / kPage) * 4;
-  if (smem > 200 * 1024) {
-    set_error("attn_prefill: max_kv_len=%d needs %zu bytes of shared memory for the page list", p.max_kv_len, smem);
+  const int pages = (p.max_kv_len + kPage - 1) / kPage;
+  if (pages > kPfMaxPages) {
+    set_error("attn_prefill: max_kv_len=%d is more than %d pages", p.max_kv_len, kPfMaxPages);
     return B200_E_UNSUPPORTED;
   }
-  // Two CTAs per SM (a budget of 128 registers, some spilled) while the page list leaves room: the kernel waits on
-  // dependent integer arithmetic, and four warps per scheduler hide more of it than two (1.73 -> 1.58 ms on 16
-  // prompts of U[100,1024] tokens).  B200_PREFILL_OCC2=0 keeps one CTA of 250 registers per SM.
-  static int occ2 = -1;
-  if (occ2 < 0) {
-    const char* ev = getenv("B200_PREFILL_OCC2");
-    occ2 = (ev && ev[0] == '0') ? 0 : 1;
-  }
+  const size_t smem = (size_t)kPfStages * kPfStageBytes + sizeof(PfShared) + (size_t)(pages < kPfListPages ? pages : kPfListPages) * 4;
   const int tiles = (max_q_len + TQ - 1) / TQ;
-  if (occ2 == 1 && smem <= 100 * 1024) {
-    cudaError_t e2 = cudaFuncSetAttribute(attn_prefill_kernel<G, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e2 != cudaSuccess) {
-      set_error("attn_prefill: cudaFuncSetAttribute: %s", cudaGetErrorString(e2));
-      return B200_E_CUDA;
-    }
-    attn_prefill_kernel<G, 2><<<dim3(tiles, p.kv_heads, batch), kPfThreads, smem, st>>>(p);
-    return check_launch("attn_prefill");
-  }
   cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) {
     set_error("attn_prefill: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     return B200_E_CUDA;
   }
-  attn_prefill_kernel<G><<<dim3(tiles, p.kv_heads, batch), kPfThreads, smem, st>>>(p);
+  launch_pdl(attn_prefill_kernel<G>, dim3(tiles, p.kv_heads, batch), dim3(kPfThreads), smem, st, p);
   return check_launch("attn_prefill");
 }
 

@@ -244,6 +244,27 @@ def test_tiled_prefill_vs_oracle(q_heads, kv_heads):
     eq(run_extend(case, pool, 512, cluster=1, impl="cluster").cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("shift,extreme", [(21, True), (22, True), (23, False), (33, False), (62, False), (63, False)])
+@pytest.mark.parametrize("q_heads", [1, 4])
+def test_tiled_prefill_at_the_limits_of_the_plain_scores(shift, extreme, q_heads):
+    """Score shifts (q_shift + k_shift - 48) around 22 .. 62, where scores take the short form, with the largest products that
+    int8 codes and multipliers give (they saturate below 22), over lengths around a stage of 64 keys and a tile of rows."""
+    kv_lens, q_lens = [1, 63, 64, 65, 129, 200], [1, 63, 64, 17, 129, 5]
+    case = _extend_case(90 + shift, kv_lens, q_lens, q_heads, 1, 40, uniform=True)
+    case["qs"][:] = shift + 48 - 36
+    if extreme:
+        case["q8"][:, :, :] = -128
+        case["k8"][::2] = -128
+        case["k8"][1::2] = 127
+        case["qm"][:] = 2**31 - 1
+        case["km"][:] = 2**31 - 1
+        case["pool"].store_codes(case["loc"], case["k8"], case["v8"], case["km"].astype(np.int64), case["ks"].astype(np.int64),
+                                 case["vm"].astype(np.int64), case["vs"].astype(np.int64))
+    pool = device_pool(case, 40, 1)
+    want = oattn.paged_attention(case["q8"], case["qm"], case["qs"], case["pool"], case["tables"], kv_lens, q_lens)
+    eq(run_extend(case, pool, 208, impl="tiled").cpu().numpy(), want)
+
+
 @pytest.mark.parametrize("kv_len,q_len", [(1024, 1024), (3584, 512)])
 def test_tiled_prefill_long_prompts_vs_oracle(kv_len, q_len):
     """A 1024-token prompt without a prefix, and 512 new tokens over a 3072-token cached prefix."""

@@ -111,3 +111,27 @@ def test_quant_estimate_only_differs_from_the_division_inside_the_tie_band():
             np.testing.assert_array_equal(r[far], exact[far])
             checked += int(far.sum())
     assert checked > 1_000_000
+
+
+def test_prefill_score_and_exponential_forms():
+    """The prefill kernel's short forms: the exponential's table index and shift from one wide multiply-add, and the rounding
+    shift of a score that cannot saturate."""
+    from oracle import attention as oattn
+    from oracle import luts
+    rng = np.random.default_rng(6)
+    row_max = rng.integers(-2**31, 2**31, 400000)
+    nx = np.concatenate([np.arange(200000), rng.integers(0, 2**21, 100000), rng.integers(0, 2**32, 100000)])
+    score = np.maximum(row_max - nx, -2**31)
+    v = score * -94548 + (row_max * 94548 - 1 + 2**32)
+    shift, idx = v >> 32, (v & 0xFFFFFFFF) >> 22
+    assert shift.min() >= 0
+    table = luts.exp2_attn().astype(np.int64)[::-1] >> 13
+    got = np.where(shift < 32, table[idx] >> np.minimum(shift, 31), 0)
+    want = oattn.exp_q15_16(np.clip(score - row_max, -(1 << 30), 0).astype(np.int32))
+    assert np.array_equal(got, want)
+    dot = np.concatenate([[2**21, -2**21, 0, 1, -1], rng.integers(-2**21, 2**21 + 1, 200000)])
+    mul = np.concatenate([[2**30, 2**30, 1, 1, 1], rng.integers(-2**30, 2**30 + 1, 200000)])
+    for s in (22, 23, 32, 33, 34, 62):
+        t = (dot * mul) >> (s - 1)
+        assert np.abs(t).max() < 2**31
+        assert np.array_equal((t + 1) >> 1, oattn.mul_shift(dot, mul, s))
