@@ -79,6 +79,9 @@ FLOAT_SIGNATURES: dict[str, list] = {
     "b200f_gemm_splits": [L, L, L, L, I],
     "b200f_gemm": [P, P, P, I, I, L, L, L, L, L, L, L, L, L, L, I, L, I, F, F, P],
     "b200f_gemm_status": [P, I],
+    "b200f_gemm_f32_ws_bytes": [L, L, L, L],
+    "b200f_gemm_f32": [P, P, P, L, L, L, L, L, L, L, L, L, L, I, F, F, P, P],
+    "b200f_gemm_f32_status": [P, I],
     "b200f_embed_bigram": [P, P, P, P, P, P, P, P, P, P, I, L, I, L, L, L, L, L, P],
     "b200f_sublayer_end": [P, I, L, P, I, L, P, P, P, P, P, P, P, P, I, L, P, P, P, I, L, I, L, F, P],
     "b200f_gated_silu": [P, I, L, L, P, I, L, I, L, P],
@@ -102,7 +105,7 @@ FLOAT_SIGNATURES: dict[str, list] = {
 }
 _SHARED = ("b200_last_error_string", "b200_decode_prepare")      # in every library
 _RESTYPES = {"b200_last_error_string": c_char_p, "b200_attn_workspace_bytes": ctypes.c_size_t,
-             "b200_tp_block_bytes": ctypes.c_size_t, "b200f_latent_attn_ws_floats": ctypes.c_size_t,
+             "b200_tp_block_bytes": ctypes.c_size_t, "b200f_latent_attn_ws_floats": ctypes.c_size_t, "b200f_gemm_f32_ws_bytes": ctypes.c_size_t,
              "b200f_grouped_attn_ws_floats": ctypes.c_size_t, "b200f_memory_scan_ws_bytes": ctypes.c_size_t}
 
 _libs: dict[str, ctypes.CDLL] = {}

@@ -1,0 +1,356 @@
+// 32-bit linears on the bf16 tensor cores.
+//
+//   out[b][t, j] = act( sum_k x[b][t, k] * w[b][j, k] )          operands, products and result in 32 bits
+//
+// An fp32 number is the sum of three bf16 numbers (8 + 8 + 8 bits of fraction, each rounded to nearest); of the nine products of
+// two such sums the six above 2^-24 of the largest are formed: hi hi, hi mid, mid hi, mid mid, hi lo, lo hi.  split_parts_kernel
+// writes the parts of both operands, gemm_f32x3_kernel multiplies them: tcgen05.mma kind::f16 with fp32 accumulators in
+// tensor memory, operands staged by TMA, small products first.  The tensor core's accumulation rounds less well than an
+// fma (a chain over K = 1024 loses a factor of two against fp32 units; so does one over 128 that comes back to small products), so
+// the accumulator starts afresh with every 64 of K and the pieces are added in registers, rounded to nearest.  Error against 64
+// bits, standard normal operands, 2-norm over 2-norm: K = 64 0.8e-7 (fp32 units 1.4e-7), 256 0.9e-7 (2.9e-7), 1024 1.1e-7 (5.7e-7),
+// 4096 1.7e-7 (11e-7).
+//
+// What bounds it: six bf16 products are a sixth of the bf16 peak, four times what the fp32 units can do; below that, the
+// operands' way from L2 (96 KB for 24 instructions of 128 x 128 x 16).
+//
+// Infinities and NaN do not survive the split (inf = inf + NaN + NaN): split_parts_kernel reports whether it met any, and the
+// linear is then computed value by value in the order of the plain kernel.
+#include "float_common.cuh"
+#include "umma.cuh"
+
+namespace b200 {
+
+constexpr int kXM = 128, kXN = 128, kXK = 64;       // tile; values of K per stage
+constexpr int kXPlane = 128 * 128;                  // bytes of one operand part in a stage: 128 rows x 64 bf16
+constexpr int kXStageBytes = 6 * kXPlane;
+constexpr int kXStages = 2;
+constexpr int kXEpiWarps = 8;
+constexpr int kXThreads = 64 + 32 * kXEpiWarps;
+constexpr int kXPitch = 20;                         // words per staged row of 16: 16-byte aligned, conflict-free both ways
+constexpr int kXSplitBlocks = 592;                  // CTAs of the splitting kernel at most, one report each
+
+struct X3Operand {
+  const float* src;
+  int64_t rows, pitch, bstride;                     // rows of one batch
+  bf16* dst;                                        // [3][batch][rows][dst_pitch]
+  int vec;                                          // rows start on 16-byte boundaries
+};
+struct X3Params {
+  X3Operand x, w;
+  float* out;
+  int M, N, K, batch, kp;                           // kp: pitch of the parts
+  int64_t out_pitch, out_bstride;
+  int act;
+  float act_a, act_b;
+  int vec;
+  unsigned* met;                                    // [split_blocks] a CTA of the splitting kernel met an infinity or a NaN
+  int split_blocks;
+};
+
+// Three bf16 numbers whose sum is v to 24 bits.  (Rounding up to infinity: the truncated number instead.)
+__device__ __forceinline__ void split3(float v, unsigned short (&o)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    bf16 h = __float2bfloat16_rn(v);
+    if (i == 0 && (__bfloat16_as_ushort(h) & 0x7fff) == 0x7f80) h = __ushort_as_bfloat16((unsigned short)(__float_as_uint(v) >> 16));
+    o[i] = __bfloat16_as_ushort(h);
+    v -= __bfloat162float(h);
+  }
+}
+
+__global__ void __launch_bounds__(256)
+split_parts_kernel(const X3Params p) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int quads = (p.K + 3) / 4;
+  const int64_t nx = (int64_t)p.batch * p.x.rows * quads, total = nx + (int64_t)p.batch * p.w.rows * quads;
+  bool met = false;
+  for (int64_t i = blockIdx.x * 256ll + threadIdx.x; i < total; i += gridDim.x * 256ll) {
+    const bool is_w = i >= nx;
+    const X3Operand& o = is_w ? p.w : p.x;
+    const int64_t j = is_w ? i - nx : i, r = j / quads, b = r / o.rows;
+    const int k = (int)(j - r * quads) * 4;
+    const float* src = o.src + b * o.bstride + (r - b * o.rows) * o.pitch + k;
+    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (o.vec && k + 3 < p.K) {
+      const float4 f = __ldg(reinterpret_cast<const float4*>(src));
+      v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+    } else {
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if (k + c < p.K) v[c] = __ldg(src + c);
+    }
+    unsigned short part[4][3];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      met |= (__float_as_uint(v[c]) & 0x7f800000u) == 0x7f800000u;
+      split3(v[c], part[c]);
+    }
+    const int64_t plane = (int64_t)p.batch * o.rows * p.kp;
+#pragma unroll
+    for (int s = 0; s < 3; ++s)                     // (kp is a multiple of 8: the quad fits its row)
+      *reinterpret_cast<uint2*>(o.dst + s * plane + r * p.kp + k) =
+          make_uint2(part[0][s] | ((unsigned)part[1][s] << 16), part[2][s] | ((unsigned)part[3][s] << 16));
+  }
+  const int any = __syncthreads_or(met);
+  if (threadIdx.x == 0) p.met[blockIdx.x] = any ? 1u : 0u;
+}
+
+__device__ __forceinline__ void umma_bf16x3(unsigned tmem_d, uint64_t desc_a, uint64_t desc_b, unsigned idesc, unsigned accumulate) {
+  asm volatile(
+      "{\n.reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
+      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+__global__ void __launch_bounds__(kXThreads, 1)
+gemm_f32x3_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const X3Params p) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + kXStages * kXStageBytes);   // full[S], empty[S], tfull[2], tempty[2]
+  unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * kXStages + 4);
+  int* stage_all = reinterpret_cast<int*>(tmem_slot + 4);
+  __shared__ int plain_s;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int num_kb = (p.K + kXK - 1) / kXK;
+  const int m_tiles = (p.M + kXM - 1) / kXM, n_tiles = (p.N + kXN - 1) / kXN;
+  const int num_tiles = p.batch * n_tiles * m_tiles;
+  const unsigned full0 = smem_u32(bars), empty0 = smem_u32(bars + kXStages);
+  const unsigned tfull0 = smem_u32(bars + 2 * kXStages), tempty0 = smem_u32(bars + 2 * kXStages + 2);
+
+  if (warp == 0 && lane == 0) {
+    for (int s = 0; s < kXStages; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(tfull0 + 8 * s, 1);
+      mbar_init(tempty0 + 8 * s, kXEpiWarps);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    plain_s = 0;
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2 * kXN) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  pdl_launch_dependents();
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const unsigned tmem_base = *tmem_slot;
+  pdl_wait();
+
+  if (warp == 0) {
+    if (lane == 0) {
+      unsigned it = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+        const int m_blk = tile % m_tiles, r = tile / m_tiles, n_blk = r % n_tiles, b = r / n_tiles;
+        for (int kb = 0; kb < num_kb; ++kb, ++it) {
+          const unsigned s = it % kXStages, ph = (it / kXStages) & 1;
+          ok = mbar_wait(empty0 + 8 * s, ph ^ 1, 1);
+          if (!ok) break;
+          mbar_expect_tx(full0 + 8 * s, kXStageBytes);
+          const unsigned dst = smem_u32(tiles + s * kXStageBytes);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            tma_load_3d(dst + i * kXPlane, &map_x, kb * kXK, m_blk * kXM, i * p.batch + b, full0 + 8 * s);
+            tma_load_3d(dst + (3 + i) * kXPlane, &map_w, kb * kXK, n_blk * kXN, i * p.batch + b, full0 + 8 * s);
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      // D = f32, A = B = bf16, both K-major
+      constexpr unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(kXN >> 3) << 17) | ((unsigned)(kXM >> 4) << 24);
+      unsigned it = 0;                               // one accumulation per stage
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+        for (int kb = 0; kb < num_kb; ++kb, ++it) {
+          const unsigned slot = it & 1, aph = (it >> 1) & 1, s = it % kXStages, ph = (it / kXStages) & 1;
+          ok = mbar_wait(tempty0 + 8 * slot, aph ^ 1, 4) && mbar_wait(full0 + 8 * s, ph, 2);
+          if (!ok) break;
+          tcgen05_fence_after();
+          const unsigned tmem_d = tmem_base + slot * kXN, base = smem_u32(tiles + s * kXStageBytes);
+          constexpr int ax[6] = {2, 1, 0, 1, 0, 0}, bw[6] = {0, 1, 2, 0, 1, 0};
+#pragma unroll
+          for (int t = 0; t < 6; ++t) {
+            const uint64_t da = make_smem_desc(base + ax[t] * kXPlane), db = make_smem_desc(base + (3 + bw[t]) * kXPlane);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) umma_bf16x3(tmem_d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (t > 0 || k > 0) ? 1u : 0u);
+          }
+          tcgen05_commit(empty0 + 8 * s);
+          tcgen05_commit(tfull0 + 8 * slot);
+        }
+      }
+    }
+  } else {
+    const int q = warp & 3, half = (warp - 2) >> 2, et = threadIdx.x - 64;
+    int* stage = stage_all + (warp - 2) * (32 * kXPitch);
+    unsigned met = 0;
+    for (int i = et; i < p.split_blocks; i += 32 * kXEpiWarps) met |= p.met[i];
+    if (met) plain_s = 1;
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * kXEpiWarps) : "memory");
+    const bool plain = plain_s != 0;
+    unsigned lc = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+      const int m_blk = tile % m_tiles, r = tile / m_tiles, n_blk = r % n_tiles, b = r / n_tiles;
+      float acc[2][32];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int j = 0; j < 32; ++j) acc[h][j] = 0.0f;
+      for (int kb = 0; kb < num_kb; ++kb, ++lc) {
+        const unsigned slot = lc & 1, aph = (lc >> 1) & 1;
+        if (ok) ok = mbar_wait(tfull0 + 8 * slot, aph, 3);
+        __syncwarp();
+        tcgen05_fence_after();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          int v[32];
+          tmem_ld_32x32(tmem_base + ((unsigned)(q * 32) << 16) + slot * kXN + (unsigned)(half * 64 + h * 32), v);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) acc[h][j] += __int_as_float(v[j]);
+        }
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(tempty0 + 8 * slot);
+      }
+      const int row0 = m_blk * kXM + q * 32, col0 = n_blk * kXN + half * 64;
+      if (plain && row0 + lane < p.M) {              // an operand is not finite
+        const float* xr = p.x.src + (int64_t)b * p.x.bstride + (int64_t)(row0 + lane) * p.x.pitch;
+#pragma unroll 1
+        for (int j = 0; j < 64 && col0 + j < p.N; ++j) {
+          const float* wr = p.w.src + (int64_t)b * p.w.bstride + (int64_t)(col0 + j) * p.w.pitch;
+          float s = 0.0f;
+          for (int k = 0; k < p.K; ++k) s = fmaf(xr[k], wr[k], s);
+#pragma unroll
+          for (int i = 0; i < 64; ++i)
+            if (i == j) acc[i >> 5][i & 31] = s;
+        }
+      }
+      if (p.act == B200F_ACT_XIELU) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int j = 0; j < 32; ++j) acc[h][j] = xielu_f32(acc[h][j], p.act_a, p.act_b);
+      }
+      float* out = p.out + (int64_t)b * p.out_bstride;
+      const int rr = lane >> 2, cc = (lane & 3) * 4;
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {                  // 16 columns at a time through the warp's staging tile
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 16; j += 4)
+          *reinterpret_cast<float4*>(stage + lane * kXPitch + j) =
+              make_float4(acc[h >> 1][16 * (h & 1) + j], acc[h >> 1][16 * (h & 1) + j + 1], acc[h >> 1][16 * (h & 1) + j + 2], acc[h >> 1][16 * (h & 1) + j + 3]);
+        __syncwarp();
+#pragma unroll
+        for (int it = 0; it < 4; ++it) {
+          const int row = row0 + it * 8 + rr, col = col0 + 16 * h + cc;
+          if (!ok || row >= p.M || col >= p.N) continue;
+          const float4 o = *reinterpret_cast<const float4*>(stage + (it * 8 + rr) * kXPitch + cc);
+          float* dst = out + (int64_t)row * p.out_pitch + col;
+          if (p.vec && col + 3 < p.N) {
+            *reinterpret_cast<float4*>(dst) = o;
+          } else {
+            dst[0] = o.x;
+            if (col + 1 < p.N) dst[1] = o.y;
+            if (col + 2 < p.N) dst[2] = o.z;
+            if (col + 3 < p.N) dst[3] = o.w;
+          }
+        }
+      }
+    }
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tcgen05_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * kXN) : "memory");
+  }
+}
+
+// ----------------------------------------------------------------------------- host side
+static int64_t x3_pitch(int64_t k) { return (k + 7) / 8 * 8; }
+static int64_t x3_bytes(int64_t rows, int64_t k, int64_t batch) { return (3 * batch * rows * x3_pitch(k) * 2 + 127) / 128 * 128; }
+
+static bool x3_map(CUtensorMap* map, const bf16* base, int64_t rows, int64_t K, int64_t kp, int64_t batch) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)(3 * batch)};
+  const cuuint64_t strides[2] = {(cuuint64_t)kp * 2, (cuuint64_t)(rows * kp) * 2};
+  const cuuint32_t box[3] = {(cuuint32_t)kXK, 128, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+}  // namespace b200
+
+using namespace b200;
+
+extern "C" size_t b200f_gemm_f32_ws_bytes(int64_t m, int64_t n, int64_t k, int64_t batch) {
+  if (m <= 0 || n <= 0 || k <= 0 || batch <= 0 || batch > 65535 / 3 || m >= (1ll << 31) || n >= (1ll << 31) || k >= (1ll << 31)) return 0;
+  // Few rows against many weight rows: the fp32 units read the weights once (4 bytes each) and fill the GPU with a tile of 64 x 64
+  // per CTA, the split moves 10 bytes of each (m = 16, n = 32768, k = 1024: 155 us against 177).  Everywhere else that kernel has too
+  // few CTAs (m = 16, n = 4608: 70 us against 51; n = 1024, k = 4096: 265 against 90) or too many products (m = 1400, n = 4608: 406
+  // against 92).
+  if (m <= 8) return 0;                             // gemv.cuh
+  if (m <= 64 && batch * ((n + 63) / 64) >= 2 * sm_count()) return 0;
+  return (size_t)(x3_bytes(m, k, batch) + x3_bytes(n, k, batch) + kXSplitBlocks * 4);
+}
+
+extern "C" int b200f_gemm_f32(const float* x, const float* w, float* out, int64_t m, int64_t n, int64_t k, int64_t batch, int64_t x_pitch,
+                              int64_t x_bstride, int64_t w_pitch, int64_t w_bstride, int64_t out_pitch, int64_t out_bstride, int act,
+                              float act_a, float act_b, void* ws, b200_stream_t s) {
+  B200_REQUIRE(x && w && out && ws, B200_E_NULL, "gemm_f32: null pointer");
+  B200_REQUIRE(b200f_gemm_f32_ws_bytes(m, n, k, batch) != 0, B200_E_SHAPE, "gemm_f32: m=%lld n=%lld k=%lld batch=%lld", (long long)m,
+               (long long)n, (long long)k, (long long)batch);
+  B200_REQUIRE(x_pitch >= k && w_pitch >= k && out_pitch >= n, B200_E_SHAPE, "gemm_f32: a row pitch is shorter than its row");
+  B200_REQUIRE(act == B200F_ACT_NONE || act == B200F_ACT_XIELU, B200_E_UNSUPPORTED, "gemm_f32: activation %d", act);
+  B200_REQUIRE((reinterpret_cast<uintptr_t>(ws) & 127u) == 0, B200_E_ALIGN, "gemm_f32: the workspace must be 128-byte aligned");
+  cudaStream_t st = (cudaStream_t)s;
+  unsigned char* at = (unsigned char*)ws;
+  X3Params p;
+  auto rows16 = [&](const float* base, int64_t pitch, int64_t bstride) { return aligned16(base) && pitch % 4 == 0 && (batch == 1 || bstride % 4 == 0); };
+  p.x = {x, m, x_pitch, x_bstride, (bf16*)at, rows16(x, x_pitch, x_bstride)};
+  at += x3_bytes(m, k, batch);
+  p.w = {w, n, w_pitch, w_bstride, (bf16*)at, rows16(w, w_pitch, w_bstride)};
+  at += x3_bytes(n, k, batch);
+  p.met = (unsigned*)at;
+  p.out = out; p.M = (int)m; p.N = (int)n; p.K = (int)k; p.batch = (int)batch; p.kp = (int)x3_pitch(k);
+  p.out_pitch = out_pitch; p.out_bstride = out_bstride; p.act = act; p.act_a = act_a; p.act_b = act_b;
+  p.vec = rows16(out, out_pitch, out_bstride);
+  const int64_t quads = batch * (m + n) * ((k + 3) / 4), blocks = (quads + 255) / 256;
+  p.split_blocks = (int)(blocks < kXSplitBlocks ? blocks : kXSplitBlocks);
+  CUtensorMap mx, mw;
+  B200_REQUIRE(x3_map(&mx, p.x.dst, m, k, p.kp, batch) && x3_map(&mw, p.w.dst, n, k, p.kp, batch), B200_E_CUDA, "gemm_f32: cuTensorMapEncodeTiled failed");
+  launch_pdl(split_parts_kernel, dim3(p.split_blocks), dim3(256), 0, st, p);
+  if (const int rc = check_launch("gemm_f32 (parts)")) return rc;
+  constexpr size_t smem = (size_t)kXStages * kXStageBytes + 1024 + (2 * kXStages + 4) * 8 + 16 + kXEpiWarps * 32 * kXPitch * 4;
+  static_assert(smem <= 227 * 1024, "shared memory budget");
+  const cudaError_t e = cudaFuncSetAttribute(gemm_f32x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  B200_REQUIRE(e == cudaSuccess, B200_E_CUDA, "gemm_f32: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  const int64_t tiles = batch * ((m + kXM - 1) / kXM) * ((n + kXN - 1) / kXN);
+  launch_pdl(gemm_f32x3_kernel, dim3((unsigned)(tiles < sm_count() ? tiles : sm_count())), dim3(kXThreads), smem, st, mx, mw, p);
+  return check_launch("gemm_f32");
+}
+
+extern "C" int b200f_gemm_f32_status(int* out_host, int reset) {
+  B200_REQUIRE(out_host, B200_E_NULL, "gemm_f32_status: null pointer");
+  cudaError_t e = cudaMemcpyFromSymbol(out_host, g_gemm_status, sizeof(int));
+  if (e == cudaSuccess && reset) {
+    const int zero = 0;
+    e = cudaMemcpyToSymbol(g_gemm_status, &zero, sizeof(int));
+  }
+  B200_REQUIRE(e == cudaSuccess, B200_E_CUDA, "gemm_f32_status: %s", cudaGetErrorString(e));
+  return B200_OK;
+}

@@ -56,6 +56,19 @@ def _check_vec(name: str, t: torch.Tensor, n: int) -> None:
 
 
 # ----------------------------------------------------------------------------- linears
+def _gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, T: int, n: int, k: int, batch: int, strides, parts: int = 1, act: int = ACT_NONE,
+          act_a: float = 0.0, act_b: float = 0.0) -> None:
+    """``strides``: row pitch and batch stride of x, of w and of out."""
+    if x.dtype == torch.float32:
+        need = query("b200f_gemm_f32_ws_bytes", T, n, k, batch) if act != ACT_GATED_SILU else 0
+        if need:
+            ws = torch.empty(need, dtype=torch.uint8, device=x.device)
+            call("b200f_gemm_f32", ptr(x), ptr(w), ptr(out), T, n, k, batch, *strides, act, act_a, act_b, ptr(ws), stream())
+            return
+    call("b200f_gemm", ptr(x), ptr(w), ptr(out), dtype_code(x.dtype), int(out.dtype == torch.float32), T, n, k, batch, *strides, parts, T * n, act,
+         act_a, act_b, stream())
+
+
 def linear(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, out_f32: bool = False, act: int = ACT_NONE,
            act_a: float = 0.0, act_b: float = 0.0) -> torch.Tensor:
     """act(x w^T) for rows x [T, k] and weight rows w [n, k]; with ACT_GATED_SILU (bf16) the weight rows alternate, 16 gates
@@ -66,9 +79,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
     n = w.shape[0]
     if out is None:
         out = rows(T, n // 2 if act == ACT_GATED_SILU else n, torch.float32 if out_f32 else x.dtype, x.device)
-    out_f32 = out.dtype == torch.float32
-    call("b200f_gemm", ptr(x), ptr(w), ptr(out), dtype_code(x.dtype), int(out_f32), T, n, k, 1, _pitch(x), 0, _pitch(w), 0,
-         _pitch(out), 0, 1, 0, act, act_a, act_b, stream())
+    _gemm(x, w, out, T, n, k, 1, (_pitch(x), 0, _pitch(w), 0, _pitch(out), 0), 1, act, act_a, act_b)
     return out
 
 
@@ -80,8 +91,7 @@ def linear_parts(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     n, code = w.shape[0], dtype_code(x.dtype)
     parts = query("b200f_gemm_splits", T, n, k, 1, code)
     out = torch.empty((parts, T, n), dtype=torch.float32, device=x.device)
-    call("b200f_gemm", ptr(x), ptr(w), ptr(out), code, 1, T, n, k, 1, _pitch(x), 0, _pitch(w), 0, n, 0, parts, T * n, ACT_NONE,
-         0.0, 0.0, stream())
+    _gemm(x, w, out, T, n, k, 1, (_pitch(x), 0, _pitch(w), 0, n, 0), parts)
     return out
 
 
@@ -98,14 +108,13 @@ def head_linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     if x.stride(2) != 1 or w.stride(2) != 1 or out.stride(2) != 1:
         raise ValueError("head_linear: rows must be contiguous")
     require_cuda(x, w, out)
-    call("b200f_gemm", ptr(x), ptr(w), ptr(out), dtype_code(x.dtype), int(out.dtype == torch.float32), T, n, k, H, x.stride(0), x.stride(1),
-         w.stride(1), w.stride(0), out.stride(0), out.stride(1), 1, 0, ACT_NONE, 0.0, 0.0, stream())
+    _gemm(x, w, out, T, n, k, H, (x.stride(0), x.stride(1), w.stride(1), w.stride(0), out.stride(0), out.stride(1)))
 
 
 def check_status() -> None:
     """Raises if a bounded wait inside a linear, the latent attention kernel or the chunked scan has expired since the last
     check.  Synchronises with the device."""
-    for name, what in (("b200f_gemm_status", "a bf16 linear"), ("b200f_latent_attn_status", "the latent attention kernel"),
+    for name, what in (("b200f_gemm_status", "a bf16 linear"), ("b200f_gemm_f32_status", "a 32-bit linear"), ("b200f_latent_attn_status", "the latent attention kernel"),
                        ("b200f_memory_scan_status", "the scan of a matrix memory")):
         st = ctypes.c_int(0)
         call(name, ctypes.byref(st), 1)

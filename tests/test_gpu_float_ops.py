@@ -61,6 +61,40 @@ def test_linear(dtype, m, n, k):
     fo.check_status()
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (3, 130, 63), (127, 128, 64), (128, 129, 65), (129, 127, 128), (300, 257, 200), (64, 512, 1500)])
+def test_linear_f32_in_three_parts(m, n, k):
+    """32-bit linears as products of three bf16 parts: sizes around the tiles (128 rows, 128 columns, 64 and 128 of K), operands of
+    all magnitudes, and rows that are not on 16-byte boundaries.  A product's error is below 2^-22 of it (three parts hold 24
+    bits; what is dropped is below 3 * 2^-26), a chain of 24 accumulations adds up to an ulp of its running sum each, most of them while that
+    is small: 4e-7 of what random operands add up to, |x| |w| / sqrt(k); a missing lowest part would be over 1e-6."""
+    g = torch.Generator(device="cuda").manual_seed(m * n + k)
+    x = torch.randn((m, k + 3), device="cuda", generator=g)[:, :k]
+    w = torch.randn((n, k + 3), device="cuda", generator=g)[:, 3:] * torch.exp2(torch.randint(-20, 20, (n, 1), device="cuda", generator=g).float())
+    want = x.double() @ w.double().T
+    got = fo.linear(x, w).double()
+    assert ((got - want).norm(dim=0) <= 4e-7 * k ** -0.5 * x.double().norm() * w.double().norm(dim=1)).all()
+    assert ((got - want).abs() <= 2.0 ** -20 * (x.double().abs() @ w.double().abs().T)).all()
+    parts = fo.linear_parts(x, w)
+    assert torch.equal(parts.sum(0), got.float())
+
+
+def test_linear_f32_keeps_infinities_nans_and_the_largest_numbers():
+    x, w = torch.randn((130, 70), device="cuda"), torch.randn((140, 70), device="cuda")
+    top = torch.finfo(torch.float32).max
+    x[5], x[6, 3] = 0.0, top
+    x[6, :3], x[6, 4:] = 0.0, 0.0
+    x[5, 7] = top
+    w[9] = 0.0
+    w[9, 3] = w[9, 7] = 1.0
+    got = fo.linear(x, w)
+    assert got[5, 9] == top and got[6, 9] == top and torch.isfinite(got[:5]).all()
+    x[0, 0], x[1, 1], x[2, 2], w[3, 4] = float("inf"), float("-inf"), float("nan"), float("inf")
+    got, want = fo.linear(x, w), (x.double() @ w.double().T).float()
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    assert torch.equal(got[torch.isinf(got)], want[torch.isinf(got)])
+    close(got[10:, 10:], host(want[10:, 10:]), torch.float32)
+
+
 def test_linear_splits_k_for_few_rows():
     g = torch.Generator().manual_seed(5)
     x, w = rows_of(g, 4, 4096, torch.bfloat16), rows_of(g, 256, 4096, torch.bfloat16)
