@@ -145,7 +145,7 @@ qkv_prepare_kernel(const int32_t* __restrict__ positions, const int32_t* __restr
       rope_row(src, is_q ? q_norm_w : k_norm_w, positions[t], cos_sin, max_pos, with_fwht, lane, a0, a1, b0, b1);
     }
     int m = max(max(0, abs_wrap(a0)), max(abs_wrap(a1), max(abs_wrap(b0), abs_wrap(b1))));
-    m = max(1, warp_max(m));
+    m = max(1, __reduce_max_sync(FULL_MASK, m));
     if (PENDING) {   // after a reduction over the loaded values: zeros for the next GEMM's partial sums
       __syncwarp();
       pending_clear2(pl, t, heads * kD, h * kD + 2 * lane);
@@ -179,7 +179,7 @@ qkv_prepare_kernel(const int32_t* __restrict__ positions, const int32_t* __restr
     const int hh = h - q_heads - kv_heads;
     const int4 b = PENDING ? pv : *reinterpret_cast<const int4*>(v + t * v_pitch + (int64_t)hh * kD + 4 * lane);
     int mv = max(max(0, abs_wrap(b.x)), max(abs_wrap(b.y), max(abs_wrap(b.z), abs_wrap(b.w))));
-    mv = max(1, warp_max(mv));
+    mv = max(1, __reduce_max_sync(FULL_MASK, mv));
     if (PENDING) {
       __syncwarp();
       pending_clear4(pl, t, heads * kD, h * kD + 4 * lane);

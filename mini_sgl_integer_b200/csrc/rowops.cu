@@ -343,14 +343,6 @@ __device__ __forceinline__ void fwht128_group(int (&val)[16], int lane8) {
   }
 }
 
-// The n = 128 scale rsr15(y * 2896).  2896 = 16 * 181, so (16a +- 2^14) >> 15 == (a +- 2^10) >> 11 with a = y * 181
-// (64 bits), and for y < 0 floor((a - 2^10) / 2^11) == floor((a + 2^10) / 2^11) - 1: one wide multiply-add, one
-// funnel shift (the result fits: |result| < |y|) and the sign word.
-__device__ __forceinline__ int fwht_scale128(int y) {
-  const long long a = (long long)y * 181LL + 1024LL;
-  return (int)__funnelshift_r((unsigned)a, (unsigned)(a >> 32), 11) + (y >> 31);
-}
-
 // FWHT-128 butterflies without saturation: valid when every input satisfies |v| < 2^24, so that
 // no partial sum can leave int32 (seven stages add seven bits).
 __device__ __forceinline__ void fwht128_group_nosat(int (&val)[16], int lane8) {

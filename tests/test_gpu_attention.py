@@ -440,6 +440,23 @@ def test_fused_qkv_preparation_equals_the_separate_steps():
         eq(a.meta(0).cpu().numpy(), b.meta(0).cpu().numpy())
 
 
+@pytest.mark.parametrize("top", [2**21, 2**22 - 1, 2**22, 2**25, 2**31 - 1])
+def test_rotation_at_the_limit_of_the_plain_stages(top):
+    """Rows whose largest value lies around 2^22, up to which no stage of the rotation or the butterflies can saturate."""
+    from mini_sgl_integer_b200.kernel import fixed_point as fp
+    from oracle import fixed_point as ofp
+    rng = np.random.default_rng(top % 1000)
+    x = rng.integers(-top, top + 1, (6, 4, 128)).astype(np.int32)
+    x[0] = top                                                   # every butterfly adds up
+    x[1, :, ::2], x[1, :, 1::2] = top, -top
+    cache = np.full((8, 128), 23170, dtype=np.int32)             # 45 degrees: both halves of a pair add up
+    cache[0] = 32767
+    pos = np.arange(6, dtype=np.int32)
+    want, _ = ofp.rope_fwht_q15(pos, x, x[:, :1], cache)
+    got, _ = fp.rope_fwht_int_q15(d(pos), d(x), d(x[:, :1]), d(cache))
+    eq(got.cpu().numpy().reshape(want.shape), want.astype(np.int32))
+
+
 def test_decode_seeded_sweep_of_shapes_and_options():
     """Random batches, group sizes, cluster sizes, row orders and output forms, both implementations."""
     rng = np.random.default_rng(2024)
