@@ -102,7 +102,7 @@ B200_API int b200f_latent_prepare(const float* qd, int splits, int64_t split_str
  * visible keys i - window < j <= i (window 0: all j <= i), softmax whose denominator also has exp(sink[h]);
  * out[i, h] = sum_j p cache[j][0 .. kv_rank).  out [tokens, heads, out_pitch].
  * key_splits > 1 needs ws of b200f_latent_attn_ws_floats floats.  simple != 0 selects the plain kernel (always for
- * B200F_F32 and for sizes the tensor-core kernel does not take). */
+ * B200F_F32 decode steps and for sizes the tiled kernels do not take). */
 B200_API size_t b200f_latent_attn_ws_floats(int64_t tokens, int heads, int kv_rank, int key_splits);
 B200_API int b200f_latent_attn_splits(int64_t tokens, int batch, int max_q, int max_kv, int heads, int kv_rank,
                                       int rot_dim, int window, int dtype);

@@ -12,7 +12,8 @@
 //                         the columns of the output, and meet at two named barriers per tile.  Scores, softmax and
 //                         accumulators are fp32.  Long key ranges of small batches are split over CTAs and merged by
 //                         latent_merge_kernel.
-// latent_attn_kernel      any size, any type, one CTA per (token, head); the 32-bit path.
+// latent_attn_f32_kernel  32-bit prompts, on the fp32 units.
+// latent_attn_kernel      any size, any type, one CTA per (token, head); 32-bit decode steps.
 #include "float_common.cuh"
 #include "umma.cuh"
 
@@ -169,6 +170,229 @@ latent_attn_kernel(const AttnParams p, const T* __restrict__ q_lat, const T* __r
   }
   T* dst = out + (t * p.heads + h) * p.out_pitch;
   for (int i = threadIdx.x; i < p.kv_rank; i += 128) dst[i] = from_f32<T>(o[i] / l);
+}
+
+// ---------------------------------------------------------------------------------------------------
+// 32-bit prompts: 32 rows (tokens x heads that share their keys) against tiles of 32 keys, on the fp32 units.  One CTA per
+// (token, head) read every key 16 times over and kept one load in flight: 1673 us for five prompts of 60 .. 500 tokens with
+// 16 heads of 288 columns, where the multiplications alone take 62 us.  Here a key row is fetched once per 32 rows and
+// comes from shared memory as float4: a thread holds 4 x 4 scores over a quarter of the columns (8 loads for 32 packed
+// multiply-adds, so the multiply-adds are the bound, and the short chains lose no digits), then 8 rows x 4 columns of the
+// output (3 loads for 32): 205 us now, and 100 instead of 206 us for two tokens of one sequence with 700 keys.
+constexpr int kF32Rows = 32, kF32Keys = 32, kF32Threads = 256;
+constexpr int kF32PartPitch = kF32Keys + 4;
+static __host__ __device__ int f32_pitch(int d) { return ((d + 31) & ~31) + 4; }     // float4 rows 4 banks apart
+static size_t f32_smem(int d, int stages) {
+  return sizeof(float) * ((size_t)(kF32Rows + stages * kF32Keys) * f32_pitch(d) + (size_t)4 * kF32Rows * kF32PartPitch +
+                          (size_t)kF32Keys * kF32PartPitch + kF32Rows) + sizeof(unsigned) * kF32Rows;
+}
+
+// NC: pieces of 256 output columns; STAGES 2: the next tile arrives while one is worked on.
+template <int NC, int STAGES>
+__global__ void __launch_bounds__(kF32Threads, NC == 1 ? 2 : 1)
+latent_attn_f32_kernel(const AttnParams p, const float* __restrict__ q_lat, const float* __restrict__ cache, float* __restrict__ out) {
+  constexpr int R = kF32Rows, NK = kF32Keys, PP = kF32PartPitch;
+  extern __shared__ __align__(16) float smf[];
+  const int D = p.kv_rank + p.rot_dim, ld = f32_pitch(D), d4 = D >> 2;
+  float* qs = smf;                                 // [R][ld]
+  float* ks = qs + R * ld;                         // [STAGES][NK][ld]
+  float* part = ks + STAGES * NK * ld;             // [4][R][PP] scores of a quarter of the columns
+  float* pt = part + 4 * R * PP;                   // [NK][PP] weights, a row per key
+  float* row_alpha = pt + NK * PP;                 // [R]: factor of the tile, in the end 1 / sum
+  unsigned* row_vis = reinterpret_cast<unsigned*>(row_alpha + R);   // [R] keys of the tile that a row sees
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int q_tile = gridDim.x - 1 - blockIdx.x, hg = blockIdx.y, seq = blockIdx.z;   // the longest rows first
+  const int start = p.seq_start[seq], count = p.seq_start[seq + 1] - start;
+  const int tok0 = q_tile * p.tokens_per_cta;
+  if (tok0 >= count) return;
+  const int ntok = min(p.tokens_per_cta, count - tok0);
+  const int h0 = hg * p.heads_per_cta, nh = min(p.heads_per_cta, p.heads - h0), rows = ntok * nh;
+  const int pos0 = p.kv_lens[seq] - count + tok0;
+  const int key_lo = first_key(pos0, p.window), key_hi = pos0 + ntok;
+  const int tiles = (key_hi - key_lo + NK - 1) / NK;
+  const int32_t* pages = p.page_table + (int64_t)seq * p.table_pitch;
+
+  auto copy_tile = [&](int tile) {                 // rows behind the last key repeat it (they are masked)
+    float* dst = ks + (tile % STAGES) * NK * ld;
+#pragma unroll
+    for (int j = 0; j < NK / 8; ++j) {
+      const int r = warp * (NK / 8) + j, key = min(key_lo + tile * NK + r, key_hi - 1);
+      const float* src = cache + ((int64_t)__ldg(pages + key / kPage) * kPage + key % kPage) * p.lat_pitch;
+      const unsigned to = smem_u32(dst + r * ld);
+      for (int c = lane; c < d4; c += 32) cp_async16(to + 16 * c, src + 4 * c);
+    }
+    cp_async_commit();
+  };
+  copy_tile(0);
+  for (int r = warp; r < R; r += 8) {
+    const int tok = r < rows ? r / nh : 0;
+    const float4* src = reinterpret_cast<const float4*>(q_lat + ((int64_t)(start + tok0 + tok) * p.heads + h0 + (r < rows ? r - tok * nh : 0)) * p.lat_pitch);
+    for (int c = lane; c < d4; c += 32) *reinterpret_cast<float4*>(qs + r * ld + 4 * c) = r < rows ? src[c] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  }
+
+  // scores: thread (ty, tx) of quarter kg has rows ty + 8 i and keys tx + 8 j
+  const int kg = tid >> 6, tx = tid & 7, ty = (tid >> 3) & 7;
+  const int c_per = (d4 + 3) >> 2, c_lo = min(kg * c_per, d4), c_hi = min(c_lo + c_per, d4);
+  // softmax: row sr, keys 4 sk ..
+  const int sr = tid >> 3, sk = 4 * (tid & 7);
+  const int pos = pos0 + sr / nh, vis_hi = sr < rows ? pos : -1, vis_lo = p.window > 0 ? pos - p.window + 1 : 0;
+  const float sink2 = sr < rows ? p.sink[h0 + sr % nh] * kLog2e : 0.0f;
+  float m = sink2, l = tid % 8 == 0 ? 1.0f : 0.0f;  // the sink is a key without a value whose score is sink2
+  // output: rows r0 .., columns 256 n + c0 ..
+  const int r0 = 8 * (tid >> 6), c0 = 4 * (tid & 63);
+  float acc[NC][8][4];
+#pragma unroll
+  for (int n = 0; n < NC; ++n)
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) acc[n][i][k] = 0.0f;
+
+  for (int tile = 0; tile < tiles; ++tile) {
+    const float* kt = ks + (tile % STAGES) * NK * ld;
+    if (STAGES > 1 && tile + 1 < tiles) {
+      copy_tile(tile + 1);
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
+    }
+    __syncthreads();
+    {
+      f32x2 s[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[i][j] = 0ull;
+      const float *qp = qs + ty * ld, *kp = kt + tx * ld;
+#pragma unroll 2
+      for (int c = c_lo; c < c_hi; ++c) {
+        ulonglong2 a[4], b[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          a[i] = *reinterpret_cast<const ulonglong2*>(qp + 8 * i * ld + 4 * c);
+          b[i] = *reinterpret_cast<const ulonglong2*>(kp + 8 * i * ld + 4 * c);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) s[i][j] = fma2(a[i].y, b[j].y, fma2(a[i].x, b[j].x, s[i][j]));
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 v = unpack2(s[i][j]);
+          part[(kg * R + ty + 8 * i) * PP + tx + 8 * j] = v.x + v.y;
+        }
+    }
+    __syncthreads();
+    bool odd = false;                              // a score that is not finite: some key entry or query may not be
+    {
+      float v[4];
+      const float* src = part + sr * PP + sk;
+      const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + R * PP);
+      const float4 c = *reinterpret_cast<const float4*>(src + 2 * R * PP), d = *reinterpret_cast<const float4*>(src + 3 * R * PP);
+      v[0] = (a.x + b.x) + (c.x + d.x); v[1] = (a.y + b.y) + (c.y + d.y);
+      v[2] = (a.z + b.z) + (c.z + d.z); v[3] = (a.w + b.w) + (c.w + d.w);
+      unsigned vis = 0;
+      float mn = m;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int key = key_lo + tile * NK + sk + k;
+        odd |= !(fabsf(v[k]) < INFINITY);
+        const bool seen = key <= vis_hi && key >= vis_lo;
+        vis |= (seen ? 1u : 0u) << (sk + k);
+        v[k] = seen ? v[k] * p.scale2 : -INFINITY;
+        mn = fmaxf(mn, v[k]);
+      }
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) {
+        mn = fmaxf(mn, __shfl_xor_sync(FULL_MASK, mn, o));
+        vis |= __shfl_xor_sync(FULL_MASK, vis, o);
+      }
+      const float mu = mn == -INFINITY ? 0.0f : mn;  // nothing seen so far: every weight is 0
+      const float alpha = exp2f(m - mu);
+      m = mn;
+      float e = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float w = exp2f(v[k] - mu);
+        pt[(sk + k) * PP + sr] = w;
+        e += w;
+      }
+      l = fmaf(l, alpha, e);
+      if (sk == 0) {
+        row_alpha[sr] = alpha;
+        row_vis[sr] = vis;
+      }
+    }
+    const bool careful = __syncthreads_or(odd);
+    // output: the tile's sum first, then one addition to the scaled total
+#pragma unroll
+    for (int n = 0; n < NC; ++n) {
+      const int col = 256 * n + c0;
+      if (col >= p.kv_rank) continue;
+      float t[8][4];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) t[i][k] = 0.0f;
+      const float *vp = kt + col, *wp = pt + r0;
+      if (!careful) {
+#pragma unroll 4
+        for (int j = 0; j < NK; ++j) {
+          const float4 x = *reinterpret_cast<const float4*>(vp + j * ld);
+          const float4 wa = *reinterpret_cast<const float4*>(wp + j * PP), wb = *reinterpret_cast<const float4*>(wp + j * PP + 4);
+          const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            t[i][0] = fmaf(w[i], x.x, t[i][0]); t[i][1] = fmaf(w[i], x.y, t[i][1]);
+            t[i][2] = fmaf(w[i], x.z, t[i][2]); t[i][3] = fmaf(w[i], x.w, t[i][3]);
+          }
+        }
+      } else {                                     // only the keys that a row sees: 0 times infinity must not reach the others
+        for (int j = 0; j < NK; ++j) {
+          const float4 x = *reinterpret_cast<const float4*>(vp + j * ld);
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if ((row_vis[r0 + i] >> j) & 1u) {
+              const float w = wp[j * PP + i];
+              t[i][0] = fmaf(w, x.x, t[i][0]); t[i][1] = fmaf(w, x.y, t[i][1]);
+              t[i][2] = fmaf(w, x.z, t[i][2]); t[i][3] = fmaf(w, x.w, t[i][3]);
+            }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float al = row_alpha[r0 + i];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[n][i][k] = fmaf(acc[n][i][k], al, t[i][k]);
+      }
+    }
+    __syncthreads();
+    if (STAGES == 1 && tile + 1 < tiles) copy_tile(tile + 1);
+  }
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) l += __shfl_xor_sync(FULL_MASK, l, o);
+  if (sk == 0) row_alpha[sr] = l;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = r0 + i;
+    if (r >= rows) continue;
+    const int tok = r / nh;
+    float* dst = out + ((int64_t)(start + tok0 + tok) * p.heads + h0 + r - tok * nh) * p.out_pitch;
+    const float sum = row_alpha[r];
+#pragma unroll
+    for (int n = 0; n < NC; ++n) {
+      const int col = 256 * n + c0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (col + k < p.kv_rank) dst[col + k] = acc[n][i][k] / sum;
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -547,6 +771,14 @@ static int launch_mma(const AttnParams& p, const bf16* q, const bf16* cache, bf1
   return check_launch("latent_attn");
 }
 
+template <int NC, int STAGES>
+static int launch_f32(const AttnParams& p, const float* q, const float* cache, float* out, dim3 grid, size_t smem, cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute(latent_attn_f32_kernel<NC, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  B200_REQUIRE(e == cudaSuccess, B200_E_CUDA, "latent_attn: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  launch_pdl(latent_attn_f32_kernel<NC, STAGES>, grid, dim3(kF32Threads), smem, st, p, q, cache, out);
+  return check_launch("latent_attn (32-bit)");
+}
+
 static int tiles_for(int max_q, int max_kv, int window, int tokens_per_cta) {
   int64_t span = max_kv;
   if (window > 0 && span > (int64_t)window + tokens_per_cta - 1) span = (int64_t)window + tokens_per_cta - 1;
@@ -612,6 +844,21 @@ extern "C" int b200f_latent_attn(const void* q_lat, const void* cache, const int
                scale * kLog2e, key_splits, ws, 1, heads, 1};
   const AttnPlan pl = (dtype == B200F_BF16 && !simple && lat_pitch % 8 == 0 && out_pitch % 2 == 0 && aligned16(q_lat) && aligned16(cache))
                           ? plan_attn(max_q, heads, kv_rank, rot_dim) : AttnPlan{0, 0, 0, 0, 0, 0};
+  // 32-bit prompts: whole float4 columns, up to 768 of them for the output (accumulators), 32 rows and keys in shared memory
+  const int D = kv_rank + rot_dim, f32_stages = f32_smem(D, 2) <= 227 * 1024 ? 2 : 1;
+  if (dtype == B200F_F32 && !simple && seq_start && max_q > 1 && D % 4 == 0 && lat_pitch % 4 == 0 && kv_rank <= 768 && aligned16(q_lat) &&
+      aligned16(cache) && f32_smem(D, f32_stages) <= 227 * 1024) {
+    p.splits = 1;
+    p.heads_per_cta = heads < kF32Rows ? heads : kF32Rows;
+    p.tokens_per_cta = kF32Rows / p.heads_per_cta;
+    p.head_groups = (heads + p.heads_per_cta - 1) / p.heads_per_cta;
+    const dim3 grid((unsigned)((max_q + p.tokens_per_cta - 1) / p.tokens_per_cta), (unsigned)p.head_groups, (unsigned)batch);
+    const float *q = (const float*)q_lat, *kc = (const float*)cache;
+    const size_t smem = f32_smem(D, f32_stages);
+    if (kv_rank <= 256) return f32_stages == 2 ? launch_f32<1, 2>(p, q, kc, (float*)out, grid, smem, st) : launch_f32<1, 1>(p, q, kc, (float*)out, grid, smem, st);
+    if (kv_rank <= 512) return f32_stages == 2 ? launch_f32<2, 2>(p, q, kc, (float*)out, grid, smem, st) : launch_f32<2, 1>(p, q, kc, (float*)out, grid, smem, st);
+    return launch_f32<3, 1>(p, q, kc, (float*)out, grid, smem, st);
+  }
   if (pl.mt == 0) {
     const size_t smem = (size_t)(2 * kv_rank + rot_dim + 128 + 8) * sizeof(float);
     B200_REQUIRE(smem <= 227 * 1024, B200_E_UNSUPPORTED, "latent_attn: kv_rank %d is too large", kv_rank);

@@ -347,6 +347,35 @@ def test_latent_attention_prompts_portions_and_decode(dtype, simple, heads, rank
         close(out[..., :rank], want, dtype, 3e-5, 1.5e-2)
 
 
+@pytest.mark.parametrize("heads,rank,rot,window", [(16, 256, 32, 0), (1, 36, 0, 7), (33, 64, 20, 40), (12, 300, 24, 0), (16, 512, 64, 100), (3, 700, 96, 0)])
+def test_latent_attention_32_bit_prompts(heads, rank, rot, window):
+    """One and two pieces in flight, one to three pieces of output columns, rows that do not fill a tile; against 64 bits and
+    the plain kernel, whose error it may exceed by rounding in the last place only.  A key that is not finite reaches the
+    rows that see it and no other."""
+    rng = np.random.default_rng(rank)
+    kv_lens, q_lens, scale = [70, 1, 33, 200], [70, 1, 2, 65], (rank + rot) ** -0.5
+    cache, table, keys, qs, q_lat = attention_case(rng, kv_lens, q_lens, heads, rank, rot, torch.float32)
+    sink, starts = rng.standard_normal(heads) * 2, i32(np.concatenate([[0], np.cumsum(q_lens)]))
+    want = attention_reference(keys, qs, kv_lens, q_lens, heads, rank, window or None, scale, sink)
+    outs = {}
+
+    def run(simple):
+        out = torch.full((sum(q_lens), heads, fo.pad8(rank)), 5.0, device="cuda")
+        fo.latent_attention(q_lat, cache, table, i32(kv_lens), starts, dev(sink), out, rank, rot, window, scale, max(q_lens), max(kv_lens), simple=simple)
+        return out[..., :rank]
+    for simple in (False, True):
+        outs[simple] = run(simple)
+        close(outs[simple], want, torch.float32, 3e-5)
+    size = {k: np.sqrt(np.mean((host(v) - want) ** 2)) for k, v in outs.items()}
+    assert size[False] <= 1.2 * size[True] + 2.0 ** -24 * np.sqrt(np.mean(want ** 2))
+    t, at = 20, host(table)[0]                                  # token 20 of the first prompt
+    cache[int(at[t // 16]), t % 16, rank // 2] = float("inf")
+    got, plain = run(False), run(True)
+    assert bool((torch.isfinite(got) == torch.isfinite(plain)).all())
+    seen = slice(t, min(70, t + (window or 70)))
+    assert not bool(torch.isfinite(got[seen]).all(2).any()) and bool(torch.isfinite(got[:t]).all()) and bool(torch.isfinite(got[70:]).all())
+
+
 @pytest.mark.parametrize("heads,rank,rot", [(8, 64, 16), (40, 128, 32)])
 @pytest.mark.parametrize("splits", [2, 5, 11])
 def test_latent_attention_with_split_keys(heads, rank, rot, splits):
