@@ -6,14 +6,14 @@
 //   out[t, n]  = sat32(mul_shift(acc, (x_mul[t] * w_mul[n]) >> 32, x_shift[t] + w_shift[n] - 48))
 //
 // Both operands are K-major (x8 [M, K] and w8 [N, K] row-major), which is what the UMMA wants.
-// A tile is 128 x BN outputs (BN = 256 at large M, down to 32 at decode sizes):
+// A tile of the one-CTA kernel is 128 x BN outputs (BN tokens, 32 .. 256):
 //   warp 0        TMA producer (one lane): A tile 128 x 128 B and B tile BN x 128 B per k-block
 //   warp 1        allocates tensor memory; one lane issues the MMAs (4 per k-block, K = 32 each)
 //   warps 2..9    epilogue: two per 32-lane quarter of the accumulator tile, half the columns each
 // The kernel is persistent (one CTA per SM walks a strided list of tiles) and keeps two accumulator
 // copies in tensor memory, so the epilogue of one tile overlaps the MMAs of the next.
 //
-// Decode sizes (M <= 256 tokens) run "weights-stationary" (template flag WS): the operands swap
+// Decode sizes (M <= 256 tokens) run "weights-stationary", prompts of few tiles too: the operands swap
 // roles - 128 weight rows are the UMMA's M side, all the tokens its N side - so every weight byte
 // crosses HBM once and a tile's accumulators are out^T.  A thread then holds one weight channel and 32
 // tokens, and the store of a token's 32 channels by a warp is one contiguous 128 bytes.  When the
@@ -65,6 +65,8 @@ struct GemmParams {
                             // (one tile each, finished in the GEMM kernel); `splits` applies to the blocks after them
   int32_t* partial;         // splits > 1: int32 [M, N] that the parts are added into (zeroed before the launch)
   int split_col0;           // first output channel that belongs to a split block
+  int tok_tile, tok_tiles;  // two-CTA weights-stationary kernel: tokens per tile (a multiple of 32) and tiles of them; its
+                            // blocks are (block of weight rows, token tile), the tiles of one block side by side
   int n_peers;              // > 0: tensor-parallel reduction - every part is added into each of these [M, N] buffers
   int32_t* peer[8];         //      (this rank's and its peers', mapped into this process: NVLink peer memory)
   int tp_on;                // the peers' buffers are the accumulator halves of tensor-parallel exchange blocks: the
@@ -127,11 +129,11 @@ __device__ __forceinline__ void store_chunk(int32_t* stage, int lane, const int 
   }
 }
 
-// Persistent kernel: CTA c computes tiles c, c + gridDim.x, ...  (tile -> n block outer, m block inner,
-// so the CTAs running at the same time share one block of weight rows in L2).  The accumulator
+// Persistent weights-stationary kernel: CTA c computes tiles c, c + gridDim.x, ... of (block of 128 weight rows, part of K),
+// all tokens wide.  The accumulator
 // lives in tensor memory twice (2 x BN columns): while the epilogue warps drain one copy, the MMA
 // warp already fills the other with the next tile.
-template <int BN, int STAGES, bool WS>
+template <int BN, int STAGES>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  const GemmParams p) {
@@ -143,15 +145,11 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   // barriers: full[S], empty[S], tmem_full[2], tmem_empty[2]
   uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + STAGES * kStageBytes);
   unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * STAGES + 4);
-  int32_t* col_scale = reinterpret_cast<int32_t*>(tmem_slot + 4);   // [2 slots][mul BN | shift BN]
-  int32_t* stage_all = col_scale + 4 * BN;                          // [epilogue warps][32][kStagePitch]
+  int32_t* tok_scale = reinterpret_cast<int32_t*>(tmem_slot + 4);   // [2 slots][mul BN | shift BN] per token
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_kb = (p.K + kBK - 1) / kBK;
-  // WS: a tile is (block of 128 weight rows, part of K); otherwise (block of BN weight rows, block of 128 tokens)
-  const int m_tiles = WS ? 1 : (p.M + kBM - 1) / kBM;
-  const int n_tiles = WS ? (p.N + kBM - 1) / kBM : (p.N + BN - 1) / BN;
-  const int num_tiles = WS ? p.full_blocks + (n_tiles - p.full_blocks) * p.splits : m_tiles * n_tiles;
+  const int num_tiles = p.full_blocks + ((p.N + kBM - 1) / kBM - p.full_blocks) * p.splits;
   const unsigned full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES);
   const unsigned tfull0 = smem_u32(bars + 2 * STAGES), tempty0 = smem_u32(bars + 2 * STAGES + 2);
 
@@ -178,7 +176,7 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   pdl_wait();               // barriers, tensor memory and descriptors are set up; the operands come from earlier kernels
   // exchange-block mode: word offset, inside this rank's block, of the accumulator half in use
   int64_t tp_acc_off = 0;
-  if (WS && p.tp_on) {
+  if (p.tp_on) {
     const TpLayout l = tp_layout(p.tp.m_max, p.tp.n);
     const int half = *reinterpret_cast<volatile int32_t*>(p.tp.base[p.tp.rank] + 1) & 1;
     tp_acc_off = l.acc + (int64_t)half * l.acc_half;
@@ -189,20 +187,15 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       unsigned it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        int n_blk = tile / m_tiles, m_blk = tile - n_blk * m_tiles, kb0 = 0, kb1 = num_kb;
-        if (WS) {
-          const WsTile t = ws_tile(p, tile, num_kb);
-          n_blk = t.n_blk; kb0 = t.kb0; kb1 = t.kb1;
-        }
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        const WsTile t = ws_tile(p, tile, num_kb);
+        for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
           const unsigned s = it % STAGES, ph = (it / STAGES) & 1;
           ok = mbar_wait(empty0 + 8 * s, ph ^ 1, 1);
           if (!ok) break;
           mbar_expect_tx(full0 + 8 * s, kStageBytes);
           const unsigned a_dst = smem_u32(tiles + s * kStageBytes);
-          // map_a always feeds the 128-row operand: token rows, or weight rows in WS mode (map_b: all tokens)
-          tma_load_2d(a_dst, &map_a, kb * kBK, (WS ? n_blk : m_blk) * kBM, full0 + 8 * s);
-          tma_load_2d(a_dst + kABytes, &map_b, kb * kBK, WS ? 0 : n_blk * BN, full0 + 8 * s);
+          tma_load_2d(a_dst, &map_a, kb * kBK, t.n_blk * kBM, full0 + 8 * s);
+          tma_load_2d(a_dst + kABytes, &map_b, kb * kBK, 0, full0 + 8 * s);
         }
       }
     }
@@ -217,12 +210,8 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         if (!ok) break;
         tcgen05_fence_after();
         const unsigned tmem_d = tmem_base + slot * BN;
-        int kb0 = 0, kb1 = num_kb;
-        if (WS) {
-          const WsTile t = ws_tile(p, tile, num_kb);
-          kb0 = t.kb0; kb1 = t.kb1;
-        }
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        const WsTile t = ws_tile(p, tile, num_kb);
+        for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
           const unsigned s = it % STAGES, ph = (it / STAGES) & 1;
           ok = mbar_wait(full0 + 8 * s, ph, 2);
           if (!ok) break;
@@ -233,7 +222,7 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           for (int k = 0; k < kBK / kUmmaK; ++k) {
             // the next 32 bytes of K inside the swizzle row: start address + 32 (encoded >> 4)
             umma_i8(tmem_d, da + (uint64_t)(k * kUmmaK >> 4), db + (uint64_t)(k * kUmmaK >> 4), idesc,
-                    (kb > kb0 || k > 0) ? 1u : 0u);
+                    (kb > t.kb0 || k > 0) ? 1u : 0u);
           }
           tcgen05_commit(empty0 + 8 * s);   // frees the stage once these MMAs have read it
         }
@@ -248,118 +237,66 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const int q = warp & 3;
     const int half = (warp - 2) >> 2;
     const int et = threadIdx.x - 64;   // 0 .. 32 * kEpiWarps - 1
-    int32_t* stage = stage_all + (warp - 2) * (32 * kStagePitch);
     unsigned lt = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++lt) {
-      const int n_blk = tile / m_tiles, m_blk = tile - n_blk * m_tiles;
       const unsigned slot = lt & 1, aph = (lt >> 1) & 1;
-      int32_t* cs = col_scale + slot * 2 * BN;
-      if (WS) {
-        // rows of the accumulator tile are weight channels, columns are tokens
-        const WsTile wt = ws_tile(p, tile, num_kb);
-        const int ch = wt.n_blk * kBM + q * 32 + lane;
-        const bool direct = !wt.split && p.n_peers == 0;
-        const bool empty_part = wt.kb0 >= wt.kb1;      // a part of K with no k-blocks: nothing was accumulated
-        if (direct && p.out_q15) {
-          for (int c = et; c < BN; c += 32 * kEpiWarps) {
-            const int t = min(c, p.M - 1);
-            int tm, ts;
-            if (p.x_absmax) absmax_to_ms_dev(__ldg(p.x_absmax + t), &tm, &ts);
-            else { tm = __ldg(p.x_mul + t); ts = __ldg(p.x_shift + t); }
-            cs[c] = tm;
-            cs[BN + c] = ts - 48;
-          }
-        }
-        int wm = 0, ws = 0;
-        if (ch < p.N && direct && p.out_q15) { wm = __ldg(p.w_mul + ch); ws = p.w_shift ? __ldg(p.w_shift + ch) : 31; }
-        epilogue_bar_sync();
-        if (ok) ok = mbar_wait(tfull0 + 8 * slot, aph, 3);
-        tcgen05_fence_after();
-#pragma unroll 1
-        for (int c0 = half * 32; c0 < BN; c0 += 64) {
-          int v[32];
-          tmem_ld_32x32(tmem_base + ((unsigned)(q * 32) << 16) + slot * BN + (unsigned)c0, v);
-          if (!ok || c0 >= p.M || ch >= p.N || empty_part) continue;
-          if (p.tp_on) {
-            // exchange-block mode: the parts are added into the rank's OWN accumulators (L2 atomics); the peers fetch
-            // them from there once this kernel has signalled
-            int32_t* dst = p.tp.base[p.tp.rank] + tp_acc_off;
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (c0 + j < p.M) atomicAdd(dst + (int64_t)(c0 + j) * p.N + ch, v[j]);
-          } else if (p.n_peers > 0) {
-            // tensor-parallel sum: the tile's partial sums go straight into every rank's accumulator (a warp's
-            // 32 channels of one token are one 128-byte reduction over NVLink); integer adds commute, so every
-            // rank ends up with the same bits whatever the arrival order
-            for (int r = 0; r < p.n_peers; ++r) {
-              int32_t* dst = p.peer[r];
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (c0 + j < p.M) atomicAdd(dst + (int64_t)(c0 + j) * p.N + ch, v[j]);
-            }
-          } else if (!direct) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (c0 + j < p.M) atomicAdd(p.partial + (int64_t)(c0 + j) * p.N + ch, v[j]);   // result unused: a reduction
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              if (c0 + j < p.M) {
-                const int64_t o = (int64_t)(c0 + j) * p.N + ch;
-                if (p.acc_out) p.acc_out[o] = v[j];
-                if (p.out_q15) p.out_q15[o] = requant_one(v[j], __mulhi(cs[c0 + j], wm), cs[BN + c0 + j] + ws);
-              }
-            }
-          }
-        }
-        tcgen05_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(tempty0 + 8 * slot);
-        continue;
-      }
-      const int row = m_blk * kBM + q * 32 + lane;
-      // the tile's per-column scales go to shared memory once (double-buffered by accumulator slot)
-      if (p.out_q15) {
+      int32_t* cs = tok_scale + slot * 2 * BN;
+      // rows of the accumulator tile are weight channels, columns are tokens
+      const WsTile wt = ws_tile(p, tile, num_kb);
+      const int ch = wt.n_blk * kBM + q * 32 + lane;
+      const bool direct = !wt.split && p.n_peers == 0;
+      const bool empty_part = wt.kb0 >= wt.kb1;      // a part of K with no k-blocks: nothing was accumulated
+      if (direct && p.out_q15) {
         for (int c = et; c < BN; c += 32 * kEpiWarps) {
-          const int col = min(n_blk * BN + c, p.N - 1);
-          cs[c] = __ldg(p.w_mul + col);
-          cs[BN + c] = (p.w_shift ? __ldg(p.w_shift + col) : 31) - 48;   // x_shift + w_shift - 48 later
+          const int t = min(c, p.M - 1);
+          int tm, ts;
+          if (p.x_absmax) absmax_to_ms_dev(__ldg(p.x_absmax + t), &tm, &ts);
+          else { tm = __ldg(p.x_mul + t); ts = __ldg(p.x_shift + t); }
+          cs[c] = tm;
+          cs[BN + c] = ts - 48;
         }
       }
-      int xm = 0, xs = 0;
-      if (row < p.M && p.out_q15) {
-        if (p.x_absmax) absmax_to_ms_dev(__ldg(p.x_absmax + row), &xm, &xs);
-        else { xm = __ldg(p.x_mul + row); xs = __ldg(p.x_shift + row); }
-      }
+      int wm = 0, ws = 0;
+      if (ch < p.N && direct && p.out_q15) { wm = __ldg(p.w_mul + ch); ws = p.w_shift ? __ldg(p.w_shift + ch) : 31; }
       epilogue_bar_sync();
       if (ok) ok = mbar_wait(tfull0 + 8 * slot, aph, 3);
       tcgen05_fence_after();
 #pragma unroll 1
-      for (int c0 = half * 32; c0 < BN; c0 += 64) {   // the quarter's two warps take alternate 32-column chunks
+      for (int c0 = half * 32; c0 < BN; c0 += 64) {
         int v[32];
         tmem_ld_32x32(tmem_base + ((unsigned)(q * 32) << 16) + slot * BN + (unsigned)c0, v);
-        const int col0 = n_blk * BN + c0;
-        if (!ok || col0 >= p.N) continue;   // warp-uniform
-        // A thread holds 32 columns of ONE row; storing that directly would touch 32 rows per
-        // instruction.  The chunk goes through a padded shared-memory tile so that each store
-        // instruction writes four rows of 128 contiguous bytes.
-        const int r_base = m_blk * kBM + q * 32;
-        const bool vec = (p.N & 3) == 0;
-        if (p.acc_out) {
-          store_chunk(stage, lane, v, p.acc_out, r_base, col0, p.M, p.N, vec);
-        }
-        if (p.out_q15) {
+        if (!ok || c0 >= p.M || ch >= p.N || empty_part) continue;
+        if (p.tp_on) {
+          // exchange-block mode: the parts are added into the rank's OWN accumulators (L2 atomics); the peers fetch
+          // them from there once this kernel has signalled
+          int32_t* dst = p.tp.base[p.tp.rank] + tp_acc_off;
 #pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            const int4 wm = *reinterpret_cast<const int4*>(cs + c0 + j);
-            const int4 ws = *reinterpret_cast<const int4*>(cs + BN + c0 + j);
-            v[j + 0] = requant_one(v[j + 0], __mulhi(xm, wm.x), xs + ws.x);
-            v[j + 1] = requant_one(v[j + 1], __mulhi(xm, wm.y), xs + ws.y);
-            v[j + 2] = requant_one(v[j + 2], __mulhi(xm, wm.z), xs + ws.z);
-            v[j + 3] = requant_one(v[j + 3], __mulhi(xm, wm.w), xs + ws.w);
+          for (int j = 0; j < 32; ++j)
+            if (c0 + j < p.M) atomicAdd(dst + (int64_t)(c0 + j) * p.N + ch, v[j]);
+        } else if (p.n_peers > 0) {
+          // tensor-parallel sum: the tile's partial sums go straight into every rank's accumulator (a warp's
+          // 32 channels of one token are one 128-byte reduction over NVLink); integer adds commute, so every
+          // rank ends up with the same bits whatever the arrival order
+          for (int r = 0; r < p.n_peers; ++r) {
+            int32_t* dst = p.peer[r];
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (c0 + j < p.M) atomicAdd(dst + (int64_t)(c0 + j) * p.N + ch, v[j]);
           }
-          store_chunk(stage, lane, v, p.out_q15, r_base, col0, p.M, p.N, vec);
+        } else if (!direct) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (c0 + j < p.M) atomicAdd(p.partial + (int64_t)(c0 + j) * p.N + ch, v[j]);   // result unused: a reduction
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            if (c0 + j < p.M) {
+              const int64_t o = (int64_t)(c0 + j) * p.N + ch;
+              if (p.acc_out) p.acc_out[o] = v[j];
+              if (p.out_q15) p.out_q15[o] = requant_one(v[j], __mulhi(cs[c0 + j], wm), cs[BN + c0 + j] + ws);
+            }
+          }
         }
       }
       // this warp has read its quarter of the accumulator copy: hand it back to the MMA warp
@@ -376,7 +313,7 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   }
   // exchange-block mode: nothing was written into a peer's memory, so only the CTA that arrives last pays a
   // system-scope fence before the flag stores (each CTA orders its own additions with a device-scope fence)
-  if (WS && p.tp_on && threadIdx.x == 0) {
+  if (p.tp_on && threadIdx.x == 0) {
     __threadfence();
     tp_signal_if_last(p.tp, 1, gridDim.x, false);
   }
@@ -575,9 +512,9 @@ template <int STAGES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads2, 1)
 gemm_w8a8_2sm_ws_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                         const GemmParams p) {
-  constexpr int BN = 256;                      // token columns of the pair's tile; each CTA stages BN / 2 token rows
+  constexpr int BN = 256;                      // most token columns of the pair's tile; each CTA stages half of them
   constexpr int kABytes = kBM * kBK;           // 128 weight rows
-  constexpr int kBBytes = (BN / 2) * kBK;      // 128 token rows
+  constexpr int kBBytes = (BN / 2) * kBK;      // room for 128 token rows
   constexpr int kStageBytes = kABytes + kBBytes;
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~uintptr_t(1023));
@@ -592,7 +529,8 @@ gemm_w8a8_2sm_ws_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const int num_kb = (p.K + kBK - 1) / kBK;
   const int w_blocks = (p.N + 2 * kBM - 1) / (2 * kBM);
-  const int num_tiles = p.full_blocks + (w_blocks - p.full_blocks) * p.splits;
+  const int tn = p.tok_tile;
+  const int num_tiles = p.full_blocks + (w_blocks * p.tok_tiles - p.full_blocks) * p.splits;
   const unsigned full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES);
   const unsigned tfull0 = smem_u32(bars + 2 * STAGES), tempty0 = smem_u32(bars + 2 * STAGES + 2);
 
@@ -625,21 +563,22 @@ gemm_w8a8_2sm_ws_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
         const WsTile t = ws_tile(p, tile, num_kb);
+        const int n_blk = t.n_blk / p.tok_tiles, tok0 = (t.n_blk - n_blk * p.tok_tiles) * tn;
         for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
           const unsigned s = it % STAGES, ph = (it / STAGES) & 1;
           ok = mbar_wait(empty0 + 8 * s, ph ^ 1, 1);
           if (!ok) break;
-          if (leader) mbar_expect_tx(full0 + 8 * s, 2 * kStageBytes);
+          if (leader) mbar_expect_tx(full0 + 8 * s, 2 * kABytes + tn * kBK);
           const unsigned a_dst = smem_u32(tiles + s * kStageBytes);
           const unsigned lbar = (full0 + 8 * s) & kPeerBitMask;
-          tma_load_2d_2sm(a_dst, &map_w, kb * kBK, t.n_blk * 2 * kBM + (int)rank * kBM, lbar);
-          tma_load_2d_2sm(a_dst + kABytes, &map_x, kb * kBK, (int)rank * (BN / 2), lbar);
+          tma_load_2d_2sm(a_dst, &map_w, kb * kBK, n_blk * 2 * kBM + (int)rank * kBM, lbar);
+          tma_load_2d_2sm(a_dst + kABytes, &map_x, kb * kBK, tok0 + (int)rank * (tn / 2), lbar);
         }
       }
     }
   } else if (warp == 1) {
     if (lane == 0 && leader) {
-      constexpr unsigned idesc = make_idesc(2 * kBM, BN);
+      const unsigned idesc = make_idesc(2 * kBM, tn);
       unsigned it = 0, lt = 0;
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++lt) {
@@ -674,13 +613,14 @@ gemm_w8a8_2sm_ws_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     for (int tile = pair; tile < num_tiles; tile += num_pairs, ++lt) {
       const WsTile t = ws_tile(p, tile, num_kb);
       const unsigned slot = lt & 1, aph = (lt >> 1) & 1;
-      const int ch = t.n_blk * 2 * kBM + (int)rank * kBM + q * 32 + lane;
+      const int n_blk = t.n_blk / p.tok_tiles, tok0 = (t.n_blk - n_blk * p.tok_tiles) * tn, toks = min(tn, p.M - tok0);
+      const int ch = n_blk * 2 * kBM + (int)rank * kBM + q * 32 + lane;
       const bool direct = !t.split;
       const bool empty_part = t.kb0 >= t.kb1;      // a part of K with no k-blocks: nothing was accumulated
       int32_t* cs = tok_scale + slot * 2 * BN;
       if (direct && p.out_q15) {
-        for (int c = et; c < BN; c += 32 * kEpiWarps2) {
-          const int tk = min(c, p.M - 1);
+        for (int c = et; c < tn; c += 32 * kEpiWarps2) {
+          const int tk = min(tok0 + c, p.M - 1);
           int tm, ts;
           if (p.x_absmax) absmax_to_ms_dev(__ldg(p.x_absmax + tk), &tm, &ts);
           else { tm = __ldg(p.x_mul + tk); ts = __ldg(p.x_shift + tk); }
@@ -694,20 +634,20 @@ gemm_w8a8_2sm_ws_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
       if (ok) ok = mbar_wait(tfull0 + 8 * slot, aph, 3);
       tcgen05_fence_after();
 #pragma unroll 1
-      for (int c0 = part * 32; c0 < BN; c0 += 32 * (kEpiWarps2 / 4)) {
-        if (!ok || c0 >= p.M || empty_part) continue;   // warp-uniform
+      for (int c0 = part * 32; c0 < tn; c0 += 32 * (kEpiWarps2 / 4)) {
+        if (!ok || c0 >= toks || empty_part) continue;   // warp-uniform
         int v[32];
         tmem_ld_32x32(tmem_base + ((unsigned)(q * 32) << 16) + slot * BN + (unsigned)c0, v);
         if (ch >= p.N) continue;
         if (!direct) {
 #pragma unroll
           for (int j = 0; j < 32; ++j)
-            if (c0 + j < p.M) atomicAdd(p.partial + (int64_t)(c0 + j) * p.N + ch, v[j]);   // result unused: a reduction
+            if (c0 + j < toks) atomicAdd(p.partial + (int64_t)(tok0 + c0 + j) * p.N + ch, v[j]);   // result unused: a reduction
         } else {
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            if (c0 + j < p.M) {
-              const int64_t o = (int64_t)(c0 + j) * p.N + ch;
+            if (c0 + j < toks) {
+              const int64_t o = (int64_t)(tok0 + c0 + j) * p.N + ch;
               if (p.acc_out) p.acc_out[o] = v[j];
               if (p.out_q15) p.out_q15[o] = requant_one(v[j], __mulhi(cs[c0 + j], wm), cs[BN + c0 + j] + ws);
             }
@@ -1009,19 +949,18 @@ static bool make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN, int STAGES, bool WS = false>
+template <int BN, int STAGES>
 static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, cudaStream_t st) {
-  constexpr size_t smem = (size_t)STAGES * (kBM * kBK + BN * kBK) + 1024 + (2 * STAGES + 4) * 8 + 16 + 4 * BN * 4 + kEpiWarps * 32 * kStagePitch * 4;
+  constexpr size_t smem = (size_t)STAGES * (kBM * kBK + BN * kBK) + 1024 + (2 * STAGES + 4) * 8 + 16 + 4 * BN * 4;
   static_assert(smem <= 227 * 1024, "shared memory budget");
-  cudaError_t e = cudaFuncSetAttribute(gemm_w8a8_kernel<BN, STAGES, WS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(gemm_w8a8_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) {
     set_error("gemm_w8a8: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     return B200_E_CUDA;
   }
-  const int tiles = WS ? p.full_blocks + ((p.N + kBM - 1) / kBM - p.full_blocks) * p.splits
-                       : ((p.N + BN - 1) / BN) * ((p.M + kBM - 1) / kBM);
+  const int tiles = p.full_blocks + ((p.N + kBM - 1) / kBM - p.full_blocks) * p.splits;
   const int grid = tiles < sm_count() ? tiles : sm_count();
-  launch_pdl(gemm_w8a8_kernel<BN, STAGES, WS>, dim3(grid), dim3(kGemmThreads), smem, st, ma, mb, p);
+  launch_pdl(gemm_w8a8_kernel<BN, STAGES>, dim3(grid), dim3(kGemmThreads), smem, st, ma, mb, p);
   return check_launch("gemm_w8a8");
 }
 
@@ -1051,10 +990,28 @@ static int launch_gemm_2sm_ws(const CUtensorMap& mw, const CUtensorMap& mx, cons
     set_error("gemm_w8a8: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     return B200_E_CUDA;
   }
-  const int tiles = p.full_blocks + ((p.N + 2 * kBM - 1) / (2 * kBM) - p.full_blocks) * p.splits;
+  const int tiles = p.full_blocks + ((p.N + 2 * kBM - 1) / (2 * kBM) * p.tok_tiles - p.full_blocks) * p.splits;
   const int pairs = tiles < sm_count() / 2 ? tiles : sm_count() / 2;
   launch_pdl(gemm_w8a8_2sm_ws_kernel<STAGES>, dim3(2 * pairs), dim3(kGemmThreads2), smem, st, mw, mx, p);
   return check_launch("gemm_w8a8 (two-CTA weights-stationary tiles)");
+}
+
+// Token tiles and parts of K of a prompt whose 256 x 256 tiles would leave CTA pairs idle; returns the parts.
+// A tile costs about (256 weight rows + its tokens) per k-block, what it moves into shared memory, so with whole-K
+// tiles the narrowest tokens tiles that still run at once are the best, down to 96 tokens (333 x 6144 x 4096: 30.8 us on single
+// CTAs, 25.6 with three tiles, 30.7 with two).  From 48 k-blocks on, splitting K beats narrowing the tiles although the
+// parts are added in memory and requantised by another kernel (333 x 4096 x 12288: 65.5 us on single CTAs, 43.0 with four whole-K
+// tiles, 35.8 with two tiles in two parts; 16 and 32 k-blocks: splitting loses or ties).
+static int prompt_tiles(GemmParams* p, int w_blocks, int num_kb, int pairs) {
+  const int fewest = (p->M + 255) / 256;
+  int tiles = fewest, splits = 1;
+  if (num_kb >= 48) splits = pairs / (w_blocks * fewest) < 4 ? pairs / (w_blocks * fewest) : 4;
+  while (splits > 1 && (splits - 1) * ((num_kb + splits - 1) / splits) >= num_kb) --splits;     // no empty part
+  if (splits <= 1)
+    while (w_blocks * (tiles + 1) <= pairs && (p->M + tiles) / (tiles + 1) >= 96) ++tiles;
+  p->tok_tile = ((p->M + tiles - 1) / tiles + 31) / 32 * 32;
+  p->tok_tiles = (p->M + p->tok_tile - 1) / p->tok_tile;
+  return splits;
 }
 
 static bool pair_ws_enabled() {
@@ -1091,6 +1048,7 @@ static int gemm_impl(const int8_t* x8, const int8_t* w8, const int32_t* x_absmax
   p.x_absmax = x_absmax; p.x_mul = x_mul; p.x_shift = x_shift; p.w_mul = w_mul; p.w_shift = w_shift;
   p.out_q15 = out_q15; p.acc_out = acc_out; p.M = (int)m; p.N = (int)n; p.K = (int)k;
   p.splits = 1; p.full_blocks = 0; p.partial = nullptr; p.n_peers = 0; p.tp_on = 0; p.split_col0 = 0;
+  p.tok_tile = 256; p.tok_tiles = 1;
   cudaStream_t st = (cudaStream_t)s;
   const int num_kb = (int)((k + kBK - 1) / kBK);
   // 65..256 tokens: CTA pairs on blocks of 256 weight rows (each CTA stages half of the 256-token tile; rows beyond
@@ -1099,10 +1057,14 @@ static int gemm_impl(const int8_t* x8, const int8_t* w8, const int32_t* x_absmax
   // 4 % at 96 and 128 tokens, 1 % at 64, nothing at 48.  B200_GEMM_PAIR_MIN moves the boundary.)
   static int pair_min = -1;
   if (pair_min < 0) { const char* e = getenv("B200_GEMM_PAIR_MIN"); pair_min = e ? atoi(e) : 65; }
-  const bool pair_ws = m >= pair_min && m <= 256 && pair_ws_enabled();
-  const int block_rows = pair_ws ? 2 * kBM : kBM, units = pair_ws ? sm_count() / 2 : sm_count();
+  // More tokens, but fewer 256 x 256 tiles than CTA pairs (one prompt's qkv, o and down projections): the same kernel with
+  // several token tiles, see prompt_tiles.
+  const int pairs = sm_count() / 2;
+  const bool prompt_ws = m > 256 && (m + 255) / 256 * ((n + 255) / 256) < pairs;
+  const bool pair_ws = prompt_ws || (m >= pair_min && m <= 256 && pair_ws_enabled());
+  const int block_rows = pair_ws ? 2 * kBM : kBM, units = pair_ws ? pairs : sm_count();
   const int w_blocks = (int)((n + block_rows - 1) / block_rows);
-  if (pair_ws || m <= 128 || (m <= 256 && w_blocks < sm_count())) {
+  if (m <= 256 || prompt_ws) {
     // decode sizes: weights-stationary, K split so that about one CTA (pair) per SM (pair) streams the weights
     // With more blocks than units the whole waves run unsplit and only the blocks of the last, partial wave are
     // split, so that it costs a fraction of a wave instead of a whole one.
@@ -1112,8 +1074,10 @@ static int gemm_impl(const int8_t* x8, const int8_t* w8, const int32_t* x_absmax
     splits = splits < 1 ? 1 : (splits > 8 ? 8 : splits);
     while (splits > 1 && num_kb / splits < 4) --splits;
     while (splits > 1 && (splits - 1) * ((num_kb + splits - 1) / splits) >= num_kb) --splits;   // no empty part
+    if (prompt_ws) splits = prompt_tiles(&p, w_blocks, num_kb, pairs);
+    else p.tok_tile = (int)((m + 31) / 32 * 32);
     p.splits = splits;
-    p.full_blocks = splits > 1 ? w_blocks - split_blocks : 0;
+    p.full_blocks = splits > 1 && !prompt_ws ? w_blocks - split_blocks : 0;
     const int64_t col0 = (int64_t)p.full_blocks * block_rows;     // first column that parts are added into
     p.split_col0 = (int)col0;
     if (splits > 1) {
@@ -1136,38 +1100,24 @@ static int gemm_impl(const int8_t* x8, const int8_t* w8, const int32_t* x_absmax
     }
     const int bn = m <= 32 ? 32 : (m <= 64 ? 64 : (m <= 128 ? 128 : 256));
     B200_REQUIRE(make_map(&ma, w8, n, k, kBM), B200_E_CUDA, "gemm_w8a8: cuTensorMapEncodeTiled failed for w8");
-    B200_REQUIRE(make_map(&mb, x8, m, k, pair_ws ? kBM : bn), B200_E_CUDA, "gemm_w8a8: cuTensorMapEncodeTiled failed for x8");
+    B200_REQUIRE(make_map(&mb, x8, m, k, pair_ws ? p.tok_tile / 2 : bn), B200_E_CUDA, "gemm_w8a8: cuTensorMapEncodeTiled failed for x8");
     int rc;
     if (pair_ws) {
       rc = launch_gemm_2sm_ws<6>(ma, mb, p, st);
     } else switch (bn) {
-      case 256: rc = launch_gemm<256, 4, true>(ma, mb, p, st); break;
-      case 128: rc = launch_gemm<128, 6, true>(ma, mb, p, st); break;
-      case 64: rc = launch_gemm<64, 8, true>(ma, mb, p, st); break;
-      default: rc = launch_gemm<32, 10, true>(ma, mb, p, st); break;
+      case 256: rc = launch_gemm<256, 4>(ma, mb, p, st); break;
+      case 128: rc = launch_gemm<128, 6>(ma, mb, p, st); break;
+      case 64: rc = launch_gemm<64, 8>(ma, mb, p, st); break;
+      default: rc = launch_gemm<32, 10>(ma, mb, p, st); break;
     }
     if (rc != B200_OK || splits == 1 || !out_q15) return rc;
     launch_pdl(splitk_epilogue_kernel, dim3((unsigned)((n - col0 + 1023) / 1024), (unsigned)m), dim3(256), 0, st, p.partial, p, zero_ws ? 1 : 0);
     return check_launch("gemm_w8a8 (split-K epilogue)");
   }
   B200_REQUIRE(make_map(&ma, x8, m, k, kBM), B200_E_CUDA, "gemm_w8a8: cuTensorMapEncodeTiled failed for x8");
-  // large problems: 256 x 256 tiles on CTA pairs, when there are enough of them to occupy every pair
-  if (((m + 2 * kBM - 1) / (2 * kBM)) * ((n + 255) / 256) >= sm_count() / 2) {
-    B200_REQUIRE(make_map(&mb, w8, n, k, kBM), B200_E_CUDA, "gemm_w8a8: cuTensorMapEncodeTiled failed for w8");
-    return launch_gemm_2sm<5>(ma, mb, p, st);
-  }
-  // tile width: wide tiles for throughput at large M; narrow ones at decode sizes so that enough CTAs
-  // stream the weights (one m block there, so the tile count is n / BN)
-  const int64_t m_tiles = (m + kBM - 1) / kBM;
-  int bn = 256;
-  while (bn > 32 && m_tiles * ((n + bn - 1) / bn) < sm_count()) bn >>= 1;
-  B200_REQUIRE(make_map(&mb, w8, n, k, bn), B200_E_CUDA, "gemm_w8a8: cuTensorMapEncodeTiled failed for w8");
-  switch (bn) {
-    case 256: return launch_gemm<256, 4>(ma, mb, p, st);
-    case 128: return launch_gemm<128, 6>(ma, mb, p, st);
-    case 64: return launch_gemm<64, 8>(ma, mb, p, st);
-    default: return launch_gemm<32, 10>(ma, mb, p, st);
-  }
+  // large problems: 256 x 256 tiles on CTA pairs
+  B200_REQUIRE(make_map(&mb, w8, n, k, kBM), B200_E_CUDA, "gemm_w8a8: cuTensorMapEncodeTiled failed for w8");
+  return launch_gemm_2sm<5>(ma, mb, p, st);
 }
 
 extern "C" int b200_gemm_w8a8(const int8_t* x8, const int8_t* w8, const int32_t* x_mul, const int32_t* x_shift,
@@ -1274,10 +1224,10 @@ extern "C" int b200_gemm_w8a8_reduce_peers(const int8_t* x8, const int8_t* w8, i
   B200_REQUIRE(make_map(&mb, x8, m, k, bn), B200_E_CUDA, "gemm_w8a8_reduce_peers: cuTensorMapEncodeTiled failed for x8");
   cudaStream_t st = (cudaStream_t)s;
   switch (bn) {
-    case 256: return launch_gemm<256, 4, true>(ma, mb, p, st);
-    case 128: return launch_gemm<128, 6, true>(ma, mb, p, st);
-    case 64: return launch_gemm<64, 8, true>(ma, mb, p, st);
-    default: return launch_gemm<32, 10, true>(ma, mb, p, st);
+    case 256: return launch_gemm<256, 4>(ma, mb, p, st);
+    case 128: return launch_gemm<128, 6>(ma, mb, p, st);
+    case 64: return launch_gemm<64, 8>(ma, mb, p, st);
+    default: return launch_gemm<32, 10>(ma, mb, p, st);
   }
 }
 
@@ -1316,10 +1266,10 @@ extern "C" int b200_gemm_w8a8_tp(const b200_tp_block* blk, const int8_t* x8, con
   B200_REQUIRE(make_map(&mb, x8, m, k, bn), B200_E_CUDA, "gemm_w8a8_tp: cuTensorMapEncodeTiled failed for x8");
   cudaStream_t st = (cudaStream_t)s;
   switch (bn) {
-    case 256: return launch_gemm<256, 4, true>(ma, mb, p, st);
-    case 128: return launch_gemm<128, 6, true>(ma, mb, p, st);
-    case 64: return launch_gemm<64, 8, true>(ma, mb, p, st);
-    default: return launch_gemm<32, 10, true>(ma, mb, p, st);
+    case 256: return launch_gemm<256, 4>(ma, mb, p, st);
+    case 128: return launch_gemm<128, 6>(ma, mb, p, st);
+    case 64: return launch_gemm<64, 8>(ma, mb, p, st);
+    default: return launch_gemm<32, 10>(ma, mb, p, st);
   }
 }
 

@@ -83,6 +83,13 @@ def test_pair_weights_stationary_tiles(M, N, K):
     run_case(M, N, K, M + N + K, per_channel_shift=True)
 
 
+@pytest.mark.parametrize("M,N,K", [(257, 520, 6400), (333, 6144, 512), (333, 1000, 6160), (600, 260, 6144), (1100, 4096, 256), (2100, 132, 272), (18900, 40, 144)])
+def test_prompts_of_few_tiles(M, N, K):
+    """More than 256 tokens on fewer 256 x 256 tiles than CTA pairs: several token tiles of 96 .. 256 tokens against a block of
+    weight rows, whole-K or (from 48 k-blocks) in up to four parts; ragged last tiles of both kinds."""
+    run_case(M, N, K, M + N + K, per_channel_shift=True)
+
+
 @pytest.mark.parametrize("M,N,K", [(300, 512, 1024), (64, 1024, 2048), (256, 20000, 256)])
 def test_token_scale_from_absmax(M, N, K):
     """The entry point that takes the row kernels' integer absmax derives the same (multiplier, shift)."""
