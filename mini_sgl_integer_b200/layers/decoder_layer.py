@@ -15,7 +15,7 @@ from typing import Optional
 
 import torch
 
-from ..attention import Int8PagedKVCache, decode_attention_int8_paged, extend_attention_int8_paged, qkv_rope_quant_store
+from ..attention import Int8PagedKVCache, NewTokens, decode_attention_int8_paged, extend_attention_int8_paged, qkv_rope_quant_store
 from ..kernel import fixed_point as fp
 from ..kernel.pending import PENDING_MAX_ROWS, PendingLinear
 from ..distributed import DistributedCommunicator
@@ -82,7 +82,7 @@ class Qwen3DecoderLayerInteger:
         self.exchange = exchange
 
     def forward_codes(self, codes: torch.Tensor, absmax: torch.Tensor, residual: torch.Tensor, batch: AttnBatch,
-                      next_norm_weight: torch.Tensor):
+                      next_norm_weight: torch.Tensor, new: Optional[NewTokens] = None):
         """The layer between two norms, for tensor-parallel steps on an exchange block: takes the int8 codes and
         absmax of ITS input norm (all token rows) and returns those of the NEXT norm (``next_norm_weight``: the next
         layer's input_layernorm or the model's final norm).  Each row-split linear is finished, added to the
@@ -98,7 +98,7 @@ class Qwen3DecoderLayerInteger:
                                                batch.kv_lens, batch.max_kv_len, row_order=batch.row_order)
         else:
             attn = extend_attention_int8_paged(q8, q_mul, q_shift, self.pool, self.layer_id, batch.page_table,
-                                               batch.kv_lens, batch.q_lens, batch.max_kv_len)
+                                               batch.kv_lens, batch.q_lens, batch.max_kv_len, new=new)
         codes, absmax = self.exchange.row_parallel_norm_quant(m, w["o"], attn.view(T, self.hq * 128), residual, w["post_norm"])
         gate_up = m.apply_quantised(w["gate_up"], codes, absmax)
         if self.inter % 128 == 0 and T <= 256 and self.hadamard_block in (0, 128):
@@ -109,12 +109,13 @@ class Qwen3DecoderLayerInteger:
         return self.exchange.row_parallel_norm_quant(m, w["down"], act, residual, next_norm_weight)
 
     def forward_q15(self, x_q15, residual_q15: Optional[torch.Tensor], batch: AttnBatch,
-                    trace: Optional[dict] = None, defer_down: bool = False):
+                    trace: Optional[dict] = None, defer_down: bool = False, new: Optional[NewTokens] = None):
         """Returns (x_out, residual_out), both Q15.16 int32 [tokens, hidden].
 
         At decode sizes on one GPU the qkv and o projections are left pending (kernel/pending.py) and finished by
         the kernels that read them; with ``defer_down`` the down projection is returned pending too, for the next
-        layer's (or the final) add + RMSNorm + quant, and ``x_q15`` may be such a pending linear."""
+        layer's (or the final) add + RMSNorm + quant, and ``x_q15`` may be such a pending linear.  ``new``: what the
+        step's layers share about its new tokens (attention.new_tokens)."""
         pending_in = isinstance(x_q15, PendingLinear)
         if not pending_in:
             fp.assert_q15(x_q15, "x_q15")
@@ -149,7 +150,7 @@ class Qwen3DecoderLayerInteger:
                                                batch.kv_lens, batch.max_kv_len, row_order=batch.row_order)
         else:
             attn = extend_attention_int8_paged(q8, q_mul, q_shift, self.pool, self.layer_id, batch.page_table,
-                                               batch.kv_lens, batch.q_lens, batch.max_kv_len)
+                                               batch.kv_lens, batch.q_lens, batch.max_kv_len, new=new)
         t["attn"] = attn
         if self.exchange is not None and self.exchange.fits(T, self.hidden):
             rowp = lambda l, x: self.exchange.row_parallel_q15(m, l, x)

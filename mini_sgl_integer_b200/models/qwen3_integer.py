@@ -15,7 +15,7 @@ from typing import Optional
 import torch
 
 from .._lib import call, ptr, require_cuda, stream
-from ..attention import Int8PagedKVCache
+from ..attention import Int8PagedKVCache, new_tokens
 from ..distributed import DistributedCommunicator
 from ..kernel import fixed_point as fp
 from ..layers.decoder_layer import AttnBatch, Qwen3DecoderLayerInteger, _Linear
@@ -174,6 +174,7 @@ class Qwen3ModelInteger:
         if self.comm.size > 1 and not self.embed_replicated:
             x = self.comm.all_reduce(x)
         T = x.shape[0]
+        new = new_tokens(batch.q_lens, T) if batch.q_lens is not None and self.layers else None
         if self.exchange is not None and self.exchange.size > 1 and self.exchange.fits(T, self.cfg.hidden) and self.layers:
             # tensor parallel on an exchange block: the rows of the residual stream have owners, and every row-split
             # linear is finished together with the norm that follows it (Qwen3DecoderLayerInteger.forward_codes)
@@ -182,11 +183,11 @@ class Qwen3ModelInteger:
             residual = x.contiguous()                       # layer 0's residual is its input; updated in place from here on
             for i, layer in enumerate(self.layers):
                 nw = self.layers[i + 1].w["input_norm"] if i + 1 < len(self.layers) else self.w["final_norm"]
-                codes, absmax = layer.forward_codes(codes, absmax, residual, batch, nw)
+                codes, absmax = layer.forward_codes(codes, absmax, residual, batch, nw, new=new)
             return codes, absmax
         residual = None
         for layer in self.layers:
-            x, residual = layer.forward_q15(x, residual, batch, defer_down=True)
+            x, residual = layer.forward_q15(x, residual, batch, defer_down=True, new=new)
         codes, _, absmax, _, _ = fp.fused_add_rmsnorm_quant(x, residual, self.w["final_norm"])
         return codes, absmax
 
