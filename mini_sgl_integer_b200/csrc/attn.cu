@@ -887,14 +887,14 @@ static int attn_common(const int8_t* q, const int32_t* q_mul, const int32_t* q_s
                (long long)table_pitch, max_pages);
   B200_REQUIRE(aligned16(q) && aligned16(k_codes) && aligned16(v_codes) && aligned16(meta), B200_E_ALIGN,
                "attn_decode: q and pool buffers must be 16-byte aligned");
-  // Configuration: the per-CTA fixed work (set-up, exchanges) is paid once per CTA, so the fewest CTAs per
-  // (row, KV head) whose slice state still lets two CTAs share an SM win; one CTA with single ring slots
-  // is preferred, then the smallest cluster with two slots per warp, then whatever fits at all.
   auto slice_keys = [&](int c) { return ((((max_pages + c - 1) / c) * kPage + 31) / 32) * 32; };
   // Configuration.  Set-up, barriers and the final exchange are paid per CTA and a lone CTA needs no
-  // cluster barrier, so one CTA per (row, KV head) wins whenever its slice state lets two CTAs share an
-  // SM - with two ring slots per warp if that still fits, else one; longer contexts take the smallest
-  // cluster whose slices fit at all (fewer CTAs beat deeper rings in every measurement).
+  // cluster barrier, so with enough rows to fill the SMs one CTA per (row, KV head) wins whenever its slice state lets
+  // two CTAs share an SM - with two ring slots per warp if that still fits, else one; longer contexts take the
+  // smallest cluster whose slices fit at all (fewer CTAs beat deeper rings in every measurement).  Fewer rows are latency: a
+  // row's CTAs double while no more than 256 of them are resident and each keeps four pages (eight KV heads, one row of 777 keys:
+  // 13.6 us with one CTA, 9.3 with eight; 8 rows: 16.0, 11.8 with four, 20.8 with eight; 16 rows of 500 keys: 12.8, 12.2 with two;
+  // 37 rows x 4 KV heads of 900 keys: 16.0, 17.4 with two; one row of 100 keys: 8.3, 9.1 with two).
   const int G_static = 1536 + G * kD * 4 + 1024;   // the kernel's static shared arrays plus the per-CTA reserve
   const size_t two_per_sm = (size_t)(233472 / 2 - G_static);
   auto fits2 = [&](int c, int st) { return decode_smem_bytes(G, slice_keys(c), st) <= two_per_sm; };
@@ -902,6 +902,7 @@ static int attn_common(const int8_t* q, const int32_t* q_mul, const int32_t* q_s
   if (cluster == 0) {
     cluster = 1;
     while (cluster < 8 && !fits2(cluster, 1)) cluster *= 2;   // fewest CTAs per row first, ring depth second
+    while (cluster < 8 && (int64_t)batch * kv_heads * cluster * 2 <= 256 && max_pages / (2 * cluster) >= 4) cluster *= 2;
     stages = fits2(cluster, 2) ? 2 : 1;
   } else {
     B200_REQUIRE(cluster == 1 || cluster == 2 || cluster == 4 || cluster == 8, B200_E_UNSUPPORTED,

@@ -112,6 +112,18 @@ def test_decode_auto_cluster_long_context_and_clamp():
     eq(codes.cpu().numpy(), wc); eq(absmax.cpu().numpy(), wm)
 
 
+@pytest.mark.parametrize("rows,keys", [(1, 127), (1, 128), (1, 511), (1, 513), (5, 300), (16, 140), (17, 140), (32, 200)])
+def test_decode_of_few_rows_spread_over_more_ctas(rows, keys):
+    """Around the lines where a row's CTAs double (four pages per CTA, 256 CTAs): the bits of one CTA per row and KV head."""
+    lens = [max(1, keys - 7 * (i % 5)) for i in range(rows)]
+    case = make_case(keys, lens, 16, 8, 16 * rows + 20)
+    pool = device_pool(case, 16 * rows + 20, 8)
+    want = run_decode(case, pool, keys, 1, impl="cluster").cpu().numpy()
+    eq(run_decode(case, pool, keys, impl="cluster").cpu().numpy(), want)
+    if rows == 1:
+        eq(want, oracle_decode(case))
+
+
 def test_decode_zero_length_sequences_give_zero():
     case = make_case(9, [0, 20, 0], 4, 2, 8)
     pool = device_pool(case, 8, 2)
