@@ -173,6 +173,17 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   __syncthreads();
   tcgen05_fence_after();
   const unsigned tmem_base = *tmem_slot;
+  // The first weights on their way into L2 while the kernel before this one still runs (weights do not depend on it, but a
+  // prefetch reads nothing, so it is safe even if they did).  Eight k-blocks per CTA are 19 MB over the SMs, what the memory delivers
+  // meanwhile; more delays the other kernel's own traffic, as any does to the larger batches of the pair kernel (256 tokens:
+  // 9.54 -> 9.59 ms).  1.4B-shaped decode step of 37 rows: 1875 -> 1803 us.
+  if (warp == 2 && lane == 0) {
+    int left = kAheadBlocks;
+    for (int tile = blockIdx.x; tile < num_tiles && left > 0; tile += gridDim.x) {
+      const WsTile t = ws_tile(p, tile, num_kb);
+      for (int kb = t.kb0; kb < t.kb1 && left > 0; ++kb, --left) tma_prefetch_2d(&map_a, kb * kBK, t.n_blk * kBM);
+    }
+  }
   pdl_wait();               // barriers, tensor memory and descriptors are set up; the operands come from earlier kernels
   // exchange-block mode: word offset, inside this rank's block, of the accumulator half in use
   int64_t tp_acc_off = 0;
@@ -508,7 +519,7 @@ gemm_w8a8_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 // weights-stationary list in blocks of 256 weight rows: whole-K tiles for the first full_blocks, `splits` parts of K
 // for the rest, whose partial sums are added into `partial` with reductions (a warp's 32 lanes are 32 consecutive
 // channels of one token: one 128-byte reduction per instruction).
-template <int STAGES>
+template <int STAGES, bool NARROW>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads2, 1)
 gemm_w8a8_2sm_ws_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                         const GemmParams p) {
@@ -529,8 +540,8 @@ gemm_w8a8_2sm_ws_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const int num_kb = (p.K + kBK - 1) / kBK;
   const int w_blocks = (p.N + 2 * kBM - 1) / (2 * kBM);
-  const int tn = p.tok_tile;
-  const int num_tiles = p.full_blocks + (w_blocks * p.tok_tiles - p.full_blocks) * p.splits;
+  const int tn = NARROW ? p.tok_tile : BN, tok_tiles = NARROW ? p.tok_tiles : 1;
+  const int num_tiles = p.full_blocks + (w_blocks * tok_tiles - p.full_blocks) * p.splits;
   const unsigned full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES);
   const unsigned tfull0 = smem_u32(bars + 2 * STAGES), tempty0 = smem_u32(bars + 2 * STAGES + 2);
 
@@ -563,7 +574,7 @@ gemm_w8a8_2sm_ws_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
         const WsTile t = ws_tile(p, tile, num_kb);
-        const int n_blk = t.n_blk / p.tok_tiles, tok0 = (t.n_blk - n_blk * p.tok_tiles) * tn;
+        const int n_blk = t.n_blk / tok_tiles, tok0 = (t.n_blk - n_blk * tok_tiles) * tn;
         for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
           const unsigned s = it % STAGES, ph = (it / STAGES) & 1;
           ok = mbar_wait(empty0 + 8 * s, ph ^ 1, 1);
@@ -613,7 +624,7 @@ gemm_w8a8_2sm_ws_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     for (int tile = pair; tile < num_tiles; tile += num_pairs, ++lt) {
       const WsTile t = ws_tile(p, tile, num_kb);
       const unsigned slot = lt & 1, aph = (lt >> 1) & 1;
-      const int n_blk = t.n_blk / p.tok_tiles, tok0 = (t.n_blk - n_blk * p.tok_tiles) * tn, toks = min(tn, p.M - tok0);
+      const int n_blk = t.n_blk / tok_tiles, tok0 = (t.n_blk - n_blk * tok_tiles) * tn, toks = min(tn, p.M - tok0);
       const int ch = n_blk * 2 * kBM + (int)rank * kBM + q * 32 + lane;
       const bool direct = !t.split;
       const bool empty_part = t.kb0 >= t.kb1;      // a part of K with no k-blocks: nothing was accumulated
@@ -980,19 +991,19 @@ static int launch_gemm_2sm(const CUtensorMap& ma, const CUtensorMap& mb, const G
   return check_launch("gemm_w8a8 (two-CTA tiles)");
 }
 
-template <int STAGES>
+template <int STAGES, bool NARROW>
 static int launch_gemm_2sm_ws(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p, cudaStream_t st) {
   constexpr int BN = 256;
   constexpr size_t smem = (size_t)STAGES * (kBM * kBK + (BN / 2) * kBK) + 1024 + (2 * STAGES + 4) * 8 + 16 + 4 * BN * 4;
   static_assert(smem <= 227 * 1024, "shared memory budget");
-  cudaError_t e = cudaFuncSetAttribute(gemm_w8a8_2sm_ws_kernel<STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(gemm_w8a8_2sm_ws_kernel<STAGES, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) {
     set_error("gemm_w8a8: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     return B200_E_CUDA;
   }
   const int tiles = p.full_blocks + ((p.N + 2 * kBM - 1) / (2 * kBM) * p.tok_tiles - p.full_blocks) * p.splits;
   const int pairs = tiles < sm_count() / 2 ? tiles : sm_count() / 2;
-  launch_pdl(gemm_w8a8_2sm_ws_kernel<STAGES>, dim3(2 * pairs), dim3(kGemmThreads2), smem, st, mw, mx, p);
+  launch_pdl(gemm_w8a8_2sm_ws_kernel<STAGES, NARROW>, dim3(2 * pairs), dim3(kGemmThreads2), smem, st, mw, mx, p);
   return check_launch("gemm_w8a8 (two-CTA weights-stationary tiles)");
 }
 
@@ -1103,7 +1114,7 @@ static int gemm_impl(const int8_t* x8, const int8_t* w8, const int32_t* x_absmax
     B200_REQUIRE(make_map(&mb, x8, m, k, pair_ws ? p.tok_tile / 2 : bn), B200_E_CUDA, "gemm_w8a8: cuTensorMapEncodeTiled failed for x8");
     int rc;
     if (pair_ws) {
-      rc = launch_gemm_2sm_ws<6>(ma, mb, p, st);
+      rc = p.tok_tile < 256 || p.tok_tiles > 1 ? launch_gemm_2sm_ws<6, true>(ma, mb, p, st) : launch_gemm_2sm_ws<6, false>(ma, mb, p, st);
     } else switch (bn) {
       case 256: rc = launch_gemm<256, 4>(ma, mb, p, st); break;
       case 128: rc = launch_gemm<128, 6>(ma, mb, p, st); break;

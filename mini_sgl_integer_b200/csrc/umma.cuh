@@ -49,6 +49,12 @@ __device__ __forceinline__ void tma_load_3d(unsigned dst, const CUtensorMap* map
       ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
       : "memory");
 }
+constexpr int kAheadBlocks = 8;     // k-blocks of weights that a CTA of a decode-size GEMM requests into L2 before its wait
+
+// The box on its way into L2 only: nothing is read, so this may run before pdl_wait() whoever writes the operand.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int c0, int c1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(map), "r"(c0), "r"(c1) : "memory");
+}
 __device__ __forceinline__ void tcgen05_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tcgen05_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tcgen05_commit(unsigned bar) {
