@@ -515,6 +515,80 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, const 
     }
 }
 
+// Up to eight rows in 32 bits: what counts is streaming the weights once, which tiles of 64 x 64 on few CTAs did at a tenth of the
+// memory's rate and the split into bf16 parts at a third (it writes and reads 6 bytes for each 4).  A CTA has four weight
+// rows; its threads stride over K, so every lane has four loads of 16 bytes in flight, and the sums meet in the end.  One row,
+// 1024 x 4096 weights: 357 -> 8.5 us; 32768 x 1024: 153 -> 21.5 (20.6 at the memory's rate); eight rows: 370 -> 9.4 and 154 -> 59 us, where the
+// loads of x bound it.
+constexpr int kGemvRows = 4, kGemvThreads = 128;
+
+template <int M, int VEC>
+__global__ void __launch_bounds__(kGemvThreads)
+gemv_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, const FGemmParams p, int64_t x_pitch, int64_t x_bstride,
+                int64_t w_pitch, int64_t w_bstride) {
+  constexpr int R = kGemvRows;
+  __shared__ float part[kGemvThreads / 32][R * M];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int n0 = blockIdx.x * R, b = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float *xr[M], *wr[R];
+#pragma unroll
+  for (int m = 0; m < M; ++m) xr[m] = x + (int64_t)b * x_bstride + min(m, p.M - 1) * x_pitch;
+#pragma unroll
+  for (int r = 0; r < R; ++r) wr[r] = w + (int64_t)b * w_bstride + min(n0 + r, p.N - 1) * w_pitch;
+  float acc[R][M] = {};
+  const int body = p.K / VEC * VEC;
+#pragma unroll 2
+  for (int c = threadIdx.x * VEC; c < body; c += kGemvThreads * VEC) {
+    float wv[R][VEC];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (VEC == 4) *reinterpret_cast<float4*>(wv[r]) = __ldg(reinterpret_cast<const float4*>(wr[r] + c));
+      else wv[r][0] = __ldg(wr[r] + c);
+    }
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      float xv[VEC];
+      if (VEC == 4) *reinterpret_cast<float4*>(xv) = *reinterpret_cast<const float4*>(xr[m] + c);
+      else xv[0] = xr[m][c];
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) acc[r][m] = fmaf(wv[r][k], xv[k], acc[r][m]);
+    }
+  }
+  if (VEC > 1 && body + (int)threadIdx.x < p.K) {          // the columns behind the last group of four
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+#pragma unroll
+      for (int r = 0; r < R; ++r) acc[r][m] = fmaf(wr[r][body + threadIdx.x], xr[m][body + threadIdx.x], acc[r][m]);
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const float v = warp_sum(acc[r][m]);
+      if (lane == 0) part[warp][r * M + m] = v;
+    }
+  __syncthreads();
+  if (threadIdx.x >= R * M) return;
+  const int r = threadIdx.x / M, m = threadIdx.x % M;
+  if (m >= p.M || n0 + r >= p.N) return;
+  float v = (part[0][threadIdx.x] + part[1][threadIdx.x]) + (part[2][threadIdx.x] + part[3][threadIdx.x]);
+  if (p.act == B200F_ACT_XIELU) v = xielu_f32(v, p.act_a, p.act_b);
+  reinterpret_cast<float*>(p.out)[(int64_t)b * p.out_bstride + m * p.out_pitch + n0 + r] = v;
+}
+
+template <int M>
+static int launch_gemv(const float* x, const float* w, const FGemmParams& p, int64_t x_pitch, int64_t x_bstride, int64_t w_pitch,
+                       int64_t w_bstride, cudaStream_t st) {
+  const dim3 grid((unsigned)((p.N + kGemvRows - 1) / kGemvRows), (unsigned)p.batch);
+  const bool vec = aligned16(x) && aligned16(w) && x_pitch % 4 == 0 && w_pitch % 4 == 0 && (p.batch == 1 || (x_bstride % 4 == 0 && w_bstride % 4 == 0));
+  if (vec) launch_pdl(gemv_f32_kernel<M, 4>, grid, dim3(kGemvThreads), 0, st, x, w, p, x_pitch, x_bstride, w_pitch, w_bstride);
+  else launch_pdl(gemv_f32_kernel<M, 1>, grid, dim3(kGemvThreads), 0, st, x, w, p, x_pitch, x_bstride, w_pitch, w_bstride);
+  return check_launch("gemm (fp32, few rows)");
+}
+
 // ----------------------------------------------------------------------------- host side
 // bf16 operand [batch][rows, K] (pitches in values, multiples of 8); box = 64 values of K x box_rows rows, 128-byte swizzle.
 static bool make_map_bf16(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int64_t batch, int64_t pitch,
@@ -591,6 +665,13 @@ extern "C" int b200f_gemm(const void* x, const void* w, void* out, int dtype, in
   p.out_pitch = out_pitch; p.out_bstride = out_bstride; p.splits = splits; p.split_stride = split_stride;
   p.act = act; p.act_a = act_a; p.act_b = act_b;
   if (dtype == B200F_F32) {
+    if (m <= 8) {
+      const float *xf = (const float*)x, *wf = (const float*)w;
+      if (m == 1) return launch_gemv<1>(xf, wf, p, x_pitch, x_bstride, w_pitch, w_bstride, st);
+      if (m == 2) return launch_gemv<2>(xf, wf, p, x_pitch, x_bstride, w_pitch, w_bstride, st);
+      if (m <= 4) return launch_gemv<4>(xf, wf, p, x_pitch, x_bstride, w_pitch, w_bstride, st);
+      return launch_gemv<8>(xf, wf, p, x_pitch, x_bstride, w_pitch, w_bstride, st);
+    }
     const dim3 grid((unsigned)((n + 63) / 64), (unsigned)((m + 63) / 64), (unsigned)batch);
     B200_REQUIRE(grid.y < 65536 && grid.z < 65536, B200_E_SHAPE, "gemm: too many rows or batches");
     launch_pdl(gemm_f32_kernel, grid, dim3(256), 0, st, (const float*)x, (const float*)w, p, x_pitch, x_bstride, w_pitch, w_bstride);

@@ -303,7 +303,7 @@ extern "C" size_t b200f_gemm_f32_ws_bytes(int64_t m, int64_t n, int64_t k, int64
   // per CTA, the split moves 10 bytes of each (m = 16, n = 32768, k = 1024: 155 us against 177).  Everywhere else that kernel has too
   // few CTAs (m = 16, n = 4608: 70 us against 51; n = 1024, k = 4096: 265 against 90) or too many products (m = 1400, n = 4608: 406
   // against 92).
-  if (m <= 8) return 0;                             // gemv.cuh
+  if (m <= 8) return 0;                             // b200f_gemm has a kernel of its own for these
   if (m <= 64 && batch * ((n + 63) / 64) >= 2 * sm_count()) return 0;
   return (size_t)(x3_bytes(m, k, batch) + x3_bytes(n, k, batch) + kXSplitBlocks * 4);
 }

@@ -78,6 +78,25 @@ def test_linear_f32_in_three_parts(m, n, k):
     assert torch.equal(parts.sum(0), got.float())
 
 
+@pytest.mark.parametrize("m,n,k,pad,batch", [(1, 1, 3, 0, 1), (1, 5, 512, 0, 1), (2, 7, 515, 0, 1), (3, 130, 1030, 2, 1), (4, 4, 4, 1, 1), (5, 33, 129, 0, 3),
+                                             (8, 1030, 2048, 0, 1), (8, 66, 511, 4, 2), (9, 66, 511, 4, 2)])
+def test_linear_f32_of_few_rows(m, n, k, pad, batch):
+    """Up to eight rows stream the weights: four weight rows per CTA, whole and ragged groups of four columns, rows that do not
+    begin on 16 bytes, heads as batches.  Chains are k / 128 long and the rest is a tree: 2^-22 of the sum of magnitudes."""
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    x = torch.randn((m, batch, k + pad), device="cuda", generator=g)[..., :k]
+    w = torch.randn((batch, n, k + pad), device="cuda", generator=g)[..., :k]
+    out = torch.full((m, batch, n + 3), 7.0, device="cuda")
+    fo.head_linear(x, w, out[..., :n])
+    want = torch.einsum("mbk,bnk->mbn", x.double(), w.double())
+    size = torch.einsum("mbk,bnk->mbn", x.double().abs(), w.double().abs())
+    assert ((out[..., :n].double() - want).abs() <= 2.0 ** -22 * size).all() and bool((out[..., n:] == 7.0).all())
+    if batch == 1:
+        got = fo.linear(x[:, 0] / k ** 0.5, w[0], act=fo.ACT_XIELU, act_a=0.7, act_b=1.1).double()
+        z = (x[:, 0] / k ** 0.5).double() @ w[0].double().T
+        close(got, host(torch.where(z > 0, 0.7 * z * z + z / 2, 1.1 * (torch.expm1(z.clamp(max=0)) - z.clamp(max=0)) + z / 2)), torch.float32)
+
+
 def test_linear_f32_keeps_infinities_nans_and_the_largest_numbers():
     x, w = torch.randn((130, 70), device="cuda"), torch.randn((140, 70), device="cuda")
     top = torch.finfo(torch.float32).max
