@@ -6,7 +6,7 @@ from typing import NamedTuple
 import torch
 
 from .. import _lib
-from .._lib import call, ptr, require_cuda, stream
+from .._lib import call, i32, ptr, require_cuda, stream
 from .kv_pool import HEAD_DIM, Int8PagedKVCache
 
 _WORKSPACES: dict = {}
@@ -70,9 +70,8 @@ def decode_attention_int8_paged(q8: torch.Tensor, q_mul: torch.Tensor, q_shift: 
         raise ValueError(f"q8 must be [batch, q_heads, {HEAD_DIM}], got shape {tuple(q8.shape)}")
     require_cuda(q8, q_mul, q_shift, page_table, kv_lens)
     batch, q_heads, _ = q8.shape
-    c = lambda t: t.to(torch.int32).contiguous()
     q8 = q8.contiguous()
-    q_mul, q_shift, page_table, kv_lens = c(q_mul), c(q_shift), c(page_table), c(kv_lens)
+    q_mul, q_shift, page_table, kv_lens = i32(q_mul), i32(q_shift), i32(page_table), i32(kv_lens)
     if page_table.ndim != 2 or page_table.shape[0] != batch:
         raise ValueError(f"page_table must be [batch, pitch], got shape {tuple(page_table.shape)}")
     o32 = torch.empty((batch, q_heads, HEAD_DIM), dtype=torch.int32, device=q8.device) if out_q15 else None
@@ -86,9 +85,10 @@ def decode_attention_int8_paged(q8: torch.Tensor, q_mul: torch.Tensor, q_shift: 
         _paged_ws(q8, q_mul, q_shift, pool, layer_id, page_table, kv_lens, None, None, o32, o8, om, batch, q_heads,
                   max_kv_len, workspace)
     else:
+        row_order = i32(row_order)
         call("b200_attn_decode", ptr(q8), ptr(q_mul), ptr(q_shift), ptr(pool.k_cache(layer_id)),
              ptr(pool.v_cache(layer_id)), ptr(pool.meta(layer_id)), ptr(page_table), page_table.stride(0),
-             ptr(kv_lens), ptr(None if row_order is None else row_order.to(torch.int32).contiguous()), ptr(o32), ptr(o8),
+             ptr(kv_lens), ptr(row_order), ptr(o32), ptr(o8),
              ptr(om), batch, q_heads, pool.kv_heads, pool.num_pages, int(max_kv_len), int(cluster), stream())
     if out_q15 and out_int8:
         return o32, o8, om
@@ -117,16 +117,15 @@ def prefill_attention_int8_paged(q8: torch.Tensor, q_mul: torch.Tensor, q_shift:
         raise ValueError(f"q8 must be [tokens, q_heads, {HEAD_DIM}], got shape {tuple(q8.shape)}")
     require_cuda(q8, q_mul, q_shift, page_table, kv_lens, q_lens, q_start)
     rows, q_heads, _ = q8.shape
-    c = lambda t: t.to(torch.int32).contiguous()
     q8 = q8.contiguous()
-    q_mul, q_shift, page_table, kv_lens, q_lens = c(q_mul), c(q_shift), c(page_table), c(kv_lens), c(q_lens)
+    q_mul, q_shift, page_table, kv_lens, q_lens = i32(q_mul), i32(q_shift), i32(page_table), i32(kv_lens), i32(q_lens)
     batch = kv_lens.shape[0]
     if page_table.ndim != 2 or page_table.shape[0] != batch or q_lens.shape[0] != batch:
         raise ValueError(f"page_table [batch, pitch], kv_lens and q_lens [batch] expected, got {tuple(page_table.shape)}, "
                          f"{tuple(kv_lens.shape)}, {tuple(q_lens.shape)}")
     if q_start is None:
         q_start = torch.cumsum(q_lens, 0, dtype=torch.int32) - q_lens
-    q_start = c(q_start)
+    q_start = i32(q_start)
     o32 = torch.empty((rows, q_heads, HEAD_DIM), dtype=torch.int32, device=q8.device) if out_q15 else None
     o8 = torch.empty((rows, q_heads, HEAD_DIM), dtype=torch.int8, device=q8.device) if out_int8 else None
     om = torch.empty((rows, q_heads), dtype=torch.int32, device=q8.device) if out_int8 else None
@@ -149,7 +148,7 @@ class NewTokens(NamedTuple):
 
 def new_tokens(q_lens: torch.Tensor, rows: int) -> NewTokens:
     """Sums q_lens, compares the total with the query rows and reads the longest back from the device, once for all layers
-    of a step (a read-back per layer kept the host from running ahead: 14.8 -> 11.9 ms for one prompt of 333 tokens through 36 layers)."""
+    of a step (a read-back per layer drained the device 36 times in an 8B-shaped step)."""
     q_lens = q_lens.to(torch.int32).contiguous()
     total, longest = (int(v) for v in torch.stack((q_lens.sum(), q_lens.max() if q_lens.numel() else q_lens.sum())).tolist())
     if total != rows:
@@ -183,9 +182,8 @@ def extend_attention_int8_paged(q8: torch.Tensor, q_mul: torch.Tensor, q_shift: 
         raise ValueError(f"q8 must be [tokens, q_heads, {HEAD_DIM}], got shape {tuple(q8.shape)}")
     require_cuda(q8, q_mul, q_shift, page_table, kv_lens, q_lens)
     rows, q_heads, _ = q8.shape
-    c = lambda t: t.to(torch.int32).contiguous()
     q8 = q8.contiguous()
-    q_mul, q_shift, page_table, kv_lens, q_lens = c(q_mul), c(q_shift), c(page_table), c(kv_lens), c(q_lens)
+    q_mul, q_shift, page_table, kv_lens, q_lens = i32(q_mul), i32(q_shift), i32(page_table), i32(kv_lens), i32(q_lens)
     if new is None:
         new = new_tokens(q_lens, rows)
     if impl in ("auto", "tiled"):
@@ -238,15 +236,15 @@ def qkv_rope_quant_store(positions: torch.Tensor, qkv_q15: torch.Tensor, q_heads
         if pl.acc.shape[1] != (q_heads + 2 * hk) * HEAD_DIM:
             raise ValueError(f"qkv width {pl.acc.shape[1]} != (q_heads + 2*kv_heads)*{HEAD_DIM}")
         require_cuda(positions, pl.acc, out_loc, cos_sin_cache_q15, q_norm_weight, k_norm_weight)
-        c = lambda t: None if t is None else t.to(torch.int32).contiguous()
         q8 = torch.empty((tokens, q_heads, HEAD_DIM), dtype=torch.int8, device=pl.acc.device)
         q_mul = torch.empty((tokens, q_heads), dtype=torch.int32, device=pl.acc.device)
         q_shift = torch.empty_like(q_mul)
-        cache = c(cos_sin_cache_q15)
+        positions, cache, out_loc = i32(positions), i32(cos_sin_cache_q15), i32(out_loc)
+        q_norm_weight, k_norm_weight = i32(q_norm_weight), i32(k_norm_weight)
         if tokens:
-            call("b200_qkv_prepare_pending", ptr(c(positions)), ptr(pl.acc), ptr(pl.x_absmax), ptr(pl.weight_mul),
-                 ptr(pl.weight_shift), ptr(cache), cache.shape[0], ptr(c(q_norm_weight)), ptr(c(k_norm_weight)),
-                 ptr(c(out_loc)), ptr(pool.k_cache(layer_id)), ptr(pool.v_cache(layer_id)), ptr(pool.meta(layer_id)),
+            call("b200_qkv_prepare_pending", ptr(positions), ptr(pl.acc), ptr(pl.x_absmax), ptr(pl.weight_mul),
+                 ptr(pl.weight_shift), ptr(cache), cache.shape[0], ptr(q_norm_weight), ptr(k_norm_weight),
+                 ptr(out_loc), ptr(pool.k_cache(layer_id)), ptr(pool.v_cache(layer_id)), ptr(pool.meta(layer_id)),
                  ptr(q8), ptr(q_mul), ptr(q_shift), tokens, q_heads, hk, pool.num_pages, int(with_fwht), stream())
         return q8, q_mul, q_shift
     if qkv_q15.dtype != torch.int32 or qkv_q15.ndim != 2:
@@ -259,14 +257,14 @@ def qkv_rope_quant_store(positions: torch.Tensor, qkv_q15: torch.Tensor, q_heads
     tokens, pitch = qkv_q15.shape[0], qkv_q15.stride(0)
     qd, kd = q_heads * HEAD_DIM, hk * HEAD_DIM
     q, k, v = qkv_q15[:, :qd], qkv_q15[:, qd:qd + kd], qkv_q15[:, qd + kd:]
-    c = lambda t: None if t is None else t.to(torch.int32).contiguous()
     q8 = torch.empty((tokens, q_heads, HEAD_DIM), dtype=torch.int8, device=qkv_q15.device)
     q_mul = torch.empty((tokens, q_heads), dtype=torch.int32, device=qkv_q15.device)
     q_shift = torch.empty_like(q_mul)
-    cache = c(cos_sin_cache_q15)
+    positions, cache, out_loc = i32(positions), i32(cos_sin_cache_q15), i32(out_loc)
+    q_norm_weight, k_norm_weight = i32(q_norm_weight), i32(k_norm_weight)
     if tokens:
-        call("b200_qkv_prepare_q15", ptr(c(positions)), ptr(q), pitch, ptr(k), pitch, ptr(v), pitch, ptr(cache),
-             cache.shape[0], ptr(c(q_norm_weight)), ptr(c(k_norm_weight)), ptr(c(out_loc)), ptr(pool.k_cache(layer_id)),
+        call("b200_qkv_prepare_q15", ptr(positions), ptr(q), pitch, ptr(k), pitch, ptr(v), pitch, ptr(cache),
+             cache.shape[0], ptr(q_norm_weight), ptr(k_norm_weight), ptr(out_loc), ptr(pool.k_cache(layer_id)),
              ptr(pool.v_cache(layer_id)), ptr(pool.meta(layer_id)), ptr(q8), ptr(q_mul), ptr(q_shift), tokens, q_heads, hk,
              pool.num_pages, int(with_fwht), stream())
     return q8, q_mul, q_shift

@@ -19,7 +19,7 @@ from typing import Callable, Optional
 
 import torch
 
-from .._lib import call, ptr, require_cuda, stream
+from .._lib import call, i32, ptr, require_cuda, stream
 from ..kernel.fixed_point import absmax_to_mul_shift, assert_q15, per_token_quant_int8_from_q15
 from ..kernel.pending import PENDING_MAX_ROWS, PendingLinear, zero_workspace
 
@@ -64,6 +64,10 @@ def weight_scale_to_mul_shift(weight_scale: torch.Tensor) -> tuple[torch.Tensor,
     return (torch.tensor(mul, dtype=torch.int32, device=dev), torch.tensor(sh, dtype=torch.int32, device=dev))
 
 
+def _flat(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    return i32(t if t is None or t.ndim == 1 else t.reshape(-1))
+
+
 def int8_gemm_q15(x8: torch.Tensor, x_mul: Optional[torch.Tensor], x_shift: Optional[torch.Tensor], w8: torch.Tensor,
                   w_mul: torch.Tensor, w_shift: Optional[torch.Tensor] = None, *, want_q15: bool = True,
                   want_acc: bool = False, x_absmax: Optional[torch.Tensor] = None):
@@ -81,12 +85,11 @@ def int8_gemm_q15(x8: torch.Tensor, x_mul: Optional[torch.Tensor], x_shift: Opti
     m, k = x8.shape
     n = w8.shape[0]
     x8, w8 = x8.contiguous(), w8.contiguous()
-    c = lambda t: None if t is None else t.reshape(-1).to(torch.int32).contiguous()
-    x_mul, x_shift, w_mul, w_shift = c(x_mul), c(x_shift), c(w_mul), c(w_shift)
+    x_mul, x_shift, w_mul, w_shift = _flat(x_mul), _flat(x_shift), _flat(w_mul), _flat(w_shift)
     out = torch.empty((m, n), dtype=torch.int32, device=x8.device) if want_q15 else None
     acc = torch.empty((m, n), dtype=torch.int32, device=x8.device) if want_acc else None
     if m > 0 and x_absmax is not None:
-        call("b200_gemm_w8a8_absmax", ptr(x8), ptr(w8), ptr(c(x_absmax)), ptr(w_mul), ptr(w_shift), ptr(out), ptr(acc),
+        call("b200_gemm_w8a8_absmax", ptr(x8), ptr(w8), ptr(_flat(x_absmax)), ptr(w_mul), ptr(w_shift), ptr(out), ptr(acc),
              m, n, k, stream())
     elif m > 0:
         call("b200_gemm_w8a8", ptr(x8), ptr(w8), ptr(x_mul), ptr(x_shift), ptr(w_mul), ptr(w_shift), ptr(out),
@@ -141,16 +144,16 @@ class W8A8Int8LinearMethod:
         """The GEMM half of apply_weights_q15 for activations already quantised by a fused row kernel."""
         if getattr(layer, "weight_mul", None) is None:
             self.process_weights_after_loading(layer)
-        x8 = codes.reshape(-1, codes.shape[-1])
+        x8 = codes if codes.ndim == 2 else codes.reshape(-1, codes.shape[-1])
         m, n = x8.shape[0], layer.weight.shape[0]
         if 0 < m <= PENDING_MAX_ROWS and x8.is_contiguous() and layer.weight.is_contiguous() and layer.weight_shift is not None:
             # decode sizes: split-K parts go into a workspace that is kept zero, which saves the clearing launch
             out = torch.empty((m, n), dtype=torch.int32, device=x8.device)
             require_cuda(x8, layer.weight, absmax, layer.weight_mul, layer.weight_shift)
-            call("b200_gemm_w8a8_absmax_ws", ptr(x8), ptr(layer.weight), ptr(absmax.reshape(-1).to(torch.int32).contiguous()), ptr(layer.weight_mul),
+            call("b200_gemm_w8a8_absmax_ws", ptr(x8), ptr(layer.weight), ptr(_flat(absmax)), ptr(layer.weight_mul),
                  ptr(layer.weight_shift), ptr(out), ptr(zero_workspace(x8.device, m, n)), m, n, x8.shape[1], stream())
         else:
-            out = int8_gemm_q15(x8, None, None, layer.weight, layer.weight_mul, layer.weight_shift, x_absmax=absmax.reshape(-1))
+            out = int8_gemm_q15(x8, None, None, layer.weight, layer.weight_mul, layer.weight_shift, x_absmax=absmax)
         if bias is not None:
             out = self._add_bias(out, bias)
         return out
@@ -173,7 +176,7 @@ class W8A8Int8LinearMethod:
         m, n2 = x8.shape[0], layer.weight.shape[0]
         out = torch.empty((m, n2 // 2), dtype=torch.int32, device=x8.device)
         if m:
-            call("b200_gemm_gate_up_silu", ptr(x8), ptr(layer.weight), ptr(absmax.reshape(-1).to(torch.int32).contiguous()),
+            call("b200_gemm_gate_up_silu", ptr(x8), ptr(layer.weight), ptr(_flat(absmax)),
                  ptr(layer.weight_mul), ptr(layer.weight_shift), ptr(out), ptr(zero_workspace(x8.device, m, n2)), m, n2,
                  x8.shape[1], stream())
         return out
@@ -189,7 +192,7 @@ class W8A8Int8LinearMethod:
         ws = zero_workspace(x8.device, m, n)
         if m:
             call("b200_gemm_w8a8_acc_ws", ptr(x8), ptr(layer.weight.contiguous()), ptr(ws), m, n, x8.shape[1], stream())
-        return PendingLinear(ws, absmax.reshape(-1).to(torch.int32).contiguous(), layer.weight_mul, layer.weight_shift)
+        return PendingLinear(ws, _flat(absmax), layer.weight_mul, layer.weight_shift)
 
     @staticmethod
     def _add_bias(out: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
