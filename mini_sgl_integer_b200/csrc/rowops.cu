@@ -133,21 +133,21 @@ rmsnorm_rows_kernel(const int32_t* __restrict__ x, const int32_t* __restrict__ r
 
   int4* no = norm_out ? reinterpret_cast<int4*>(norm_out + row * H) : nullptr;
   int m2 = 0;
+  auto apply = [&](auto element) {
 #pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int idx = threadIdx.x + i * blockDim.x;
-    if (FULL || idx < nvec) {
-      const int4 ww = kEarlyGain ? gain[i] : __ldg(wr + idx);
-      int4 o;
-      o.x = nr.zero ? 0 : norm_apply(v[i].x, inv, ww.x, nr.p);
-      o.y = nr.zero ? 0 : norm_apply(v[i].y, inv, ww.y, nr.p);
-      o.z = nr.zero ? 0 : norm_apply(v[i].z, inv, ww.z, nr.p);
-      o.w = nr.zero ? 0 : norm_apply(v[i].w, inv, ww.w, nr.p);
-      v[i] = o;
-      if (no) no[idx] = o;
-      m2 = max(max(m2, abs_wrap(o.x)), max(abs_wrap(o.y), max(abs_wrap(o.z), abs_wrap(o.w))));
+    for (int i = 0; i < VPT; ++i) {
+      const int idx = threadIdx.x + i * blockDim.x;
+      if (FULL || idx < nvec) {
+        const int4 ww = kEarlyGain ? gain[i] : __ldg(wr + idx);
+        const int4 o = make_int4(element(v[i].x, ww.x), element(v[i].y, ww.y), element(v[i].z, ww.z), element(v[i].w, ww.w));
+        v[i] = o;
+        if (no) no[idx] = o;
+        m2 = max(max(m2, abs_wrap(o.x)), max(abs_wrap(o.y), max(abs_wrap(o.z), abs_wrap(o.w))));
+      }
     }
-  }
+  };
+  if (nr.p >= 14) apply([&](int x1, int w1) { return norm_apply_high(x1, inv, w1, nr.p - 14); });
+  else apply([&](int x1, int w1) { return nr.zero ? 0 : norm_apply(x1, inv, w1, nr.p); });
   if (codes == nullptr) return;
   m2 = max(1, block_max(m2, red32));
   const float mf = __int2float_rn(m2);

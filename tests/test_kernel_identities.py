@@ -135,3 +135,17 @@ def test_prefill_score_and_exponential_forms():
         t = (dot * mul) >> (s - 1)
         assert np.abs(t).max() < 2**31
         assert np.array_equal((t + 1) >> 1, oattn.mul_shift(dot, mul, s))
+
+
+def test_norm_product_from_its_upper_words():
+    """Rows with p >= 14: (v * inv * w, wrapped to 64 bits) >> (p + 18), saturated, is the upper word of the wrapped product >> (p - 14)."""
+    rng = np.random.default_rng(8)
+    n, word = 60000, 2**32 - 1
+    edge = lambda: np.where(rng.random(n) < 0.2, rng.choice([-2**31, -2**31 + 1, -1, 0, 1, 2**31 - 1], n), rng.integers(-2**31, 2**31, n)).tolist()
+    for v, inv, w, p in zip(edge(), edge(), edge(), rng.integers(14, 32, n).tolist()):
+        a = v * inv
+        b = (a * w + 2**63) % 2**64 - 2**63
+        want = max(-2**31, min(2**31 - 1, b >> (p + 18)))
+        lo, hi = a & word, (a >> 32) & word
+        top = (((lo * (w & word)) >> 32) - (lo if w < 0 else 0) + hi * (w & word)) & word
+        assert (top - ((top >> 31) << 32)) >> (p - 14) == want
