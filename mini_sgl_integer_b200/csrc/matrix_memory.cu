@@ -456,23 +456,29 @@ memory_scan_kernel(const MemoryParams p, const T* __restrict__ rows) {
   }
 }
 
-// Log gates (f, i) of a prompt batch to (f + m_(t-1) - m_t, exp(i - m_t), exp(-m_t)); a warp per (sequence, head).
-__global__ void __launch_bounds__(32)
+// Log gates (f, i) of a prompt batch to (f + m_(t-1) - m_t, exp(i - m_t), exp(-m_t)); a CTA per (sequence, head), a warp per 32
+// tokens of a stretch.  One warp per (sequence, head) was a chain of 32 tokens after 32: 56 us for 3500 tokens.  The warps' maps
+// m -> max(m + a, b) are composed one after the other as that chain did, so the bits are the same.
+constexpr int kRunningWarps = 16;
+__global__ void __launch_bounds__(32 * kRunningWarps)
 running_max_kernel(const MemoryPrepare p) {
+  __shared__ float2 maps[2][kRunningWarps];
   pdl_launch_dependents();
   pdl_wait();
-  const int h = blockIdx.x, seq = blockIdx.y, lane = threadIdx.x;
+  const int h = blockIdx.x, seq = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t t0 = p.seq_start[seq], t1 = p.seq_start[seq + 1];
   if (t0 >= t1) return;
   float* ms = p.norm_state + ((int64_t)p.slots[seq] * p.heads + h) * (p.norm_dim + 1) + p.norm_dim;
   float m = p.positions[t0] > 0 ? *ms : 0.0f;
   const float4 none = make_float4(0.0f, -INFINITY, 0.0f, 0.0f);         // leaves the maximum alone
   auto load = [&](int64_t t) { return t < t1 ? p.gates[t * p.heads + h] : none; };
-  float4 next[2] = {load(t0 + lane), load(t0 + 32 + lane)};
-  for (int64_t base = t0; base < t1; base += 32) {
-    const float4 g = next[0];
-    next[0] = next[1];
-    next[1] = load(base + 64 + lane);
+  constexpr int kStretch = 32 * kRunningWarps;
+  float4 next = load(t0 + threadIdx.x);
+  int buf = 0;
+  for (int64_t base = t0; base < t1; base += kStretch, buf ^= 1) {
+    const int64_t t = base + threadIdx.x;
+    const float4 g = next;
+    next = load(t + kStretch);
     float a = g.x, b = g.y;                              // m -> max(m + a, b), composed over the lanes up to this one
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -482,13 +488,21 @@ running_max_kernel(const MemoryPrepare p) {
         a += pa;
       }
     }
-    const float after = fmaxf(m + a, b);
+    if (lane == 31) maps[buf][warp] = make_float2(a, b);
+    __syncthreads();
+    float mine = m;
+#pragma unroll
+    for (int w = 0; w < kRunningWarps; ++w) {
+      if (w == warp) mine = m;
+      const float2 f = maps[buf][w];
+      m = fmaxf(m + f.x, f.y);
+    }
+    const float after = fmaxf(mine + a, b);
     float before = __shfl_up_sync(FULL_MASK, after, 1);
-    if (lane == 0) before = m;
-    m = __shfl_sync(FULL_MASK, after, 31);
-    if (base + lane < t1) p.gates[(base + lane) * p.heads + h] = make_float4(fminf(g.x + before - after, 0.0f), expf(g.y - after), expf(-after), 0.0f);
+    if (lane == 0) before = mine;
+    if (t < t1) p.gates[t * p.heads + h] = make_float4(fminf(g.x + before - after, 0.0f), expf(g.y - after), expf(-after), 0.0f);
   }
-  if (lane == 0) *ms = m;
+  if (threadIdx.x == 0) *ms = m;
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -1482,7 +1496,7 @@ static int launch_prepare(MemoryPrepare p, T* out, int batch, cudaStream_t st) {
     rc = check_launch("memory_prepare (convolution state)");
   }
   if (rc == B200_OK && p.kind == B200F_MEMORY_EXP) {
-    launch_pdl(running_max_kernel, dim3((unsigned)p.heads, (unsigned)batch), dim3(32), 0, st, p);
+    launch_pdl(running_max_kernel, dim3((unsigned)p.heads, (unsigned)batch), dim3(32 * kRunningWarps), 0, st, p);
     rc = check_launch("memory_prepare (running maximum)");
   }
   return rc;
