@@ -85,6 +85,63 @@ latent_prepare_kernel(const PrepareParams p, T* __restrict__ qn, T* __restrict__
     row[p.kv_rank + i] = from_f32<T>(rotated([&](int k) { return at(d0 + p.kv_rank + k); }, i, p.rot_dims, cs));
 }
 
+// The same four columns at a time, for sizes and pitches that are multiples of four.  All columns of a token's queries are spread
+// over the CTA at once (a warp per head walked its columns one by one, two loads in flight), and a thread keeps its four
+// columns of the latent between the sum of squares and the result.  8186 tokens x (16 heads of 192 + 576): 113 -> 80 us; 256 tokens in four
+// parts: 13.9 -> 8.0; one token in six parts: 10.0 -> 6.0.
+constexpr int kPrepareThreads = 256;
+template <typename T>
+__global__ void __launch_bounds__(kPrepareThreads)
+latent_prepare_vec_kernel(const PrepareParams p, T* __restrict__ qn, T* __restrict__ q_lat, T* __restrict__ cache) {
+  __shared__ float scratch[32];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int64_t t = blockIdx.x;
+  const int tid = threadIdx.x;
+  const float* src = p.qd + t * p.qd_pitch;
+  const int pos = min(max(p.positions[t], 0), p.max_pos - 1);
+  const float* cs = p.rot_dims ? p.rope + (int64_t)pos * p.rot_dims : nullptr;
+  const int half = p.rot_dims >> 1;
+  // columns i .. i + 3 of a rotated vector
+  auto rotated4 = [&](const float* v, int i) {
+    const float4 a = part_sum4(v + i, p.splits, p.split_stride);
+    if (i >= p.rot_dims) return a;
+    const bool low = i < half;
+    const float4 o = part_sum4(v + (low ? i + half : i - half), p.splits, p.split_stride);
+    const float4 c = *reinterpret_cast<const float4*>(cs + (low ? i : i - half)), s = *reinterpret_cast<const float4*>(cs + half + (low ? i : i - half));
+    return low ? make_float4(a.x * c.x - o.x * s.x, a.y * c.y - o.y * s.y, a.z * c.z - o.z * s.z, a.w * c.w - o.w * s.w)
+               : make_float4(a.x * c.x + o.x * s.x, a.y * c.y + o.y * s.y, a.z * c.z + o.z * s.z, a.w * c.w + o.w * s.w);
+  };
+  const int lat = p.kv_rank + p.rot_dim, d4 = p.dim >> 2, per = d4 + (p.rot_dim >> 2);
+  const int64_t d0 = (int64_t)p.heads * p.head_pitch;
+  const bool own = p.dkv_norm && 4 * tid < p.kv_rank;
+  float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (own) x = part_sum4(src + d0 + 4 * tid, p.splits, p.split_stride);
+#pragma unroll 2
+  for (int i = tid; i < p.heads * per; i += kPrepareThreads) {
+    const int h = i / per, c = i - h * per;
+    const float* q = src + (int64_t)h * p.head_pitch;
+    if (c < d4) store4(qn + (t * p.heads + h) * p.qn_pitch + 4 * c, part_sum4(q + 4 * c, p.splits, p.split_stride));
+    else store4(q_lat + (t * p.heads + h) * p.lat_pitch + p.kv_rank + 4 * (c - d4), rotated4(q + p.dim, 4 * (c - d4)));
+  }
+  if (p.lat_pitch > lat)
+    for (int i = tid; i < p.heads * (p.lat_pitch - lat); i += kPrepareThreads) {
+      const int h = i / (p.lat_pitch - lat);
+      q_lat[(t * p.heads + h) * p.lat_pitch + lat + i - h * (p.lat_pitch - lat)] = from_f32<T>(0.0f);
+    }
+  if (!p.dkv_norm) return;
+  const float ss = block_sum(fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w))), scratch);
+  const float inv = 1.0f / sqrtf(ss / (float)p.kv_rank + p.eps);
+  const int64_t loc = p.out_loc[t];
+  if (loc < 0 || loc >= p.cache_rows) return;
+  T* row = cache + loc * p.lat_pitch;
+  if (own) {
+    const float4 w = *reinterpret_cast<const float4*>(p.dkv_norm + 4 * tid);
+    store4(row + 4 * tid, make_float4(x.x * inv * w.x, x.y * inv * w.y, x.z * inv * w.z, x.w * inv * w.w));
+  }
+  for (int i = 4 * tid; i < p.rot_dim; i += 4 * kPrepareThreads) store4(row + p.kv_rank + i, rotated4(src + d0 + p.kv_rank, i));
+}
+
 // ---------------------------------------------------------------------------------------------------
 struct AttnParams {
   const int32_t* page_table;
@@ -804,6 +861,16 @@ extern "C" int b200f_latent_prepare(const float* qd, int splits, int64_t split_s
   B200_REQUIRE(qd && positions && qn && q_lat && (!rot_dims || rope) && (!dkv_norm || (cache && out_loc)), B200_E_NULL, "latent_prepare: null pointer");
   PrepareParams p{qd, splits, split_stride, qd_pitch, positions, out_loc, rope, rot_dims, max_pos, dkv_norm, eps, heads, dim, rot_dim,
                   kv_rank, head_pitch, qn_pitch, lat_pitch, cache_rows};
+  const bool vec = dim % 4 == 0 && rot_dim % 4 == 0 && rot_dims % 8 == 0 && kv_rank % 4 == 0 && kv_rank <= 4 * kPrepareThreads && head_pitch % 4 == 0 &&
+                   qn_pitch % 4 == 0 && lat_pitch % 4 == 0 && qd_pitch % 4 == 0 && (splits == 1 || split_stride % 4 == 0) && (int64_t)heads * head_pitch < (1ll << 31) &&
+                   aligned16(qd) && aligned16(rope) && aligned16(dkv_norm) && aligned16(qn) && aligned16(q_lat) && aligned16(cache);
+  if (vec) {
+    if (dtype == B200F_BF16)
+      launch_pdl(latent_prepare_vec_kernel<bf16>, dim3((unsigned)tokens), dim3(kPrepareThreads), 0, (cudaStream_t)s, p, (bf16*)qn, (bf16*)q_lat, (bf16*)cache);
+    else
+      launch_pdl(latent_prepare_vec_kernel<float>, dim3((unsigned)tokens), dim3(kPrepareThreads), 0, (cudaStream_t)s, p, (float*)qn, (float*)q_lat, (float*)cache);
+    return check_launch("latent_prepare");
+  }
   if (dtype == B200F_BF16)
     launch_pdl(latent_prepare_kernel<bf16>, dim3((unsigned)tokens), dim3(256), 0, (cudaStream_t)s, p, (bf16*)qn, (bf16*)q_lat, (bf16*)cache);
   else

@@ -310,6 +310,37 @@ def test_latent_prepare(dtype, own):
         assert bool((cache == 0).all())
 
 
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("H,dim,rot,dims,rank,parts", [(3, 20, 16, 8, 36, 2), (16, 128, 64, 64, 512, 1), (5, 4, 8, 8, 1024, 3), (2, 8, 4, 0, 4, 1), (1, 64, 32, 16, 1028, 1)])
+def test_latent_prepare_four_columns_at_a_time(dtype, H, dim, rot, dims, rank, parts):
+    """Sizes that are multiples of four: rotations of part of the columns and of none, latents up to and beyond what a CTA holds,
+    sums of parts, locations outside the cache."""
+    from mini_sgl_integer_b200.layers.rotary_float import rotary_table
+    from mini_sgl_integer_b200.models.config import RotarySpec, YarnScaling
+    rng = np.random.default_rng(rank)
+    T, eps, sc = 11, 1e-2, ROT["scaling"]
+    rope = rotary_table(RotarySpec(dims, 5000.0, YarnScaling(sc["factor"], sc["original"], sc["fast"], sc["slow"])), 300, "cuda") if dims else None
+    n, lat = H * (dim + rot) + rank + rot, fo.pad8(rank + rot)
+    qd, pos, w = rng.standard_normal((parts, T, n)) * 0.3, rng.integers(0, 300, T), rng.standard_normal(rank)
+    loc = rng.permutation(5 * 16)[:T]
+    loc[4], loc[5] = -1, 5 * 16
+    qn = torch.zeros(T, H, fo.pad8(dim), dtype=dtype, device="cuda")
+    ql = torch.full((T, H, lat), 9.0, dtype=dtype, device="cuda")
+    cache = torch.zeros(5, 16, lat, dtype=dtype, device="cuda")
+    fo.latent_prepare(dev(qd), i32(pos), i32(loc), rope, dev(w), eps, qn, ql, cache, H, dim, rot, rank)
+    full = dev(qd).double().sum(0).cpu().numpy()
+    turn = (lambda v: S.rotate(v, pos, dict(ROT, dims=dims, base=5000.0))) if dims else (lambda v: v)
+    q, d = full[:, :H * (dim + rot)].reshape(T, H, dim + rot), full[:, H * (dim + rot):]
+    close(qn[..., :dim], q[..., :dim], dtype)
+    close(ql[..., rank:rank + rot], turn(q[..., dim:]), dtype)
+    assert bool((ql[..., :rank] == 9.0).all()) and bool((ql[..., rank + rot:] == 0.0).all())
+    kept = [i for i in range(T) if 0 <= loc[i] < 80]
+    rows = cache.view(-1, lat)[loc[kept].tolist()]
+    close(rows[:, :rank], S.rms_norm(d[:, :rank], w, eps)[kept], dtype)
+    close(rows[:, rank:rank + rot], turn(d[:, rank:])[kept], dtype)
+    assert int((cache.view(-1, lat).abs().sum(1) > 0).sum()) == len(kept)
+
+
 def attention_case(rng, kv_lens, q_lens, heads, rank, rot, dtype, spike=True):
     """Latent rows in shuffled pages, queries, and a spike: one key far back that a head attends to almost alone."""
     lat, pages = fo.pad8(rank + rot), [-(-n // 16) for n in kv_lens]
