@@ -110,7 +110,7 @@ __device__ __forceinline__ void store_pack(bf16* p, const Pack<VEC>& a) {
   }
 }
 
-template <typename T, int VEC, int NV>
+template <typename T, int VEC, int NV, bool EARLY>
 __global__ void sublayer_end_kernel(const SublayerEnd p, T* __restrict__ x_out_t) {
   __shared__ float scratch[32];
   pdl_launch_dependents();
@@ -121,6 +121,54 @@ __global__ void sublayer_end_kernel(const SublayerEnd p, T* __restrict__ x_out_t
   int col[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) col[i] = (i * blockDim.x + threadIdx.x) * VEC;
+  // the sum of the depth average's earlier planes
+  auto plane_sum = [&](int c) {
+    Pack<VEC> a;
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) a.v[k] = 0.0f;
+    const float* h = p.hist + base + c;
+    int j = 0;
+    for (; j + 4 <= p.planes; j += 4) {            // four planes in flight
+      Pack<VEC> b[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) b[u] = load_pack<VEC>(h + (int64_t)(j + u) * p.plane_stride);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float cu = __ldg(p.coef + j + u);
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) a.v[k] = fmaf(cu, b[u].v[k], a.v[k]);
+      }
+    }
+    for (; j < p.planes; ++j) {
+      const Pack<VEC> b = load_pack<VEC>(h + (int64_t)j * p.plane_stride);
+      const float cu = __ldg(p.coef + j);
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) a.v[k] = fmaf(cu, b.v[k], a.v[k]);
+    }
+    return a;
+  };
+  // EARLY: what the sums of squares do not need is requested in front of them.  A decode row is a chain of memory latencies (y,
+  // then stream and gain, then planes, then the next gain); this saves two of them: decode steps of Sefevik 0.3B 613 -> 598 us, 1.4B
+  // with 256 rows 1527 -> 1516.  The registers cost many rows their occupancy (8186 rows: 52.6 -> 64.0 us) and wide ones do not have them.
+  constexpr int E = EARLY ? NV : 1;
+  Pack<VEC> x0[E], w0[E], a0[E], f0[E];
+  if (EARLY) {
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      if (col[i] >= p.width) continue;
+      if (p.y) {
+        if (p.x_in) x0[i] = load_pack<VEC>(p.x_in + base + col[i]);
+        w0[i] = load_pack<VEC>(p.norm_w + col[i]);
+      }
+      if (p.final_w) f0[i] = load_pack<VEC>(p.final_w + col[i]);
+    }
+  }
+  auto early_planes = [&]() {
+    if (!EARLY || !p.coef) return;
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+      if (col[i] < p.width) a0[i] = plane_sum(col[i]);
+  };
   // the sum of a stack of parts and its sum of squares
   auto take = [&](const float* y, int splits, int64_t stride, Pack<VEC> (&a)[NV]) {
     float ss = 0.0f;
@@ -140,6 +188,7 @@ __global__ void sublayer_end_kernel(const SublayerEnd p, T* __restrict__ x_out_t
   };
   if (p.y) {
     float ss = take(p.y, p.splits, p.split_stride, r);
+    early_planes();
     if (p.y2) {
       Pack<VEC> r2[NV];
       const float ss2 = block_sum(take(p.y2, p.splits2, p.split_stride2, r2), scratch);
@@ -164,8 +213,8 @@ __global__ void sublayer_end_kernel(const SublayerEnd p, T* __restrict__ x_out_t
       Pack<VEC> x;
 #pragma unroll
       for (int k = 0; k < VEC; ++k) x.v[k] = 0.0f;
-      if (p.x_in) x = load_pack<VEC>(p.x_in + base + col[i]);
-      const Pack<VEC> w = load_pack<VEC>(p.norm_w + col[i]);
+      if (p.x_in) x = EARLY ? x0[EARLY ? i : 0] : load_pack<VEC>(p.x_in + base + col[i]);
+      const Pack<VEC> w = EARLY ? w0[EARLY ? i : 0] : load_pack<VEC>(p.norm_w + col[i]);
 #pragma unroll
       for (int k = 0; k < VEC; ++k) r[i].v[k] = fmaf(r[i].v[k] * inv, w.v[k], x.v[k]);
     }
@@ -173,6 +222,7 @@ __global__ void sublayer_end_kernel(const SublayerEnd p, T* __restrict__ x_out_t
 #pragma unroll
     for (int i = 0; i < NV; ++i)
       if (col[i] < p.width) r[i] = load_pack<VEC>(p.x_in + base + col[i]);
+    early_planes();
   }
   if (p.add) {
 #pragma unroll
@@ -189,28 +239,7 @@ __global__ void sublayer_end_kernel(const SublayerEnd p, T* __restrict__ x_out_t
     for (int i = 0; i < NV; ++i) {
       if (col[i] >= p.width) continue;
       if (p.hist_out) store_pack<VEC>(p.hist_out + base + col[i], r[i]);
-      Pack<VEC> a;
-#pragma unroll
-      for (int k = 0; k < VEC; ++k) a.v[k] = 0.0f;
-      const float* h = p.hist + base + col[i];
-      int j = 0;
-      for (; j + 4 <= p.planes; j += 4) {          // four planes in flight
-        Pack<VEC> b[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) b[u] = load_pack<VEC>(h + (int64_t)(j + u) * p.plane_stride);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float c = __ldg(p.coef + j + u);
-#pragma unroll
-          for (int k = 0; k < VEC; ++k) a.v[k] = fmaf(c, b[u].v[k], a.v[k]);
-        }
-      }
-      for (; j < p.planes; ++j) {
-        const Pack<VEC> b = load_pack<VEC>(h + (int64_t)j * p.plane_stride);
-        const float c = __ldg(p.coef + j);
-#pragma unroll
-        for (int k = 0; k < VEC; ++k) a.v[k] = fmaf(c, b.v[k], a.v[k]);
-      }
+      const Pack<VEC> a = EARLY ? a0[EARLY ? i : 0] : plane_sum(col[i]);
 #pragma unroll
       for (int k = 0; k < VEC; ++k) r[i].v[k] = fmaf(c_new, r[i].v[k], a.v[k]);
     }
@@ -233,7 +262,7 @@ __global__ void sublayer_end_kernel(const SublayerEnd p, T* __restrict__ x_out_t
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       if (col[i] >= p.width) continue;
-      const Pack<VEC> w = load_pack<VEC>(p.final_w + col[i]);
+      const Pack<VEC> w = EARLY ? f0[EARLY ? i : 0] : load_pack<VEC>(p.final_w + col[i]);
 #pragma unroll
       for (int k = 0; k < VEC; ++k) r[i].v[k] = r[i].v[k] * inv * w.v[k];
     }
@@ -331,10 +360,13 @@ static int launch_sublayer_end(const SublayerEnd& p, T* x_out_t, int64_t rows, c
   while (threads < 1024 && threads * 4 < groups) threads *= 2;
   const int nv = (groups + threads - 1) / threads;
   const dim3 grid((unsigned)rows), block(threads);
-  if (nv <= 1) launch_pdl(sublayer_end_kernel<T, VEC, 1>, grid, block, 0, st, p, x_out_t);
-  else if (nv <= 2) launch_pdl(sublayer_end_kernel<T, VEC, 2>, grid, block, 0, st, p, x_out_t);
-  else if (nv <= 4) launch_pdl(sublayer_end_kernel<T, VEC, 4>, grid, block, 0, st, p, x_out_t);
-  else if (nv <= 8) launch_pdl(sublayer_end_kernel<T, VEC, 8>, grid, block, 0, st, p, x_out_t);
+  const bool few = rows <= 592;                     // up to about four rows per SM
+  if (nv <= 1 && few) launch_pdl(sublayer_end_kernel<T, VEC, 1, true>, grid, block, 0, st, p, x_out_t);
+  else if (nv <= 2 && few) launch_pdl(sublayer_end_kernel<T, VEC, 2, true>, grid, block, 0, st, p, x_out_t);
+  else if (nv <= 1) launch_pdl(sublayer_end_kernel<T, VEC, 1, false>, grid, block, 0, st, p, x_out_t);
+  else if (nv <= 2) launch_pdl(sublayer_end_kernel<T, VEC, 2, false>, grid, block, 0, st, p, x_out_t);
+  else if (nv <= 4) launch_pdl(sublayer_end_kernel<T, VEC, 4, false>, grid, block, 0, st, p, x_out_t);
+  else if (nv <= 8) launch_pdl(sublayer_end_kernel<T, VEC, 8, false>, grid, block, 0, st, p, x_out_t);
   else {
     set_error("sublayer_end: width %d is above the kernel's %d", p.width, 8 * 1024 * VEC);
     return B200_E_UNSUPPORTED;

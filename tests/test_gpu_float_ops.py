@@ -201,6 +201,29 @@ def test_sublayer_end(dtype, width, parts):
         close(xt, S.rms_norm(want, fw, eps), dtype)
 
 
+@pytest.mark.parametrize("width", [3, 40, 1024, 2048, 1027])
+def test_sublayer_end_of_few_and_many_rows(width):
+    """Up to 592 rows request streams, gains and planes in front of the sums: the bits of the form for more rows, for every
+    combination of what may be left out, also where the stream is updated in place."""
+    g = torch.Generator(device="cuda").manual_seed(width)
+    rnd = lambda *n: torch.randn(n, device="cuda", generator=g)
+    T, few, parts, planes = 593, 592, 3, 5
+    y, y2, x, hist, coef = rnd(parts, T, width), rnd(1, T, width), rnd(T, width), rnd(planes + 1, T, width), rnd(planes + 1)
+    w, w1, w2, fw, add = (rnd(width) for _ in range(5))
+    cut = lambda t: None if t is None else t[..., :few, :].contiguous()
+    for has_y, mean, avg, final, plus, stream in [(1, 0, 0, 1, 0, 1), (1, 1, 0, 1, 1, 1), (1, 0, 1, 1, 0, 1), (0, 0, 1, 0, 1, 1), (1, 0, 1, 0, 0, 0), (0, 0, 0, 1, 0, 1)]:
+        outs = []
+        for c in (lambda t: None if t is None else t.clone(), cut):
+            xs, h = c(x) if stream else None, c(hist)
+            xo = xs if xs is not None else torch.empty_like(c(x))
+            xt = torch.zeros(xo.shape[0], fo.pad8(width), dtype=torch.bfloat16, device="cuda")[:, :width]
+            kw = dict(hist=h, planes=planes, coef=coef, hist_out=h[planes]) if avg else {}
+            fo.sublayer_end(c(y) if has_y else None, xs, w if has_y else None, 1e-3, xo, xt, torch.bfloat16, final_w=fw if final else None,
+                            mean_with=(w1, c(y2), w2) if mean else None, add=add if plus else None, **kw)
+            outs.append((xo[:few], xt[:few], h[planes, :few]))
+        assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
 @pytest.mark.parametrize("dtype", DT)
 @pytest.mark.parametrize("n", [40, 133, 2052])
 def test_xielu(dtype, n):
