@@ -40,10 +40,11 @@ B200_API int b200f_gemm(const void* x, const void* w, void* out, int dtype, int 
                         float act_b, b200_stream_t s);
 B200_API int b200f_gemm_status(int* out_host, int reset);    /* synchronises with the device */
 
-/* ---- 32-bit linear on the tensor cores: operands as sums of three bf16 numbers, fp32 accumulation restarted every 128 of K;
- * closer to the exact result than a chain of fp32 fmas.  ws: b200f_gemm_f32_ws_bytes bytes, 128-byte aligned; 0 where
- * b200f_gemm is to be used instead. */
-B200_API size_t b200f_gemm_f32_ws_bytes(int64_t m, int64_t n, int64_t k, int64_t batch);
+/* ---- 32-bit linear whose sums may be taken in any order (b200f_gemm gives each output one chain over K, the same bits in every
+ * batch).  Up to eight rows on the fp32 units, more on the tensor cores: operands as sums of three bf16 numbers, fp32 accumulation
+ * restarted every 64 of K; closer to the exact result than a chain of fp32 fmas.  ws: b200f_gemm_f32_ws_bytes bytes, 128-byte
+ * aligned (NULL for 0); negative where b200f_gemm is to be used instead. */
+B200_API int64_t b200f_gemm_f32_ws_bytes(int64_t m, int64_t n, int64_t k, int64_t batch);
 B200_API int b200f_gemm_f32(const float* x, const float* w, float* out, int64_t m, int64_t n, int64_t k, int64_t batch, int64_t x_pitch,
                             int64_t x_bstride, int64_t w_pitch, int64_t w_bstride, int64_t out_pitch, int64_t out_bstride,
                             int act, float act_a, float act_b, void* ws, b200_stream_t s);

@@ -105,7 +105,7 @@ FLOAT_SIGNATURES: dict[str, list] = {
 }
 _SHARED = ("b200_last_error_string", "b200_decode_prepare")      # in every library
 _RESTYPES = {"b200_last_error_string": c_char_p, "b200_attn_workspace_bytes": ctypes.c_size_t,
-             "b200_tp_block_bytes": ctypes.c_size_t, "b200f_latent_attn_ws_floats": ctypes.c_size_t, "b200f_gemm_f32_ws_bytes": ctypes.c_size_t,
+             "b200_tp_block_bytes": ctypes.c_size_t, "b200f_latent_attn_ws_floats": ctypes.c_size_t, "b200f_gemm_f32_ws_bytes": ctypes.c_int64,
              "b200f_grouped_attn_ws_floats": ctypes.c_size_t, "b200f_memory_scan_ws_bytes": ctypes.c_size_t}
 
 _libs: dict[str, ctypes.CDLL] = {}

@@ -13,7 +13,9 @@
 //   * in between: one CTA per 128 x BN tile.
 // Every wait is bounded as in the int8 kernels.
 //
-// fp32 operands (B200F_F32) use a plain shared-memory tiled FFMA kernel: true 32-bit products.
+// fp32 operands (B200F_F32): true 32-bit products, every sum one chain over K.  Up to eight rows stream the weights (chain_f32_kernel),
+// more go through shared-memory tiles (gemm_f32_kernel); both give a row the same bits.  (float_gemm32.cu has forms that
+// round otherwise, for callers that do not need that.)
 #include "float_common.cuh"
 #include "umma.cuh"
 
@@ -515,77 +517,94 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, const 
     }
 }
 
-// Up to eight rows in 32 bits: what counts is streaming the weights once, which tiles of 64 x 64 on few CTAs did at a tenth of the
-// memory's rate and the split into bf16 parts at a third (it writes and reads 6 bytes for each 4).  A CTA has four weight
-// rows; its threads stride over K, so every lane has four loads of 16 bytes in flight, and the sums meet in the end.  One row,
-// 1024 x 4096 weights: 357 -> 8.5 us; 32768 x 1024: 153 -> 21.5 (20.6 at the memory's rate); eight rows: 370 -> 9.4 and 154 -> 59 us, where the
-// loads of x bound it.
-constexpr int kGemvRows = 4, kGemvThreads = 128;
+// Up to eight rows in 32 bits: what counts is streaming the weights once, which the 64 x 64 tiles above do on few CTAs at a tenth of the
+// memory's rate.  Every sum is the same chain over K as there, so a row's result does not depend on how many rows there are.  A warp has eight weight rows and up to eight rows of x, a lane one or two of these sums; both operands come through
+// a ring in shared memory, since a lane's own walk along a row of weights would touch 32 rows per load.  What bounds it: the issue of
+// loads and multiply-adds (two float4 from shared memory per four of them), and with few weight rows the chain, four cycles per value
+// of K.  WARPS 1 where CTAs of four warps would not occupy every SM twice.  One row, 1024 x 4096 weights: 357 us with the tiles, 27 here;
+// 32768 x 1024: 153, 53; eight rows: 370, 31 and 154, 52.
+constexpr int kChainStages = 4;
 
-template <int M, int VEC>
-__global__ void __launch_bounds__(kGemvThreads)
-gemv_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, const FGemmParams p, int64_t x_pitch, int64_t x_bstride,
-                int64_t w_pitch, int64_t w_bstride) {
-  constexpr int R = kGemvRows;
-  __shared__ float part[kGemvThreads / 32][R * M];
-  pdl_launch_dependents();
-  pdl_wait();
-  const int n0 = blockIdx.x * R, b = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const float *xr[M], *wr[R];
-#pragma unroll
-  for (int m = 0; m < M; ++m) xr[m] = x + (int64_t)b * x_bstride + min(m, p.M - 1) * x_pitch;
-#pragma unroll
-  for (int r = 0; r < R; ++r) wr[r] = w + (int64_t)b * w_bstride + min(n0 + r, p.N - 1) * w_pitch;
-  float acc[R][M] = {};
-  const int body = p.K / VEC * VEC;
-#pragma unroll 2
-  for (int c = threadIdx.x * VEC; c < body; c += kGemvThreads * VEC) {
-    float wv[R][VEC];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      if (VEC == 4) *reinterpret_cast<float4*>(wv[r]) = __ldg(reinterpret_cast<const float4*>(wr[r] + c));
-      else wv[r][0] = __ldg(wr[r] + c);
-    }
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      float xv[VEC];
-      if (VEC == 4) *reinterpret_cast<float4*>(xv) = *reinterpret_cast<const float4*>(xr[m] + c);
-      else xv[0] = xr[m][c];
-#pragma unroll
-      for (int r = 0; r < R; ++r)
-#pragma unroll
-        for (int k = 0; k < VEC; ++k) acc[r][m] = fmaf(wv[r][k], xv[k], acc[r][m]);
-    }
-  }
-  if (VEC > 1 && body + (int)threadIdx.x < p.K) {          // the columns behind the last group of four
-#pragma unroll
-    for (int m = 0; m < M; ++m)
-#pragma unroll
-      for (int r = 0; r < R; ++r) acc[r][m] = fmaf(wr[r][body + threadIdx.x], xr[m][body + threadIdx.x], acc[r][m]);
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const float v = warp_sum(acc[r][m]);
-      if (lane == 0) part[warp][r * M + m] = v;
-    }
-  __syncthreads();
-  if (threadIdx.x >= R * M) return;
-  const int r = threadIdx.x / M, m = threadIdx.x % M;
-  if (m >= p.M || n0 + r >= p.N) return;
-  float v = (part[0][threadIdx.x] + part[1][threadIdx.x]) + (part[2][threadIdx.x] + part[3][threadIdx.x]);
-  if (p.act == B200F_ACT_XIELU) v = xielu_f32(v, p.act_a, p.act_b);
-  reinterpret_cast<float*>(p.out)[(int64_t)b * p.out_bstride + m * p.out_pitch + n0 + r] = v;
+__device__ __forceinline__ void cp_async_part(unsigned dst, const float* src, int bytes, bool vec) {       // the rest becomes zero
+  if (vec) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
-template <int M>
-static int launch_gemv(const float* x, const float* w, const FGemmParams& p, int64_t x_pitch, int64_t x_bstride, int64_t w_pitch,
+// MPL: rows of x per lane.
+template <int MPL, int WARPS, bool VEC>
+__global__ void __launch_bounds__(32 * WARPS)
+chain_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, const FGemmParams p, int64_t x_pitch, int64_t x_bstride,
+                 int64_t w_pitch, int64_t w_bstride) {
+  constexpr int W = 8 * WARPS, ROWS = W + 4 * MPL, COLS = WARPS == 1 ? 128 : 64, STEP = VEC ? 4 : 1, CHUNKS = COLS / STEP;
+  constexpr int STRIDE = VEC ? 32 * WARPS / CHUNKS : 1, PER = VEC ? (ROWS + STRIDE - 1) / STRIDE : 1;     // rows of a thread's copies
+  __shared__ __align__(16) float ring[kChainStages][ROWS][COLS + 4];       // rows 4 banks apart: conflict-free float4 loads
+  pdl_launch_dependents();
+  pdl_wait();
+  const int n0 = blockIdx.x * W, b = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  x += (int64_t)b * x_bstride;
+  w += (int64_t)b * w_bstride;
+  const int stages = (p.K + COLS - 1) / COLS;
+  auto row_of = [&](int r) { return r < W ? w + (int64_t)min(n0 + r, p.N - 1) * w_pitch : x + (int64_t)min(r - W, p.M - 1) * x_pitch; };
+  const int vr = threadIdx.x / CHUNKS, vc = threadIdx.x % CHUNKS * STEP;
+  const float* src[PER];
+#pragma unroll
+  for (int j = 0; j < PER; ++j) src[j] = row_of(min(vr + j * STRIDE, ROWS - 1));
+  auto issue = [&](int stage) {
+    if (stage < stages) {
+      const int k0 = stage * COLS;
+      float(*to)[COLS + 4] = ring[stage % kChainStages];
+      if constexpr (VEC) {
+        const int left = max(0, min(4, p.K - k0 - vc)), at = left > 0 ? k0 + vc : 0;
+#pragma unroll
+        for (int j = 0; j < PER; ++j)
+          if (vr + j * STRIDE < ROWS) cp_async_part(smem_u32(&to[vr + j * STRIDE][vc]), src[j] + at, 4 * left, true);
+      } else {
+        for (int i = threadIdx.x; i < ROWS * COLS; i += 32 * WARPS) {
+          const int r = i / COLS, k = k0 + i % COLS;
+          cp_async_part(smem_u32(&to[r][i % COLS]), row_of(r) + min(k, p.K - 1), k < p.K ? 4 : 0, false);
+        }
+      }
+    }
+    cp_async_commit();
+  };
+  for (int j = 0; j < kChainStages - 1; ++j) issue(j);
+  const int r = warp * 8 + (lane & 7), m0 = lane >> 3;
+  const int end = (p.K + 15) & ~15;                 // (the tiles above add up whole steps of 16)
+  float acc[MPL] = {};
+  for (int stage = 0; stage < stages; ++stage) {
+    cp_async_wait<kChainStages - 2>();
+    if (WARPS > 1) __syncthreads(); else __syncwarp();          // this stage has landed for everybody, the one before is free
+    issue(stage + kChainStages - 1);
+    const float(*s)[COLS + 4] = ring[stage % kChainStages];
+    const int cols = min(COLS, end - stage * COLS);
+#pragma unroll 4
+    for (int c = 0; c < cols; c += 4) {
+      const float4 a = *reinterpret_cast<const float4*>(&s[r][c]);
+#pragma unroll
+      for (int j = 0; j < MPL; ++j) {
+        const float4 v = *reinterpret_cast<const float4*>(&s[W + m0 + 4 * j][c]);
+        acc[j] = fmaf(v.w, a.w, fmaf(v.z, a.z, fmaf(v.y, a.y, fmaf(v.x, a.x, acc[j]))));
+      }
+    }
+  }
+  cp_async_wait<0>();
+  if (n0 + r >= p.N) return;
+#pragma unroll
+  for (int j = 0; j < MPL; ++j) {
+    const int m = m0 + 4 * j;
+    if (m >= p.M) continue;
+    const float v = p.act == B200F_ACT_XIELU ? xielu_f32(acc[j], p.act_a, p.act_b) : acc[j];
+    reinterpret_cast<float*>(p.out)[(int64_t)b * p.out_bstride + (int64_t)m * p.out_pitch + n0 + r] = v;
+  }
+}
+
+template <int MPL, int WARPS>
+static int launch_chain(const float* x, const float* w, const FGemmParams& p, int64_t x_pitch, int64_t x_bstride, int64_t w_pitch,
                        int64_t w_bstride, cudaStream_t st) {
-  const dim3 grid((unsigned)((p.N + kGemvRows - 1) / kGemvRows), (unsigned)p.batch);
+  const dim3 grid((unsigned)((p.N + 8 * WARPS - 1) / (8 * WARPS)), (unsigned)p.batch);
   const bool vec = aligned16(x) && aligned16(w) && x_pitch % 4 == 0 && w_pitch % 4 == 0 && (p.batch == 1 || (x_bstride % 4 == 0 && w_bstride % 4 == 0));
-  if (vec) launch_pdl(gemv_f32_kernel<M, 4>, grid, dim3(kGemvThreads), 0, st, x, w, p, x_pitch, x_bstride, w_pitch, w_bstride);
-  else launch_pdl(gemv_f32_kernel<M, 1>, grid, dim3(kGemvThreads), 0, st, x, w, p, x_pitch, x_bstride, w_pitch, w_bstride);
+  if (vec) launch_pdl(chain_f32_kernel<MPL, WARPS, true>, grid, dim3(32 * WARPS), 0, st, x, w, p, x_pitch, x_bstride, w_pitch, w_bstride);
+  else launch_pdl(chain_f32_kernel<MPL, WARPS, false>, grid, dim3(32 * WARPS), 0, st, x, w, p, x_pitch, x_bstride, w_pitch, w_bstride);
   return check_launch("gemm (fp32, few rows)");
 }
 
@@ -667,10 +686,9 @@ extern "C" int b200f_gemm(const void* x, const void* w, void* out, int dtype, in
   if (dtype == B200F_F32) {
     if (m <= 8) {
       const float *xf = (const float*)x, *wf = (const float*)w;
-      if (m == 1) return launch_gemv<1>(xf, wf, p, x_pitch, x_bstride, w_pitch, w_bstride, st);
-      if (m == 2) return launch_gemv<2>(xf, wf, p, x_pitch, x_bstride, w_pitch, w_bstride, st);
-      if (m <= 4) return launch_gemv<4>(xf, wf, p, x_pitch, x_bstride, w_pitch, w_bstride, st);
-      return launch_gemv<8>(xf, wf, p, x_pitch, x_bstride, w_pitch, w_bstride, st);
+      const bool wide = batch * ((n + 31) / 32) >= 2 * sm_count();
+      if (m <= 4) return wide ? launch_chain<1, 4>(xf, wf, p, x_pitch, x_bstride, w_pitch, w_bstride, st) : launch_chain<1, 1>(xf, wf, p, x_pitch, x_bstride, w_pitch, w_bstride, st);
+      return wide ? launch_chain<2, 4>(xf, wf, p, x_pitch, x_bstride, w_pitch, w_bstride, st) : launch_chain<2, 1>(xf, wf, p, x_pitch, x_bstride, w_pitch, w_bstride, st);
     }
     const dim3 grid((unsigned)((n + 63) / 64), (unsigned)((m + 63) / 64), (unsigned)batch);
     B200_REQUIRE(grid.y < 65536 && grid.z < 65536, B200_E_SHAPE, "gemm: too many rows or batches");

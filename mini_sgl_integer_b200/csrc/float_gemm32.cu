@@ -1,6 +1,9 @@
-// 32-bit linears on the bf16 tensor cores.
+// 32-bit linears whose sums may be taken in any order: closer to the exact ones than a chain over K, but rounded otherwise for
+// other numbers of rows.  (float_gemm.cu has the chains.)
 //
 //   out[b][t, j] = act( sum_k x[b][t, k] * w[b][j, k] )          operands, products and result in 32 bits
+//
+// Up to eight rows stream the weights through the fp32 units (gemv_f32_kernel); more run on the bf16 tensor cores.
 //
 // An fp32 number is the sum of three bf16 numbers (8 + 8 + 8 bits of fraction, each rounded to nearest); of the nine products of
 // two such sums the six above 2^-24 of the largest are formed: hi hi, hi mid, mid hi, mid mid, hi lo, lo hi.  split_parts_kernel
@@ -278,6 +281,77 @@ gemm_f32x3_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   }
 }
 
+// Up to eight rows in 32 bits: what counts is streaming the weights once, which tiles of 64 x 64 on few CTAs did at a tenth of the
+// memory's rate and the split into bf16 parts at a third (it writes and reads 6 bytes for each 4).  A CTA has four weight
+// rows; its threads stride over K, so every lane has four loads of 16 bytes in flight, and the sums meet in the end.  One row,
+// 1024 x 4096 weights: 357 -> 8.5 us; 32768 x 1024: 153 -> 21.5 (20.6 at the memory's rate); eight rows: 370 -> 9.4 and 154 -> 59 us, where the
+// loads of x bound it.
+constexpr int kGemvRows = 4, kGemvThreads = 128;
+
+template <int M, int VEC>
+__global__ void __launch_bounds__(kGemvThreads)
+gemv_f32_kernel(const X3Params p) {
+  constexpr int R = kGemvRows;
+  __shared__ float part[kGemvThreads / 32][R * M];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int n0 = blockIdx.x * R, b = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float *xr[M], *wr[R];
+#pragma unroll
+  for (int m = 0; m < M; ++m) xr[m] = p.x.src + (int64_t)b * p.x.bstride + min(m, p.M - 1) * p.x.pitch;
+#pragma unroll
+  for (int r = 0; r < R; ++r) wr[r] = p.w.src + (int64_t)b * p.w.bstride + min(n0 + r, p.N - 1) * p.w.pitch;
+  float acc[R][M] = {};
+  const int body = p.K / VEC * VEC;
+#pragma unroll 2
+  for (int c = threadIdx.x * VEC; c < body; c += kGemvThreads * VEC) {
+    float wv[R][VEC];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (VEC == 4) *reinterpret_cast<float4*>(wv[r]) = __ldg(reinterpret_cast<const float4*>(wr[r] + c));
+      else wv[r][0] = __ldg(wr[r] + c);
+    }
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      float xv[VEC];
+      if (VEC == 4) *reinterpret_cast<float4*>(xv) = *reinterpret_cast<const float4*>(xr[m] + c);
+      else xv[0] = xr[m][c];
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) acc[r][m] = fmaf(wv[r][k], xv[k], acc[r][m]);
+    }
+  }
+  if (VEC > 1 && body + (int)threadIdx.x < p.K) {          // the columns behind the last group of four
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+#pragma unroll
+      for (int r = 0; r < R; ++r) acc[r][m] = fmaf(wr[r][body + threadIdx.x], xr[m][body + threadIdx.x], acc[r][m]);
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const float v = warp_sum(acc[r][m]);
+      if (lane == 0) part[warp][r * M + m] = v;
+    }
+  __syncthreads();
+  if (threadIdx.x >= R * M) return;
+  const int r = threadIdx.x / M, m = threadIdx.x % M;
+  if (m >= p.M || n0 + r >= p.N) return;
+  float v = (part[0][threadIdx.x] + part[1][threadIdx.x]) + (part[2][threadIdx.x] + part[3][threadIdx.x]);
+  if (p.act == B200F_ACT_XIELU) v = xielu_f32(v, p.act_a, p.act_b);
+  p.out[(int64_t)b * p.out_bstride + m * p.out_pitch + n0 + r] = v;
+}
+
+template <int M>
+static int launch_gemv(const X3Params& p, cudaStream_t st) {
+  const dim3 grid((unsigned)((p.N + kGemvRows - 1) / kGemvRows), (unsigned)p.batch);
+  if (p.x.vec && p.w.vec) launch_pdl(gemv_f32_kernel<M, 4>, grid, dim3(kGemvThreads), 0, st, p);
+  else launch_pdl(gemv_f32_kernel<M, 1>, grid, dim3(kGemvThreads), 0, st, p);
+  return check_launch("gemm_f32 (few rows)");
+}
+
 // ----------------------------------------------------------------------------- host side
 static int64_t x3_pitch(int64_t k) { return (k + 7) / 8 * 8; }
 static int64_t x3_bytes(int64_t rows, int64_t k, int64_t batch) { return (3 * batch * rows * x3_pitch(k) * 2 + 127) / 128 * 128; }
@@ -297,25 +371,27 @@ static bool x3_map(CUtensorMap* map, const bf16* base, int64_t rows, int64_t K, 
 
 using namespace b200;
 
-extern "C" size_t b200f_gemm_f32_ws_bytes(int64_t m, int64_t n, int64_t k, int64_t batch) {
-  if (m <= 0 || n <= 0 || k <= 0 || batch <= 0 || batch > 65535 / 3 || m >= (1ll << 31) || n >= (1ll << 31) || k >= (1ll << 31)) return 0;
+extern "C" int64_t b200f_gemm_f32_ws_bytes(int64_t m, int64_t n, int64_t k, int64_t batch) {
+  if (m <= 0 || n <= 0 || k <= 0 || batch <= 0 || batch > 65535 / 3 || m >= (1ll << 31) || n >= (1ll << 31) || k >= (1ll << 31)) return -1;
+  if (m <= 8) return 0;
   // Few rows against many weight rows: the fp32 units read the weights once (4 bytes each) and fill the GPU with a tile of 64 x 64
   // per CTA, the split moves 10 bytes of each (m = 16, n = 32768, k = 1024: 155 us against 177).  Everywhere else that kernel has too
   // few CTAs (m = 16, n = 4608: 70 us against 51; n = 1024, k = 4096: 265 against 90) or too many products (m = 1400, n = 4608: 406
   // against 92).
-  if (m <= 8) return 0;                             // b200f_gemm has a kernel of its own for these
-  if (m <= 64 && batch * ((n + 63) / 64) >= 2 * sm_count()) return 0;
-  return (size_t)(x3_bytes(m, k, batch) + x3_bytes(n, k, batch) + kXSplitBlocks * 4);
+  if (m <= 64 && batch * ((n + 63) / 64) >= 2 * sm_count()) return -1;
+  return x3_bytes(m, k, batch) + x3_bytes(n, k, batch) + kXSplitBlocks * 4;
 }
 
 extern "C" int b200f_gemm_f32(const float* x, const float* w, float* out, int64_t m, int64_t n, int64_t k, int64_t batch, int64_t x_pitch,
                               int64_t x_bstride, int64_t w_pitch, int64_t w_bstride, int64_t out_pitch, int64_t out_bstride, int act,
                               float act_a, float act_b, void* ws, b200_stream_t s) {
-  B200_REQUIRE(x && w && out && ws, B200_E_NULL, "gemm_f32: null pointer");
-  B200_REQUIRE(b200f_gemm_f32_ws_bytes(m, n, k, batch) != 0, B200_E_SHAPE, "gemm_f32: m=%lld n=%lld k=%lld batch=%lld", (long long)m,
+  B200_REQUIRE(x && w && out, B200_E_NULL, "gemm_f32: null pointer");
+  const int64_t need = b200f_gemm_f32_ws_bytes(m, n, k, batch);
+  B200_REQUIRE(need >= 0, B200_E_SHAPE, "gemm_f32: m=%lld n=%lld k=%lld batch=%lld", (long long)m,
                (long long)n, (long long)k, (long long)batch);
   B200_REQUIRE(x_pitch >= k && w_pitch >= k && out_pitch >= n, B200_E_SHAPE, "gemm_f32: a row pitch is shorter than its row");
   B200_REQUIRE(act == B200F_ACT_NONE || act == B200F_ACT_XIELU, B200_E_UNSUPPORTED, "gemm_f32: activation %d", act);
+  B200_REQUIRE(need == 0 || ws, B200_E_NULL, "gemm_f32: no workspace");
   B200_REQUIRE((reinterpret_cast<uintptr_t>(ws) & 127u) == 0, B200_E_ALIGN, "gemm_f32: the workspace must be 128-byte aligned");
   cudaStream_t st = (cudaStream_t)s;
   unsigned char* at = (unsigned char*)ws;
@@ -329,6 +405,7 @@ extern "C" int b200f_gemm_f32(const float* x, const float* w, float* out, int64_
   p.out = out; p.M = (int)m; p.N = (int)n; p.K = (int)k; p.batch = (int)batch; p.kp = (int)x3_pitch(k);
   p.out_pitch = out_pitch; p.out_bstride = out_bstride; p.act = act; p.act_a = act_a; p.act_b = act_b;
   p.vec = rows16(out, out_pitch, out_bstride);
+  if (need == 0) return m == 1 ? launch_gemv<1>(p, st) : m == 2 ? launch_gemv<2>(p, st) : m <= 4 ? launch_gemv<4>(p, st) : launch_gemv<8>(p, st);
   const int64_t quads = batch * (m + n) * ((k + 3) / 4), blocks = (quads + 255) / 256;
   p.split_blocks = (int)(blocks < kXSplitBlocks ? blocks : kXSplitBlocks);
   CUtensorMap mx, mw;

@@ -57,12 +57,12 @@ def _check_vec(name: str, t: torch.Tensor, n: int) -> None:
 
 # ----------------------------------------------------------------------------- linears
 def _gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, T: int, n: int, k: int, batch: int, strides, parts: int = 1, act: int = ACT_NONE,
-          act_a: float = 0.0, act_b: float = 0.0) -> None:
+          act_a: float = 0.0, act_b: float = 0.0, chained: bool = False) -> None:
     """``strides``: row pitch and batch stride of x, of w and of out."""
-    if x.dtype == torch.float32:
-        need = query("b200f_gemm_f32_ws_bytes", T, n, k, batch) if act != ACT_GATED_SILU else 0
-        if need:
-            ws = torch.empty(need, dtype=torch.uint8, device=x.device)
+    if x.dtype == torch.float32 and not chained:
+        need = query("b200f_gemm_f32_ws_bytes", T, n, k, batch) if act != ACT_GATED_SILU else -1
+        if need >= 0:
+            ws = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None
             call("b200f_gemm_f32", ptr(x), ptr(w), ptr(out), T, n, k, batch, *strides, act, act_a, act_b, ptr(ws), stream())
             return
     call("b200f_gemm", ptr(x), ptr(w), ptr(out), dtype_code(x.dtype), int(out.dtype == torch.float32), T, n, k, batch, *strides, parts, T * n, act,
@@ -70,28 +70,30 @@ def _gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, T: int, n: int, k
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, out_f32: bool = False, act: int = ACT_NONE,
-           act_a: float = 0.0, act_b: float = 0.0) -> torch.Tensor:
+           act_a: float = 0.0, act_b: float = 0.0, chained: bool = False) -> torch.Tensor:
     """act(x w^T) for rows x [T, k] and weight rows w [n, k]; with ACT_GATED_SILU (bf16) the weight rows alternate, 16 gates
-    and 16 values, and the result has n / 2 columns."""
+    and 16 values, and the result has n / 2 columns.  ``chained``: in 32 bits every sum is one chain over k, and a row's result
+    does not depend on the others; without it the sums are closer to the exact ones, but rounded otherwise for other numbers of rows."""
     _check_rows("x", x, x.dtype)
     _check_rows("w", w, x.dtype, x.shape[1])
     T, k = x.shape
     n = w.shape[0]
     if out is None:
         out = rows(T, n // 2 if act == ACT_GATED_SILU else n, torch.float32 if out_f32 else x.dtype, x.device)
-    _gemm(x, w, out, T, n, k, 1, (_pitch(x), 0, _pitch(w), 0, _pitch(out), 0), 1, act, act_a, act_b)
+    _gemm(x, w, out, T, n, k, 1, (_pitch(x), 0, _pitch(w), 0, _pitch(out), 0), 1, act, act_a, act_b, chained)
     return out
 
 
-def linear_parts(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
-    """x w^T as fp32 partial sums [parts, T, n]; several parts at decode sizes where the weight alone cannot occupy the GPU."""
+def linear_parts(x: torch.Tensor, w: torch.Tensor, chained: bool = False) -> torch.Tensor:
+    """x w^T as fp32 partial sums [parts, T, n]; several parts at decode sizes where the weight alone cannot occupy the GPU.
+    ``chained``: as for ``linear``."""
     _check_rows("x", x, x.dtype)
     _check_rows("w", w, x.dtype, x.shape[1])
     T, k = x.shape
     n, code = w.shape[0], dtype_code(x.dtype)
     parts = query("b200f_gemm_splits", T, n, k, 1, code)
     out = torch.empty((parts, T, n), dtype=torch.float32, device=x.device)
-    _gemm(x, w, out, T, n, k, 1, (_pitch(x), 0, _pitch(w), 0, n, 0), parts)
+    _gemm(x, w, out, T, n, k, 1, (_pitch(x), 0, _pitch(w), 0, n, 0), parts, chained=chained)
     return out
 
 

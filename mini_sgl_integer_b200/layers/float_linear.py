@@ -38,11 +38,13 @@ def padded_rows(w: torch.Tensor, dtype: torch.dtype, device) -> torch.Tensor:
 
 class FloatLinear(BaseOP):
     """W x without bias; ``weight`` may be several checkpoint tensors stacked along the output.  ``pad_out``: zero rows are
-    added up to a multiple of it, so that the rows of the output start on aligned addresses."""
+    added up to a multiple of it, so that the rows of the output start on aligned addresses.  ``chained``: in 32 bits, the same
+    order of the sums for every batch (fo.linear)."""
 
-    def __init__(self, in_features: int, out_features: Sequence[int], names: Sequence[str], dtype: torch.dtype, device, pad_out: int = 1):
+    def __init__(self, in_features: int, out_features: Sequence[int], names: Sequence[str], dtype: torch.dtype, device, pad_out: int = 1,
+                 chained: bool = False):
         self._in, self._outs, self._names, self._pad = in_features, tuple(out_features), tuple(names), -sum(out_features) % pad_out
-        self._dtype, self._device = dtype, device
+        self._dtype, self._device, self._chained = dtype, device, chained
         self.weight = torch.empty(0)
 
     def load_state_dict(self, state_dict: StateDict, *, prefix: str = "", _internal: bool = False) -> None:
@@ -52,11 +54,11 @@ class FloatLinear(BaseOP):
         self.weight = padded_rows(parts[0] if len(parts) == 1 else torch.cat([p.to(self._device) for p in parts]), self._dtype, self._device)
 
     def forward(self, x: torch.Tensor, out_f32: bool = False) -> torch.Tensor:
-        return fo.linear(x, self.weight, out_f32=out_f32)
+        return fo.linear(x, self.weight, out_f32=out_f32, chained=self._chained)
 
     def parts(self, x: torch.Tensor) -> torch.Tensor:
         """The output as fp32 partial sums [parts, rows, out] for a kernel that adds them."""
-        return fo.linear_parts(x, self.weight)
+        return fo.linear_parts(x, self.weight, self._chained)
 
 
 class XieluMLP(BaseOP):
@@ -93,10 +95,10 @@ class GatedSiluMLP(BaseOP):
 
     BLOCK = 16
 
-    def __init__(self, hidden: int, ff: int, dtype: torch.dtype, device):
-        self._hidden, self._ff, self._dtype, self._device = hidden, ff, dtype, device
+    def __init__(self, hidden: int, ff: int, dtype: torch.dtype, device, chained: bool = False):
+        self._hidden, self._ff, self._dtype, self._device, self._chained = hidden, ff, dtype, device, chained
         self.weight = torch.empty(0)
-        self.down = FloatLinear(ff, [hidden], ["down"], dtype, device)
+        self.down = FloatLinear(ff, [hidden], ["down"], dtype, device, chained=chained)
 
     def load_state_dict(self, state_dict: StateDict, *, prefix: str = "", _internal: bool = False) -> None:
         blocks = -(-self._ff // self.BLOCK)
@@ -115,5 +117,5 @@ class GatedSiluMLP(BaseOP):
         if x.dtype == torch.bfloat16 and fo.query("b200f_gemm_splits", T, w.shape[0], x.shape[1], 1, fo.dtype_code(x.dtype)) == 1:
             fo.linear(x, w, out=act, act=fo.ACT_GATED_SILU)                                    # in the linear's epilogue
         else:
-            fo.gated_silu(fo.linear_parts(x, w), act)
+            fo.gated_silu(fo.linear_parts(x, w, self._chained), act)
         return self.down.parts(act[:, :self._ff])

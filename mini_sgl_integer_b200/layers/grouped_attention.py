@@ -18,7 +18,7 @@ from .float_linear import FloatLinear, take_f32
 class GroupedAttention(BaseOP):
     def __init__(self, cfg: GroupedAttentionConfig, hidden: int, eps: float, dtype: torch.dtype, device):
         self._cfg, self._eps, self._device = cfg, eps, device
-        self.o = FloatLinear(cfg.heads * cfg.vdim, [hidden], ["o"], dtype, device)
+        self.o = FloatLinear(cfg.heads * cfg.vdim, [hidden], ["o"], dtype, device, chained=True)
 
     def projections(self) -> List[Tuple[str, int]]:
         c = self._cfg

@@ -25,7 +25,7 @@ class MatrixMemory(BaseOP):
         self._heads, self._qk, self._dim, self._vdim, self._eps, self._device = heads, qk_heads, dim, vdim, eps, device
         self._q_scale, self._cap, self._group = 1.0, 0.0, vdim
         self._conv_w = self._conv_b = self._skip = None
-        self.o = FloatLinear(heads * vdim, [hidden], ["o"], dtype, device)
+        self.o = FloatLinear(heads * vdim, [hidden], ["o"], dtype, device, chained=True)
 
     def projections(self) -> List[Tuple[str, int]]:
         raise NotImplementedError

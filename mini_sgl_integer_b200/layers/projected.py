@@ -20,7 +20,7 @@ class ProjectedMixers(BaseOP):
             for name, n in mixer.projections():
                 names.append(prefix + name)
                 sizes.append(n)
-        self.proj = FloatLinear(hidden, sizes, names, dtype, device, pad_out=8)
+        self.proj = FloatLinear(hidden, sizes, names, dtype, device, pad_out=8, chained=True)
 
     def load_state_dict(self, state_dict: StateDict, *, prefix: str = "", _internal: bool = False) -> None:
         self.proj.load_state_dict(state_dict, prefix=prefix)

@@ -8,6 +8,10 @@ Layers start .. stop - 1 may run several times with the same weights; a vector o
 and every run has its own cache and state.  The stream x is fp32 and updated in place; a sublayer's last linear stays a
 stack of partial sums, and one kernel finishes it: output norm, residual add, the vector of a pass that begins, and the
 norm in front of the next linear, whose result is in the model's dtype.
+
+In 32 bits the linears sum in one order whatever the batch (``chained``).  At a request's first token an mLSTM head reads out one
+key; where that is nearly orthogonal to the query the readout is tiny, and the norm of the head brings it back to size one together
+with the rounding of everything in front of it: another order of the linears' sums moves outputs by up to 5e-5.
 """
 from __future__ import annotations
 
@@ -38,7 +42,7 @@ class DerelornLayer(BaseOP):
         else:
             sides = [("", MLSTM(m, *args) if layer.type == "mlstm" else GatedDelta(m, *args))]
         self.mix = ProjectedMixers(hidden, sides, dtype, device)
-        self.mlp: Optional[GatedSiluMLP] = GatedSiluMLP(hidden, layer.mlp.ff, dtype, device) if layer.mlp is not None else None
+        self.mlp: Optional[GatedSiluMLP] = GatedSiluMLP(hidden, layer.mlp.ff, dtype, device, chained=True) if layer.mlp is not None else None
 
     def load_state_dict(self, state_dict: StateDict, *, prefix: str = "", _internal: bool = False) -> None:
         gain = lambda name: take_f32(state_dict, prefix + name, (self._hidden,), self._device)
@@ -73,7 +77,7 @@ class DerelornForCausalLM(HybridForCausalLM):
         fo.dtype_code(dtype)
         self._runs = config.runs
         self.layers = OPList([DerelornLayer(config, l, dtype, self._device) for l in config.layers])
-        self.head = FloatLinear(config.hidden_size, [config.vocab_size], ["head"], dtype, self._device)
+        self.head = FloatLinear(config.hidden_size, [config.vocab_size], ["head"], dtype, self._device, chained=True)
 
     def load_state_dict(self, state_dict: StateDict, *, prefix: str = "", _internal: bool = False) -> None:
         c = self._config

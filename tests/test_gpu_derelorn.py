@@ -84,6 +84,25 @@ def test_prompt_portions_and_decoding(name, dtype):
     e.check_status()
 
 
+@pytest.mark.parametrize("name", ["one layer", "wide heads", "mixed", "odd sizes"])
+def test_a_request_in_32_bits_does_not_depend_on_the_others(name):
+    """Short prompts, where a head's readout of one nearly orthogonal key is rounding brought back to size one: each request's
+    logits are the same bits alone and beside others, for prompts and for the tokens after them."""
+    rng = np.random.default_rng(3)
+    prompts = [rng.integers(0, CONFIGS[name]["vocab"], n).tolist() for n in (8, 3, 8, 2, 12, 40)]
+    e = engine(name, "float32")
+    alone = []
+    for p in prompts:
+        r = e.open()
+        alone.append((e.step([r], [p]).clone(), e.step([r], [p[:1]]).clone()))
+        e.close(r)
+    reqs = [e.open() for _ in prompts]
+    first = e.step(reqs, prompts).clone()
+    second = e.step(reqs, [p[:1] for p in prompts]).clone()
+    for i, (a, b) in enumerate(alone):
+        assert torch.equal(first[i], a[0]) and torch.equal(second[i], b[0]), i
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("name", ["mixed", "odd sizes", "loop over everything"])
 def test_decoding_from_the_first_token(name, dtype):

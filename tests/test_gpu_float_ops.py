@@ -97,6 +97,23 @@ def test_linear_f32_of_few_rows(m, n, k, pad, batch):
         close(got, host(torch.where(z > 0, 0.7 * z * z + z / 2, 1.1 * (torch.expm1(z.clamp(max=0)) - z.clamp(max=0)) + z / 2)), torch.float32)
 
 
+@pytest.mark.parametrize("n,k,pad", [(1, 1, 0), (7, 15, 1), (8, 16, 0), (33, 17, 3), (40, 63, 0), (9, 64, 4), (24, 129, 3), (130, 65, 3), (66, 1030, 2), (9480, 260, 0), (9477, 70, 1)])
+def test_chained_linear_f32_gives_a_row_the_same_bits_in_every_batch(n, k, pad):
+    """Sums that are one chain over k, whatever kernel the number of rows selects (1 .. 4, 5 .. 8, more) and however the rows lie:
+    around a step (16) and a stage (64, 128) of K, a warp's weight rows (8), CTAs of one and of four warps (from 9441 weight rows on)."""
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    x = torch.randn((70, k + pad), device="cuda", generator=g)[:, :k]
+    w = torch.randn((n, k + pad), device="cuda", generator=g)[:, pad:]
+    kw = dict(act=fo.ACT_XIELU, act_a=0.7, act_b=1.1)
+    want, act = fo.linear(x, w, chained=True), fo.linear(x, w, chained=True, **kw)
+    exact, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert ((want.double() - exact).abs() <= (k + 1) * 2.0 ** -24 * size).all()
+    for m in (1, 2, 3, 4, 5, 8, 9, 33, 65):
+        assert torch.equal(fo.linear(x[:m], w, chained=True), want[:m]), m
+        assert torch.equal(fo.linear_parts(x[3:3 + m], w, chained=True)[0], want[3:3 + m]), m
+        assert torch.equal(fo.linear(x[:m], w, chained=True, **kw), act[:m]), m
+
+
 def test_linear_f32_keeps_infinities_nans_and_the_largest_numbers():
     x, w = torch.randn((130, 70), device="cuda"), torch.randn((140, 70), device="cuda")
     top = torch.finfo(torch.float32).max
