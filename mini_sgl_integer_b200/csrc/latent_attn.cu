@@ -36,6 +36,10 @@ struct PrepareParams {
   int64_t cache_rows;
 };
 
+// First and second half of a rotated pair; the two kernels below round in the same places.
+__device__ __forceinline__ float turn_low(float a, float o, float c, float s) { return fmaf(-o, s, __fmul_rn(a, c)); }
+__device__ __forceinline__ float turn_high(float a, float o, float c, float s) { return fmaf(o, s, __fmul_rn(a, c)); }
+
 // Entry i of a rotated vector whose unrotated entries `load` returns.
 template <typename F>
 __device__ __forceinline__ float rotated(const F& load, int i, int rot_dims, const float* cs) {
@@ -43,7 +47,7 @@ __device__ __forceinline__ float rotated(const F& load, int i, int rot_dims, con
   const int half = rot_dims >> 1;
   const int k = i < half ? i : i - half;
   const float c = cs[k], s = cs[half + k];
-  return i < half ? load(i) * c - load(i + half) * s : load(i) * c + load(i - half) * s;
+  return i < half ? turn_low(load(i), load(i + half), c, s) : turn_high(load(i), load(i - half), c, s);
 }
 
 template <typename T>
@@ -87,13 +91,16 @@ latent_prepare_kernel(const PrepareParams p, T* __restrict__ qn, T* __restrict__
 
 // The same four columns at a time, for sizes and pitches that are multiples of four.  All columns of a token's queries are spread
 // over the CTA at once (a warp per head walked its columns one by one, two loads in flight), and a thread keeps its four
-// columns of the latent between the sum of squares and the result.  8186 tokens x (16 heads of 192 + 576): 113 -> 80 us; 256 tokens in four
-// parts: 13.9 -> 8.0; one token in six parts: 10.0 -> 6.0.
+// columns of the latent between the sum of squares and the result.  Rotations round and squares are added up (through shared
+// memory) as in the kernel above: otherwise some of the cache's bf16 entries fall to the other side.  16 heads of 192 + 576
+// columns, with the launch: 8186 tokens 123 -> 94 us (88 without that order); 256 tokens in four parts 29.5 -> 18.4; one token in six
+// parts 29.4 -> 17.1.
 constexpr int kPrepareThreads = 256;
 template <typename T>
 __global__ void __launch_bounds__(kPrepareThreads)
 latent_prepare_vec_kernel(const PrepareParams p, T* __restrict__ qn, T* __restrict__ q_lat, T* __restrict__ cache) {
   __shared__ float scratch[32];
+  __shared__ __align__(16) float latent[4 * kPrepareThreads];
   pdl_launch_dependents();
   pdl_wait();
   const int64_t t = blockIdx.x;
@@ -109,14 +116,15 @@ latent_prepare_vec_kernel(const PrepareParams p, T* __restrict__ qn, T* __restri
     const bool low = i < half;
     const float4 o = part_sum4(v + (low ? i + half : i - half), p.splits, p.split_stride);
     const float4 c = *reinterpret_cast<const float4*>(cs + (low ? i : i - half)), s = *reinterpret_cast<const float4*>(cs + half + (low ? i : i - half));
-    return low ? make_float4(a.x * c.x - o.x * s.x, a.y * c.y - o.y * s.y, a.z * c.z - o.z * s.z, a.w * c.w - o.w * s.w)
-               : make_float4(a.x * c.x + o.x * s.x, a.y * c.y + o.y * s.y, a.z * c.z + o.z * s.z, a.w * c.w + o.w * s.w);
+    return low ? make_float4(turn_low(a.x, o.x, c.x, s.x), turn_low(a.y, o.y, c.y, s.y), turn_low(a.z, o.z, c.z, s.z), turn_low(a.w, o.w, c.w, s.w))
+               : make_float4(turn_high(a.x, o.x, c.x, s.x), turn_high(a.y, o.y, c.y, s.y), turn_high(a.z, o.z, c.z, s.z), turn_high(a.w, o.w, c.w, s.w));
   };
   const int lat = p.kv_rank + p.rot_dim, d4 = p.dim >> 2, per = d4 + (p.rot_dim >> 2);
   const int64_t d0 = (int64_t)p.heads * p.head_pitch;
   const bool own = p.dkv_norm && 4 * tid < p.kv_rank;
   float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   if (own) x = part_sum4(src + d0 + 4 * tid, p.splits, p.split_stride);
+  *reinterpret_cast<float4*>(latent + 4 * tid) = x;
 #pragma unroll 2
   for (int i = tid; i < p.heads * per; i += kPrepareThreads) {
     const int h = i / per, c = i - h * per;
@@ -130,7 +138,10 @@ latent_prepare_vec_kernel(const PrepareParams p, T* __restrict__ qn, T* __restri
       q_lat[(t * p.heads + h) * p.lat_pitch + lat + i - h * (p.lat_pitch - lat)] = from_f32<T>(0.0f);
     }
   if (!p.dkv_norm) return;
-  const float ss = block_sum(fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w))), scratch);
+  __syncthreads();
+  float ss = 0.0f;
+  for (int i = tid; i < p.kv_rank; i += kPrepareThreads) ss = fmaf(latent[i], latent[i], ss);
+  ss = block_sum(ss, scratch);
   const float inv = 1.0f / sqrtf(ss / (float)p.kv_rank + p.eps);
   const int64_t loc = p.out_loc[t];
   if (loc < 0 || loc >= p.cache_rows) return;

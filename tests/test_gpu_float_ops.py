@@ -437,6 +437,27 @@ def test_latent_attention_prompts_portions_and_decode(dtype, simple, heads, rank
         close(out[..., :rank], want, dtype, 3e-5, 1.5e-2)
 
 
+@pytest.mark.parametrize("H,dim,rot,dims,rank,parts", [(16, 64, 32, 32, 256, 1), (3, 20, 16, 8, 260, 2), (2, 8, 8, 8, 1024, 3)])
+def test_latent_prepare_forms_give_the_same_bits(H, dim, rot, dims, rank, parts):
+    """The form for four columns at a time against the one for single columns (which a table of angles off 16-byte boundaries
+    selects), in 32 bits, where every rounding shows."""
+    from mini_sgl_integer_b200.layers.rotary_float import rotary_table
+    from mini_sgl_integer_b200.models.config import RotarySpec, YarnScaling
+    T, sc = 300, ROT["scaling"]
+    g = torch.Generator(device="cuda").manual_seed(rank)
+    rope = rotary_table(RotarySpec(dims, 5000.0, YarnScaling(sc["factor"], sc["original"], sc["fast"], sc["slow"])), T, "cuda")
+    off = torch.empty(rope.numel() + 1, device="cuda")[1:].view(rope.shape).copy_(rope)
+    qd = torch.randn((parts, T, H * (dim + rot) + rank + rot), device="cuda", generator=g)
+    w, at = torch.randn(rank, device="cuda", generator=g), i32(range(T))
+    outs = []
+    for table in (rope, off):
+        qn, ql = torch.zeros(T, H, fo.pad8(dim), device="cuda"), torch.zeros(T, H, fo.pad8(rank + rot), device="cuda")
+        cache = torch.zeros(19, 16, fo.pad8(rank + rot), device="cuda")
+        fo.latent_prepare(qd, at, at, table, w, 1e-5, qn, ql, cache, H, dim, rot, rank)
+        outs.append((qn, ql, cache))
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
 @pytest.mark.parametrize("heads,rank,rot,window", [(16, 256, 32, 0), (1, 36, 0, 7), (33, 64, 20, 40), (12, 300, 24, 0), (16, 512, 64, 100), (3, 700, 96, 0)])
 def test_latent_attention_32_bit_prompts(heads, rank, rot, window):
     """One and two pieces in flight, one to three pieces of output columns, rows that do not fill a tile; against 64 bits and
