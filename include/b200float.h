@@ -42,7 +42,8 @@ B200_API int b200f_gemm_status(int* out_host, int reset);    /* synchronises wit
 
 /* ---- 32-bit linear whose sums may be taken in any order (b200f_gemm gives each output one chain over K, the same bits in every
  * batch).  Up to eight rows on the fp32 units, more on the tensor cores: operands as sums of three bf16 numbers, fp32 accumulation
- * restarted every 64 of K; closer to the exact result than a chain of fp32 fmas.  ws: b200f_gemm_f32_ws_bytes bytes, 128-byte
+ * restarted every 64 of K; closer to the exact result than a chain of fp32 fmas.  Outputs that those parts cannot give (not finite,
+ * or of operands or results below 2^-110), and only these, are computed as b200f_gemm does.  ws: b200f_gemm_f32_ws_bytes bytes, 128-byte
  * aligned (NULL for 0); negative where b200f_gemm is to be used instead. */
 B200_API int64_t b200f_gemm_f32_ws_bytes(int64_t m, int64_t n, int64_t k, int64_t batch);
 B200_API int b200f_gemm_f32(const float* x, const float* w, float* out, int64_t m, int64_t n, int64_t k, int64_t batch, int64_t x_pitch,

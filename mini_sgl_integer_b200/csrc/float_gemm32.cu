@@ -17,8 +17,11 @@
 // What bounds it: six bf16 products are a sixth of the bf16 peak, four times what the fp32 units can do; below that, the
 // operands' way from L2 (96 KB for 24 instructions of 128 x 128 x 16).
 //
-// Infinities and NaN do not survive the split (inf = inf + NaN + NaN): split_parts_kernel reports whether it met any, and the
-// linear is then computed value by value in the order of the plain kernel.
+// What the parts cannot give is computed again on the fp32 units, as the chain over K of float_gemm.cu: outputs that are not finite (an
+// operand that is not, inf = inf + NaN + NaN, or finite products of leading parts above the largest number) or almost
+// subnormal, and the rows and columns of operands below 2^-110, whose lowest part bf16 cannot hold.  Each output is judged by
+// itself, so such a row leaves the other rows' bits alone; a block of 64 x 64 outputs that holds one costs a CTA what it costs
+// gemm_f32_kernel.  1400 x 4608 x 1024: 87 us, 239 with one NaN, 787 with nothing else (gemm_f32_kernel 419).
 #include "float_common.cuh"
 #include "umma.cuh"
 
@@ -31,12 +34,15 @@ constexpr int kXStages = 2;
 constexpr int kXEpiWarps = 8;
 constexpr int kXThreads = 64 + 32 * kXEpiWarps;
 constexpr int kXPitch = 20;                         // words per staged row of 16: 16-byte aligned, conflict-free both ways
-constexpr int kXSplitBlocks = 592;                  // CTAs of the splitting kernel at most, one report each
+constexpr unsigned kXTiny = (127u - 110u) << 23;    // 2^-110: from here on three bf16 numbers hold all 24 bits
+constexpr unsigned kXInf = 0x7f800000u;
 
 struct X3Operand {
   const float* src;
   int64_t rows, pitch, bstride;                     // rows of one batch
   bf16* dst;                                        // [3][batch][rows][dst_pitch]
+  unsigned* odd;                                    // [batch][rows] the parts of one of the row's values do not add up to it; a byte for each
+                                                    // of `pieces` warps that split the row
   int vec;                                          // rows start on 16-byte boundaries
 };
 struct X3Params {
@@ -47,9 +53,15 @@ struct X3Params {
   int act;
   float act_a, act_b;
   int vec;
-  unsigned* met;                                    // [split_blocks] a CTA of the splitting kernel met an infinity or a NaN
-  int split_blocks;
+  int pieces;                                       // 1 or 4: few rows are split by four warps each
+  unsigned odd_mask;
 };
+
+// Neither zero nor within [2^-110, infinity).
+__device__ __forceinline__ bool odd_value(float v) {
+  const unsigned u = __float_as_uint(v) & 0x7fffffffu;
+  return u != 0u && u - kXTiny >= kXInf - kXTiny;
+}
 
 // Three bf16 numbers whose sum is v to 24 bits.  (Rounding up to infinity: the truncated number instead.)
 __device__ __forceinline__ void split3(float v, unsigned short (&o)[3]) {
@@ -62,42 +74,47 @@ __device__ __forceinline__ void split3(float v, unsigned short (&o)[3]) {
   }
 }
 
+// A warp per row; four for each of few rows, half a warp for short ones.
 __global__ void __launch_bounds__(256)
 split_parts_kernel(const X3Params p) {
   pdl_launch_dependents();
   pdl_wait();
-  const int quads = (p.K + 3) / 4;
-  const int64_t nx = (int64_t)p.batch * p.x.rows * quads, total = nx + (int64_t)p.batch * p.w.rows * quads;
-  bool met = false;
-  for (int64_t i = blockIdx.x * 256ll + threadIdx.x; i < total; i += gridDim.x * 256ll) {
-    const bool is_w = i >= nx;
-    const X3Operand& o = is_w ? p.w : p.x;
-    const int64_t j = is_w ? i - nx : i, r = j / quads, b = r / o.rows;
-    const int k = (int)(j - r * quads) * 4;
-    const float* src = o.src + b * o.bstride + (r - b * o.rows) * o.pitch + k;
-    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (o.vec && k + 3 < p.K) {
-      const float4 f = __ldg(reinterpret_cast<const float4*>(src));
-      v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-    } else {
+  const int quads = (p.K + 3) / 4, lanes = quads <= 16 ? 16 : 32, per = 256 / lanes, lane = threadIdx.x & (lanes - 1);
+  const int64_t nx = (int64_t)p.batch * p.x.rows, total = (nx + (int64_t)p.batch * p.w.rows) * p.pieces;
+  for (int64_t base = (int64_t)blockIdx.x * per; base < total; base += (int64_t)gridDim.x * per) {
+    const int64_t at = min(base + threadIdx.x / lanes, total - 1);      // (behind the end: the last one again, to the same values)
+    const int64_t i = p.pieces == 1 ? at : at >> 2;
+    const int piece = p.pieces == 1 ? 0 : (int)(at & 3);
+    const X3Operand& o = i >= nx ? p.w : p.x;
+    const int64_t r = i >= nx ? i - nx : i, b = r / o.rows, plane = (int64_t)p.batch * o.rows * p.kp;
+    const float* src = o.src + b * o.bstride + (r - b * o.rows) * o.pitch;
+    bf16* dst = o.dst + r * p.kp;
+    bool odd = false;
+#pragma unroll 4
+    for (int q = lane + lanes * piece; q < quads; q += lanes * p.pieces) {
+      const int k = 4 * q;
+      float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      if (o.vec && k + 3 < p.K) {
+        const float4 f = __ldg(reinterpret_cast<const float4*>(src + k));
+        v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+      } else {
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if (k + c < p.K) v[c] = __ldg(src + c);
+        for (int c = 0; c < 4; ++c)
+          if (k + c < p.K) v[c] = __ldg(src + k + c);
+      }
+      unsigned short part[4][3];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        odd |= odd_value(v[c]);
+        split3(v[c], part[c]);
+      }
+#pragma unroll
+      for (int s = 0; s < 3; ++s)                   // (kp is a multiple of 8: the quad fits its row)
+        *reinterpret_cast<uint2*>(dst + s * plane + k) = make_uint2(part[0][s] | ((unsigned)part[1][s] << 16), part[2][s] | ((unsigned)part[3][s] << 16));
     }
-    unsigned short part[4][3];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      met |= (__float_as_uint(v[c]) & 0x7f800000u) == 0x7f800000u;
-      split3(v[c], part[c]);
-    }
-    const int64_t plane = (int64_t)p.batch * o.rows * p.kp;
-#pragma unroll
-    for (int s = 0; s < 3; ++s)                     // (kp is a multiple of 8: the quad fits its row)
-      *reinterpret_cast<uint2*>(o.dst + s * plane + r * p.kp + k) =
-          make_uint2(part[0][s] | ((unsigned)part[1][s] << 16), part[2][s] | ((unsigned)part[3][s] << 16));
+    const unsigned votes = __ballot_sync(FULL_MASK, odd) >> (threadIdx.x & 31 & ~(lanes - 1)) & (lanes == 16 ? 0xffffu : ~0u);
+    if (lane == 0) reinterpret_cast<unsigned char*>(o.odd + r)[piece] = votes != 0;
   }
-  const int any = __syncthreads_or(met);
-  if (threadIdx.x == 0) p.met[blockIdx.x] = any ? 1u : 0u;
 }
 
 __device__ __forceinline__ void umma_bf16x3(unsigned tmem_d, uint64_t desc_a, uint64_t desc_b, unsigned idesc, unsigned accumulate) {
@@ -109,14 +126,84 @@ __device__ __forceinline__ void umma_bf16x3(unsigned tmem_d, uint64_t desc_a, ui
       : "memory");
 }
 
+__device__ __forceinline__ void epilogue_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kXEpiWarps) : "memory"); }
+__device__ __forceinline__ bool epilogue_any(bool v) {
+  unsigned r;
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 q, %1, 0;\nbar.red.or.pred p, 1, %2, q;\nselp.u32 %0, 1, 0, p;\n}"
+               : "=r"(r) : "r"((unsigned)v), "n"(32 * kXEpiWarps) : "memory");
+  return r != 0;
+}
+
+// The epilogue warps go over this CTA's tiles once more, 64 x 64 outputs at a time with 4 x 4 per thread as in gemm_f32_kernel, and
+// replace the outputs that the parts could not give.
+__device__ __forceinline__ void chain_again(const X3Params& p, int* smem, int et, int num_tiles, int m_tiles, int n_tiles) {
+  float(*xs)[68] = reinterpret_cast<float(*)[68]>(smem), (*ws)[68] = xs + 16;
+  static_assert(2 * 16 * 68 <= kXEpiWarps * 32 * kXPitch, "two tiles of 16 x 64 in the staging area");
+  const int tx = et & 15, ty = et >> 4;
+  for (int block = 4 * blockIdx.x; block < 4 * num_tiles; block = (block & 3) < 3 ? block + 1 : block - 3 + 4 * (int)gridDim.x) {
+    const int tile = block >> 2, m_blk = tile % m_tiles, r = tile / m_tiles, n_blk = r % n_tiles, b = r / n_tiles;
+    const int m0 = m_blk * kXM + 64 * (block & 1), n0 = n_blk * kXN + 32 * (block & 2);
+    if (m0 >= p.M || n0 >= p.N) continue;            // (the same for all threads)
+    float* out = p.out + (int64_t)b * p.out_bstride;
+    unsigned need = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
+        if (m < p.M && n < p.N && (((p.x.odd[(int64_t)b * p.M + m] | p.w.odd[(int64_t)b * p.N + n]) & p.odd_mask) || odd_value(out[(int64_t)m * p.out_pitch + n])))
+          need |= 1u << (4 * i + j);
+      }
+    if (!epilogue_any(need != 0)) continue;
+    // a thread fetches four columns of one row of either operand, a step ahead
+    const int fr = et >> 2, fk = 4 * (et & 3);
+    auto fetch = [&](const X3Operand& o, int row, int k) {
+      float4 f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (row >= o.rows || k >= p.K) return f;
+      const float* src = o.src + (int64_t)b * o.bstride + row * o.pitch + k;
+      if (o.vec && k + 3 < p.K) return __ldg(reinterpret_cast<const float4*>(src));
+      f.x = src[0];
+      if (k + 1 < p.K) f.y = src[1];
+      if (k + 2 < p.K) f.z = src[2];
+      if (k + 3 < p.K) f.w = src[3];
+      return f;
+    };
+    float4 fx = fetch(p.x, m0 + fr, fk), fw = fetch(p.w, n0 + fr, fk);
+    float acc[4][4] = {};
+    for (int k0 = 0; k0 < p.K; k0 += 16) {
+      xs[fk][fr] = fx.x; xs[fk + 1][fr] = fx.y; xs[fk + 2][fr] = fx.z; xs[fk + 3][fr] = fx.w;
+      ws[fk][fr] = fw.x; ws[fk + 1][fr] = fw.y; ws[fk + 2][fr] = fw.z; ws[fk + 3][fr] = fw.w;
+      epilogue_barrier();
+      fx = fetch(p.x, m0 + fr, k0 + 16 + fk);
+      fw = fetch(p.w, n0 + fr, k0 + 16 + fk);
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        const float4 a = *reinterpret_cast<const float4*>(&xs[k][ty * 4]), c = *reinterpret_cast<const float4*>(&ws[k][tx * 4]);
+        const float av[4] = {a.x, a.y, a.z, a.w}, cv[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], cv[j], acc[i][j]);
+      }
+      epilogue_barrier();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if ((need >> (4 * i + j)) & 1u)
+          out[(int64_t)(m0 + ty * 4 + i) * p.out_pitch + n0 + tx * 4 + j] = p.act == B200F_ACT_XIELU ? xielu_f32(acc[i][j], p.act_a, p.act_b) : acc[i][j];
+  }
+}
+
 __global__ void __launch_bounds__(kXThreads, 1)
-gemm_f32x3_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const X3Params p) {
+gemm_f32x3_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ X3Params p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + kXStages * kXStageBytes);   // full[S], empty[S], tfull[2], tempty[2]
   unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * kXStages + 4);
   int* stage_all = reinterpret_cast<int*>(tmem_slot + 4);
-  __shared__ int plain_s;
+  __shared__ int again_s;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_kb = (p.K + kXK - 1) / kXK;
@@ -135,7 +222,7 @@ gemm_f32x3_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       mbar_init(tempty0 + 8 * s, kXEpiWarps);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    plain_s = 0;
+    again_s = 0;
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2 * kXN) : "memory");
@@ -196,15 +283,14 @@ gemm_f32x3_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   } else {
     const int q = warp & 3, half = (warp - 2) >> 2, et = threadIdx.x - 64;
     int* stage = stage_all + (warp - 2) * (32 * kXPitch);
-    unsigned met = 0;
-    for (int i = et; i < p.split_blocks; i += 32 * kXEpiWarps) met |= p.met[i];
-    if (met) plain_s = 1;
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * kXEpiWarps) : "memory");
-    const bool plain = plain_s != 0;
     unsigned lc = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
       const int m_blk = tile % m_tiles, r = tile / m_tiles, n_blk = r % n_tiles, b = r / n_tiles;
+      const int row0 = m_blk * kXM + q * 32, col0 = n_blk * kXN + half * 64;
+      const unsigned *ox = p.x.odd + (int64_t)b * p.M, *ow = p.w.odd + (int64_t)b * p.N;
+      const unsigned odd = (row0 + lane < p.M ? ox[row0 + lane] : 0u) | (col0 + lane < p.N ? ow[col0 + lane] : 0u) |
+                           (col0 + 32 + lane < p.N ? ow[col0 + 32 + lane] : 0u);
       float acc[2][32];
 #pragma unroll
       for (int h = 0; h < 2; ++h)
@@ -226,25 +312,18 @@ gemm_f32x3_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         __syncwarp();
         if (lane == 0) mbar_arrive(tempty0 + 8 * slot);
       }
-      const int row0 = m_blk * kXM + q * 32, col0 = n_blk * kXN + half * 64;
-      if (plain && row0 + lane < p.M) {              // an operand is not finite
-        const float* xr = p.x.src + (int64_t)b * p.x.bstride + (int64_t)(row0 + lane) * p.x.pitch;
-#pragma unroll 1
-        for (int j = 0; j < 64 && col0 + j < p.N; ++j) {
-          const float* wr = p.w.src + (int64_t)b * p.w.bstride + (int64_t)(col0 + j) * p.w.pitch;
-          float s = 0.0f;
-          for (int k = 0; k < p.K; ++k) s = fmaf(xr[k], wr[k], s);
-#pragma unroll
-          for (int i = 0; i < 64; ++i)
-            if (i == j) acc[i >> 5][i & 31] = s;
-        }
-      }
       if (p.act == B200F_ACT_XIELU) {
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
           for (int j = 0; j < 32; ++j) acc[h][j] = xielu_f32(acc[h][j], p.act_a, p.act_b);
       }
+      bool again = (odd & p.odd_mask) != 0;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int j = 0; j < 32; ++j) again |= odd_value(acc[h][j]);
+      if (again) again_s = 1;
       float* out = p.out + (int64_t)b * p.out_bstride;
       const int rr = lane >> 2, cc = (lane & 3) * 4;
 #pragma unroll
@@ -272,6 +351,8 @@ gemm_f32x3_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         }
       }
     }
+    epilogue_barrier();
+    if (again_s) chain_again(p, stage_all, et, num_tiles, m_tiles, n_tiles);      // behind all tiles: no wait of the pipeline spans it
   }
   tcgen05_fence_before();
   __syncthreads();
@@ -379,7 +460,7 @@ extern "C" int64_t b200f_gemm_f32_ws_bytes(int64_t m, int64_t n, int64_t k, int6
   // few CTAs (m = 16, n = 4608: 70 us against 51; n = 1024, k = 4096: 265 against 90) or too many products (m = 1400, n = 4608: 406
   // against 92).
   if (m <= 64 && batch * ((n + 63) / 64) >= 2 * sm_count()) return -1;
-  return x3_bytes(m, k, batch) + x3_bytes(n, k, batch) + kXSplitBlocks * 4;
+  return x3_bytes(m, k, batch) + x3_bytes(n, k, batch) + 4 * batch * (m + n);
 }
 
 extern "C" int b200f_gemm_f32(const float* x, const float* w, float* out, int64_t m, int64_t n, int64_t k, int64_t batch, int64_t x_pitch,
@@ -397,20 +478,23 @@ extern "C" int b200f_gemm_f32(const float* x, const float* w, float* out, int64_
   unsigned char* at = (unsigned char*)ws;
   X3Params p;
   auto rows16 = [&](const float* base, int64_t pitch, int64_t bstride) { return aligned16(base) && pitch % 4 == 0 && (batch == 1 || bstride % 4 == 0); };
-  p.x = {x, m, x_pitch, x_bstride, (bf16*)at, rows16(x, x_pitch, x_bstride)};
+  p.x = {x, m, x_pitch, x_bstride, (bf16*)at, nullptr, rows16(x, x_pitch, x_bstride)};
   at += x3_bytes(m, k, batch);
-  p.w = {w, n, w_pitch, w_bstride, (bf16*)at, rows16(w, w_pitch, w_bstride)};
+  p.w = {w, n, w_pitch, w_bstride, (bf16*)at, nullptr, rows16(w, w_pitch, w_bstride)};
   at += x3_bytes(n, k, batch);
-  p.met = (unsigned*)at;
+  p.x.odd = (unsigned*)at;
+  p.w.odd = p.x.odd + batch * m;
   p.out = out; p.M = (int)m; p.N = (int)n; p.K = (int)k; p.batch = (int)batch; p.kp = (int)x3_pitch(k);
   p.out_pitch = out_pitch; p.out_bstride = out_bstride; p.act = act; p.act_a = act_a; p.act_b = act_b;
   p.vec = rows16(out, out_pitch, out_bstride);
   if (need == 0) return m == 1 ? launch_gemv<1>(p, st) : m == 2 ? launch_gemv<2>(p, st) : m <= 4 ? launch_gemv<4>(p, st) : launch_gemv<8>(p, st);
-  const int64_t quads = batch * (m + n) * ((k + 3) / 4), blocks = (quads + 255) / 256;
-  p.split_blocks = (int)(blocks < kXSplitBlocks ? blocks : kXSplitBlocks);
+  // a few thousand warps keep the memory busy; below that, rows of several hundred values are worth four
+  p.pieces = batch * (m + n) <= 16 * sm_count() && k > 256 ? 4 : 1;
+  p.odd_mask = p.pieces == 4 ? ~0u : 0xffu;
+  const int64_t blocks = (batch * (m + n) * p.pieces + (k <= 64 ? 15 : 7)) / (k <= 64 ? 16 : 8), most = 16 * sm_count();
   CUtensorMap mx, mw;
   B200_REQUIRE(x3_map(&mx, p.x.dst, m, k, p.kp, batch) && x3_map(&mw, p.w.dst, n, k, p.kp, batch), B200_E_CUDA, "gemm_f32: cuTensorMapEncodeTiled failed");
-  launch_pdl(split_parts_kernel, dim3(p.split_blocks), dim3(256), 0, st, p);
+  launch_pdl(split_parts_kernel, dim3((unsigned)(blocks < most ? blocks : most)), dim3(256), 0, st, p);
   if (const int rc = check_launch("gemm_f32 (parts)")) return rc;
   constexpr size_t smem = (size_t)kXStages * kXStageBytes + 1024 + (2 * kXStages + 4) * 8 + 16 + kXEpiWarps * 32 * kXPitch * 4;
   static_assert(smem <= 227 * 1024, "shared memory budget");

@@ -218,6 +218,36 @@ def test_sublayer_end(dtype, width, parts):
         close(xt, S.rms_norm(want, fw, eps), dtype)
 
 
+@pytest.mark.parametrize("m,n,k", [(9, 40, 24), (130, 140, 70), (1300, 2000, 600)])
+def test_linear_f32_outside_the_range_of_three_parts(m, n, k):
+    """What the sum of three bf16 numbers cannot hold, in one row or column of a linear of one tile, of ragged ones, and of more
+    tiles than SMs: values that are not finite, finite products of the largest, sums that overflow, operands and outputs next to
+    the subnormals.  These outputs have the bits of the chain over k, all others those that they have without such values."""
+    g = torch.Generator(device="cuda").manual_seed(m)
+    x, w, at = torch.randn((m, k), device="cuda", generator=g), torch.randn((n, k), device="cuda", generator=g), torch.arange(k, device="cuda")
+    act = dict(act=fo.ACT_XIELU, act_a=0.7, act_b=1.1)
+    inner = (slice(6, m - 1), slice(4, n - 1))
+    plain, plain_act = fo.linear(x, w)[inner], fo.linear(x, w, **act)[inner]
+    assert not torch.equal(plain, fo.linear(x, w, chained=True)[inner])
+    one = lambda c, v: torch.where(at == c, v, 0.0)
+    x[0] *= 2.0 ** -112
+    x[1, 7] = 2.0 ** -126
+    x[2] = one(3, float("inf"))
+    x[3, 5], x[m - 1, k - 1] = float("-inf"), float("nan")
+    x[4] = one(2, 1.998 * 2.0 ** 64)
+    x[5] = torch.where(x[5] > 0, 1e30, 0.998e30)
+    w[1], w[2], w[3] = one(2, 2.0 ** 63), 1e30, -1.001e30
+    w[n - 1] *= 2.0 ** -118
+    for args, untouched in (({}, plain), (act, plain_act)):
+        got, chain = fo.linear(x, w, **args), fo.linear(x, w, chained=True, **args)
+        same = (got == chain) | (torch.isnan(got) & torch.isnan(chain))
+        assert bool(same[[0, 1, 2, 3, m - 1]].all()) and bool(same[:, n - 1].all()) and bool(same[4:6, 1:4].all())
+        assert torch.equal(got[inner], untouched)
+        assert bool(torch.isnan(got[m - 1]).all()) and bool(torch.isinf(got[5, 2])) and (args or bool(torch.isfinite(got[4, 1])))
+    assert torch.equal(fo.linear(x * 2.0 ** -60, w * 2.0 ** -60)[inner], fo.linear(x * 2.0 ** -60, w * 2.0 ** -60, chained=True)[inner])
+    fo.check_status()
+
+
 @pytest.mark.parametrize("width", [3, 40, 1024, 2048, 1027])
 def test_sublayer_end_of_few_and_many_rows(width):
     """Up to 592 rows request streams, gains and planes in front of the sums: the bits of the form for more rows, for every
