@@ -293,7 +293,7 @@ latent_attn_f32_kernel(const AttnParams p, const float* __restrict__ q_lat, cons
     }
     cp_async_commit();
   };
-  copy_tile(0);
+  if (tiles > 0) copy_tile(0);                     // (a length below the new tokens leaves rows without keys)
   for (int r = warp; r < R; r += 8) {
     const int tok = r < rows ? r / nh : 0;
     const float4* src = reinterpret_cast<const float4*>(q_lat + ((int64_t)(start + tok0 + tok) * p.heads + h0 + (r < rows ? r - tok * nh : 0)) * p.lat_pitch);
@@ -924,7 +924,7 @@ extern "C" int b200f_latent_attn(const void* q_lat, const void* cache, const int
                           ? plan_attn(max_q, heads, kv_rank, rot_dim) : AttnPlan{0, 0, 0, 0, 0, 0};
   // 32-bit prompts: whole float4 columns, up to 768 of them for the output (accumulators), 32 rows and keys in shared memory
   const int D = kv_rank + rot_dim, f32_stages = f32_smem(D, 2) <= 227 * 1024 ? 2 : 1;
-  if (dtype == B200F_F32 && !simple && seq_start && max_q > 1 && D % 4 == 0 && lat_pitch % 4 == 0 && kv_rank <= 768 && aligned16(q_lat) &&
+  if (dtype == B200F_F32 && !simple && seq_start && max_q > 1 && batch <= 65535 && D % 4 == 0 && lat_pitch % 4 == 0 && kv_rank <= 768 && aligned16(q_lat) &&
       aligned16(cache) && f32_smem(D, f32_stages) <= 227 * 1024) {
     p.splits = 1;
     p.heads_per_cta = heads < kF32Rows ? heads : kF32Rows;

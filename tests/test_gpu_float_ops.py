@@ -517,6 +517,24 @@ def test_latent_attention_32_bit_prompts(heads, rank, rot, window):
     assert not bool(torch.isfinite(got[seen]).all(2).any()) and bool(torch.isfinite(got[:t]).all()) and bool(torch.isfinite(got[70:]).all())
 
 
+@pytest.mark.parametrize("window", [0, 5])
+def test_latent_attention_32_bit_prompts_longer_than_their_keys(window):
+    """Lengths below the number of new tokens: the rows in front of the first key have none and give zeros, as in the plain form;
+    whole tiles of them touch no page."""
+    heads, rank, rot, q_lens, kv_lens = 8, 36, 8, [9, 70, 3], [0, 6, 3]
+    g = torch.Generator(device="cuda").manual_seed(window)
+    q = torch.randn((sum(q_lens), heads, fo.pad8(rank + rot)), device="cuda", generator=g)
+    cache = torch.randn((2, 16, fo.pad8(rank + rot)), device="cuda", generator=g)
+    table, starts, sink = i32([[0], [1], [0]]), i32(np.concatenate([[0], np.cumsum(q_lens)])), torch.randn(heads, device="cuda", generator=g)
+    outs = []
+    for simple in (False, True):
+        out = torch.full((sum(q_lens), heads, fo.pad8(rank)), 5.0, device="cuda")
+        fo.latent_attention(q, cache, table, i32(kv_lens), starts, sink, out, rank, rot, window, 0.3, max(q_lens), max(kv_lens), simple=simple)
+        outs.append(out[..., :rank])
+    close(outs[0], host(outs[1]), torch.float32)
+    assert not bool(outs[0][:9].any()) and not bool(outs[0][9:73].any()) and bool(outs[0][73:].any(2).all())
+
+
 @pytest.mark.parametrize("heads,rank,rot", [(8, 64, 16), (40, 128, 32)])
 @pytest.mark.parametrize("splits", [2, 5, 11])
 def test_latent_attention_with_split_keys(heads, rank, rot, splits):
