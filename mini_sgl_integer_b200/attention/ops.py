@@ -140,20 +140,23 @@ def prefill_attention_int8_paged(q8: torch.Tensor, q_mul: torch.Tensor, q_shift:
 
 
 class NewTokens(NamedTuple):
-    """What a step of new tokens needs to know of its q_lens: the row of each sequence's first one, and the longest."""
+    """What a step of new tokens needs to know of them: how many each sequence has (a copy), the row of its first one, the longest
+    and the rows in all."""
 
+    q_lens: torch.Tensor
     q_start: torch.Tensor
     longest: int
+    rows: int
 
 
 def new_tokens(q_lens: torch.Tensor, rows: int) -> NewTokens:
     """Sums q_lens, compares the total with the query rows and reads the longest back from the device, once for all layers
     of a step (a read-back per layer drained the device 36 times in an 8B-shaped step)."""
-    q_lens = q_lens.to(torch.int32).contiguous()
+    q_lens = q_lens.to(torch.int32, copy=True).contiguous()
     total, longest = (int(v) for v in torch.stack((q_lens.sum(), q_lens.max() if q_lens.numel() else q_lens.sum())).tolist())
     if total != rows:
         raise ValueError(f"sum(q_lens)={total} does not match the {rows} query rows")
-    return NewTokens(torch.cumsum(q_lens, 0, dtype=torch.int32) - q_lens, longest)
+    return NewTokens(q_lens, torch.cumsum(q_lens, 0, dtype=torch.int32) - q_lens, longest, rows)
 
 
 def extend_attention_int8_paged(q8: torch.Tensor, q_mul: torch.Tensor, q_shift: torch.Tensor,
@@ -173,19 +176,23 @@ def extend_attention_int8_paged(q8: torch.Tensor, q_mul: torch.Tensor, q_shift: 
     tokens); "cluster" = the decode kernel launched once per query row, "split" = its workspace passes (each row
     re-reads its keys: only for a handful of new tokens per sequence).  All three give the same bits.
 
-    ``new``: `new_tokens(q_lens, tokens)` of the same step, for callers that run many layers on one batch; without it
-    the lengths are summed and read back here, which waits for everything the device has been given so far.
+    ``new``: `new_tokens(q_lens, tokens)` of the same step, for callers that run many layers on one batch; its lengths are
+    those that count then.  Without it they are summed and read back here, which waits for everything the device has been
+    given so far.
     """
     if q8.dtype != torch.int8:
         raise TypeError(f"q8 must be int8, got {q8.dtype}")
     if q8.ndim != 3 or q8.shape[-1] != HEAD_DIM:
         raise ValueError(f"q8 must be [tokens, q_heads, {HEAD_DIM}], got shape {tuple(q8.shape)}")
-    require_cuda(q8, q_mul, q_shift, page_table, kv_lens, q_lens)
     rows, q_heads, _ = q8.shape
+    if new is not None and (new.rows != rows or new.q_lens.shape[0] != kv_lens.shape[0]):
+        raise ValueError(f"new is of {new.q_lens.shape[0]} sequences and {new.rows} rows, not of {kv_lens.shape[0]} and {rows}")
+    require_cuda(q8, q_mul, q_shift, page_table, kv_lens, q_lens)
     q8 = q8.contiguous()
-    q_mul, q_shift, page_table, kv_lens, q_lens = i32(q_mul), i32(q_shift), i32(page_table), i32(kv_lens), i32(q_lens)
+    q_mul, q_shift, page_table, kv_lens = i32(q_mul), i32(q_shift), i32(page_table), i32(kv_lens)
     if new is None:
         new = new_tokens(q_lens, rows)
+    q_lens = new.q_lens
     if impl in ("auto", "tiled"):
         return prefill_attention_int8_paged(q8, q_mul, q_shift, pool, layer_id, page_table, kv_lens, q_lens, max_kv_len,
                                             new.longest, out_q15=out_q15, out_int8=out_int8, q_start=new.q_start)

@@ -141,3 +141,22 @@ def test_context_rules():
     with pytest.raises(RuntimeError, match="No active batch"):
         ctx.batch
     core.set_global_ctx(None)
+
+
+def test_new_tokens_of_another_batch_are_refused():
+    """What the layers of a step share about its new tokens has to be of this batch: the kernels take rows from it unchecked."""
+    from mini_sgl_integer_b200.attention import extend_attention_int8_paged, new_tokens
+    lens = torch.tensor([3, 5], dtype=torch.int32)
+    new = new_tokens(lens, 8)
+    lens[:] = 0                                                     # (a copy was taken)
+    assert new.q_lens.tolist() == [3, 5] and new.q_start.tolist() == [0, 3] and new.longest == 5
+    with pytest.raises(ValueError, match="query rows"):
+        new_tokens(torch.tensor([3, 5]), 9)
+    call = lambda rows, seqs: extend_attention_int8_paged(
+        torch.zeros((rows, 4, 128), dtype=torch.int8), torch.ones((rows, 4)), torch.ones((rows, 4)), None, 0,
+        torch.zeros((seqs, 1)), torch.full((seqs,), 8), torch.full((seqs,), 1), 16, new=new)
+    for rows, seqs in ((7, 2), (9, 2), (8, 1), (8, 3)):
+        with pytest.raises(ValueError, match="new is of 2 sequences and 8 rows"):
+            call(rows, seqs)
+    with pytest.raises(RuntimeError, match="CUDA"):                 # of this batch: on to the device check
+        call(8, 2)
