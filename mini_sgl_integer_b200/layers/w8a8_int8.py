@@ -85,11 +85,11 @@ def int8_gemm_q15(x8: torch.Tensor, x_mul: Optional[torch.Tensor], x_shift: Opti
     m, k = x8.shape
     n = w8.shape[0]
     x8, w8 = x8.contiguous(), w8.contiguous()
-    x_mul, x_shift, w_mul, w_shift = _flat(x_mul), _flat(x_shift), _flat(w_mul), _flat(w_shift)
+    x_mul, x_shift, w_mul, w_shift, x_absmax = _flat(x_mul), _flat(x_shift), _flat(w_mul), _flat(w_shift), _flat(x_absmax)
     out = torch.empty((m, n), dtype=torch.int32, device=x8.device) if want_q15 else None
     acc = torch.empty((m, n), dtype=torch.int32, device=x8.device) if want_acc else None
     if m > 0 and x_absmax is not None:
-        call("b200_gemm_w8a8_absmax", ptr(x8), ptr(w8), ptr(_flat(x_absmax)), ptr(w_mul), ptr(w_shift), ptr(out), ptr(acc),
+        call("b200_gemm_w8a8_absmax", ptr(x8), ptr(w8), ptr(x_absmax), ptr(w_mul), ptr(w_shift), ptr(out), ptr(acc),
              m, n, k, stream())
     elif m > 0:
         call("b200_gemm_w8a8", ptr(x8), ptr(w8), ptr(x_mul), ptr(x_shift), ptr(w_mul), ptr(w_shift), ptr(out),
@@ -150,8 +150,9 @@ class W8A8Int8LinearMethod:
             # decode sizes: split-K parts go into a workspace that is kept zero, which saves the clearing launch
             out = torch.empty((m, n), dtype=torch.int32, device=x8.device)
             require_cuda(x8, layer.weight, absmax, layer.weight_mul, layer.weight_shift)
-            call("b200_gemm_w8a8_absmax_ws", ptr(x8), ptr(layer.weight), ptr(_flat(absmax)), ptr(layer.weight_mul),
-                 ptr(layer.weight_shift), ptr(out), ptr(zero_workspace(x8.device, m, n)), m, n, x8.shape[1], stream())
+            absmax, ws = _flat(absmax), zero_workspace(x8.device, m, n)      # (a converted absmax has to outlive the workspace's allocation)
+            call("b200_gemm_w8a8_absmax_ws", ptr(x8), ptr(layer.weight), ptr(absmax), ptr(layer.weight_mul),
+                 ptr(layer.weight_shift), ptr(out), ptr(ws), m, n, x8.shape[1], stream())
         else:
             out = int8_gemm_q15(x8, None, None, layer.weight, layer.weight_mul, layer.weight_shift, x_absmax=absmax)
         if bias is not None:
@@ -176,9 +177,9 @@ class W8A8Int8LinearMethod:
         m, n2 = x8.shape[0], layer.weight.shape[0]
         out = torch.empty((m, n2 // 2), dtype=torch.int32, device=x8.device)
         if m:
-            call("b200_gemm_gate_up_silu", ptr(x8), ptr(layer.weight), ptr(_flat(absmax)),
-                 ptr(layer.weight_mul), ptr(layer.weight_shift), ptr(out), ptr(zero_workspace(x8.device, m, n2)), m, n2,
-                 x8.shape[1], stream())
+            absmax, ws = _flat(absmax), zero_workspace(x8.device, m, n2)
+            call("b200_gemm_gate_up_silu", ptr(x8), ptr(layer.weight), ptr(absmax), ptr(layer.weight_mul), ptr(layer.weight_shift),
+                 ptr(out), ptr(ws), m, n2, x8.shape[1], stream())
         return out
 
     def apply_pending(self, layer, codes: torch.Tensor, absmax: torch.Tensor) -> PendingLinear:

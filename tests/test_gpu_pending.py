@@ -3,6 +3,8 @@ zero, add + RMSNorm + quant and the q/k/v preparation reading exact accumulators
 materialised path (itself checked against the oracle elsewhere) and of the oracle, and leave the workspace zero."""
 from __future__ import annotations
 
+from types import SimpleNamespace
+
 import numpy as np
 import pytest
 import torch
@@ -157,3 +159,26 @@ def test_gate_up_with_silu_in_the_epilogue(m, inter, k, block):
         np.testing.assert_array_equal(got_absmax.cpu().numpy().reshape(-1), want_absmax.reshape(-1))
     ref = fp.silu_mul_fwht_quant(meth.apply_quantised(layer, d(codes), d(absmax)), block)
     assert torch.equal(ref[0], got_codes) and torch.equal(ref[1], got_scale) and torch.equal(ref[2], got_absmax)
+
+
+@pytest.mark.parametrize("fused", [False, True])
+def test_an_absmax_of_another_type_outlives_the_first_workspace(fused):
+    """The first linear of a width allocates its workspace, and clears it, behind the conversion of the absmax to int32: the
+    converted copy must not have been given back by then."""
+    from mini_sgl_integer_b200.kernel import pending
+    from mini_sgl_integer_b200.layers.w8a8_int8 import W8A8Int8LinearMethod
+    g = torch.Generator(device="cuda").manual_seed(3)
+    n, k, method = 256, 256, W8A8Int8LinearMethod()
+    layer = SimpleNamespace(weight=torch.randint(-127, 128, (n, k), dtype=torch.int8, device="cuda", generator=g),
+                            weight_scale=torch.full((n, 1), 0.01, device="cuda"), input_scale=None)
+    method.process_weights_after_loading(layer)
+    codes = torch.randint(-127, 128, (3, k), dtype=torch.int8, device="cuda", generator=g)
+    absmax = torch.tensor([70000, 90000, 65536], dtype=torch.int32, device="cuda")
+    run = method.apply_gate_up_silu if fused else method.apply_quantised
+    want, wide = run(layer, codes, absmax), absmax.to(torch.int64)
+    for key in [key for key in pending._workspaces if key[1] == n]:
+        del pending._workspaces[key]
+    held = [torch.empty(128, dtype=torch.int32, device="cuda")]      # no gap of the copy's size is left, and behind it there is room
+    while held[-1].data_ptr() % (2 << 20) and len(held) < 20000:
+        held.append(torch.empty(128, dtype=torch.int32, device="cuda"))
+    assert torch.equal(run(layer, codes, wide), want)
