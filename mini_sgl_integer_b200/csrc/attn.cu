@@ -228,6 +228,7 @@ constexpr int kDecodeWarps = 8;
 constexpr int kDecodeThreads = kDecodeWarps * 32;
 static_assert(kDecodeThreads >= kD, "the output stage maps one thread to one d");
 constexpr int kVPrefetchPages = 64;         // V pages per CTA requested into L2 during the exponential pass
+constexpr int kAlonePages = 16;                      // rows of up to 256 keys are one CTA's work
 constexpr int kRingSlot = kSlotBytes + 384; // a pair of pages plus their two scale blocks (2 x 160 B), 128-byte granular
 // Both contractions run on the integer tensor-core MMA with the long dimension on M:
 //   dots^T [16 keys x 8 heads] = K page [16 x 128] . Q^T [128 x 8]        (4 k-steps of 32 d)
@@ -316,7 +317,10 @@ attn_decode_kernel(const DecodeParams p) {
   const int L_all = max(0, min(p.kv_lens[seq], p.max_kv_len));
   const int L = p.row_limit ? max(0, min(p.row_limit[b], L_all)) : L_all;
   const int n_pages = (L + kPage - 1) / kPage;
-  const int Ce = C;   // CTAs that work on this row
+  // CTAs that work on this row: a short one is done sooner by one CTA than by several that wait for each other (below), and the launch
+  // only knows a bound of the lengths
+  const int Ce = n_pages <= kAlonePages && n_pages * kPage <= S ? 1 : C;
+  if (rank >= Ce) return;
   // a CTA on its own needs no cluster barrier (and the plain one is cheaper)
   auto row_sync = [&]() { if (Ce > 1) cluster.sync(); else __syncthreads(); };
   const int ppc = (n_pages + Ce - 1) / Ce;               // pages per CTA
@@ -893,8 +897,11 @@ static int attn_common(const int8_t* q, const int32_t* q_mul, const int32_t* q_s
   // two CTAs share an SM - with two ring slots per warp if that still fits, else one; longer contexts take the
   // smallest cluster whose slices fit at all (fewer CTAs beat deeper rings in every measurement).  Fewer rows are latency: a
   // row's CTAs double while no more than 256 of them are resident and each keeps four pages (eight KV heads, one row of 777 keys:
-  // 13.6 us with one CTA, 9.3 with eight; 8 rows: 16.0, 11.8 with four, 20.8 with eight; 16 rows of 500 keys: 12.8, 12.2 with two;
-  // 37 rows x 4 KV heads of 900 keys: 16.0, 17.4 with two; one row of 100 keys: 8.3, 9.1 with two).
+  // 12.9 us with one CTA, 8.7 with eight; 8 rows: 14.6, 11.4 with four, 19.7 with eight; 16 rows of 500 keys: 12.8, 12.2 with two;
+  // 37 rows x 4 KV heads of 900 keys: 16.0, 17.4 with two).  Up to kAlonePages one CTA is faster (one row of 200 keys: 7.9 us, 8.5
+  // with two or more; 8 rows: 8.8, 9.7; 400 keys: 9.6, 8.4 with four, and 10.5, 9.9): such bounds stay at one, and such rows
+  // under a larger bound are left to the first CTA of their cluster (one row of 100 keys under 4096: 7.7 us, 8.5 with all eight; 8 rows:
+  // 8.8, 9.6).
   const int G_static = 1536 + G * kD * 4 + 1024;   // the kernel's static shared arrays plus the per-CTA reserve
   const size_t two_per_sm = (size_t)(233472 / 2 - G_static);
   auto fits2 = [&](int c, int st) { return decode_smem_bytes(G, slice_keys(c), st) <= two_per_sm; };
@@ -902,7 +909,7 @@ static int attn_common(const int8_t* q, const int32_t* q_mul, const int32_t* q_s
   if (cluster == 0) {
     cluster = 1;
     while (cluster < 8 && !fits2(cluster, 1)) cluster *= 2;   // fewest CTAs per row first, ring depth second
-    while (cluster < 8 && (int64_t)batch * kv_heads * cluster * 2 <= 256 && max_pages / (2 * cluster) >= 4) cluster *= 2;
+    while (cluster < 8 && max_pages > kAlonePages && (int64_t)batch * kv_heads * cluster * 2 <= 256 && max_pages / (2 * cluster) >= 4) cluster *= 2;
     stages = fits2(cluster, 2) ? 2 : 1;
   } else {
     B200_REQUIRE(cluster == 1 || cluster == 2 || cluster == 4 || cluster == 8, B200_E_UNSUPPORTED,

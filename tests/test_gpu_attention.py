@@ -256,6 +256,23 @@ def test_tiled_prefill_vs_oracle(q_heads, kv_heads):
     eq(run_extend(case, pool, 512, cluster=1, impl="cluster").cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("cluster", [0, 2, 4, 8])
+def test_short_rows_under_a_large_bound_are_one_ctas_work(cluster):
+    """Around 256 keys, up to which the first CTA of a row's cluster works alone, beside longer rows; and rows that see few of
+    their sequence's many keys, whose V scales all count."""
+    lens = [1, 16, 17, 255, 256, 257, 272, 600]
+    case = make_case(5, lens, 16, 4, 160)
+    pool = device_pool(case, 160, 4)
+    want = oracle_decode(case)
+    for bound in (600, 2048):
+        eq(run_decode(case, pool, bound, cluster, impl="cluster").cpu().numpy(), want)
+    kv_lens, q_lens = [600, 290, 40], [30, 285, 40]
+    case = _extend_case(6, kv_lens, q_lens, 8, 2, 100)
+    pool = device_pool(case, 100, 2)
+    want = oattn.paged_attention(case["q8"], case["qm"], case["qs"], case["pool"], case["tables"], kv_lens, q_lens)
+    eq(run_extend(case, pool, 640, cluster, impl="cluster").cpu().numpy(), want)
+
+
 @pytest.mark.parametrize("shift,extreme", [(21, True), (22, True), (23, False), (33, False), (62, False), (63, False)])
 @pytest.mark.parametrize("q_heads", [1, 4])
 def test_tiled_prefill_at_the_limits_of_the_plain_scores(shift, extreme, q_heads):
