@@ -1010,13 +1010,14 @@ static int launch_gemm_2sm_ws(const CUtensorMap& mw, const CUtensorMap& mx, cons
 // Token tiles and parts of K of a prompt whose 256 x 256 tiles would leave CTA pairs idle; returns the parts.
 // A tile costs about (256 weight rows + its tokens) per k-block, what it moves into shared memory, so with whole-K
 // tiles the narrowest tokens tiles that still run at once are the best, down to 96 tokens (333 x 6144 x 4096: 30.8 us on single
-// CTAs, 25.6 with three tiles, 30.7 with two).  From 48 k-blocks on, splitting K beats narrowing the tiles although the
+// CTAs, 25.6 with three tiles, 30.7 with two).  From 40 k-blocks on, splitting K beats narrowing the tiles although the
 // parts are added in memory and requantised by another kernel (333 x 4096 x 12288: 65.5 us on single CTAs, 43.0 with four whole-K
-// tiles, 35.8 with two tiles in two parts; 16 and 32 k-blocks: splitting loses or ties).
+// tiles, 35.8 with two tiles in two parts).  Below, it depends on the shape (split, whole): 1000 x 2048 with 16, 32, 36 and 40 k-blocks
+// 16.5, 13.8; 19.0, 18.4; 19.7, 19.6; 20.3, 20.7; 333 x 4096 with 16, 24 and 40 14.3, 13.5; 15.5, 15.9; 18.0, 20.6.
 static int prompt_tiles(GemmParams* p, int w_blocks, int num_kb, int pairs) {
   const int fewest = (p->M + 255) / 256;
   int tiles = fewest, splits = 1;
-  if (num_kb >= 48) splits = pairs / (w_blocks * fewest) < 4 ? pairs / (w_blocks * fewest) : 4;
+  if (num_kb >= 40) splits = pairs / (w_blocks * fewest) < 4 ? pairs / (w_blocks * fewest) : 4;
   while (splits > 1 && (splits - 1) * ((num_kb + splits - 1) / splits) >= num_kb) --splits;     // no empty part
   if (splits <= 1)
     while (w_blocks * (tiles + 1) <= pairs && (p->M + tiles) / (tiles + 1) >= 96) ++tiles;
