@@ -469,6 +469,26 @@ def test_fused_qkv_preparation_equals_the_separate_steps():
         eq(a.meta(0).cpu().numpy(), b.meta(0).cpu().numpy())
 
 
+def test_tiled_prefill_beyond_the_page_list():
+    """Around 131072 keys, from where on a tile reads its page ids where they are: the bits of the row-at-a-time passes.  The pages of
+    a small pool serve all sequences, many times over."""
+    from mini_sgl_integer_b200.attention import Int8PagedKVCache, extend_attention_int8_paged
+    g = torch.Generator(device="cuda").manual_seed(4)
+    kv_lens, q_lens, pages, bound = [131072, 131073, 133000], [17, 3, 40], 97, 133008
+    pool = Int8PagedKVCache(1, 1, 128, pages, "cuda")
+    rnd = lambda lo, hi, shape, dtype: torch.randint(lo, hi, shape, device="cuda", generator=g, dtype=dtype)
+    for codes in (pool.k_cache(0), pool.v_cache(0)):
+        codes.copy_(rnd(-127, 128, codes.shape, torch.int8))
+    meta = pool.meta(0)
+    meta[:, :, :32] = rnd(2**30, 2**31 - 1, (*meta.shape[:2], 32), torch.int32)
+    meta[:, :, 32:36] = rnd(35, 39, (*meta.shape[:2], 16), torch.int8).view(torch.int32)
+    meta[:, :, 36:40] = rnd(36, 40, (*meta.shape[:2], 16), torch.int8).view(torch.int32)
+    T, table = sum(q_lens), rnd(0, pages, (3, bound // 16), torch.int32)
+    q8, qm, qs = rnd(-127, 128, (T, 4, 128), torch.int8), rnd(2**30, 2**31 - 1, (T, 4), torch.int32), rnd(43, 46, (T, 4), torch.int32)
+    run = lambda impl: extend_attention_int8_paged(q8, qm, qs, pool, 0, table, d(np.array(kv_lens, np.int32)), d(np.array(q_lens, np.int32)), bound, impl=impl)
+    eq(run("tiled").cpu().numpy(), run("split").cpu().numpy())
+
+
 @pytest.mark.parametrize("top", [2**21, 2**22 - 1, 2**22, 2**25, 2**31 - 1])
 def test_rotation_at_the_limit_of_the_plain_stages(top):
     """Rows whose largest value lies around 2^22, up to which no stage of the rotation or the butterflies can saturate."""
