@@ -16,12 +16,14 @@
 // walked three times per tile - row maxima, sums of exponentials, then probabilities and PV - and the scores
 // are recomputed each time.  K is therefore read three times and V once per tile, from L2 after the first touch.
 //
-// What bounds it is integer issue: about 35 instructions per score over the three walks.  The general steps (64-bit
-// rounding shifts with saturation, clamps, a table in global memory) took 194, at a quarter of the issue slots; they
+// What bounds it is the latency of dependent integer steps: 115 thread instructions per causal score over the three walks (masked
+// corners of tiles and set-up included), issued on 39 % of the cycles by four warps per scheduler, which wait for fixed
+// latencies and, half as long, for shared memory (128 registers a thread, 8 words of it spilled).  The general steps (64-bit
+// rounding shifts with saturation, clamps, a table in global memory) took 194 instructions on 27 % of the cycles; they
 // remain for scales whose scores could saturate.  Otherwise a score is one wide multiply, one shift and a rounding
 // step, and its exponential one wide multiply-add: with nx = max - score, P = 94548 nx - 1 + 2^32 has the shift in
 // its high word and, read backwards, the table index on top of its low word (tests/test_kernel_identities.py).
-// 15 prompts of 100 .. 1000 tokens, 32 / 8 heads: 0.78 ms a layer, 1.77 ms with the general steps and one warp per 16 rows.
+// 15 prompts of 100 .. 1000 tokens, 32 / 8 heads: 0.80 ms a layer, 1.77 ms with the general steps and one warp per 16 rows.
 #include "attn_common.cuh"
 #include "luts.cuh"
 
