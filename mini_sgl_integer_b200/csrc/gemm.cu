@@ -13,7 +13,7 @@
 // The kernel is persistent (one CTA per SM walks a strided list of tiles) and keeps two accumulator
 // copies in tensor memory, so the epilogue of one tile overlaps the MMAs of the next.
 //
-// Decode sizes (M <= 256 tokens) run "weights-stationary", prompts of few tiles too: the operands swap
+// Decode sizes (M <= 256 tokens) run "weights-stationary" (template flag WS), most prompts of few tiles too: the operands swap
 // roles - 128 weight rows are the UMMA's M side, all the tokens its N side - so every weight byte
 // crosses HBM once and a tile's accumulators are out^T.  A thread then holds one weight channel and 32
 // tokens, and the store of a token's 32 channels by a warp is one contiguous 128 bytes.  When the
@@ -129,11 +129,11 @@ __device__ __forceinline__ void store_chunk(int32_t* stage, int lane, const int 
   }
 }
 
-// Persistent weights-stationary kernel: CTA c computes tiles c, c + gridDim.x, ... of (block of 128 weight rows, part of K),
-// all tokens wide.  The accumulator
+// Persistent kernel: CTA c computes tiles c, c + gridDim.x, ...; weights-stationary of (block of 128 weight rows, part of K), all
+// tokens wide, else of (block of BN weight rows, block of 128 tokens), the tokens inside.  The accumulator
 // lives in tensor memory twice (2 x BN columns): while the epilogue warps drain one copy, the MMA
 // warp already fills the other with the next tile.
-template <int BN, int STAGES>
+template <int BN, int STAGES, bool WS>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  const GemmParams p) {
@@ -145,11 +145,19 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   // barriers: full[S], empty[S], tmem_full[2], tmem_empty[2]
   uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + STAGES * kStageBytes);
   unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * STAGES + 4);
-  int32_t* tok_scale = reinterpret_cast<int32_t*>(tmem_slot + 4);   // [2 slots][mul BN | shift BN] per token
+  int32_t* col_scale = reinterpret_cast<int32_t*>(tmem_slot + 4);   // [2 slots][mul BN | shift BN] per column: token or channel
+  int32_t* stage_all = col_scale + 4 * BN;                          // not WS: [epilogue warps][32][kStagePitch]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_kb = (p.K + kBK - 1) / kBK;
-  const int num_tiles = p.full_blocks + ((p.N + kBM - 1) / kBM - p.full_blocks) * p.splits;
+  const int m_tiles = WS ? 1 : (p.M + kBM - 1) / kBM;
+  const int num_tiles = WS ? p.full_blocks + ((p.N + kBM - 1) / kBM - p.full_blocks) * p.splits : m_tiles * ((p.N + BN - 1) / BN);
+  auto tile_of = [&](int tile) {                    // (n_blk counts 128-row blocks, or BN-row blocks with the token block in m_blk)
+    if (WS) return ws_tile(p, tile, num_kb);
+    WsTile t;
+    t.n_blk = tile / m_tiles; t.kb0 = 0; t.kb1 = num_kb; t.split = false;
+    return t;
+  };
   const unsigned full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES);
   const unsigned tfull0 = smem_u32(bars + 2 * STAGES), tempty0 = smem_u32(bars + 2 * STAGES + 2);
 
@@ -177,17 +185,17 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   // prefetch reads nothing, so it is safe even if they did).  Eight k-blocks per CTA are 19 MB over the SMs, what the memory delivers
   // meanwhile; more delays the other kernel's own traffic, as any does to the larger batches of the pair kernel (256 tokens:
   // 9.54 -> 9.59 ms).  1.4B-shaped decode step of 37 rows: 1875 -> 1803 us.
-  if (warp == 2 && lane == 0) {
+  if (WS && warp == 2 && lane == 0) {
     int left = kAheadBlocks;
     for (int tile = blockIdx.x; tile < num_tiles && left > 0; tile += gridDim.x) {
-      const WsTile t = ws_tile(p, tile, num_kb);
+      const WsTile t = tile_of(tile);
       for (int kb = t.kb0; kb < t.kb1 && left > 0; ++kb, --left) tma_prefetch_2d(&map_a, kb * kBK, t.n_blk * kBM);
     }
   }
   pdl_wait();               // barriers, tensor memory and descriptors are set up; the operands come from earlier kernels
   // exchange-block mode: word offset, inside this rank's block, of the accumulator half in use
   int64_t tp_acc_off = 0;
-  if (p.tp_on) {
+  if (WS && p.tp_on) {
     const TpLayout l = tp_layout(p.tp.m_max, p.tp.n);
     const int half = *reinterpret_cast<volatile int32_t*>(p.tp.base[p.tp.rank] + 1) & 1;
     tp_acc_off = l.acc + (int64_t)half * l.acc_half;
@@ -198,15 +206,17 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       unsigned it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const WsTile t = ws_tile(p, tile, num_kb);
+        const WsTile t = tile_of(tile);
+        const int a_row = (WS ? t.n_blk : tile - t.n_blk * m_tiles) * kBM, b_row = WS ? 0 : t.n_blk * BN;
         for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
           const unsigned s = it % STAGES, ph = (it / STAGES) & 1;
           ok = mbar_wait(empty0 + 8 * s, ph ^ 1, 1);
           if (!ok) break;
           mbar_expect_tx(full0 + 8 * s, kStageBytes);
           const unsigned a_dst = smem_u32(tiles + s * kStageBytes);
-          tma_load_2d(a_dst, &map_a, kb * kBK, t.n_blk * kBM, full0 + 8 * s);
-          tma_load_2d(a_dst + kABytes, &map_b, kb * kBK, 0, full0 + 8 * s);
+          // map_a always feeds the 128-row operand: weight rows in WS mode (map_b: all tokens), else token rows
+          tma_load_2d(a_dst, &map_a, kb * kBK, a_row, full0 + 8 * s);
+          tma_load_2d(a_dst + kABytes, &map_b, kb * kBK, b_row, full0 + 8 * s);
         }
       }
     }
@@ -221,7 +231,7 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         if (!ok) break;
         tcgen05_fence_after();
         const unsigned tmem_d = tmem_base + slot * BN;
-        const WsTile t = ws_tile(p, tile, num_kb);
+        const WsTile t = tile_of(tile);
         for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
           const unsigned s = it % STAGES, ph = (it / STAGES) & 1;
           ok = mbar_wait(full0 + 8 * s, ph, 2);
@@ -252,9 +262,53 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++lt) {
       const unsigned slot = lt & 1, aph = (lt >> 1) & 1;
-      int32_t* cs = tok_scale + slot * 2 * BN;
+      int32_t* cs = col_scale + slot * 2 * BN;
+      const WsTile wt = tile_of(tile);
+      if (!WS) {
+        // rows of the accumulator tile are tokens, columns are weight channels, whose scales go to shared memory once
+        const int row0 = (tile - wt.n_blk * m_tiles) * kBM + q * 32, row = row0 + lane;
+        if (p.out_q15)
+          for (int c = et; c < BN; c += 32 * kEpiWarps) {
+            const int col = min(wt.n_blk * BN + c, p.N - 1);
+            cs[c] = __ldg(p.w_mul + col);
+            cs[BN + c] = (p.w_shift ? __ldg(p.w_shift + col) : 31) - 48;   // x_shift + w_shift - 48 later
+          }
+        int xm = 0, xs = 0;
+        if (row < p.M && p.out_q15) {
+          if (p.x_absmax) absmax_to_ms_dev(__ldg(p.x_absmax + row), &xm, &xs);
+          else { xm = __ldg(p.x_mul + row); xs = __ldg(p.x_shift + row); }
+        }
+        epilogue_bar_sync();
+        if (ok) ok = mbar_wait(tfull0 + 8 * slot, aph, 3);
+        tcgen05_fence_after();
+        int32_t* stage = stage_all + (warp - 2) * (32 * kStagePitch);
+#pragma unroll 1
+        for (int c0 = half * 32; c0 < BN; c0 += 64) {   // the quarter's two warps take alternate 32-column chunks
+          int v[32];
+          tmem_ld_32x32(tmem_base + ((unsigned)(q * 32) << 16) + slot * BN + (unsigned)c0, v);
+          const int col0 = wt.n_blk * BN + c0;
+          if (!ok || col0 >= p.N) continue;             // warp-uniform
+          // (a thread has 32 columns of one row: through a padded tile, so that a store writes four rows of 128 bytes)
+          const bool vec = (p.N & 3) == 0;
+          if (p.acc_out) store_chunk(stage, lane, v, p.acc_out, row0, col0, p.M, p.N, vec);
+          if (p.out_q15) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              const int4 wm = *reinterpret_cast<const int4*>(cs + c0 + j), ws = *reinterpret_cast<const int4*>(cs + BN + c0 + j);
+              v[j + 0] = requant_one(v[j + 0], __mulhi(xm, wm.x), xs + ws.x);
+              v[j + 1] = requant_one(v[j + 1], __mulhi(xm, wm.y), xs + ws.y);
+              v[j + 2] = requant_one(v[j + 2], __mulhi(xm, wm.z), xs + ws.z);
+              v[j + 3] = requant_one(v[j + 3], __mulhi(xm, wm.w), xs + ws.w);
+            }
+            store_chunk(stage, lane, v, p.out_q15, row0, col0, p.M, p.N, vec);
+          }
+        }
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(tempty0 + 8 * slot);
+        continue;
+      }
       // rows of the accumulator tile are weight channels, columns are tokens
-      const WsTile wt = ws_tile(p, tile, num_kb);
       const int ch = wt.n_blk * kBM + q * 32 + lane;
       const bool direct = !wt.split && p.n_peers == 0;
       const bool empty_part = wt.kb0 >= wt.kb1;      // a part of K with no k-blocks: nothing was accumulated
@@ -324,7 +378,7 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   }
   // exchange-block mode: nothing was written into a peer's memory, so only the CTA that arrives last pays a
   // system-scope fence before the flag stores (each CTA orders its own additions with a device-scope fence)
-  if (p.tp_on && threadIdx.x == 0) {
+  if (WS && p.tp_on && threadIdx.x == 0) {
     __threadfence();
     tp_signal_if_last(p.tp, 1, gridDim.x, false);
   }
@@ -960,18 +1014,19 @@ static bool make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, bool WS = true>
 static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, cudaStream_t st) {
-  constexpr size_t smem = (size_t)STAGES * (kBM * kBK + BN * kBK) + 1024 + (2 * STAGES + 4) * 8 + 16 + 4 * BN * 4;
+  constexpr size_t smem = (size_t)STAGES * (kBM * kBK + BN * kBK) + 1024 + (2 * STAGES + 4) * 8 + 16 + 4 * BN * 4 + (WS ? 0 : kEpiWarps * 32 * kStagePitch * 4);
   static_assert(smem <= 227 * 1024, "shared memory budget");
-  cudaError_t e = cudaFuncSetAttribute(gemm_w8a8_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(gemm_w8a8_kernel<BN, STAGES, WS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) {
     set_error("gemm_w8a8: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     return B200_E_CUDA;
   }
-  const int tiles = p.full_blocks + ((p.N + kBM - 1) / kBM - p.full_blocks) * p.splits;
+  const int tiles = WS ? p.full_blocks + ((p.N + kBM - 1) / kBM - p.full_blocks) * p.splits
+                       : ((p.N + BN - 1) / BN) * ((p.M + kBM - 1) / kBM);
   const int grid = tiles < sm_count() ? tiles : sm_count();
-  launch_pdl(gemm_w8a8_kernel<BN, STAGES>, dim3(grid), dim3(kGemmThreads), smem, st, ma, mb, p);
+  launch_pdl(gemm_w8a8_kernel<BN, STAGES, WS>, dim3(grid), dim3(kGemmThreads), smem, st, ma, mb, p);
   return check_launch("gemm_w8a8");
 }
 
@@ -1010,21 +1065,29 @@ static int launch_gemm_2sm_ws(const CUtensorMap& mw, const CUtensorMap& mx, cons
 // Token tiles and parts of K of a prompt whose 256 x 256 tiles would leave CTA pairs idle; returns the parts.
 // A tile costs about (256 weight rows + its tokens) per k-block, what it moves into shared memory, so with whole-K
 // tiles the narrowest tokens tiles that still run at once are the best, down to 96 tokens (333 x 6144 x 4096: 30.8 us on single
-// CTAs, 25.6 with three tiles, 30.7 with two).  From 40 k-blocks on, splitting K beats narrowing the tiles although the
+// CTAs, 25.6 with three tiles, 30.7 with two); beyond 128 tokens the epilogue takes a second turn (257 x 2048 x 512: 14.5 us with two
+// tiles of 160, 9.9 with three of 96).  From 40 k-blocks on, splitting K beats narrowing the tiles although the
 // parts are added in memory and requantised by another kernel (333 x 4096 x 12288: 65.5 us on single CTAs, 43.0 with four whole-K
 // tiles, 35.8 with two tiles in two parts).  Below, it depends on the shape (split, whole): 1000 x 2048 with 16, 32, 36 and 40 k-blocks
-// 16.5, 13.8; 19.0, 18.4; 19.7, 19.6; 20.3, 20.7; 333 x 4096 with 16, 24 and 40 14.3, 13.5; 15.5, 15.9; 18.0, 20.6.
-static int prompt_tiles(GemmParams* p, int w_blocks, int num_kb, int pairs) {
+// 16.5, 13.8; 19.0, 18.4; 19.7, 19.6; 20.3, 20.7; 333 x 4096 with 16, 24 and 40 14.3, 13.5; 15.5, 15.9; 18.0, 20.6; where four parts fit
+// (one_wave, see lone_prompt) from 20 on: 300 x 1024 with 16, 20 and 32 10.8, 12.8; 11.1, 13.9; 12.0, 17.3.
+static int prompt_tiles(GemmParams* p, int w_blocks, int num_kb, int pairs, bool one_wave) {
   const int fewest = (p->M + 255) / 256;
   int tiles = fewest, splits = 1;
-  if (num_kb >= 40) splits = pairs / (w_blocks * fewest) < 4 ? pairs / (w_blocks * fewest) : 4;
+  if (num_kb >= (one_wave ? 20 : 40)) splits = pairs / (w_blocks * fewest) < 4 ? pairs / (w_blocks * fewest) : 4;
   while (splits > 1 && (splits - 1) * ((num_kb + splits - 1) / splits) >= num_kb) --splits;     // no empty part
+  auto per_tile = [&](int n) { return (p->M + n - 1) / n; };
   if (splits <= 1)
-    while (w_blocks * (tiles + 1) <= pairs && (p->M + tiles) / (tiles + 1) >= 96) ++tiles;
-  p->tok_tile = ((p->M + tiles - 1) / tiles + 31) / 32 * 32;
+    while (w_blocks * (tiles + 1) <= pairs && per_tile(tiles + 1) >= (per_tile(tiles) > 128 ? 64 : 96)) ++tiles;
+  p->tok_tile = (per_tile(tiles) + 31) / 32 * 32;
   p->tok_tiles = (p->M + p->tok_tile - 1) / p->tok_tile;
   return splits;
 }
+
+// Prompts that stay on single CTAs with narrow tiles of 128 tokens: where all tiles of 32 weight rows run at once and K is too short to be
+// split (300 x 512: 6.0 us with 1 k-block, 10.2 with 16, 14.6 with 32; on pairs 9.2, 13.4, 18.2 whole and 11.2 in four parts), and, with K short, where a
+// pair's second half would have no weight rows (15000 x 128 with 1 and 16 k-blocks: 10.1, 16.3 us; on pairs 15.3, 19.9; with 32: 26.2, 25.2).
+static bool lone_prompt(int64_t m, int64_t n, int num_kb, bool one_wave) { return (one_wave && num_kb < 20) || (n <= kBM && num_kb <= 16); }
 
 static bool pair_ws_enabled() {
   static int on = -1;
@@ -1072,7 +1135,9 @@ static int gemm_impl(const int8_t* x8, const int8_t* w8, const int32_t* x_absmax
   // More tokens, but fewer 256 x 256 tiles than CTA pairs (one prompt's qkv, o and down projections): the same kernel with
   // several token tiles, see prompt_tiles.
   const int pairs = sm_count() / 2;
-  const bool prompt_ws = m > 256 && (m + 255) / 256 * ((n + 255) / 256) < pairs;
+  const bool one_wave = (m + kBM - 1) / kBM * ((n + 31) / 32) <= sm_count();
+  const bool few_tiles = m > 256 && (m + 255) / 256 * ((n + 255) / 256) < pairs;
+  const bool prompt_ws = few_tiles && !lone_prompt(m, n, num_kb, one_wave);
   const bool pair_ws = prompt_ws || (m >= pair_min && m <= 256 && pair_ws_enabled());
   const int block_rows = pair_ws ? 2 * kBM : kBM, units = pair_ws ? pairs : sm_count();
   const int w_blocks = (int)((n + block_rows - 1) / block_rows);
@@ -1086,7 +1151,7 @@ static int gemm_impl(const int8_t* x8, const int8_t* w8, const int32_t* x_absmax
     splits = splits < 1 ? 1 : (splits > 8 ? 8 : splits);
     while (splits > 1 && num_kb / splits < 4) --splits;
     while (splits > 1 && (splits - 1) * ((num_kb + splits - 1) / splits) >= num_kb) --splits;   // no empty part
-    if (prompt_ws) splits = prompt_tiles(&p, w_blocks, num_kb, pairs);
+    if (prompt_ws) splits = prompt_tiles(&p, w_blocks, num_kb, pairs, one_wave);
     else p.tok_tile = (int)((m + 31) / 32 * 32);
     p.splits = splits;
     p.full_blocks = splits > 1 && !prompt_ws ? w_blocks - split_blocks : 0;
@@ -1127,6 +1192,11 @@ static int gemm_impl(const int8_t* x8, const int8_t* w8, const int32_t* x_absmax
     return check_launch("gemm_w8a8 (split-K epilogue)");
   }
   B200_REQUIRE(make_map(&ma, x8, m, k, kBM), B200_E_CUDA, "gemm_w8a8: cuTensorMapEncodeTiled failed for x8");
+  if (few_tiles) {                     // (tiles of 64 weight rows where those of 128 tokens occupy every SM)
+    const int bn = (m + kBM - 1) / kBM * ((n + 63) / 64) < sm_count() ? 32 : 64;
+    B200_REQUIRE(make_map(&mb, w8, n, k, bn), B200_E_CUDA, "gemm_w8a8: cuTensorMapEncodeTiled failed for w8");
+    return bn == 32 ? launch_gemm<32, 10, false>(ma, mb, p, st) : launch_gemm<64, 8, false>(ma, mb, p, st);
+  }
   // large problems: 256 x 256 tiles on CTA pairs
   B200_REQUIRE(make_map(&mb, w8, n, k, kBM), B200_E_CUDA, "gemm_w8a8: cuTensorMapEncodeTiled failed for w8");
   return launch_gemm_2sm<5>(ma, mb, p, st);

@@ -83,10 +83,13 @@ def test_pair_weights_stationary_tiles(M, N, K):
     run_case(M, N, K, M + N + K, per_channel_shift=True)
 
 
-@pytest.mark.parametrize("M,N,K", [(257, 520, 6400), (333, 6144, 512), (333, 1000, 6160), (300, 520, 4992), (300, 520, 5008), (600, 260, 6144), (1100, 4096, 256), (2100, 132, 272), (18900, 40, 144)])
+@pytest.mark.parametrize("M,N,K", [(257, 520, 6400), (333, 6144, 512), (333, 1000, 6160), (333, 2000, 4992), (333, 2000, 5008), (257, 2048, 512),
+                                   (300, 520, 2432), (300, 520, 2448), (257, 1024, 144), (300, 36, 16), (700, 768, 272), (700, 772, 272), (2100, 130, 272),
+                                   (5000, 100, 272), (9500, 127, 2048), (9500, 128, 2064), (18688, 40, 144), (18900, 40, 144), (600, 260, 6144), (1100, 4096, 256), (2100, 132, 272)])
 def test_prompts_of_few_tiles(M, N, K):
-    """More than 256 tokens on fewer 256 x 256 tiles than CTA pairs: several token tiles of 96 .. 256 tokens against a block of
-    weight rows, whole-K or (from 40 k-blocks) in up to four parts; ragged last tiles of both kinds."""
+    """More than 256 tokens on fewer 256 x 256 tiles than CTA pairs: several token tiles of 64 .. 256 tokens against a block of
+    weight rows, whole-K or (from 40 k-blocks, or 20 for the smallest) in up to four parts; single CTAs with 32 or 64 weight rows a
+    tile where all of those run at once and K is short, or where there are at most 128 weight rows; ragged last tiles of every kind."""
     run_case(M, N, K, M + N + K, per_channel_shift=True)
 
 
