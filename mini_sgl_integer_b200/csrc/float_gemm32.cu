@@ -454,6 +454,9 @@ using namespace b200;
 
 extern "C" int64_t b200f_gemm_f32_ws_bytes(int64_t m, int64_t n, int64_t k, int64_t batch) {
   if (m <= 0 || n <= 0 || k <= 0 || batch <= 0 || batch > 65535 / 3 || m >= (1ll << 31) || n >= (1ll << 31) || k >= (1ll << 31)) return -1;
+  // Short sums: the chains' kernels have little to do and no second launch (16 of K: 2 .. 4 us, 7 .. 13 here; 9 x 4096 with 64 of K: 5.9,
+  // 7.9; 2048 x 256: 7.3, 8.6; 300 x 4096, of more tiles than SMs: 12.4, 10.0; five rows, 16384 weight rows with 64 of K: 6.3, 18.2).
+  if (k <= 32 || (k <= 64 && (m > 8 ? batch * ((m + 63) / 64) * ((n + 63) / 64) <= sm_count() : m > 4 && batch * n >= 8192))) return -1;
   if (m <= 8) return 0;
   // Few rows against many weight rows: the fp32 units read the weights once (4 bytes each) and fill the GPU with a tile of 64 x 64
   // per CTA, the split moves 10 bytes of each (m = 16, n = 32768, k = 1024: 155 us against 177).  Everywhere else that kernel has too

@@ -61,7 +61,8 @@ def test_linear(dtype, m, n, k):
     fo.check_status()
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (3, 130, 63), (127, 128, 64), (128, 129, 65), (129, 127, 128), (300, 257, 200), (64, 512, 1500)])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (3, 130, 63), (127, 128, 64), (128, 129, 65), (129, 127, 128), (300, 257, 200), (64, 512, 1500),
+                                   (700, 900, 64), (1000, 700, 33)])
 def test_linear_f32_in_three_parts(m, n, k):
     """32-bit linears as products of three bf16 parts: sizes around the tiles (128 rows, 128 columns, 64 and 128 of K), operands of
     all magnitudes, and rows that are not on 16-byte boundaries.  A product's error is below 2^-22 of it (three parts hold 24
