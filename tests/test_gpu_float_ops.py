@@ -219,7 +219,18 @@ def test_sublayer_end(dtype, width, parts):
         close(xt, S.rms_norm(want, fw, eps), dtype)
 
 
-@pytest.mark.parametrize("m,n,k", [(9, 40, 24), (130, 140, 70), (1300, 2000, 600)])
+@pytest.mark.parametrize("m,n,k,chain", [(1, 40, 32, True), (1, 40, 33, False), (2048, 700, 32, True), (9, 40, 64, True), (9, 40, 65, False), (300, 1900, 64, False),
+                                         (300, 1850, 64, True), (4, 8200, 64, False), (5, 8200, 64, True), (5, 8100, 64, False)])
+def test_linear_f32_of_short_sums_is_a_chain(m, n, k, chain):
+    """Up to 32 of K, and up to 64 with few tiles or with five to eight rows of many weight rows."""
+    g = torch.Generator(device="cuda").manual_seed(k)
+    x, w = torch.randn((m, k), device="cuda", generator=g), torch.randn((n, k), device="cuda", generator=g)
+    got = fo.linear(x, w)
+    assert torch.equal(got, fo.linear(x, w, chained=True)) == chain
+    close(got, host(x) @ host(w).T, torch.float32)
+
+
+@pytest.mark.parametrize("m,n,k", [(9, 40, 130), (130, 140, 70), (1300, 2000, 40), (1300, 2000, 600)])
 def test_linear_f32_outside_the_range_of_three_parts(m, n, k):
     """What the sum of three bf16 numbers cannot hold, in one row or column of a linear of one tile, of ragged ones, and of more
     tiles than SMs: values that are not finite, finite products of the largest, sums that overflow, operands and outputs next to
@@ -530,7 +541,7 @@ def test_latent_attention_32_bit_prompts_longer_than_their_keys(window):
     outs = []
     for simple in (False, True):
         out = torch.full((sum(q_lens), heads, fo.pad8(rank)), 5.0, device="cuda")
-        fo.latent_attention(q, cache, table, i32(kv_lens), starts, sink, out, rank, rot, window, 0.3, max(q_lens), max(kv_lens), simple=simple)
+        fo.latent_attention(q, cache, table, i32(kv_lens), starts, sink, out, rank, rot, window, 0.3, max(q_lens), 100, simple=simple)
         outs.append(out[..., :rank])
     close(outs[0], host(outs[1]), torch.float32)
     assert not bool(outs[0][:9].any()) and not bool(outs[0][9:73].any()) and bool(outs[0][73:].any(2).all())
