@@ -909,7 +909,9 @@ static int attn_common(const int8_t* q, const int32_t* q_mul, const int32_t* q_s
   if (cluster == 0) {
     cluster = 1;
     while (cluster < 8 && !fits2(cluster, 1)) cluster *= 2;   // fewest CTAs per row first, ring depth second
-    while (cluster < 8 && max_pages > kAlonePages && (int64_t)batch * kv_heads * cluster * 2 <= 256 && max_pages / (2 * cluster) >= 4) cluster *= 2;
+    // (with one query head per KV head a CTA has less to do: two of them are worth it from 640 keys on; 12 rows of 500 keys: 10.0 us, 10.7 with two)
+    const int least = G == 1 && (int64_t)batch * kv_heads * 4 > 256 ? 40 : kAlonePages + 1;
+    while (cluster < 8 && max_pages >= least && (int64_t)batch * kv_heads * cluster * 2 <= 256 && max_pages / (2 * cluster) >= 4) cluster *= 2;
     stages = fits2(cluster, 2) ? 2 : 1;
   } else {
     B200_REQUIRE(cluster == 1 || cluster == 2 || cluster == 4 || cluster == 8, B200_E_UNSUPPORTED,
