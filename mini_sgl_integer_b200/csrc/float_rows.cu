@@ -360,7 +360,9 @@ static int launch_sublayer_end(const SublayerEnd& p, T* x_out_t, int64_t rows, c
   while (threads < 1024 && threads * 4 < groups) threads *= 2;
   const int nv = (groups + threads - 1) / threads;
   const dim3 grid((unsigned)rows), block(threads);
-  const bool few = rows <= 592;                     // up to about four rows per SM
+  // up to four rows per SM, if so many CTAs of the early form's registers are resident (2048 columns: three; 592 rows of them take 5.9 us
+  // early and 4.6 late, 400 rows 3.8 and 4.5)
+  const bool few = rows <= 592 && rows * threads <= 444 * 256;
   if (nv <= 1 && few) launch_pdl(sublayer_end_kernel<T, VEC, 1, true>, grid, block, 0, st, p, x_out_t);
   else if (nv <= 2 && few) launch_pdl(sublayer_end_kernel<T, VEC, 2, true>, grid, block, 0, st, p, x_out_t);
   else if (nv <= 1) launch_pdl(sublayer_end_kernel<T, VEC, 1, false>, grid, block, 0, st, p, x_out_t);

@@ -262,11 +262,12 @@ def test_linear_f32_outside_the_range_of_three_parts(m, n, k):
 
 @pytest.mark.parametrize("width", [3, 40, 1024, 2048, 1027])
 def test_sublayer_end_of_few_and_many_rows(width):
-    """Up to 592 rows request streams, gains and planes in front of the sums: the bits of the form for more rows, for every
+    """Up to 592 rows, or 444, request streams, gains and planes in front of the sums: the bits of the form for more rows, for every
     combination of what may be left out, also where the stream is updated in place."""
     g = torch.Generator(device="cuda").manual_seed(width)
     rnd = lambda *n: torch.randn(n, device="cuda", generator=g)
-    T, few, parts, planes = 593, 592, 3, 5
+    few, parts, planes = 444 if width == 2048 else 592, 3, 5      # (2048 columns: three CTAs per SM)
+    T = few + 1
     y, y2, x, hist, coef = rnd(parts, T, width), rnd(1, T, width), rnd(T, width), rnd(planes + 1, T, width), rnd(planes + 1)
     w, w1, w2, fw, add = (rnd(width) for _ in range(5))
     cut = lambda t: None if t is None else t[..., :few, :].contiguous()
