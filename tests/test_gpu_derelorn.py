@@ -87,9 +87,10 @@ def test_prompt_portions_and_decoding(name, dtype):
 @pytest.mark.parametrize("name", ["one layer", "wide heads", "mixed", "odd sizes"])
 def test_a_request_in_32_bits_does_not_depend_on_the_others(name):
     """Short prompts, where a head's readout of one nearly orthogonal key is rounding brought back to size one: each request's
-    logits are the same bits alone and beside others, for prompts and for the tokens after them."""
+    logits are the same bits alone and beside others, for prompts and for the tokens after them.  (300 tokens: the running maximum by
+    16 warps alone, by four beside short prompts.)"""
     rng = np.random.default_rng(3)
-    prompts = [rng.integers(0, CONFIGS[name]["vocab"], n).tolist() for n in (8, 3, 8, 2, 12, 40)]
+    prompts = [rng.integers(0, CONFIGS[name]["vocab"], n).tolist() for n in (8, 3, 8, 2, 12, 300 if name == "one layer" else 40)]
     e = engine(name, "float32")
     alone = []
     for p in prompts:
