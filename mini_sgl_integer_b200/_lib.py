@@ -15,6 +15,7 @@ import torch
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "libb200int.so")
 FLOAT_LIB_PATH = os.path.join(_PKG, "libb200float.so")
+PYCALL_PATH = os.path.join(_PKG, "_pycall.abi3.so")
 
 P, I, L, F = c_void_p, c_int, c_int64, c_float
 
@@ -147,24 +148,32 @@ def library_of(name: str) -> ctypes.CDLL:
 
 
 CALLS = 0      # entry-point calls made through `call` (bench.py counts the launches of a captured step with it)
-_entries: dict[str, tuple] = {}      # name -> (entry point, its library)
+_entries: dict[str, tuple] = {}      # name -> (entry point as a native callable, the same through ctypes, its library)
 
 
 def _entry(name: str) -> tuple:
     e = _entries.get(name)
     if e is None:
+        if not os.path.exists(PYCALL_PATH):
+            raise RuntimeError(f"{PYCALL_PATH} is missing: build it with `python -m mini_sgl_integer_b200.build`")
+        from ._pycall import bind
         lib = library_of(name)
-        e = _entries[name] = (getattr(lib, name), lib)
+        slow = getattr(lib, name)
+        e = _entries[name] = (bind(name, ctypes.cast(slow, c_void_p).value) or slow, slow, lib)
     return e
 
 
 # A step outside a CUDA graph is some hundreds of calls, and a short prompt is bound by what each costs on the host: entry points
-# are looked up once, pointers and streams are plain integers.  An 8B-shaped prompt of 333 tokens, 448 launches: 11.5 -> 8.2 ms.
+# are looked up once and take their arguments without ctypes (csrc/pycall.cpp; 22 arguments 6.2 -> 0.7 us), pointers and streams are
+# plain integers.  Arguments that are objects of ctypes go through ctypes.
 def call(name: str, *args) -> None:
     global CALLS
-    fn, lib = _entry(name)
+    fn, slow, lib = _entry(name)
     CALLS += 1
-    rc = fn(*args)
+    try:
+        rc = fn(*args)
+    except (TypeError, OverflowError):
+        rc = slow(*args)
     if rc != 0:
         msg = lib.b200_last_error_string().decode("utf-8", "replace")
         raise B200Error(name, rc, msg)

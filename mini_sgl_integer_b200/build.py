@@ -2,7 +2,8 @@
 
     python -m mini_sgl_integer_b200.build [int] [float] [--force] [--verbose]
 
-``libb200int.so`` holds the integer path, ``libb200float.so`` the floating-point models; a model needs only its own.
+``libb200int.so`` holds the integer path, ``libb200float.so`` the floating-point models; a model needs only its own.  With either
+comes ``_pycall.abi3.so``, through which Python calls their entry points (compiled by g++ against Python's headers).
 nvcc cross-compiles without a GPU, so this runs on a CPU-only host as well.
 """
 from __future__ import annotations
@@ -12,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
@@ -54,7 +56,21 @@ def build_library(force: bool = False, verbose: bool = False, which: str = "int"
     os.makedirs(obj_dir, exist_ok=True)
     with open(os.path.join(obj_dir, ".lock"), "w") as lock:
         fcntl.flock(lock, fcntl.LOCK_EX)
+        _build_pycall(force)
         return _build_locked(obj_dir, force, verbose, which)
+
+
+def _build_pycall(force: bool) -> None:
+    target, src = os.path.join(PKG_DIR, "_pycall.abi3.so"), os.path.join(CSRC, "pycall.cpp")
+    if not force and not _stale(target, [src] + [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE)]):
+        return
+    part = target + ".part"
+    cmd = [os.environ.get("CXX", "g++"), "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
+           "-I" + sysconfig.get_paths()["include"], src, "-o", part]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on pycall.cpp:\n{r.stdout}")
+    os.replace(part, target)
 
 
 def _build_locked(obj_dir: str, force: bool, verbose: bool, which: str) -> str:

@@ -1,0 +1,101 @@
+// The entry points of the C libraries as Python callables, with arguments converted by the types of their declarations.
+//
+// A step outside a CUDA graph is some hundreds of entry-point calls with 10 to 30 arguments each, and ctypes takes about 0.25 us for
+// every argument (22 arguments: 6.2 us; here 0.7), more than the launch itself; a short prompt is bound by it.  Python integers, None
+// (a null pointer) and numbers are taken; anything else raises TypeError or OverflowError, and the caller goes through ctypes instead.
+// The library stays where ctypes has loaded it: `bind(name, address)` only wraps the address.
+#define PY_SSIZE_T_CLEAN
+#define Py_LIMITED_API 0x030a0000
+#include <Python.h>
+
+#include <cstring>
+#include <tuple>
+#include <type_traits>
+#include <utility>
+
+#include "../../include/b200float.h"
+#include "../../include/b200int.h"
+
+namespace {
+
+template <typename T>
+bool take(PyObject* o, T& out) {
+  if constexpr (std::is_pointer_v<T>) {
+    if (o == Py_None) {
+      out = nullptr;
+      return true;
+    }
+    out = reinterpret_cast<T>(PyLong_AsVoidPtr(o));
+  } else if constexpr (std::is_floating_point_v<T>) {
+    out = static_cast<T>(PyFloat_AsDouble(o));
+  } else {
+    const long long v = PyLong_AsLongLong(o);
+    out = static_cast<T>(v);
+    if (static_cast<long long>(out) != v) PyErr_SetString(PyExc_OverflowError, "an integer argument is too large");
+  }
+  return !PyErr_Occurred();
+}
+
+template <typename F>
+struct Call;
+template <typename R, typename... A>
+struct Call<R (*)(A...)> {
+  template <size_t... I>
+  static bool take_all(std::tuple<A...>& v, PyObject* const* args, std::index_sequence<I...>) {
+    return (take(args[I], std::get<I>(v)) && ...);
+  }
+  static PyObject* run(PyObject* self, PyObject* const* args, Py_ssize_t n) {
+    if (n != (Py_ssize_t)sizeof...(A)) return PyErr_Format(PyExc_TypeError, "%zd arguments where %zu are wanted", n, sizeof...(A));
+    std::tuple<A...> v;
+    if (!take_all(v, args, std::index_sequence_for<A...>())) return nullptr;
+    const auto f = reinterpret_cast<R (*)(A...)>(PyCapsule_GetPointer(self, nullptr));
+    if (!f) return nullptr;
+    R r;
+    Py_BEGIN_ALLOW_THREADS
+    r = std::apply(f, v);
+    Py_END_ALLOW_THREADS
+    return PyLong_FromLongLong(static_cast<long long>(r));
+  }
+};
+
+#define B200_ENTRY_POINTS(X) \
+  X(b200_to_fixed_f32) X(b200_to_fixed_bf16) X(b200_from_fixed_f32) X(b200_from_fixed_bf16) X(b200_rmsnorm_q15) X(b200_silu_mul_q15) \
+  X(b200_fwht_q15) X(b200_qk_rope_q15) X(b200_per_token_quant_q15) X(b200_absmax_to_mul_shift) X(b200_kv_store_q15) \
+  X(b200_kv_store_codes) X(b200_attn_extend) X(b200_attn_prefill) X(b200_attn_workspace_bytes) X(b200_attn_paged_ws) \
+  X(b200_attn_paged_static) X(b200_embedding_bf16_q15) X(b200_argmax_i32) X(b200_decode_prepare) X(b200_static_quant_q15) \
+  X(b200_qkv_prepare_q15) X(b200_gemm_w8a8) X(b200_gemm_w8a8_absmax) X(b200_gemm_w8a8_reduce_peers) X(b200_gemm_w8a8_absmax_ws) \
+  X(b200_gemm_w8a8_acc_ws) X(b200_gemm_gate_up_silu) X(b200_fwht_quant_q15) X(b200_rmsnorm_q15_pending) X(b200_qkv_prepare_pending) \
+  X(b200_quant_given_absmax_q15) X(b200_requant_q15) X(b200_attn_decode) X(b200_quantize_per_tensor_int8_ms) X(b200_tp_block_bytes) \
+  X(b200_tp_block_clear) X(b200_tp_absmax_put) X(b200_tp_quant_wait) X(b200_tp_absmax_quant) X(b200_gemm_w8a8_tp) \
+  X(b200_tp_requant_scatter) X(b200_tp_collect) X(b200_tp_requant_direct) X(b200_tp_all_gather) X(b200_tp_owner_norm) \
+  X(b200_tp_collect_codes) X(b200_tp_silu_absmax_quant) X(b200_tp_set_timeout_us) X(b200f_gemm_splits) X(b200f_gemm) \
+  X(b200f_gemm_f32_ws_bytes) X(b200f_gemm_f32) X(b200f_embed_bigram) X(b200f_sublayer_end) X(b200f_gated_silu) \
+  X(b200f_memory_prepare) X(b200f_memory_scan_ws_bytes) X(b200f_memory_scan) X(b200f_memory_output) X(b200f_grouped_prepare) \
+  X(b200f_grouped_attn_ws_floats) X(b200f_grouped_attn_splits) X(b200f_grouped_attn) X(b200f_xielu) X(b200f_mingru) \
+  X(b200f_latent_prepare) X(b200f_latent_attn_ws_floats) X(b200f_latent_attn_splits) X(b200f_latent_attn) X(b200f_argmax)
+
+#define AS_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&Call<decltype(&name)>::run)), METH_FASTCALL, nullptr},
+PyMethodDef g_entries[] = {B200_ENTRY_POINTS(AS_METHOD){nullptr, nullptr, 0, nullptr}};
+
+// bind(name, address): a callable, or None for a name that is not in the table.
+PyObject* bind(PyObject*, PyObject* args) {
+  const char* name;
+  unsigned long long address;
+  if (!PyArg_ParseTuple(args, "sK", &name, &address)) return nullptr;
+  for (PyMethodDef* m = g_entries; m->ml_name; ++m)
+    if (!std::strcmp(m->ml_name, name)) {
+      PyObject* at = PyCapsule_New(reinterpret_cast<void*>(address), nullptr, nullptr);
+      if (!at) return nullptr;
+      PyObject* f = PyCFunction_NewEx(m, at, nullptr);
+      Py_DECREF(at);
+      return f;
+    }
+  Py_RETURN_NONE;
+}
+
+PyMethodDef g_methods[] = {{"bind", bind, METH_VARARGS, "bind(name, address): the entry point as a callable, or None"}, {nullptr, nullptr, 0, nullptr}};
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_pycall", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__pycall(void) { return PyModule_Create(&g_module); }

@@ -271,7 +271,7 @@ def memory_prepare(y: torch.Tensor, col0: int, segments, conv_w: Optional[torch.
     if kind == MEMORY_EXP and (norm_state.dtype != torch.float32 or norm_state.shape[1] != heads or not norm_state.is_contiguous()):
         raise ValueError(f"norm_state must be contiguous fp32 [slots, {heads}, dim + 1]")
     seg = (ctypes.c_int32 * 6)(*[v for s in segments for v in s])
-    call("b200f_memory_prepare", ptr(y), parts, T * n, n, col0, ctypes.cast(seg, ctypes.c_void_p), ptr(conv_w), ptr(conv_b), taps,
+    call("b200f_memory_prepare", ptr(y), parts, T * n, n, col0, ctypes.addressof(seg), ptr(conv_w), ptr(conv_b), taps,
          ptr(conv_state) if taps > 1 else None, ptr(slots), ptr(positions), ptr(seq_start), ptr(seq_ids), ptr(out), _pitch(out), dtype_code(out.dtype),
          kind, heads, gate_cols[0], gate_cols[1], ptr(gate_a), ptr(gate_b), float(cap), ptr(gates), ptr(norm_state),
          0 if norm_state is None else norm_state.shape[2] - 1, T, slots.numel(), stream())

@@ -100,7 +100,7 @@ class CacheManager:
             return
         rows = sorted(self._dirty)
         self._dirty.clear()
-        src = self._host[rows]
-        if self.page_table.is_cuda:
-            src = src.pin_memory().to(self.page_table.device, non_blocking=True)
-        self.page_table[torch.tensor(rows, device=self.page_table.device)] = src
+        at, src = torch.tensor(rows), self._host[rows]
+        if self.page_table.is_cuda:                        # (pinned: copies from pageable memory wait for the stream)
+            at, src = (t.pin_memory().to(self.page_table.device, non_blocking=True) for t in (at, src))
+        self.page_table.index_copy_(0, at, src)

@@ -1,0 +1,48 @@
+"""Entry points called without ctypes receive the arguments that they would receive from it."""
+from __future__ import annotations
+
+import ctypes
+
+import pytest
+
+from mini_sgl_integer_b200 import _lib
+from mini_sgl_integer_b200.build import build_library
+
+build_library()
+from mini_sgl_integer_b200._pycall import bind  # noqa: E402
+
+ALL = {**_lib.SIGNATURES, **_lib.FLOAT_SIGNATURES}
+BOUND = [n for n in ALL if bind(n, 1) is not None]
+
+
+def test_everything_that_launches_is_bound():
+    assert set(ALL) - set(BOUND) == {n for n in ALL if n.endswith("_status")} | {"b200_version", "b200_last_error_string", "b200_get_lut"}
+
+
+@pytest.mark.parametrize("name", BOUND)
+def test_arguments_arrive(name):
+    types = ALL[name]
+    got = []
+    target = ctypes.CFUNCTYPE(_lib._RESTYPES.get(name, ctypes.c_int), *types)(lambda *a: got.append(a) or 7)
+    fn = bind(name, ctypes.cast(target, ctypes.c_void_p).value)
+    large = {ctypes.c_void_p: 2**63 + 5, ctypes.c_int64: -(2**62), ctypes.c_size_t: 2**62, ctypes.c_int: -(2**31), ctypes.c_float: -1.5}
+    for args in ([i + 0.25 if t is ctypes.c_float else i + 1 for i, t in enumerate(types)], [large[t] for t in types],
+                 [None if t is ctypes.c_void_p else 0 for t in types], [True] * len(types)):
+        assert fn(*args) == 7
+        assert got.pop() == tuple(args)
+    with pytest.raises(TypeError):
+        fn(*args[1:])
+    if ctypes.c_int in types:
+        with pytest.raises(OverflowError):
+            fn(*[2**31 if t is ctypes.c_int else 0 for t in types])
+    if ctypes.c_void_p in types:
+        with pytest.raises(TypeError):
+            fn(*[ctypes.c_void_p(16) if t is ctypes.c_void_p else 0 for t in types])
+    assert not got
+
+
+def test_objects_of_ctypes_go_through_ctypes():
+    with pytest.raises(_lib.B200Error):
+        _lib.call("b200_fwht_q15", ctypes.c_void_p(16), 16, 4, 96, 1, None)
+    with pytest.raises(ctypes.ArgumentError):
+        _lib.call("b200_fwht_q15", 1.5, 16, 4, 96, 1, None)
