@@ -462,6 +462,12 @@ B200_API int b200_tp_set_timeout_us(int64_t microseconds);    /* synchronises wi
  * Synchronises with the device.  No counterpart in the reference. */
 B200_API int b200_gemm_status(int* out_host, int reset);
 
+/* on != 0: from here on, until it is called with 0, the calling thread's launches use weights that no kernel of this library writes,
+ * and its GEMMs of decode size may read them while the kernels in front of them still run.  The next launch is made
+ * in full stream order, so that whatever wrote the weights earlier in the stream has completed; launches of other streams
+ * are unaffected. */
+B200_API int b200_settled_weights(int on);
+
 #ifdef __cplusplus
 }
 #endif

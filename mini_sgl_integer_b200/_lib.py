@@ -56,6 +56,7 @@ SIGNATURES: dict[str, list] = {
     "b200_rmsnorm_q15_pending": [P, P, P, P, P, P, P, P, P, P, P, L, I, P],
     "b200_qkv_prepare_pending": [P, P, P, P, P, P, I, P, P, P, P, P, P, P, P, P, L, I, I, L, I, P],
     "b200_gemm_status": [P, I],
+    "b200_settled_weights": [I],
     "b200_quant_given_absmax_q15": [P, P, P, L, I, P],
     "b200_requant_q15": [P, P, P, P, P, P, L, L, P],
     "b200_attn_decode": [P, P, P, P, P, P, P, L, P, P, P, P, P, I, I, I, L, I, I, P],
@@ -80,6 +81,7 @@ FLOAT_SIGNATURES: dict[str, list] = {
     "b200f_gemm_splits": [L, L, L, L, I],
     "b200f_gemm": [P, P, P, I, I, L, L, L, L, L, L, L, L, L, L, I, L, I, F, F, P],
     "b200f_gemm_status": [P, I],
+    "b200f_settled_weights": [I],
     "b200f_gemm_f32_ws_bytes": [L, L, L, L],
     "b200f_gemm_f32": [P, P, P, L, L, L, L, L, L, L, L, L, L, I, F, F, P, P],
     "b200f_gemm_f32_status": [P, I],
@@ -182,6 +184,21 @@ def call(name: str, *args) -> None:
 def query(name: str, *args) -> int:
     """An entry point that returns a number instead of a status."""
     return _entry(name)[0](*args)
+
+
+class settled_weights:
+    """``with settled_weights("int"):`` around a model's forward: its weights are what checkpoints or earlier work of the current stream
+    have left, and no kernel launched inside writes them, so that linears of decode size may read theirs ahead (b200_settled_weights)."""
+
+    def __init__(self, which: str):
+        self.name = "b200_settled_weights" if which == "int" else "b200f_settled_weights"
+
+    def __enter__(self):
+        query(self.name, 1)
+
+    def __exit__(self, *exc):
+        query(self.name, 0)
+        return False
 
 
 def ptr(t: torch.Tensor | None) -> int | None:

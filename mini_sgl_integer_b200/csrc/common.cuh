@@ -30,6 +30,14 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // without it, or after a kernel that never triggers, behaves as usual.
 bool pdl_enabled();
 
+// While a thread has declared the weights settled (b200_settled_weights, b200f_settled_weights), its GEMMs of decode size read them
+// before their wait.  That needs everything that wrote a weight to have completed and be visible when such a GEMM starts, which may be as
+// early as the kernels in front of it trigger.  So the scope's first launch is a plain one: it starts once all earlier
+// work of the stream has completed, and no later launch of the stream starts before it.
+void settle(bool on);
+bool settle_takes_first(cudaStream_t st);         // whether this launch has to be the plain one
+bool weights_settled(cudaStream_t st);
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -41,7 +49,7 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  cfg.numAttrs = !settle_takes_first(st) && pdl_enabled() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
@@ -249,6 +257,13 @@ __device__ __forceinline__ int requant_one(int acc, int cm, int s) {
   if (s > 0 && s < 63) return sat32(((long long)acc * (long long)cm + (1LL << (s - 1))) >> s);
   return sat32(mul_shift64((long long)acc, (long long)cm, s));
 }
+// The same with shifts outside 1 .. 62 in a function of their own, for kernels of few rows, where fetching code is much of the time.  (In the
+// epilogues of many rows the call costs more than it saves: a prompt of 333 tokens 8.15 ms inline, 8.50 with it.)
+static __device__ __noinline__ int requant_rare(int acc, int cm, int s) { return sat32(mul_shift64((long long)acc, (long long)cm, s)); }
+__device__ __forceinline__ int requant_few(int acc, int cm, int s) {
+  if (s > 0 && s < 63) return sat32(((long long)acc * (long long)cm + (1LL << (s - 1))) >> s);
+  return requant_rare(acc, cm, s);
+}
 
 // A linear's output that has not been requantised yet: the exact int32 accumulators [rows, n] (split-K parts already
 // added), the absmax of each token's input row and the weight's per-channel scales.  A row kernel that is handed this
@@ -268,7 +283,7 @@ __device__ __forceinline__ int2 pending_take2(const PendingLinear& pl, int64_t r
   const int2 wm = __ldg(reinterpret_cast<const int2*>(pl.w_mul + col));
   int2 ws = make_int2(31, 31);
   if (pl.w_shift) ws = __ldg(reinterpret_cast<const int2*>(pl.w_shift + col));
-  return make_int2(requant_one(a.x, __mulhi(xm, wm.x), xs48 + ws.x), requant_one(a.y, __mulhi(xm, wm.y), xs48 + ws.y));
+  return make_int2(requant_few(a.x, __mulhi(xm, wm.x), xs48 + ws.x), requant_few(a.y, __mulhi(xm, wm.y), xs48 + ws.y));
 }
 
 __device__ __forceinline__ void pending_clear2(const PendingLinear& pl, int64_t row, int n, int col) {
@@ -284,10 +299,10 @@ __device__ __forceinline__ int4 pending_take4(const PendingLinear& pl, int64_t r
   int4 ws = make_int4(31, 31, 31, 31);
   if (pl.w_shift) ws = __ldg(reinterpret_cast<const int4*>(pl.w_shift + col));
   int4 r;
-  r.x = requant_one(a.x, __mulhi(xm, wm.x), xs48 + ws.x);
-  r.y = requant_one(a.y, __mulhi(xm, wm.y), xs48 + ws.y);
-  r.z = requant_one(a.z, __mulhi(xm, wm.z), xs48 + ws.z);
-  r.w = requant_one(a.w, __mulhi(xm, wm.w), xs48 + ws.w);
+  r.x = requant_few(a.x, __mulhi(xm, wm.x), xs48 + ws.x);
+  r.y = requant_few(a.y, __mulhi(xm, wm.y), xs48 + ws.y);
+  r.z = requant_few(a.z, __mulhi(xm, wm.z), xs48 + ws.z);
+  r.w = requant_few(a.w, __mulhi(xm, wm.w), xs48 + ws.w);
   return r;
 }
 

@@ -39,6 +39,7 @@ struct FGemmParams {
   int64_t split_stride;
   int act;
   float act_a, act_b;
+  int early;                         // the weights are settled (weights-stationary form): the first may be loaded before the wait
   int vec;                           // out rows and batches start on 16-byte boundaries (pitch and strides allow it)
 };
 
@@ -182,6 +183,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   constexpr int kABytes = kFBM * kFKBytes;
   constexpr int kBBytes = BN * kFKBytes;
   constexpr int kStageBytes = kABytes + kBBytes;
+  constexpr bool kFew = WS && BN <= 64;        // (128 and 256 rows are no faster for it)
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + STAGES * kStageBytes);   // full[S], empty[S], tfull[2], tempty[2]
   unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * STAGES + 4);
@@ -215,8 +217,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   __syncthreads();
   tcgen05_fence_after();
   const unsigned tmem_base = *tmem_slot;
-  pdl_wait();
-
   // tile -> (batch, weight block, token block or part of K)
   auto decode_tile = [&](int tile) {
     if (WS) return f_ws_tile(p, tile, n_tiles, num_kb);
@@ -229,6 +229,19 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     return t;
   };
 
+  // Settled weights go into the free stages before the wait; behind it only the tokens are missing.
+  unsigned ahead = 0;
+  if (kFew && p.early && warp == 0 && lane == 0) {
+    for (int tile = blockIdx.x; tile < num_tiles && ahead < STAGES; tile += gridDim.x) {
+      const FWsTile t = decode_tile(tile);
+      for (int kb = t.kb0; kb < t.kb1 && ahead < STAGES; ++kb, ++ahead) {
+        mbar_expect_tx(full0 + 8 * ahead, kStageBytes);
+        tma_load_3d(smem_u32(tiles + ahead * kStageBytes), &map_a, kb * kFBK, t.n_blk * kFBM, t.b, full0 + 8 * ahead);
+      }
+    }
+  }
+  pdl_wait();
+
   if (warp == 0) {
     if (lane == 0) {
       unsigned it = 0;
@@ -237,12 +250,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const FWsTile t = decode_tile(tile);
         for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
           const unsigned s = it % STAGES, ph = (it / STAGES) & 1;
-          ok = mbar_wait(empty0 + 8 * s, ph ^ 1, 1);
-          if (!ok) break;
-          mbar_expect_tx(full0 + 8 * s, kStageBytes);
           const unsigned a_dst = smem_u32(tiles + s * kStageBytes);
-          // map_a feeds the 128-row operand: token rows, or weight rows in the weights-stationary form
-          tma_load_3d(a_dst, &map_a, kb * kFBK, (WS ? t.n_blk : t.part) * kFBM, t.b, full0 + 8 * s);
+          if (!kFew || it >= ahead) {
+            ok = mbar_wait(empty0 + 8 * s, ph ^ 1, 1);
+            if (!ok) break;
+            mbar_expect_tx(full0 + 8 * s, kStageBytes);
+            // map_a feeds the 128-row operand: token rows, or weight rows in the weights-stationary form
+            tma_load_3d(a_dst, &map_a, kb * kFBK, (WS ? t.n_blk : t.part) * kFBM, t.b, full0 + 8 * s);
+          }
           tma_load_3d(a_dst + kABytes, &map_b, kb * kFBK, WS ? 0 : t.n_blk * BN, t.b, full0 + 8 * s);
         }
       }
@@ -287,17 +302,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       __syncwarp();
       tcgen05_fence_after();
       if (WS) {
+        constexpr int CH = kFew ? 8 : 32;                      // tokens at a time: little code to fetch for few of them
         const int ch = t.n_blk * kFBM + q * 32 + lane;         // rows of the accumulator are weight rows, columns tokens
         const int64_t off = (int64_t)t.b * p.out_bstride + (int64_t)t.part * p.split_stride + ch;
 #pragma unroll 1
-        for (int c0 = half * 32; c0 < BN; c0 += 64) {
-          if (c0 >= p.M) break;
-          int v[32];
+        for (int c0 = half * CH; c0 < p.M; c0 += 2 * CH) {
+          int v[CH];
           tmem_ld_32x32(tmem_base + ((unsigned)(q * 32) << 16) + slot * BN + (unsigned)c0, v);
           if (p.act == B200F_ACT_GATED_SILU) {                   // weight rows alternate: 16 gates, 16 gated
             bf16* out = reinterpret_cast<bf16*>(p.out) + (int64_t)t.b * p.out_bstride + ((ch >> 5) * 16 + (ch & 15));
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
+            for (int j = 0; j < CH; ++j) {
               const float up = __int_as_float(__shfl_down_sync(FULL_MASK, v[j], 16));
               if (ok && lane < 16 && ch < p.N && c0 + j < p.M)
                 out[(int64_t)(c0 + j) * p.out_pitch] = __float2bfloat16_rn(silu_f32(__int_as_float(v[j])) * up);
@@ -305,17 +320,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           } else if (ok && ch < p.N) {
             if (p.act == B200F_ACT_XIELU) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] = __float_as_int(xielu_f32(__int_as_float(v[j]), p.act_a, p.act_b));
+              for (int j = 0; j < CH; ++j) v[j] = __float_as_int(xielu_f32(__int_as_float(v[j]), p.act_a, p.act_b));
             }
             if (p.out_f32) {
               float* out = reinterpret_cast<float*>(p.out) + off;
 #pragma unroll
-              for (int j = 0; j < 32; ++j)
+              for (int j = 0; j < CH; ++j)
                 if (c0 + j < p.M) out[(int64_t)(c0 + j) * p.out_pitch] = __int_as_float(v[j]);
             } else {
               bf16* out = reinterpret_cast<bf16*>(p.out) + off;
 #pragma unroll
-              for (int j = 0; j < 32; ++j)
+              for (int j = 0; j < CH; ++j)
                 if (c0 + j < p.M) out[(int64_t)(c0 + j) * p.out_pitch] = __float2bfloat16_rn(__int_as_float(v[j]));
             }
           }
@@ -683,6 +698,7 @@ extern "C" int b200f_gemm(const void* x, const void* w, void* out, int dtype, in
   p.out = out; p.out_f32 = out_f32 || dtype == B200F_F32; p.M = (int)m; p.N = (int)n; p.K = (int)k; p.batch = (int)batch;
   p.out_pitch = out_pitch; p.out_bstride = out_bstride; p.splits = splits; p.split_stride = split_stride;
   p.act = act; p.act_a = act_a; p.act_b = act_b;
+  p.early = weights_settled(st);
   if (dtype == B200F_F32) {
     if (m <= 8) {
       const float *xf = (const float*)x, *wf = (const float*)w;
@@ -731,6 +747,11 @@ extern "C" int b200f_gemm(const void* x, const void* w, void* out, int dtype, in
     case 64: return launch_bf16<64, 8, false>(ma, mb, p, st);
     default: return launch_bf16<32, 9, false>(ma, mb, p, st);
   }
+}
+
+extern "C" int b200f_settled_weights(int on) {
+  settle(on != 0);
+  return B200_OK;
 }
 
 extern "C" int b200f_gemm_status(int* out_host, int reset) {

@@ -65,6 +65,7 @@ struct GemmParams {
                             // (one tile each, finished in the GEMM kernel); `splits` applies to the blocks after them
   int32_t* partial;         // splits > 1: int32 [M, N] that the parts are added into (zeroed before the launch)
   int split_col0;           // first output channel that belongs to a split block
+  int early;                // the weights are settled: the first ones may be loaded before the wait on earlier kernels
   int tok_tile, tok_tiles;  // two-CTA weights-stationary kernel: tokens per tile (a multiple of 32) and tiles of them; its
                             // blocks are (block of weight rows, token tile), the tiles of one block side by side
   int n_peers;              // > 0: tensor-parallel reduction - every part is added into each of these [M, N] buffers
@@ -141,6 +142,7 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   constexpr int kABytes = kBM * kBK;
   constexpr int kBBytes = BN * kBK;
   constexpr int kStageBytes = kABytes + kBBytes;
+  constexpr bool kFew = WS && BN <= 64;        // what helps a few rows costs more of them time
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~uintptr_t(1023));
   // barriers: full[S], empty[S], tmem_full[2], tmem_empty[2]
   uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + STAGES * kStageBytes);
@@ -186,10 +188,26 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   // meanwhile; more delays the other kernel's own traffic, as any does to the larger batches of the pair kernel (256 tokens:
   // 9.54 -> 9.59 ms).  1.4B-shaped decode step of 37 rows: 1875 -> 1803 us.
   if (WS && warp == 2 && lane == 0) {
-    int left = kAheadBlocks;
+    int skip = kFew && p.early ? STAGES : 0, left = kAheadBlocks;
     for (int tile = blockIdx.x; tile < num_tiles && left > 0; tile += gridDim.x) {
       const WsTile t = tile_of(tile);
-      for (int kb = t.kb0; kb < t.kb1 && left > 0; ++kb, --left) tma_prefetch_2d(&map_a, kb * kBK, t.n_blk * kBM);
+      for (int kb = t.kb0; kb < t.kb1 && left > 0; ++kb) {
+        if (skip > 0) { --skip; continue; }
+        tma_prefetch_2d(&map_a, kb * kBK, t.n_blk * kBM);
+        --left;
+      }
+    }
+  }
+  // Settled weights go straight into the free stages, and behind the wait only the tokens are missing.  (From L2 to shared memory is
+  // not much faster than from HBM, so a prefetch alone leaves most of the time where it was.)
+  unsigned ahead = 0;
+  if (kFew && p.early && warp == 0 && lane == 0) {
+    for (int tile = blockIdx.x; tile < num_tiles && ahead < STAGES; tile += gridDim.x) {
+      const WsTile t = tile_of(tile);
+      for (int kb = t.kb0; kb < t.kb1 && ahead < STAGES; ++kb, ++ahead) {
+        mbar_expect_tx(full0 + 8 * ahead, kStageBytes);
+        tma_load_2d(smem_u32(tiles + ahead * kStageBytes), &map_a, kb * kBK, t.n_blk * kBM, full0 + 8 * ahead);
+      }
     }
   }
   pdl_wait();               // barriers, tensor memory and descriptors are set up; the operands come from earlier kernels
@@ -210,12 +228,14 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const int a_row = (WS ? t.n_blk : tile - t.n_blk * m_tiles) * kBM, b_row = WS ? 0 : t.n_blk * BN;
         for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
           const unsigned s = it % STAGES, ph = (it / STAGES) & 1;
-          ok = mbar_wait(empty0 + 8 * s, ph ^ 1, 1);
-          if (!ok) break;
-          mbar_expect_tx(full0 + 8 * s, kStageBytes);
           const unsigned a_dst = smem_u32(tiles + s * kStageBytes);
-          // map_a always feeds the 128-row operand: weight rows in WS mode (map_b: all tokens), else token rows
-          tma_load_2d(a_dst, &map_a, kb * kBK, a_row, full0 + 8 * s);
+          if (!kFew || it >= ahead) {
+            ok = mbar_wait(empty0 + 8 * s, ph ^ 1, 1);
+            if (!ok) break;
+            mbar_expect_tx(full0 + 8 * s, kStageBytes);
+            // map_a always feeds the 128-row operand: weight rows in WS mode (map_b: all tokens), else token rows
+            tma_load_2d(a_dst, &map_a, kb * kBK, a_row, full0 + 8 * s);
+          }
           tma_load_2d(a_dst + kABytes, &map_b, kb * kBK, b_row, full0 + 8 * s);
         }
       }
@@ -327,17 +347,20 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       epilogue_bar_sync();
       if (ok) ok = mbar_wait(tfull0 + 8 * slot, aph, 3);
       tcgen05_fence_after();
+      // (eight tokens at a time: unrolled over 32, most of the time of a few rows' tile went into fetching the code; many rows are faster
+      // with fewer accesses to tensor memory)
+      constexpr int CH = kFew ? 8 : 32;
 #pragma unroll 1
-      for (int c0 = half * 32; c0 < BN; c0 += 64) {
-        int v[32];
+      for (int c0 = half * CH; c0 < p.M; c0 += 2 * CH) {       // M <= BN
+        int v[CH];
         tmem_ld_32x32(tmem_base + ((unsigned)(q * 32) << 16) + slot * BN + (unsigned)c0, v);
-        if (!ok || c0 >= p.M || ch >= p.N || empty_part) continue;
+        if (!ok || ch >= p.N || empty_part) continue;
         if (p.tp_on) {
           // exchange-block mode: the parts are added into the rank's OWN accumulators (L2 atomics); the peers fetch
           // them from there once this kernel has signalled
           int32_t* dst = p.tp.base[p.tp.rank] + tp_acc_off;
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
+          for (int j = 0; j < CH; ++j)
             if (c0 + j < p.M) atomicAdd(dst + (int64_t)(c0 + j) * p.N + ch, v[j]);
         } else if (p.n_peers > 0) {
           // tensor-parallel sum: the tile's partial sums go straight into every rank's accumulator (a warp's
@@ -346,20 +369,21 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           for (int r = 0; r < p.n_peers; ++r) {
             int32_t* dst = p.peer[r];
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
+            for (int j = 0; j < CH; ++j)
               if (c0 + j < p.M) atomicAdd(dst + (int64_t)(c0 + j) * p.N + ch, v[j]);
           }
         } else if (!direct) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
+          for (int j = 0; j < CH; ++j)
             if (c0 + j < p.M) atomicAdd(p.partial + (int64_t)(c0 + j) * p.N + ch, v[j]);   // result unused: a reduction
         } else {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
+          for (int j = 0; j < CH; ++j) {
             if (c0 + j < p.M) {
               const int64_t o = (int64_t)(c0 + j) * p.N + ch;
               if (p.acc_out) p.acc_out[o] = v[j];
-              if (p.out_q15) p.out_q15[o] = requant_one(v[j], __mulhi(cs[c0 + j], wm), cs[BN + c0 + j] + ws);
+              if (p.out_q15) p.out_q15[o] = kFew ? requant_few(v[j], __mulhi(cs[c0 + j], wm), cs[BN + c0 + j] + ws)
+                                            : requant_one(v[j], __mulhi(cs[c0 + j], wm), cs[BN + c0 + j] + ws);
             }
           }
         }
@@ -984,10 +1008,10 @@ splitk_epilogue_kernel(int32_t* partial, const GemmParams p, int clear) {
     int4 ws = make_int4(31, 31, 31, 31);
     if (p.w_shift) ws = __ldg(reinterpret_cast<const int4*>(p.w_shift + c));
     int4 r;
-    r.x = requant_one(a.x, __mulhi(xm, wm.x), xs + ws.x);
-    r.y = requant_one(a.y, __mulhi(xm, wm.y), xs + ws.y);
-    r.z = requant_one(a.z, __mulhi(xm, wm.z), xs + ws.z);
-    r.w = requant_one(a.w, __mulhi(xm, wm.w), xs + ws.w);
+    r.x = requant_few(a.x, __mulhi(xm, wm.x), xs + ws.x);
+    r.y = requant_few(a.y, __mulhi(xm, wm.y), xs + ws.y);
+    r.z = requant_few(a.z, __mulhi(xm, wm.z), xs + ws.z);
+    r.w = requant_few(a.w, __mulhi(xm, wm.w), xs + ws.w);
     *reinterpret_cast<int4*>(p.out_q15 + o) = r;
     // behind the result's store: a store issued right behind the load of the same address waits for the load's miss
     if (clear) *reinterpret_cast<int4*>(partial + o) = make_int4(0, 0, 0, 0);
@@ -995,7 +1019,7 @@ splitk_epilogue_kernel(int32_t* partial, const GemmParams p, int clear) {
     for (int j = 0; j < 4 && c + j < p.N; ++j) {
       const int a = partial[o + j];
       if (clear) partial[o + j] = 0;
-      p.out_q15[o + j] = requant_one(a, __mulhi(xm, __ldg(p.w_mul + c + j)), xs + (p.w_shift ? __ldg(p.w_shift + c + j) : 31));
+      p.out_q15[o + j] = requant_few(a, __mulhi(xm, __ldg(p.w_mul + c + j)), xs + (p.w_shift ? __ldg(p.w_shift + c + j) : 31));
     }
   }
 }
@@ -1125,6 +1149,7 @@ static int gemm_impl(const int8_t* x8, const int8_t* w8, const int32_t* x_absmax
   p.splits = 1; p.full_blocks = 0; p.partial = nullptr; p.n_peers = 0; p.tp_on = 0; p.split_col0 = 0;
   p.tok_tile = 256; p.tok_tiles = 1;
   cudaStream_t st = (cudaStream_t)s;
+  p.early = weights_settled(st);
   const int num_kb = (int)((k + kBK - 1) / kBK);
   // 65..256 tokens: CTA pairs on blocks of 256 weight rows (each CTA stages half of the 256-token tile; rows beyond
   // the batch are zero fill that costs no traffic); fewer tokens: single CTAs on blocks of 128 weight rows with a
@@ -1245,7 +1270,7 @@ extern "C" int b200_gemm_gate_up_silu(const int8_t* x8, const int8_t* w8, const 
   GemmParams p;
   p.x_absmax = x_absmax; p.x_mul = nullptr; p.x_shift = nullptr; p.w_mul = w_mul; p.w_shift = w_shift;
   p.out_q15 = act_out; p.acc_out = nullptr; p.M = (int)m; p.N = (int)n2; p.K = (int)k;
-  p.n_peers = 0; p.tp_on = 0;
+  p.n_peers = 0; p.tp_on = 0; p.early = 0;
   const int inter = (int)(n2 / 2), w_blocks = inter / kBM, num_kb = (int)((k + kBK - 1) / kBK), units = sm_count() / 2;
   const int tail = w_blocks % units;
   const int split_blocks = w_blocks < units ? w_blocks : tail;
@@ -1288,6 +1313,7 @@ extern "C" int b200_gemm_w8a8_reduce_peers(const int8_t* x8, const int8_t* w8, i
   p.x_absmax = nullptr; p.x_mul = nullptr; p.x_shift = nullptr; p.w_mul = nullptr; p.w_shift = nullptr;
   p.out_q15 = nullptr; p.acc_out = nullptr; p.M = (int)m; p.N = (int)n; p.K = (int)k; p.partial = nullptr; p.split_col0 = 0;
   p.n_peers = n_peers;
+  p.early = 0;
   p.tp_on = 0;
   for (int r = 0; r < 8; ++r) {
     p.peer[r] = r < n_peers ? peer_acc[r] : nullptr;
@@ -1328,6 +1354,7 @@ extern "C" int b200_gemm_w8a8_tp(const b200_tp_block* blk, const int8_t* x8, con
   p.x_absmax = nullptr; p.x_mul = nullptr; p.x_shift = nullptr; p.w_mul = nullptr; p.w_shift = nullptr;
   p.out_q15 = nullptr; p.acc_out = nullptr; p.M = (int)m; p.N = (int)n; p.K = (int)k; p.partial = nullptr; p.split_col0 = 0;
   p.n_peers = 0;
+  p.early = 0;
   p.tp_on = 1;
   p.tp.rank = blk->rank; p.tp.size = blk->size; p.tp.m_max = blk->m_max; p.tp.n = blk->n;
   for (int r = 0; r < 8; ++r) {
@@ -1353,6 +1380,11 @@ extern "C" int b200_gemm_w8a8_tp(const b200_tp_block* blk, const int8_t* x8, con
     case 64: return launch_gemm<64, 8>(ma, mb, p, st);
     default: return launch_gemm<32, 10>(ma, mb, p, st);
   }
+}
+
+extern "C" int b200_settled_weights(int on) {
+  settle(on != 0);
+  return B200_OK;
 }
 
 extern "C" int b200_gemm_status(int* out_host, int reset) {

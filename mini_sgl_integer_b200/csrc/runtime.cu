@@ -24,6 +24,18 @@ bool pdl_enabled() {
   return on != 0;
 }
 
+static thread_local int g_settled = 0;               // 0 no, 1 declared, the plain launch is still to come, 2 yes
+static thread_local cudaStream_t g_settled_stream;
+
+void settle(bool on) { g_settled = on ? 1 : 0; }
+bool settle_takes_first(cudaStream_t st) {
+  if (g_settled != 1) return false;
+  g_settled = 2;
+  g_settled_stream = st;
+  return true;
+}
+bool weights_settled(cudaStream_t st) { return g_settled == 2 && g_settled_stream == st; }
+
 int check_launch(const char* what) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {

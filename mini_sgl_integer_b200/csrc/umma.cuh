@@ -77,6 +77,14 @@ __device__ __forceinline__ void tmem_ld_32x32(unsigned taddr, int (&v)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+__device__ __forceinline__ void tmem_ld_32x32(unsigned taddr, int (&v)[8]) {        // eight columns
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr)
+               : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
 // Shared-memory operand descriptor: K-major tile whose rows are 128 bytes, 128-byte swizzle.
 // Eight rows form one 1024-byte swizzle atom, so the stride between 8-row groups is 1024 bytes;
 // the leading-dimension offset is unused in this mode.  Bits: [0,14) address >> 4,

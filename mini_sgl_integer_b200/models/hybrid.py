@@ -5,6 +5,7 @@ from typing import Optional
 
 import torch
 
+from .._lib import settled_weights
 from ..core import get_global_ctx
 from ..kernel import float_ops as fo
 from ..layers.base import BaseOP
@@ -27,6 +28,7 @@ class HybridForCausalLM(BaseOP):
         rows = batch.logit_rows
         if rows is None and batch.is_prefill:
             rows = batch.attn_metadata.get_last_indices(batch.size).to(torch.int64)
-        return self.forward_tokens(batch.input_ids, batch.attn_metadata, ctx.attn_backend.kvcache, rows)
+        with settled_weights("float"):
+            return self.forward_tokens(batch.input_ids, batch.attn_metadata, ctx.attn_backend.kvcache, rows)
 
     check_status = staticmethod(fo.check_status)

@@ -14,7 +14,7 @@ from typing import Optional
 
 import torch
 
-from .._lib import call, ptr, require_cuda, stream
+from .._lib import call, ptr, require_cuda, settled_weights, stream
 from ..attention import Int8PagedKVCache, new_tokens
 from ..distributed import DistributedCommunicator
 from ..kernel import fixed_point as fp
@@ -207,11 +207,12 @@ class Qwen3ForCausalLMInteger:
     def forward(self, input_ids: torch.Tensor, batch: AttnBatch, last_indices: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Q15.16 logits int32 [rows, vocab]; ``last_indices`` selects the token rows that need logits
         (the last token of every sequence in a prefill batch, BaseAttnMetadata.get_last_indices)."""
-        codes, absmax = self.model.forward(input_ids, batch)
-        if last_indices is not None:
-            idx = last_indices.to(torch.int64)
-            codes, absmax = codes.index_select(0, idx), absmax.index_select(0, idx)
-        return self.method.apply_quantised(self.lm_head, codes, absmax)
+        with settled_weights("int"):
+            codes, absmax = self.model.forward(input_ids, batch)
+            if last_indices is not None:
+                idx = last_indices.to(torch.int64)
+                codes, absmax = codes.index_select(0, idx), absmax.index_select(0, idx)
+            return self.method.apply_quantised(self.lm_head, codes, absmax)
 
     check_status = staticmethod(check_device_status)
 
