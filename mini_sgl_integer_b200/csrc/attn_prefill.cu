@@ -13,17 +13,18 @@
 // accumulator registers: two CTAs per SM then spill.)
 //
 // The softmax is exact (LUT exponential with truncation), so nothing can be rescaled on the fly: the keys are
-// walked three times per tile - row maxima, sums of exponentials, then probabilities and PV - and the scores
-// are recomputed each time.  K is therefore read three times and V once per tile, from L2 after the first touch.
+// walked three times per tile - row maxima, sums of exponentials, then probabilities and PV.  Tensor memory, which
+// the integer MMA does not need, keeps what the next walk wants of the first kPfKept stages (512 keys): a lane's 16
+// scores per stage behind the first walk, their exponentials behind the second, in columns of its own lane.  Those stages read K
+// once and V once; behind them the scores are recomputed in each walk.
 //
-// What bounds it is the latency of dependent integer steps: 115 thread instructions per causal score over the three walks (masked
-// corners of tiles and set-up included), issued on 39 % of the cycles by four warps per scheduler, which wait for fixed
-// latencies and, half as long, for shared memory (128 registers a thread, 8 words of it spilled).  The general steps (64-bit
-// rounding shifts with saturation, clamps, a table in global memory) took 194 instructions on 27 % of the cycles; they
-// remain for scales whose scores could saturate.  Otherwise a score is one wide multiply, one shift and a rounding
+// What bounds it is the latency of dependent integer steps on four warps per scheduler (128 registers a thread, 8 words of it
+// spilled).  Recomputing every score in every walk took 115 thread instructions per causal score (masked corners of tiles and set-up
+// included); of a kept score the second walk is an exponential and a sum, the third a product and the limbs.  The general steps (64-bit
+// rounding shifts with saturation, clamps, a table in global memory) remain for scales whose scores could saturate.  Otherwise a score is one wide multiply, one shift and a rounding
 // step, and its exponential one wide multiply-add: with nx = max - score, P = 94548 nx - 1 + 2^32 has the shift in
 // its high word and, read backwards, the table index on top of its low word (tests/test_kernel_identities.py).
-// 15 prompts of 100 .. 1000 tokens, 32 / 8 heads: 0.80 ms a layer, 1.77 ms with the general steps and one warp per 16 rows.
+// 32 / 8 heads: 15 prompts of 100 .. 1000 tokens 0.59 ms a layer, 0.82 with every score recomputed; one of 333 tokens 27.8 us, 41.3.
 #include "attn_common.cuh"
 #include "luts.cuh"
 
@@ -60,6 +61,9 @@ constexpr int kPfStageBytes = kPfMeta + 4 * 192;
 constexpr int kPfNeg = (int)(-2147483647 - 1);
 constexpr int kPfListPages = 8192;                 // page ids kept in shared memory; those of longer contexts are read where they are
 constexpr int kPfMaxPages = 42624;                 // of a sequence
+// Tensor memory of a CTA: 256 of 512 columns, for two CTAs per SM.  A warp reaches the 32 lanes of its quarter; two warps share
+// each and have half of the columns, 16 for each stage.
+constexpr int kPfColumns = 256, kPfKept = kPfColumns / 2 / 16;
 
 // Shared memory behind the ring.
 struct PfShared {
@@ -69,7 +73,27 @@ struct PfShared {
   int rel[2][kPfKeys];                             // relative V scales of this stage's and the next one's keys
   unsigned long long vref;
   int ks_min, ks_max;
+  unsigned tmem;
 };
+
+// 16 words of every lane to and from its own columns.
+__device__ __forceinline__ void pf_keep(unsigned taddr, const int (&v)[2][2][4]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+               ::"r"(taddr), "r"(v[0][0][0]), "r"(v[0][0][1]), "r"(v[0][0][2]), "r"(v[0][0][3]), "r"(v[0][1][0]), "r"(v[0][1][1]), "r"(v[0][1][2]),
+                 "r"(v[0][1][3]), "r"(v[1][0][0]), "r"(v[1][0][1]), "r"(v[1][0][2]), "r"(v[1][0][3]), "r"(v[1][1][0]), "r"(v[1][1][1]), "r"(v[1][1][2]),
+                 "r"(v[1][1][3])
+               : "memory");
+}
+__device__ __forceinline__ void pf_kept(unsigned taddr, int (&v)[2][2][4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+               : "=r"(v[0][0][0]), "=r"(v[0][0][1]), "=r"(v[0][0][2]), "=r"(v[0][0][3]), "=r"(v[0][1][0]), "=r"(v[0][1][1]), "=r"(v[0][1][2]),
+                 "=r"(v[0][1][3]), "=r"(v[1][0][0]), "=r"(v[1][0][1]), "=r"(v[1][0][2]), "=r"(v[1][0][3]), "=r"(v[1][1][0]), "=r"(v[1][1][1]),
+                 "=r"(v[1][1][2]), "=r"(v[1][1][3])
+               : "r"(taddr)
+               : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void pf_keep_done() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ void mma_u8s8(int (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
   asm volatile(
@@ -104,6 +128,24 @@ attn_prefill_kernel(const PrefillParams p) {
   unsigned char* ring = smem_raw;                                                    // [stages][kPfStageBytes]
   PfShared& sh = *reinterpret_cast<PfShared*>(smem_raw + kPfStages * kPfStageBytes);
   int32_t* pages = reinterpret_cast<int32_t*>(smem_raw + kPfStages * kPfStageBytes + sizeof(PfShared));
+  // In front of the trigger: a GEMM behind this kernel allocates all columns and keeps them while it waits for it, so it may
+  // start only when every CTA here has its own.
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(&sh.tmem)), "r"(kPfColumns) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const unsigned kept = sh.tmem + ((unsigned)((warp & 3) * 32) << 16) + (warp >> 2) * (kPfColumns / 2);
+  auto release = [&]() {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(sh.tmem), "r"(kPfColumns) : "memory");
+    }
+  };
   pdl_launch_dependents();
   for (int i = tid; i < 1024; i += kPfThreads) sh.exp_lut[i] = g_exp2_attn_lut[1023 - i] >> 13;
   if (tid == 0) {
@@ -116,7 +158,10 @@ attn_prefill_kernel(const PrefillParams p) {
   const int L_all = max(0, min(p.kv_lens[b], p.max_kv_len));
   const int n_q = max(0, min(p.q_lens[b], L_all));
   const int n_tiles = (n_q + TQ - 1) / TQ;
-  if ((int)blockIdx.x >= n_tiles) return;            // whole CTA: this sequence has fewer tiles
+  if ((int)blockIdx.x >= n_tiles) {                  // whole CTA: this sequence has fewer tiles
+    release();
+    return;
+  }
   const int tile = n_tiles - 1 - (int)blockIdx.x;    // the tiles with the most keys start first
   const int t0 = tile * TQ;
   const int64_t q_row0 = p.q_start[b];
@@ -141,7 +186,7 @@ attn_prefill_kernel(const PrefillParams p) {
   const unsigned k_dst = ((c_chunk >> 3) << 7) + ((((c_chunk & 7) ^ ((c_chunk >> 3) & 1))) << 4);   // row-parity swizzle
   const int64_t chunk_off = (int64_t)kh * (kPage * kD) + (c_chunk << 4);
   const int64_t page_stride = (int64_t)p.kv_heads * (kPage * kD);
-  auto issue = [&](int stage, bool with_v) {
+  auto issue = [&](int stage, bool with_k, bool with_v) {
     if (stage < n_stages) {
       const unsigned st = ring_base + (stage % kPfStages) * kPfStageBytes;
 #pragma unroll
@@ -149,7 +194,7 @@ attn_prefill_kernel(const PrefillParams p) {
         const int pi = c_page + 2 * i, pg = 4 * stage + pi;
         if (pg < n_pages) {
           const int64_t off = page_id(pg) * page_stride + chunk_off;
-          cp_async16(st + pi * 2048 + k_dst, reinterpret_cast<const unsigned char*>(p.k_codes) + off);
+          if (with_k) cp_async16(st + pi * 2048 + k_dst, reinterpret_cast<const unsigned char*>(p.k_codes) + off);
           if (with_v) cp_async16(st + kPfV + pi * 2048 + (c_chunk << 4), reinterpret_cast<const unsigned char*>(p.v_codes) + off);
         }
       }
@@ -162,7 +207,7 @@ attn_prefill_kernel(const PrefillParams p) {
     }
     cp_async_commit();
   };
-  for (int j = 0; j < kPfStages - 1; ++j) issue(j, false);
+  for (int j = 0; j < kPfStages - 1; ++j) issue(j, true, false);
 
   // ---- over ALL keys of the sequence: the reference V scale, and the range of the K shifts
   {
@@ -260,11 +305,11 @@ attn_prefill_kernel(const PrefillParams p) {
     }
   };
   // Walks the stages; body(stage's shared memory, first key of this warp's pair of pages).
-  auto walk = [&](bool with_v, auto&& ahead, auto&& body) {
-    for (int stage = 0; stage < n_stages; ++stage) {
+  auto walk = [&](int first, bool with_v, auto&& ahead, auto&& body) {
+    for (int stage = first; stage < n_stages; ++stage) {
       cp_async_wait<kPfStages - 3>();                    // this stage and the next one
       __syncthreads();                                   // ... have landed for everybody; the stage before is free
-      issue(stage + kPfStages - 1, with_v);
+      issue(stage + kPfStages - 1, !with_v || stage + kPfStages - 1 >= kPfKept, with_v);
       ahead(stage);
       if (stage * kPfKeys < lim_any) body(ring + (stage % kPfStages) * kPfStageBytes, stage * kPfKeys + side * 32, stage);
     }
@@ -274,10 +319,11 @@ attn_prefill_kernel(const PrefillParams p) {
 
   // ---- pass 1: row maxima
   int row_max[2] = {kPfNeg, kPfNeg};
-  walk(false, [](int) {}, [&](const unsigned char* st, int key0, int) {
+  walk(0, false, [](int) {}, [&](const unsigned char* st, int key0, int stage) {
     if (key0 >= lim_any) return;
     int sc[2][2][4];
     scores(st, sc);
+    if (stage < kPfKept) pf_keep(kept + 16 * stage, sc);
     const bool all = key0 + 32 <= lim_all;
 #pragma unroll
     for (int h = 0; h < 2; ++h)
@@ -287,7 +333,8 @@ attn_prefill_kernel(const PrefillParams p) {
         for (int e = 0; e < 4; ++e)
           if (all || key0 + pg * 16 + 4 * fc + e < lim[h]) row_max[h] = max(row_max[h], sc[h][pg][e]);
   });
-  for (int j = 0; j < kPfStages - 1; ++j) issue(j, false);
+  pf_keep_done();
+  for (int j = 0; j < kPfStages - 1; ++j) issue(kPfKept + j, true, false);
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     row_max[h] = max(row_max[h], __shfl_xor_sync(FULL_MASK, row_max[h], 1));
@@ -304,12 +351,9 @@ attn_prefill_kernel(const PrefillParams p) {
     exp_c[h] = (long long)row_max[h] * 94548LL - 1LL + (1LL << 32);
   }
 
-  // ---- pass 2: sums of exponentials
+  // ---- pass 2: sums of exponentials; sc becomes the exponentials, 0 for keys that the row does not see
   unsigned row_sum[2] = {0u, 0u};
-  walk(false, [](int) {}, [&](const unsigned char* st, int key0, int) {
-    if (key0 >= lim_any) return;
-    int sc[2][2][4];
-    scores(st, sc);
+  auto exponentials = [&](int (&sc)[2][2][4], int key0) {
     const bool all = key0 + 32 <= lim_all;
 #pragma unroll
     for (int h = 0; h < 2; ++h)
@@ -318,10 +362,36 @@ attn_prefill_kernel(const PrefillParams p) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const unsigned v = pf_exp(sc[h][pg][e], exp_c[h], sh.exp_lut);
-          if (all || key0 + pg * 16 + 4 * fc + e < lim[h]) row_sum[h] += v;
+          sc[h][pg][e] = all || key0 + pg * 16 + 4 * fc + e < lim[h] ? (int)v : 0;
         }
+  };
+  auto add_up = [&](const int (&sc)[2][2][4]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int pg = 0; pg < 2; ++pg)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) row_sum[h] += (unsigned)sc[h][pg][e];
+  };
+#pragma unroll 1
+  for (int stage = 0; stage < min(n_stages, kPfKept); ++stage) {
+    const int key0 = stage * kPfKeys + side * 32;
+    if (key0 >= lim_any) break;
+    int sc[2][2][4];
+    pf_kept(kept + 16 * stage, sc);
+    exponentials(sc, key0);
+    pf_keep(kept + 16 * stage, sc);
+    add_up(sc);
+  }
+  walk(kPfKept, false, [](int) {}, [&](const unsigned char* st, int key0, int) {
+    if (key0 >= lim_any) return;
+    int sc[2][2][4];
+    scores(st, sc);
+    exponentials(sc, key0);
+    add_up(sc);
   });
-  for (int j = 0; j < kPfStages - 1; ++j) issue(j, true);
+  pf_keep_done();
+  for (int j = 0; j < kPfStages - 1; ++j) issue(j, j >= kPfKept, true);
   unsigned inv[2];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -356,14 +426,18 @@ attn_prefill_kernel(const PrefillParams p) {
   cp_async_wait<kPfStages - 2>();
   __syncthreads();                                       // the first stage; and the sums have been read
   if (tid < kPfKeys) rel_scales(0, tid);
-  walk(true, [&](int stage) {
+  walk(0, true, [&](int stage) {
     if (stage + 1 < n_stages && group == (stage & (kPfGroups - 1))) rel_scales(stage + 1, tid & (kPfKeys - 1));
   }, [&](const unsigned char* st, int key0, int stage) {
     uint4 own_hi = make_uint4(0, 0, 0, 0), own_lo = make_uint4(0, 0, 0, 0);      // [row h, page]: keys 4 fc .. 4 fc + 3 as bytes
     if (key0 < lim_any) {
       int sc[2][2][4];
-      scores(st, sc);
-      const bool all = key0 + 32 <= lim_all;
+      if (stage < kPfKept) {
+        pf_kept(kept + 16 * stage, sc);
+      } else {
+        scores(st, sc);
+        exponentials(sc, key0);
+      }
       unsigned ah[2][2], al[2][2];
 #pragma unroll
       for (int pg = 0; pg < 2; ++pg) {
@@ -374,9 +448,8 @@ attn_prefill_kernel(const PrefillParams p) {
           unsigned w[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            const unsigned pr = (pf_exp(sc[h][pg][e], exp_c[h], sh.exp_lut) * inv[h]) >> 16;
+            const unsigned pr = ((unsigned)sc[h][pg][e] * inv[h]) >> 16;
             w[e] = (pr * r[e] + 16384u) >> 15;
-            if (!(all || key0 + pg * 16 + 4 * fc + e < lim[h])) w[e] = 0u;
           }
           const unsigned w01 = __byte_perm(w[0], w[1], 0x5410), w23 = __byte_perm(w[2], w[3], 0x5410);
           ah[h][pg] = __byte_perm(w01, w23, 0x7531);
@@ -450,6 +523,7 @@ attn_prefill_kernel(const PrefillParams p) {
       }
     }
   }
+  release();
 }
 
 template <int G>
