@@ -318,6 +318,9 @@ B200_API int b200_gemm_w8a8_absmax(const int8_t* x8, const int8_t* w8, const int
  * that is ALL ZERO whenever no call is using it (allocate it zeroed once):
  *   b200_gemm_w8a8_absmax_ws  the linear of b200_gemm_w8a8_absmax; split-K parts are added into zero_ws without a
  *                             clearing launch and the requantising kernel zeroes what it read.  out_q15 != zero_ws.
+ *   b200_gemm_w8a8_absmax_tail (m <= 256) without the requantising kernel: columns that whole tiles gave are in out_q15, the others, from
+ *                             *tail_col0 (host memory; a multiple of 128, or n) on, stay exact accumulators in zero_ws, for
+ *                             b200_silu_mul_q15_tail: b200_silu_mul_q15 with codes on such a gate_up result (it zeroes them again).
  *   b200_gemm_w8a8_acc_ws     leaves the exact accumulators in zero_ws; exactly one of the two calls below must then
  *                             consume them (they zero the buffer again) before zero_ws is reused.
  *   b200_rmsnorm_q15_pending  b200_rmsnorm_q15 with x = the Q15.16 result of that linear, computed on the fly from
@@ -327,6 +330,12 @@ B200_API int b200_gemm_w8a8_absmax(const int8_t* x8, const int8_t* w8, const int
  *                             * 128], q | k | v heads side by side).
  * No reference counterpart: the reference materialises every linear's output (layers/quantization/w8a8_int8.py:242-286)
  * before RMSNorm (models/integer/qwen3_integer.py:62-80) or q/k-norm + RoPE (models/utils_integer.py:209-227) read it. */
+B200_API int b200_gemm_w8a8_absmax_tail(const int8_t* x8, const int8_t* w8, const int32_t* x_absmax, const int32_t* w_mul,
+                                        const int32_t* w_shift, int32_t* out_q15, int32_t* zero_ws, int64_t* tail_col0, int64_t m, int64_t n,
+                                        int64_t k, b200_stream_t s);
+B200_API int b200_silu_mul_q15_tail(const int32_t* gate_up, int32_t* acc, const int32_t* x_absmax, const int32_t* w_mul, const int32_t* w_shift,
+                                    int64_t tail_col0, int8_t* codes, float* scale, int32_t* absmax, int64_t rows, int inter, int fwht_block,
+                                    b200_stream_t s);
 B200_API int b200_gemm_w8a8_absmax_ws(const int8_t* x8, const int8_t* w8, const int32_t* x_absmax, const int32_t* w_mul,
                                       const int32_t* w_shift, int32_t* out_q15, int32_t* zero_ws, int64_t m, int64_t n,
                                       int64_t k, b200_stream_t s);

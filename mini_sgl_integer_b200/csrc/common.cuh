@@ -30,8 +30,8 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // without it, or after a kernel that never triggers, behaves as usual.
 bool pdl_enabled();
 
-// While a thread has declared the weights settled (b200_settled_weights, b200f_settled_weights), its GEMMs of decode size read them
-// before their wait.  That needs everything that wrote a weight to have completed and be visible when such a GEMM starts, which may be as
+// While a thread has declared weights and inputs of a step settled (b200_settled_weights, b200f_settled_weights), the kernels of a decode step read
+// them before their wait.  That needs everything that wrote them to have completed and be visible when such a kernel starts, which may be as
 // early as the kernels in front of it trigger.  So the scope's first launch is a plain one: it starts once all earlier
 // work of the stream has completed, and no later launch of the stream starts before it.
 void settle(bool on);
@@ -65,6 +65,28 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 __device__ __forceinline__ int sat32(long long v) {
   return v > 2147483647LL ? 2147483647 : (v < -2147483648LL ? (int)(-2147483647 - 1) : (int)v);
 }
+
+// Loads that stay on their side of pdl_wait().  A kernel with loads in front of its wait reads everything with these that another
+// kernel may have written: the compiler takes __ldg, __ldcs and loads through const __restrict__ pointers for loads of memory that
+// nobody writes and moves them in front of the wait with the others.
+__device__ __forceinline__ int fresh1(const int32_t* p) {
+  int v;
+  asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ int2 fresh2(const int32_t* p) {
+  int2 v;
+  asm volatile("ld.global.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ int4 fresh4(const int32_t* p) {
+  int4 v;
+  asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+
+// The 128-byte line of `p` on its way into L2: nothing is read, so this may stand in front of pdl_wait() whoever writes there.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // |x| with two's-complement wrap (|-2^31| stays -2^31), as the reference's where(x<0,-x,x).
 __device__ __forceinline__ int abs_wrap(int x) { return x < 0 ? (int)(0u - (unsigned)x) : x; }
@@ -214,7 +236,8 @@ __device__ __forceinline__ int norm_normalised_sq(int v, int p) {
 }
 // inverse_sqrt_q0_31 (rmsnorm_int_only_v2.py:89-117) of ms = ((S / H) >> 1) + 1.
 __device__ __forceinline__ int norm_inv_sqrt(long long S, int H, const int32_t* lut) {
-  int ms = (int)((S / H) >> 1) + 1;
+  // (S >= 0; a 64-bit division is some hundred cycles in the middle of the row's chain of dependent steps)
+  int ms = (int)(((H & (H - 1)) == 0 ? S >> (31 - __clz(H)) : S / H) >> 1) + 1;
   if (ms <= 0) return 0;
   int pos = 31 - __clz(ms);
   int even = ((pos + 1) >> 1) << 1;
@@ -278,12 +301,23 @@ struct PendingLinear {
   const int32_t* w_shift;     // nullable: 31 everywhere
 };
 
-__device__ __forceinline__ int2 pending_take2(const PendingLinear& pl, int64_t row, int n, int col, int xm, int xs48) {
-  const int2 a = *reinterpret_cast<const int2*>(pl.acc + row * n + col);
-  const int2 wm = __ldg(reinterpret_cast<const int2*>(pl.w_mul + col));
-  int2 ws = make_int2(31, 31);
-  if (pl.w_shift) ws = __ldg(reinterpret_cast<const int2*>(pl.w_shift + col));
+// The channels' scales, which a kernel may have before the accumulators.
+__device__ __forceinline__ void pending_scales2(const PendingLinear& pl, int col, int2& wm, int2& ws) {
+  wm = fresh2(pl.w_mul + col);
+  ws = make_int2(31, 31);
+  if (pl.w_shift) ws = fresh2(pl.w_shift + col);
+}
+__device__ __forceinline__ void pending_scales4(const PendingLinear& pl, int col, int4& wm, int4& ws) {
+  wm = fresh4(pl.w_mul + col);
+  ws = make_int4(31, 31, 31, 31);
+  if (pl.w_shift) ws = fresh4(pl.w_shift + col);
+}
+__device__ __forceinline__ int2 pending_requant2(int2 a, int2 wm, int2 ws, int xm, int xs48) {
   return make_int2(requant_few(a.x, __mulhi(xm, wm.x), xs48 + ws.x), requant_few(a.y, __mulhi(xm, wm.y), xs48 + ws.y));
+}
+__device__ __forceinline__ int4 pending_requant4(int4 a, int4 wm, int4 ws, int xm, int xs48) {
+  return make_int4(requant_few(a.x, __mulhi(xm, wm.x), xs48 + ws.x), requant_few(a.y, __mulhi(xm, wm.y), xs48 + ws.y),
+                   requant_few(a.z, __mulhi(xm, wm.z), xs48 + ws.z), requant_few(a.w, __mulhi(xm, wm.w), xs48 + ws.w));
 }
 
 __device__ __forceinline__ void pending_clear2(const PendingLinear& pl, int64_t row, int n, int col) {
@@ -293,16 +327,23 @@ __device__ __forceinline__ void pending_clear4(const PendingLinear& pl, int64_t 
   *reinterpret_cast<int4*>(pl.acc + row * n + col) = make_int4(0, 0, 0, 0);
 }
 
+__device__ __forceinline__ int2 pending_take2(const PendingLinear& pl, int64_t row, int n, int col, int xm, int xs48) {
+  const int2 a = *reinterpret_cast<const int2*>(pl.acc + row * n + col);
+  const int2 wm = __ldg(reinterpret_cast<const int2*>(pl.w_mul + col));
+  int2 ws = make_int2(31, 31);
+  if (pl.w_shift) ws = __ldg(reinterpret_cast<const int2*>(pl.w_shift + col));
+  return make_int2(requant_one(a.x, __mulhi(xm, wm.x), xs48 + ws.x), requant_one(a.y, __mulhi(xm, wm.y), xs48 + ws.y));
+}
 __device__ __forceinline__ int4 pending_take4(const PendingLinear& pl, int64_t row, int n, int col, int xm, int xs48) {
   const int4 a = *reinterpret_cast<const int4*>(pl.acc + row * n + col);
   const int4 wm = __ldg(reinterpret_cast<const int4*>(pl.w_mul + col));
   int4 ws = make_int4(31, 31, 31, 31);
   if (pl.w_shift) ws = __ldg(reinterpret_cast<const int4*>(pl.w_shift + col));
   int4 r;
-  r.x = requant_few(a.x, __mulhi(xm, wm.x), xs48 + ws.x);
-  r.y = requant_few(a.y, __mulhi(xm, wm.y), xs48 + ws.y);
-  r.z = requant_few(a.z, __mulhi(xm, wm.z), xs48 + ws.z);
-  r.w = requant_few(a.w, __mulhi(xm, wm.w), xs48 + ws.w);
+  r.x = requant_one(a.x, __mulhi(xm, wm.x), xs48 + ws.x);
+  r.y = requant_one(a.y, __mulhi(xm, wm.y), xs48 + ws.y);
+  r.z = requant_one(a.z, __mulhi(xm, wm.z), xs48 + ws.z);
+  r.w = requant_one(a.w, __mulhi(xm, wm.w), xs48 + ws.w);
   return r;
 }
 

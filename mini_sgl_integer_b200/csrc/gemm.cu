@@ -1128,10 +1128,13 @@ using namespace b200;
 
 static int gemm_impl(const int8_t* x8, const int8_t* w8, const int32_t* x_absmax, const int32_t* x_mul,
                      const int32_t* x_shift, const int32_t* w_mul, const int32_t* w_shift, int32_t* out_q15,
-                     int32_t* acc_out, int64_t m, int64_t n, int64_t k, b200_stream_t s, int32_t* zero_ws = nullptr) {
+                     int32_t* acc_out, int64_t m, int64_t n, int64_t k, b200_stream_t s, int32_t* zero_ws = nullptr,
+                     int64_t* tail_col0 = nullptr) {
   // zero_ws: a caller-kept [m, n] int32 workspace that is all zero on entry; split-K parts are added into it without
   // a clearing launch.  With a Q15.16 output the requantising kernel zeroes it again; with acc_out == zero_ws (no
   // Q15.16 output) it holds the exact accumulators on return and whoever consumes them clears it.
+  // tail_col0 (with zero_ws and a Q15.16 output): the blocks that were split stay accumulators in zero_ws, from column *tail_col0 on
+  // (n: there are none), and their consumer finishes and clears them.
   B200_REQUIRE(x8 && w8, B200_E_NULL, "gemm_w8a8: x8 or w8 is null");
   B200_REQUIRE(out_q15 || acc_out, B200_E_NULL, "gemm_w8a8: no output requested");
   B200_REQUIRE(!out_q15 || (((x_mul && x_shift) || x_absmax) && w_mul), B200_E_NULL,
@@ -1212,7 +1215,8 @@ static int gemm_impl(const int8_t* x8, const int8_t* w8, const int32_t* x_absmax
       case 64: rc = launch_gemm<64, 8>(ma, mb, p, st); break;
       default: rc = launch_gemm<32, 10>(ma, mb, p, st); break;
     }
-    if (rc != B200_OK || splits == 1 || !out_q15) return rc;
+    if (tail_col0) *tail_col0 = splits == 1 ? n : col0;
+    if (rc != B200_OK || splits == 1 || !out_q15 || tail_col0) return rc;
     launch_pdl(splitk_epilogue_kernel, dim3((unsigned)((n - col0 + 1023) / 1024), (unsigned)m), dim3(256), 0, st, p.partial, p, zero_ws ? 1 : 0);
     return check_launch("gemm_w8a8 (split-K epilogue)");
   }
@@ -1247,6 +1251,17 @@ extern "C" int b200_gemm_w8a8_absmax_ws(const int8_t* x8, const int8_t* w8, cons
   B200_REQUIRE(aligned16(zero_ws) && zero_ws != out_q15, B200_E_ALIGN,
                "gemm_w8a8_absmax_ws: the workspace must be 16-byte aligned and distinct from the output");
   return gemm_impl(x8, w8, x_absmax, nullptr, nullptr, w_mul, w_shift, out_q15, nullptr, m, n, k, s, zero_ws);
+}
+
+extern "C" int b200_gemm_w8a8_absmax_tail(const int8_t* x8, const int8_t* w8, const int32_t* x_absmax, const int32_t* w_mul,
+                                          const int32_t* w_shift, int32_t* out_q15, int32_t* zero_ws, int64_t* tail_col0, int64_t m, int64_t n,
+                                          int64_t k, b200_stream_t s) {
+  B200_REQUIRE(x_absmax && out_q15 && zero_ws && tail_col0, B200_E_NULL, "gemm_w8a8_absmax_tail: null pointer");
+  B200_REQUIRE(aligned16(zero_ws) && zero_ws != out_q15, B200_E_ALIGN,
+               "gemm_w8a8_absmax_tail: the workspace must be 16-byte aligned and distinct from the output");
+  B200_REQUIRE(m <= 256, B200_E_UNSUPPORTED, "gemm_w8a8_absmax_tail: m=%lld (at most 256)", (long long)m);
+  *tail_col0 = n;
+  return gemm_impl(x8, w8, x_absmax, nullptr, nullptr, w_mul, w_shift, out_q15, nullptr, m, n, k, s, zero_ws, tail_col0);
 }
 
 extern "C" int b200_gemm_w8a8_acc_ws(const int8_t* x8, const int8_t* w8, int32_t* zero_ws, int64_t m, int64_t n, int64_t k,

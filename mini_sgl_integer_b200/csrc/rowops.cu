@@ -4,6 +4,8 @@
 // its reductions, so every input element is read from HBM once.
 #include <cuda_bf16.h>
 
+#include <cooperative_groups.h>
+
 #include <cstdlib>
 
 #include "common.cuh"
@@ -57,16 +59,51 @@ static int elementwise_grid(int64_t n, int threads) {
 // One CTA per row; thread t owns int4 vectors t, t+T, ... (VPT of them).
 // FULL: the row is exactly blockDim.x * VPT vectors long (no bounds checks on the vector index).
 // PENDING: x is null and the row comes from a linear's exact accumulators, requantised while it is loaded.
+// Few rows are a chain of latencies: the loads, three reductions, the table, the codes.  So up to two vectors per thread (a decode
+// batch) have the table in shared memory and gains and scales on their way before the wait - in registers if they are settled
+// (`early`), else in L2, where weights streaming through have displaced them - and one barrier per reduction.
 template <int VPT, bool FULL, bool PENDING = false>
 __global__ void __launch_bounds__(1024)
 rmsnorm_rows_kernel(const int32_t* __restrict__ x, const int32_t* __restrict__ res,
                     const int32_t* __restrict__ w, int32_t* __restrict__ res_out,
                     int32_t* __restrict__ norm_out, int8_t* __restrict__ codes,
-                    float* __restrict__ scale, int32_t* __restrict__ absmax, int H, const PendingLinear pl) {
-  __shared__ long long red64[33];
-  __shared__ int red32[33];
+                    float* __restrict__ scale, int32_t* __restrict__ absmax, int H, const PendingLinear pl, int early) {
+  constexpr bool kAhead = VPT <= 2;
+  __shared__ long long red64[32];
+  __shared__ int red_a[32], red_b[32];
+  __shared__ int32_t lut_s[kAhead ? 1024 : 1];
   pdl_launch_dependents();
+  const int4* wr = reinterpret_cast<const int4*>(w);
+  int4 gain[kAhead ? VPT : 1], wm[kAhead && PENDING ? VPT : 1], ws[kAhead && PENDING ? VPT : 1];
+  auto constants = [&]() {
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int idx = threadIdx.x + i * blockDim.x, at = FULL || idx < (H >> 2) ? idx : 0;
+      gain[kAhead ? i : 0] = fresh4(w + 4 * at);
+      if (PENDING) pending_scales4(pl, 4 * at, wm[kAhead ? i : 0], ws[kAhead ? i : 0]);
+    }
+  };
+  if (kAhead) {
+    for (int i = threadIdx.x; i < 1024; i += blockDim.x) lut_s[i] = g_inv_sqrt_lut[i];
+    if (early) {
+      constants();
+    } else if (PENDING) {
+      for (int c = threadIdx.x * 32; c < H; c += blockDim.x * 32) {
+        prefetch_l2(w + c);
+        prefetch_l2(pl.w_mul + c);
+        if (pl.w_shift) prefetch_l2(pl.w_shift + c);
+      }
+    }
+  }
   pdl_wait();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  auto row_max = [&](int v, int* red) {
+    v = warp_max(v);
+    if (nw == 1) return v;
+    if (lane == 0) red[wid] = v;
+    __syncthreads();
+    return warp_max(lane < nw ? red[lane] : (int)(-2147483647 - 1));
+  };
   const int64_t row = blockIdx.x;
   const int nvec = H >> 2;
   const int4* xr = PENDING ? nullptr : reinterpret_cast<const int4*>(x + row * H);
@@ -74,22 +111,11 @@ rmsnorm_rows_kernel(const int32_t* __restrict__ x, const int32_t* __restrict__ r
   int4* ro = res ? reinterpret_cast<int4*>(res_out + row * H) : nullptr;
   int pxm = 0, pxs = 0;
   if (PENDING) {
-    absmax_to_ms_dev(__ldg(pl.x_absmax + row), &pxm, &pxs);
+    absmax_to_ms_dev(fresh1(pl.x_absmax + row), &pxm, &pxs);
     pxs -= 48;
   }
 
-  // the norm gains do not depend on the row: with few vectors per thread they are requested up front, so that their
-  // latency hides behind the first reduction instead of following the second
-  constexpr bool kEarlyGain = VPT <= 2;
-  const int4* wr = reinterpret_cast<const int4*>(w);
-  int4 gain[kEarlyGain ? VPT : 1];
-  if (kEarlyGain) {
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int idx = threadIdx.x + i * blockDim.x;
-      gain[i] = (FULL || idx < nvec) ? __ldg(wr + idx) : make_int4(0, 0, 0, 0);
-    }
-  }
+  if (kAhead && !early) constants();
 
   int4 v[VPT];
   int m = 0;
@@ -98,10 +124,11 @@ rmsnorm_rows_kernel(const int32_t* __restrict__ x, const int32_t* __restrict__ r
     const int idx = threadIdx.x + i * blockDim.x;
     int4 a = make_int4(0, 0, 0, 0);
     if (FULL || idx < nvec) {
-      if (PENDING) a = pending_take4(pl, row, H, idx * 4, pxm, pxs);
-      else a = __ldcs(xr + idx);
+      if (PENDING && kAhead) a = pending_requant4(fresh4(pl.acc + row * H + idx * 4), wm[kAhead ? i : 0], ws[kAhead ? i : 0], pxm, pxs);
+      else if (PENDING) a = pending_take4(pl, row, H, idx * 4, pxm, pxs);
+      else a = kAhead ? fresh4(x + row * H + 4 * idx) : __ldcs(xr + idx);
       if (rr) {
-        int4 b = __ldcs(rr + idx);
+        int4 b = kAhead ? fresh4(res + row * H + 4 * idx) : __ldcs(rr + idx);
         a.x = (int)((unsigned)a.x + (unsigned)b.x);
         a.y = (int)((unsigned)a.y + (unsigned)b.y);
         a.z = (int)((unsigned)a.z + (unsigned)b.z);
@@ -112,7 +139,7 @@ rmsnorm_rows_kernel(const int32_t* __restrict__ x, const int32_t* __restrict__ r
     v[i] = a;
     m = max(max(m, abs_wrap(a.x)), max(abs_wrap(a.y), max(abs_wrap(a.z), abs_wrap(a.w))));
   }
-  m = block_max(m, red32);
+  m = row_max(m, red_a);
   if (PENDING) {   // the accumulators have arrived (the reduction used them): leave zeros behind
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
@@ -128,8 +155,15 @@ rmsnorm_rows_kernel(const int32_t* __restrict__ x, const int32_t* __restrict__ r
     S += (long long)norm_normalised_sq(v[i].x, nr.p) + (long long)norm_normalised_sq(v[i].y, nr.p) +
          (long long)norm_normalised_sq(v[i].z, nr.p) + (long long)norm_normalised_sq(v[i].w, nr.p);
   }
-  S = block_sum64(S, red64);
-  const int inv = norm_inv_sqrt(S, H, g_inv_sqrt_lut);
+  S = warp_sum64(S);
+  if (nw > 1) {
+    if (lane == 0) red64[wid] = S;
+    __syncthreads();
+    S = warp_sum64(lane < nw ? red64[lane] : 0);
+  } else {
+    __syncwarp();                              // the table is the warp's own
+  }
+  const int inv = norm_inv_sqrt(S, H, kAhead ? lut_s : g_inv_sqrt_lut);
 
   int4* no = norm_out ? reinterpret_cast<int4*>(norm_out + row * H) : nullptr;
   int m2 = 0;
@@ -138,7 +172,7 @@ rmsnorm_rows_kernel(const int32_t* __restrict__ x, const int32_t* __restrict__ r
     for (int i = 0; i < VPT; ++i) {
       const int idx = threadIdx.x + i * blockDim.x;
       if (FULL || idx < nvec) {
-        const int4 ww = kEarlyGain ? gain[i] : __ldg(wr + idx);
+        const int4 ww = kAhead ? gain[kAhead ? i : 0] : __ldg(wr + idx);
         const int4 o = make_int4(element(v[i].x, ww.x), element(v[i].y, ww.y), element(v[i].z, ww.z), element(v[i].w, ww.w));
         v[i] = o;
         if (no) no[idx] = o;
@@ -149,7 +183,7 @@ rmsnorm_rows_kernel(const int32_t* __restrict__ x, const int32_t* __restrict__ r
   if (nr.p >= 14) apply([&](int x1, int w1) { return norm_apply_high(x1, inv, w1, nr.p - 14); });
   else apply([&](int x1, int w1) { return nr.zero ? 0 : norm_apply(x1, inv, w1, nr.p); });
   if (codes == nullptr) return;
-  m2 = max(1, block_max(m2, red32));
+  m2 = max(1, row_max(m2, red_b));
   const float mf = __int2float_rn(m2);
   const float my = __frcp_rn(mf);
   unsigned* co = reinterpret_cast<unsigned*>(codes + row * H);
@@ -389,11 +423,11 @@ static int silu_threads(int nblocks) {
 // row, all of them resident), quantises with the agreed value and reports it; `scale` is not written.
 // ACT = false: `gate_up` already holds SiLU(gate) * up, int32 [rows, I] (the gate_up GEMM applied it in its epilogue);
 // the kernel then only rotates and quantises.
-template <bool FWHT, bool QUANT, bool TABLE, bool TP = false, bool ACT = true>
+template <bool FWHT, bool QUANT, bool TABLE, bool TP = false, bool ACT = true, bool TAIL = false>
 __global__ void __launch_bounds__(kSiluMaxThreads, 2)
 silu_rows_kernel(const int32_t* __restrict__ gate_up, int32_t* __restrict__ q15_out,
                  int8_t* __restrict__ codes, float* __restrict__ scale,
-                 int32_t* __restrict__ absmax, int64_t rows, int I, const TpAgree agree) {
+                 int32_t* __restrict__ absmax, int64_t rows, int I, const TpAgree agree, const PendingLinear pl, int tail_col0) {
   extern __shared__ __align__(16) int32_t rowbuf[];   // QUANT: [I] results of the row; then the table
   __shared__ int red32[2][32];
   __shared__ int agree_slot;
@@ -427,6 +461,11 @@ silu_rows_kernel(const int32_t* __restrict__ gate_up, int32_t* __restrict__ q15_
       asm volatile("cp.async.bulk.prefetch.L2.global [%0], 512;" ::"l"(next + (size_t)c * 512) : "memory");
   }
 
+  int pxm = 0, pxs = 0;
+  if (TAIL) {
+    absmax_to_ms_dev(fresh1(pl.x_absmax + row), &pxm, &pxs);
+    pxs -= 48;
+  }
   int m = 0;
   unsigned small_its = 0;                        // bit `it`: the iteration's values came from the path without saturation
   for (int it = 0; it < niter; ++it) {           // the shuffles need whole warps: a warp leaves when none of its
@@ -436,8 +475,14 @@ silu_rows_kernel(const int32_t* __restrict__ gate_up, int32_t* __restrict__ q15_
     if (live_mask == 0) break;
     const bool all_live = live_mask == FULL_MASK;  // the usual case: no zero fill in front of the loads
     int val[16];
+    const bool gate_tail = TAIL && live && b * 128 >= tail_col0, up_tail = TAIL && live && I + b * 128 >= tail_col0;
     auto load = [&](int k, int4& g, int4& u) {
       const int off = b * 128 + k * 32 + lane8 * 4;
+      if (TAIL && (gate_tail || up_tail)) {
+        g = gate_tail ? pending_take4(pl, row, 2 * I, off, pxm, pxs) : __ldcs(reinterpret_cast<const int4*>(gate + off));
+        u = up_tail ? pending_take4(pl, row, 2 * I, I + off, pxm, pxs) : __ldcs(reinterpret_cast<const int4*>(up + off));
+        return;
+      }
       if (all_live) {
         g = __ldcs(reinterpret_cast<const int4*>(gate + off));
         u = ACT ? __ldcs(reinterpret_cast<const int4*>(up + off)) : make_int4(0, 0, 0, 0);
@@ -577,11 +622,127 @@ silu_rows_kernel(const int32_t* __restrict__ gate_up, int32_t* __restrict__ q15_
       }
     }
   }
+  if (TAIL) {                          // every value has been used: zeros for the next GEMM's parts
+    int32_t* acc = pl.acc + row * 2 * I;
+    for (int c = tail_col0 + 4 * threadIdx.x; c < 2 * I; c += 4 * blockDim.x) *reinterpret_cast<int4*>(acc + c) = make_int4(0, 0, 0, 0);
+  }
   if (threadIdx.x == 0) {
     if (!TP) scale[row] = quant_scale(mf);
     absmax[row] = m;
   }
   if (TP) __syncthreads();             // the agreement's shared word is reused by the next row
+  }
+}
+
+// The same for few rows: a row is a cluster of CTAs, a 128-block a warp (four values per lane, the rotation's upper five stages over the
+// lanes), and the CTAs agree on the row's absmax over distributed shared memory.  With a row per CTA most SMs idle and a chain of
+// loads, 48 shuffles and two passes takes its time; here results stay in registers.  The clusters walk the rows with their number as stride.
+// TAIL: the columns from `tail_col0` on (a multiple of 128) of the row are still the exact accumulators of the linear in front, in
+// `pl.acc` ([rows, 2 I]): requantised while they are loaded, zeroed behind.  One row of 12288 columns: 6.8 -> 2.3 us (in a chain of
+// launches); a decode step of one request (8B) 3215 -> 2811 with the other kernels' early loads.
+template <bool FWHT, bool TAIL>
+__global__ void __launch_bounds__(1024, 1)
+silu_few_rows_kernel(const int32_t* __restrict__ gate_up, int8_t* __restrict__ codes, float* __restrict__ scale,
+                     int32_t* __restrict__ absmax, int rows, int I, const PendingLinear pl, int tail_col0, int early) {
+  extern __shared__ __align__(16) uint16_t sneg_tab[];
+  __shared__ int red32[2][32];
+  __shared__ int cta_max[2][8];                         // [row parity][CTA of the cluster]
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank(), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nw = blockDim.x >> 5, b = rank * nw + warp, col = b * 128 + 4 * lane;
+  const bool live = b * 128 < I;
+  const bool gate_tail = TAIL && live && b * 128 >= tail_col0, up_tail = TAIL && live && I + b * 128 >= tail_col0;
+  pdl_launch_dependents();
+  silu_stage_table(sneg_tab);
+  int4 gm = make_int4(0, 0, 0, 0), gs = gm, um = gm, us = gm;
+  auto scales = [&]() {
+    if (gate_tail) pending_scales4(pl, col, gm, gs);
+    if (up_tail) pending_scales4(pl, I + col, um, us);
+  };
+  if (TAIL && early) scales();
+  if (C > 1) cluster.sync();                            // the peers run: their shared memory may be written
+  pdl_wait();
+  if (TAIL && !early) scales();
+  __syncthreads();
+  int slot = 0;
+  for (int row = blockIdx.x / C; row < rows; row += gridDim.x / C, slot ^= 1) {
+    const int64_t at = (int64_t)row * 2 * I + col;
+    int4 g = make_int4(0, 0, 0, 0), u = g;
+    if (live) {
+      g = fresh4((gate_tail ? pl.acc : gate_up) + at);
+      u = fresh4((up_tail ? pl.acc : gate_up) + at + I);
+    }
+    if (TAIL && (gate_tail || up_tail)) {
+      int xm, xs;
+      absmax_to_ms_dev(fresh1(pl.x_absmax + row), &xm, &xs);
+      if (gate_tail) g = pending_requant4(g, gm, gs, xm, xs - 48);
+      if (up_tail) u = pending_requant4(u, um, us, xm, xs - 48);
+    }
+    constexpr unsigned kOff = 1u << 20;                // (the row kernel above explains the small path)
+    const unsigned out = ((unsigned)g.x + kOff) | ((unsigned)u.x + kOff) | ((unsigned)g.y + kOff) | ((unsigned)u.y + kOff) |
+                         ((unsigned)g.z + kOff) | ((unsigned)u.z + kOff) | ((unsigned)g.w + kOff) | ((unsigned)u.w + kOff);
+    const bool small = !__any_sync(FULL_MASK, out >= (1u << 21));
+    int v0, v1, v2, v3;
+    if (small) {
+      v0 = silu_mul_elem_table_small(g.x, u.x, sneg_tab); v1 = silu_mul_elem_table_small(g.y, u.y, sneg_tab);
+      v2 = silu_mul_elem_table_small(g.z, u.z, sneg_tab); v3 = silu_mul_elem_table_small(g.w, u.w, sneg_tab);
+    } else {
+      v0 = silu_mul_elem_table(g.x, u.x, sneg_tab); v1 = silu_mul_elem_table(g.y, u.y, sneg_tab);
+      v2 = silu_mul_elem_table(g.z, u.z, sneg_tab); v3 = silu_mul_elem_table(g.w, u.w, sneg_tab);
+    }
+    if (FWHT) {
+      const int big = (v0 ^ (v0 >> 31)) | (v1 ^ (v1 >> 31)) | (v2 ^ (v2 >> 31)) | (v3 ^ (v3 >> 31));
+      if (small || !__any_sync(FULL_MASK, big >= (1 << 24))) {
+        const int a = v0 + v1, d = v0 - v1, e = v2 + v3, f = v2 - v3;
+        v0 = a + e; v2 = a - e; v1 = d + f; v3 = d - f;
+#pragma unroll
+        for (int bit = 0; bit < 5; ++bit) {
+          const int sign = (lane >> bit) & 1 ? -1 : 1;
+          v0 = __shfl_xor_sync(FULL_MASK, v0, 1 << bit) + sign * v0;
+          v1 = __shfl_xor_sync(FULL_MASK, v1, 1 << bit) + sign * v1;
+          v2 = __shfl_xor_sync(FULL_MASK, v2, 1 << bit) + sign * v2;
+          v3 = __shfl_xor_sync(FULL_MASK, v3, 1 << bit) + sign * v3;
+        }
+      } else {                                         // saturating butterflies, the reference's stage order
+        const int a = add_sat(v0, v1), d = sub_sat(v0, v1), e = add_sat(v2, v3), f = sub_sat(v2, v3);
+        v0 = add_sat(a, e); v2 = sub_sat(a, e); v1 = add_sat(d, f); v3 = sub_sat(d, f);
+#pragma unroll 1
+        for (int bit = 0; bit < 5; ++bit) {
+          const bool lower = ((lane >> bit) & 1) == 0;
+          int p;
+          p = __shfl_xor_sync(FULL_MASK, v0, 1 << bit); v0 = lower ? add_sat(v0, p) : sub_sat(p, v0);
+          p = __shfl_xor_sync(FULL_MASK, v1, 1 << bit); v1 = lower ? add_sat(v1, p) : sub_sat(p, v1);
+          p = __shfl_xor_sync(FULL_MASK, v2, 1 << bit); v2 = lower ? add_sat(v2, p) : sub_sat(p, v2);
+          p = __shfl_xor_sync(FULL_MASK, v3, 1 << bit); v3 = lower ? add_sat(v3, p) : sub_sat(p, v3);
+        }
+      }
+      v0 = fwht_scale128(v0); v1 = fwht_scale128(v1); v2 = fwht_scale128(v2); v3 = fwht_scale128(v3);
+    }
+    int m = warp_max(max(max(0, abs_wrap(v0)), max(abs_wrap(v1), max(abs_wrap(v2), abs_wrap(v3)))));
+    if (lane == 0) red32[slot][warp] = m;
+    __syncthreads();
+    m = warp_max(lane < nw ? red32[slot][lane] : 0);
+    if (C > 1) {
+      // (a slot is written again two rows later, when every CTA has passed the barrier of the row in between)
+      if ((int)threadIdx.x < C) *cluster.map_shared_rank(&cta_max[slot][rank], (int)threadIdx.x) = m;
+      cluster.sync();
+      m = warp_max(lane < C ? cta_max[slot][lane] : 0);
+    }
+    m = max(1, m);
+    const float mf = __int2float_rn(m), my = __frcp_rn(mf);
+    if (live) {
+      unsigned* co = reinterpret_cast<unsigned*>(codes + (int64_t)row * I) + b * 32 + lane;
+      if (m < (1 << 22)) *co = quant4_bytes_fast_small<true>(make_int4(v0, v1, v2, v3), mf, __fmul_rn(my, 127.0f));
+      else *co = pack4(quant_code_fast(v0, mf, my), quant_code_fast(v1, mf, my), quant_code_fast(v2, mf, my), quant_code_fast(v3, mf, my));
+    }
+    if (TAIL) {                                        // the values have been used: zeros for the next GEMM's parts
+      if (gate_tail) *reinterpret_cast<int4*>(pl.acc + at) = make_int4(0, 0, 0, 0);
+      if (up_tail) *reinterpret_cast<int4*>(pl.acc + at + I) = make_int4(0, 0, 0, 0);
+    }
+    if (rank == 0 && threadIdx.x == 0) {
+      scale[row] = quant_scale(mf);
+      absmax[row] = m;
+    }
   }
 }
 
@@ -766,12 +927,13 @@ extern "C" int b200_rmsnorm_q15(const int32_t* x, const int32_t* residual, const
                    aligned16(norm_out) && ((uintptr_t)codes & 3u) == 0,
                B200_E_ALIGN, "rmsnorm_q15: int32 buffers must be 16-byte aligned (codes 4-byte)");
   const PendingLinear none = {nullptr, nullptr, nullptr, nullptr};
+  const int early = weights_settled((cudaStream_t)s);
   if ((hidden >> 2) == p.threads * p.vpt) {
     DISPATCH_VPT(p.vpt, (launch_pdl(rmsnorm_rows_kernel<V, true>, dim3((unsigned)rows), dim3(p.threads), 0, (cudaStream_t)s,
-                                    x, residual, weight, residual_out, norm_out, codes, scale, absmax, hidden, none)));
+                                    x, residual, weight, residual_out, norm_out, codes, scale, absmax, hidden, none, early)));
   } else {
     DISPATCH_VPT(p.vpt, (launch_pdl(rmsnorm_rows_kernel<V, false>, dim3((unsigned)rows), dim3(p.threads), 0, (cudaStream_t)s,
-                                    x, residual, weight, residual_out, norm_out, codes, scale, absmax, hidden, none)));
+                                    x, residual, weight, residual_out, norm_out, codes, scale, absmax, hidden, none, early)));
   }
   return check_launch("rmsnorm_q15");
 }
@@ -797,12 +959,13 @@ extern "C" int b200_rmsnorm_q15_pending(int32_t* acc, const int32_t* x_absmax, c
                    aligned16(residual_out) && aligned16(norm_out) && ((uintptr_t)codes & 3u) == 0,
                B200_E_ALIGN, "rmsnorm_q15_pending: int32 buffers must be 16-byte aligned (codes 4-byte)");
   const PendingLinear pl = {acc, x_absmax, w_mul, w_shift};
+  const int early = weights_settled((cudaStream_t)s);
   if ((hidden >> 2) == p.threads * p.vpt) {
     DISPATCH_VPT(p.vpt, (launch_pdl(rmsnorm_rows_kernel<V, true, true>, dim3((unsigned)rows), dim3(p.threads), 0, (cudaStream_t)s,
-                                    (const int32_t*)nullptr, residual, weight, residual_out, norm_out, codes, scale, absmax, hidden, pl)));
+                                    (const int32_t*)nullptr, residual, weight, residual_out, norm_out, codes, scale, absmax, hidden, pl, early)));
   } else {
     DISPATCH_VPT(p.vpt, (launch_pdl(rmsnorm_rows_kernel<V, false, true>, dim3((unsigned)rows), dim3(p.threads), 0, (cudaStream_t)s,
-                                    (const int32_t*)nullptr, residual, weight, residual_out, norm_out, codes, scale, absmax, hidden, pl)));
+                                    (const int32_t*)nullptr, residual, weight, residual_out, norm_out, codes, scale, absmax, hidden, pl, early)));
   }
   return check_launch("rmsnorm_q15_pending");
 }
@@ -823,10 +986,55 @@ extern "C" int b200_per_token_quant_q15(const int32_t* x, int8_t* codes, float* 
   return check_launch("per_token_quant_q15");
 }
 
+// CTAs per row of silu_few_rows_kernel; 0: not this kernel.  It pays while about every warp of the GPU's has one block, and where a row
+// has so many that one CTA makes several turns (us, a CTA per row | this one: 12288 columns, 1 row 6.8 | 2.3, 37 rows 7.0 | 4.3, 50 rows 7.2 | 6.7, 64 rows
+// 7.4 | 7.6; 6400: 1 row 4.2 | 2.2, 64 rows 4.9 | 3.9, 100 rows 5.3 | 6.8; 3072: 148 rows 3.5 | 3.2, 200 rows 5.8 | 5.4; 25600: 1 row 14.0 | 3.1, 64 rows
+// 21.7 | 15.5, 148 rows 14.8 | 29.4).  Eight CTAs for the fewest rows, then fewer while that leaves 16 warps a CTA (6400 columns, 24 rows: 3.1
+// with eight, 2.8 with four, 3.2 with two; 3072, 37 rows: 2.9 with eight, 2.8 with four, 2.6 with two).
+static int silu_cluster(int64_t rows, int nblocks) {
+  if (nblocks > 8 * 32 || (rows * nblocks > 4800 && (nblocks <= 128 || rows > 100))) return 0;
+  int c = 8;
+  while (c > 1 && (c > nblocks || (rows * c > 64 && nblocks <= 16 * (c / 2)))) c /= 2;
+  return c;
+}
+
+template <bool FWHT, bool TAIL>
+static int launch_silu_few(const int32_t* gu, int8_t* codes, float* scale, int32_t* absmax, int64_t rows, int inter, const PendingLinear& pl,
+                           int tail_col0, int c, cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute(silu_few_rows_kernel<FWHT, TAIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSiluTableBytes);
+  B200_REQUIRE(e == cudaSuccess, B200_E_CUDA, "silu_mul_q15: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  const int threads = (inter / 128 + c - 1) / c * 32, per_sm = threads > 512 ? 2 : 4;
+  const int64_t clusters = rows < (int64_t)148 * per_sm / c ? rows : (int64_t)148 * per_sm / c;
+  const int early = weights_settled(st);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(clusters * c));
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = kSiluTableBytes;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = c;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = !settle_takes_first(st) && pdl_enabled() ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, silu_few_rows_kernel<FWHT, TAIL>, gu, codes, scale, absmax, (int)rows, inter, pl, tail_col0, early);
+  return check_launch("silu_mul_q15 (few rows)");
+}
+
 static int launch_silu(const int32_t* gu, int32_t* q15, int8_t* codes, float* scale, int32_t* absmax,
-                       int64_t rows, int inter, bool fwht, cudaStream_t st) {
+                       int64_t rows, int inter, bool fwht, cudaStream_t st, const PendingLinear* pl = nullptr, int tail_col0 = 0) {
   const bool quant = codes != nullptr;
   const int nblocks = inter / 128;
+  if (quant && !q15) {
+    const int c = silu_cluster(rows, nblocks);
+    const PendingLinear none = {nullptr, nullptr, nullptr, nullptr};
+    if (c && pl) return fwht ? launch_silu_few<true, true>(gu, codes, scale, absmax, rows, inter, *pl, tail_col0, c, st)
+                             : launch_silu_few<false, true>(gu, codes, scale, absmax, rows, inter, *pl, tail_col0, c, st);
+    if (c) return fwht ? launch_silu_few<true, false>(gu, codes, scale, absmax, rows, inter, none, 0, c, st)
+                       : launch_silu_few<false, false>(gu, codes, scale, absmax, rows, inter, none, 0, c, st);
+  }
   const int threads = silu_threads(nblocks);
   // the direct sigmoid table (38 KB) is used when it fits beside the row buffer with two CTAs per SM
   constexpr size_t kTableBytes = ((size_t)kSnegEntries * 2 + 15) / 16 * 16;
@@ -837,6 +1045,22 @@ static int launch_silu(const int32_t* gu, int32_t* q15, int8_t* codes, float* sc
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
     sms = 148;
   const unsigned grid = (unsigned)(rows < 2 * (int64_t)sms ? rows : 2 * (int64_t)sms);
+#define B200_SILU_TAIL_LAUNCH(F, T)                                                                        \
+  do {                                                                                                     \
+    cudaError_t e = cudaFuncSetAttribute(silu_rows_kernel<F, true, T, false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    if (e != cudaSuccess) {                                                                                \
+      set_error("silu_mul_q15: cudaFuncSetAttribute: %s", cudaGetErrorString(e));                          \
+      return B200_E_CUDA;                                                                                  \
+    }                                                                                                      \
+    launch_pdl(silu_rows_kernel<F, true, T, false, true, true>, dim3(grid), dim3(threads), smem, st, gu, (int32_t*)nullptr, codes, scale, absmax, rows, \
+               inter, TpAgree{}, *pl, tail_col0);                                                          \
+    return check_launch("silu_mul_q15");                                                                   \
+  } while (0)
+  if (pl) {
+    if (fwht) { if (table) B200_SILU_TAIL_LAUNCH(true, true); else B200_SILU_TAIL_LAUNCH(true, false); }
+    else { if (table) B200_SILU_TAIL_LAUNCH(false, true); else B200_SILU_TAIL_LAUNCH(false, false); }
+  }
+#undef B200_SILU_TAIL_LAUNCH
 #define B200_SILU_LAUNCH(F, Q, T)                                                                          \
   do {                                                                                                     \
     cudaError_t e = cudaFuncSetAttribute(silu_rows_kernel<F, Q, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
@@ -845,7 +1069,7 @@ static int launch_silu(const int32_t* gu, int32_t* q15, int8_t* codes, float* sc
       set_error("silu_mul_q15: cudaFuncSetAttribute: %s", cudaGetErrorString(e));                          \
       return B200_E_CUDA;                                                                                  \
     }                                                                                                      \
-    launch_pdl(silu_rows_kernel<F, Q, T>, dim3(grid), dim3(threads), smem, st, gu, q15, codes, scale, absmax, rows, inter, TpAgree{});    \
+    launch_pdl(silu_rows_kernel<F, Q, T>, dim3(grid), dim3(threads), smem, st, gu, q15, codes, scale, absmax, rows, inter, TpAgree{}, PendingLinear{}, 0);    \
   } while (0)
 #define B200_SILU_LAUNCH_T(F, Q) do { if (table) B200_SILU_LAUNCH(F, Q, true); else B200_SILU_LAUNCH(F, Q, false); } while (0)
   if (fwht && quant) B200_SILU_LAUNCH_T(true, true);
@@ -884,6 +1108,22 @@ extern "C" int b200_silu_mul_q15(const int32_t* gate_up, int32_t* q15_out, int8_
   return launch_silu(gate_up, q15_out, codes, scale, absmax, rows, inter, fwht_block == 128, st);
 }
 
+extern "C" int b200_silu_mul_q15_tail(const int32_t* gate_up, int32_t* acc, const int32_t* x_absmax, const int32_t* w_mul, const int32_t* w_shift,
+                                      int64_t tail_col0, int8_t* codes, float* scale, int32_t* absmax, int64_t rows, int inter, int fwht_block,
+                                      b200_stream_t s) {
+  B200_REQUIRE(gate_up && acc && x_absmax && w_mul && codes && scale && absmax, B200_E_NULL, "silu_mul_q15_tail: null pointer");
+  B200_REQUIRE(rows >= 0 && rows <= 256 && inter > 0 && tail_col0 >= 0 && tail_col0 <= 2 * (int64_t)inter, B200_E_SHAPE,
+               "silu_mul_q15_tail: rows=%lld (at most 256) inter=%d tail_col0=%lld", (long long)rows, inter, (long long)tail_col0);
+  B200_REQUIRE(fwht_block == 0 || fwht_block == 128, B200_E_UNSUPPORTED, "silu_mul_q15_tail: fwht_block=%d (0 or 128)", fwht_block);
+  B200_REQUIRE(inter % 128 == 0 && inter <= 49152 && tail_col0 % 128 == 0, B200_E_UNSUPPORTED,
+               "silu_mul_q15_tail: inter=%d (at most 49152) and tail_col0=%lld must be multiples of 128", inter, (long long)tail_col0);
+  if (rows == 0) return B200_OK;
+  B200_REQUIRE(aligned16(gate_up) && aligned16(acc) && aligned16(w_mul) && aligned16(w_shift) && ((uintptr_t)codes & 3u) == 0, B200_E_ALIGN,
+               "silu_mul_q15_tail: int32 buffers must be 16-byte aligned (codes 4-byte)");
+  const PendingLinear pl = {acc, x_absmax, w_mul, w_shift};
+  return launch_silu(gate_up, nullptr, codes, scale, absmax, rows, inter, fwht_block == 128, (cudaStream_t)s, &pl, (int)tail_col0);
+}
+
 extern "C" int b200_fwht_quant_q15(const int32_t* act, int8_t* codes, float* scale, int32_t* absmax, int64_t rows, int inter,
                                    int fwht_block, b200_stream_t s) {
   B200_REQUIRE(act && codes && scale && absmax, B200_E_NULL, "fwht_quant_q15: null pointer");
@@ -909,7 +1149,7 @@ extern "C" int b200_fwht_quant_q15(const int32_t* act, int8_t* codes, float* sca
       return B200_E_CUDA;                                                                                                  \
     }                                                                                                                      \
     launch_pdl(silu_rows_kernel<F, true, true, false, false>, dim3(grid), dim3(threads), smem, st, act, (int32_t*)nullptr, \
-               codes, scale, absmax, rows, inter, TpAgree{});                                                              \
+               codes, scale, absmax, rows, inter, TpAgree{}, PendingLinear{}, 0);                                          \
   } while (0)
   if (fwht_block == 128) B200_FQ_LAUNCH(true); else B200_FQ_LAUNCH(false);
 #undef B200_FQ_LAUNCH
@@ -946,7 +1186,7 @@ extern "C" int b200_tp_silu_absmax_quant(const b200_tp_block* blk, const int32_t
       return B200_E_CUDA;                                                                                             \
     }                                                                                                                 \
     launch_pdl(silu_rows_kernel<F, true, T, true>, dim3((unsigned)rows), dim3(threads), smem, st, gate_up,            \
-               (int32_t*)nullptr, codes, (float*)nullptr, absmax, (int64_t)rows, inter, agree);                       \
+               (int32_t*)nullptr, codes, (float*)nullptr, absmax, (int64_t)rows, inter, agree, PendingLinear{}, 0);   \
   } while (0)
   if (fwht_block == 128) { if (table) B200_SILU_TP_LAUNCH(true, true); else B200_SILU_TP_LAUNCH(true, false); }
   else { if (table) B200_SILU_TP_LAUNCH(false, true); else B200_SILU_TP_LAUNCH(false, false); }

@@ -370,8 +370,21 @@ def silu_mul_fwht_quant(gate_up: torch.Tensor, fwht_block: int = 128, want_q15: 
     """SiLU(gate) * up -> blocked FWHT -> per-token int8 quant, one pass over the row.
 
     Replaces silu_and_mul_int_only + apply_blockwise_fwht_q15 + per_token_quant_int8_from_q15.
-    ``fwht_block`` 0 skips the rotation.  Returns (codes, scale [..., 1], absmax [..., 1], q15 or None).
+    ``fwht_block`` 0 skips the rotation.  ``gate_up`` may be a linear with a pending tail (W8A8Int8LinearMethod.apply_tail), without
+    ``want_q15``.  Returns (codes, scale [..., 1], absmax [..., 1], q15 or None).
     """
+    from .pending import TailLinear
+    if isinstance(gate_up, TailLinear):
+        if want_q15:
+            raise ValueError("the Q15.16 activations of a linear with a pending tail are not kept")
+        out, pl = gate_up.out, gate_up.pending
+        rows, inter = out.shape[0], out.shape[1] // 2
+        codes = torch.empty((rows, inter), dtype=torch.int8, device=out.device)
+        scale = torch.empty((rows, 1), dtype=torch.float32, device=out.device)
+        absmax = torch.empty((rows, 1), dtype=torch.int32, device=out.device)
+        call("b200_silu_mul_q15_tail", ptr(out), ptr(pl.acc), ptr(pl.x_absmax), ptr(pl.weight_mul), ptr(pl.weight_shift), gate_up.tail_col0, ptr(codes),
+             ptr(scale), ptr(absmax), rows, inter, int(fwht_block), stream())
+        return codes, scale, absmax, None
     assert_q15(gate_up, "gate_up")
     if gate_up.ndim != 2:
         raise ValueError(f"gate_up must be 2D [tokens, 2*inter], got shape {tuple(gate_up.shape)}")

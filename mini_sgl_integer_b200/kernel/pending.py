@@ -20,9 +20,10 @@ import torch
 
 from .._lib import call, ptr, stream
 
-__all__ = ["PendingLinear", "zero_workspace", "workspace_scope", "reset_workspaces", "PENDING_MAX_ROWS"]
+__all__ = ["PendingLinear", "TailLinear", "zero_workspace", "workspace_scope", "reset_workspaces", "PENDING_MAX_ROWS"]
 
 PENDING_MAX_ROWS = 256          # the GEMM splits K (and needs a zeroed buffer) up to this many token rows
+TAIL_MAX_ROWS = 64              # up to here the activation finishes the split columns of gate_up
 
 _workspaces: dict = {}
 _scope = [0]
@@ -61,6 +62,19 @@ def reset_workspaces() -> None:
     leaves a buffer dirty), before the buffers are used again."""
     for buf in _workspaces.values():
         buf.zero_()
+
+
+@dataclass
+class TailLinear:
+    """A linear of decode size whose last columns are pending: those before ``tail_col0`` are Q15.16 in ``out``."""
+
+    out: torch.Tensor                       # int32 [rows, n]
+    tail_col0: int
+    pending: "PendingLinear"                # holds the columns from tail_col0 on
+
+    @property
+    def shape(self):
+        return self.out.shape
 
 
 @dataclass

@@ -14,6 +14,7 @@ kernel/fixed_point/attention_prototype.py:100-112).
 """
 from __future__ import annotations
 
+import ctypes
 import math
 from typing import Callable, Optional
 
@@ -21,7 +22,7 @@ import torch
 
 from .._lib import call, i32, ptr, require_cuda, stream
 from ..kernel.fixed_point import absmax_to_mul_shift, assert_q15, per_token_quant_int8_from_q15
-from ..kernel.pending import PENDING_MAX_ROWS, PendingLinear, zero_workspace
+from ..kernel.pending import PENDING_MAX_ROWS, PendingLinear, TailLinear, zero_workspace
 
 __all__ = ["W8A8Int8LinearMethod", "int8_gemm_q15", "weight_scale_to_mul_shift", "per_token_quant_int8_from_q15",
            "per_tensor_quant_int8_static_from_q15"]
@@ -194,6 +195,21 @@ class W8A8Int8LinearMethod:
         if m:
             call("b200_gemm_w8a8_acc_ws", ptr(x8), ptr(layer.weight.contiguous()), ptr(ws), m, n, x8.shape[1], stream())
         return PendingLinear(ws, _flat(absmax), layer.weight_mul, layer.weight_shift)
+
+    def apply_tail(self, layer, codes: torch.Tensor, absmax: torch.Tensor) -> TailLinear:
+        """apply_quantised for at most PENDING_MAX_ROWS rows; the blocks of weight rows whose sums were split over CTAs stay pending for
+        silu_mul_fwht_quant."""
+        if getattr(layer, "weight_mul", None) is None:
+            self.process_weights_after_loading(layer)
+        x8 = codes.reshape(-1, codes.shape[-1]).contiguous()
+        require_cuda(x8, layer.weight, absmax, layer.weight_mul, layer.weight_shift)
+        m, n = x8.shape[0], layer.weight.shape[0]
+        out, absmax, ws = torch.empty((m, n), dtype=torch.int32, device=x8.device), _flat(absmax), zero_workspace(x8.device, m, n)
+        tail = ctypes.c_int64(n)
+        if m:
+            call("b200_gemm_w8a8_absmax_tail", ptr(x8), ptr(layer.weight.contiguous()), ptr(absmax), ptr(layer.weight_mul), ptr(layer.weight_shift),
+                 ptr(out), ptr(ws), ctypes.addressof(tail), m, n, x8.shape[1], stream())
+        return TailLinear(out, tail.value, PendingLinear(ws, absmax, layer.weight_mul, layer.weight_shift))
 
     @staticmethod
     def _add_bias(out: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:

@@ -1,0 +1,99 @@
+"""Forms of the integer step's kernels for few rows and for prompts whose scores fit tensor memory, at the sizes where their branches meet."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import attention as oattn
+from oracle import fixed_point as ofp
+from tests.attn_util import device_pool
+from tests.test_gpu_attention import _extend_case, eq, run_extend
+from tests.test_gpu_pending import _layer, _linear_case, _workspaces_zero
+
+pytestmark = pytest.mark.gpu
+
+
+def d(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+# One to eight CTAs per row, a last CTA or warp without a block, blocks up to the kernel's limit; values that need the saturating butterflies
+@pytest.mark.parametrize("rows,inter", [(1, 128), (1, 1152), (3, 6400), (17, 12288), (64, 25600), (65, 3072), (37, 17 * 128), (2, 32768), (2, 49152)])
+@pytest.mark.parametrize("block", [0, 128])
+@pytest.mark.parametrize("top", [2**18, 2**22, 2**31 - 1])
+def test_silu_of_few_rows(rows, inter, block, top):
+    from mini_sgl_integer_b200.kernel import fixed_point as fp
+    rng = np.random.default_rng(rows + inter)
+    gu = rng.integers(-top, top, (rows, 2 * inter)).astype(np.int32)
+    gu[0, :128] = 0
+    act = ofp.silu_and_mul(gu)
+    codes, scale, absmax = ofp.per_token_quant_from_q15(ofp.blockwise_fwht_q15(act, block) if block else act)
+    got = fp.silu_mul_fwht_quant(d(gu), block)
+    np.testing.assert_array_equal(got[0].cpu().numpy(), codes)
+    np.testing.assert_array_equal(got[1].cpu().numpy().reshape(-1), np.asarray(scale).reshape(-1))
+    np.testing.assert_array_equal(got[2].cpu().numpy().reshape(-1), np.asarray(absmax).reshape(-1))
+
+
+# whole blocks only; a split tail inside the up half and across both; everything split; pairs of CTAs (more than 64 rows)
+@pytest.mark.parametrize("m,inter,k", [(1, 128, 256), (3, 6400, 2048), (1, 12288, 1024), (37, 148 * 64, 512), (64, 3072, 1024), (65, 12288, 1024), (200, 9472 + 128, 512),
+                                       (256, 1536, 2048)])
+@pytest.mark.parametrize("shift", [True, False])
+def test_activation_on_a_linear_with_a_pending_tail(m, inter, k, shift):
+    from mini_sgl_integer_b200.kernel import fixed_point as fp
+    from mini_sgl_integer_b200.layers.w8a8_int8 import W8A8Int8LinearMethod
+    codes, absmax, w8, wm, ws, acc, q15 = _linear_case(m + inter + k, m, 2 * inter, k, shift)
+    want = ofp.per_token_quant_from_q15(ofp.blockwise_fwht_q15(ofp.silu_and_mul(q15), 128))
+    layer, method = _layer(w8, wm, ws), W8A8Int8LinearMethod()
+    for _ in range(2):
+        tail = method.apply_tail(layer, d(codes), d(absmax))
+        np.testing.assert_array_equal(tail.out[:, :tail.tail_col0].cpu().numpy(), q15[:, :tail.tail_col0])
+        got = fp.silu_mul_fwht_quant(tail, 128)
+        np.testing.assert_array_equal(got[0].cpu().numpy(), want[0])
+        np.testing.assert_array_equal(got[2].cpu().numpy().reshape(-1), want[2].reshape(-1))
+        assert _workspaces_zero()
+
+
+# One short of, at and beyond the 512 keys whose scores are kept, with and without a prefix; tiles of 64, 32, 16 and 8 tokens
+@pytest.mark.parametrize("kv_heads", [1, 2, 4, 8])
+@pytest.mark.parametrize("kv_len,q_len", [(511, 511), (512, 40), (513, 513), (640, 9), (577, 300), (64, 64), (65, 1)])
+def test_tiled_prefill_around_the_kept_scores(kv_heads, kv_len, q_len):
+    kv_lens, q_lens = [kv_len, 30], [q_len, 30]
+    case = _extend_case(kv_len + q_len, kv_lens, q_lens, 8, kv_heads, 64)
+    want = oattn.paged_attention(case["q8"], case["qm"], case["qs"], case["pool"], case["tables"], kv_lens, q_lens)
+    eq(run_extend(case, device_pool(case, 64, kv_heads), 640, impl="tiled").cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("requests", [1, 5, 70])
+def test_a_step_that_reads_ahead_gives_the_bits_of_one_that_does_not(requests):
+    """Weights, gains, page tables and the keys of earlier steps are read before the wait on the kernels in front only inside a model's
+    forward; the layers by themselves wait first."""
+    from mini_sgl_integer_b200.attention import Int8PagedKVCache
+    from mini_sgl_integer_b200.layers.decoder_layer import AttnBatch
+    from mini_sgl_integer_b200.models import Qwen3ForCausalLMInteger, Qwen3IntegerConfig, random_weights
+    cfg = Qwen3IntegerConfig(3, 512, 8, 2, 1536, 1000, max_pos=256)
+    weights = random_weights(cfg, 5, generate_on_device=True)
+    g = torch.Generator(device="cuda").manual_seed(7)
+    lens = torch.randint(1, 120, (requests,), device="cuda", generator=g, dtype=torch.int32)
+    table = torch.arange(requests * 8, dtype=torch.int32, device="cuda").view(requests, 8)
+    loc = (table.gather(1, (lens - 1)[:, None].long() // 16)[:, 0] * 16 + (lens - 1) % 16).to(torch.int32)
+    ids = torch.randint(0, 1000, (requests,), device="cuda", generator=g, dtype=torch.int32)
+    batch = AttnBatch(lens - 1, loc, table, lens, None, 128)
+    out = []
+    for ahead in (True, False):
+        pool = Int8PagedKVCache(2, 3, 128, requests * 8, "cuda")
+        for i in range(3):
+            gi = torch.Generator(device="cuda").manual_seed(i)
+            for c in (pool.k_cache(i), pool.v_cache(i)):
+                c.copy_(torch.randint(-127, 128, c.shape, dtype=torch.int8, device="cuda", generator=gi))
+            meta = pool.meta(i)
+            meta[:, :, :32] = 2**30 + 12345
+            meta[:, :, 32:40] = 0x24242424
+        model = Qwen3ForCausalLMInteger(cfg, weights, pool)
+        if ahead:
+            logits = model.forward(ids, batch)
+        else:
+            codes, absmax = model.model.forward(ids, batch)
+            logits = model.method.apply_quantised(model.lm_head, codes, absmax)
+        out.append([logits] + [t.clone() for i in range(3) for t in (pool.k_cache(i), pool.v_cache(i), pool.meta(i))])
+    assert all(torch.equal(a, b) for a, b in zip(*out)) and _workspaces_zero()

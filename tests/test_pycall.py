@@ -6,10 +6,7 @@ import ctypes
 import pytest
 
 from mini_sgl_integer_b200 import _lib
-from mini_sgl_integer_b200.build import build_library
-
-build_library()
-from mini_sgl_integer_b200._pycall import bind  # noqa: E402
+from mini_sgl_integer_b200._pycall import bind
 
 ALL = {**_lib.SIGNATURES, **_lib.FLOAT_SIGNATURES}
 BOUND = [n for n in ALL if bind(n, 1) is not None]
