@@ -69,17 +69,36 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
   return warp_sum(lane < nw ? scratch[lane] : 0.0f);
 }
 
-// Sum over the parts of a split linear, in order.
+// Sum over the parts of a split linear, in order.  The linears of this library give at most kMaxParts, whose loads are all in flight
+// together: in a loop of unknown length they were two or three memory latencies, one after the other.
+constexpr int kMaxParts = 6;
 __device__ __forceinline__ float part_sum(const float* p, int splits, int64_t stride) {
   float v = p[0];
-  for (int s = 1; s < splits; ++s) v += p[(int64_t)s * stride];
+  if (splits > 1) {
+    float o[kMaxParts];
+#pragma unroll
+    for (int s = 1; s < kMaxParts; ++s) o[s] = s < splits ? p[(int64_t)s * stride] : 0.0f;
+#pragma unroll
+    for (int s = 1; s < kMaxParts; ++s)
+      if (s < splits) v += o[s];
+    for (int s = kMaxParts; s < splits; ++s) v += p[(int64_t)s * stride];
+  }
   return v;
 }
 __device__ __forceinline__ float4 part_sum4(const float* p, int splits, int64_t stride) {
   float4 v = *reinterpret_cast<const float4*>(p);
-  for (int s = 1; s < splits; ++s) {
-    const float4 o = *reinterpret_cast<const float4*>(p + (int64_t)s * stride);
-    v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+  if (splits > 1) {
+    float4 o[kMaxParts];
+#pragma unroll
+    for (int s = 1; s < kMaxParts; ++s)
+      if (s < splits) o[s] = *reinterpret_cast<const float4*>(p + (int64_t)s * stride);
+#pragma unroll
+    for (int s = 1; s < kMaxParts; ++s)
+      if (s < splits) { v.x += o[s].x; v.y += o[s].y; v.z += o[s].z; v.w += o[s].w; }
+    for (int s = kMaxParts; s < splits; ++s) {
+      const float4 t = *reinterpret_cast<const float4*>(p + (int64_t)s * stride);
+      v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+    }
   }
   return v;
 }

@@ -80,6 +80,7 @@ struct SublayerEnd {
   int width;
   int64_t t_pitch;
   float eps;
+  int early;                         // the weights are settled
 };
 
 template <int VEC>
@@ -116,11 +117,32 @@ __global__ void sublayer_end_kernel(const SublayerEnd p, T* __restrict__ x_out_t
   pdl_launch_dependents();
   const int64_t row = blockIdx.x;
   const int64_t base = row * p.width;
-  pdl_wait();
   Pack<VEC> r[NV];
   int col[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) col[i] = (i * blockDim.x + threadIdx.x) * VEC;
+  constexpr int E = EARLY ? NV : 1;
+  Pack<VEC> x0[E], w0[E], a0[E], f0[E];
+  auto gains = [&]() {
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      if (col[i] >= p.width) continue;
+      if (p.y) w0[i] = load_pack<VEC>(p.norm_w + col[i]);
+      if (p.final_w) f0[i] = load_pack<VEC>(p.final_w + col[i]);
+    }
+  };
+  if (EARLY) {               // the gains before the wait if they are settled, else on their way into L2
+    if (p.coef && threadIdx.x == 0) prefetch_l2(p.coef);
+    if (p.early) {
+      gains();
+    } else {
+      for (int c = threadIdx.x * 32; c < p.width; c += blockDim.x * 32) {
+        if (p.y) prefetch_l2(p.norm_w + c);
+        if (p.final_w) prefetch_l2(p.final_w + c);
+      }
+    }
+  }
+  pdl_wait();
   // the sum of the depth average's earlier planes
   auto plane_sum = [&](int c) {
     Pack<VEC> a;
@@ -150,18 +172,11 @@ __global__ void sublayer_end_kernel(const SublayerEnd p, T* __restrict__ x_out_t
   // EARLY: what the sums of squares do not need is requested in front of them.  A decode row is a chain of memory latencies (y,
   // then stream and gain, then planes, then the next gain); this saves two of them: decode steps of Sefevik 0.3B 613 -> 598 us, 1.4B
   // with 256 rows 1527 -> 1516.  The registers cost many rows their occupancy (8186 rows: 52.6 -> 64.0 us) and wide ones do not have them.
-  constexpr int E = EARLY ? NV : 1;
-  Pack<VEC> x0[E], w0[E], a0[E], f0[E];
   if (EARLY) {
+    if (!p.early) gains();
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-      if (col[i] >= p.width) continue;
-      if (p.y) {
-        if (p.x_in) x0[i] = load_pack<VEC>(p.x_in + base + col[i]);
-        w0[i] = load_pack<VEC>(p.norm_w + col[i]);
-      }
-      if (p.final_w) f0[i] = load_pack<VEC>(p.final_w + col[i]);
-    }
+    for (int i = 0; i < E; ++i)
+      if (p.y && p.x_in && col[i] < p.width) x0[i] = load_pack<VEC>(p.x_in + base + col[i]);
   }
   auto early_planes = [&]() {
     if (!EARLY || !p.coef) return;
@@ -176,7 +191,21 @@ __global__ void sublayer_end_kernel(const SublayerEnd p, T* __restrict__ x_out_t
     for (int i = 0; i < NV; ++i) {
       if (col[i] >= p.width) continue;
       a[i] = load_pack<VEC>(y + base + col[i]);
-      for (int s = 1; s < splits; ++s) {
+      int s = 1;
+      if (EARLY && splits > 1) {                     // (part_sum explains why)
+        Pack<VEC> o[kMaxParts];
+#pragma unroll
+        for (int u = 1; u < kMaxParts; ++u)
+          if (u < splits) o[u] = load_pack<VEC>(y + (int64_t)u * stride + base + col[i]);
+#pragma unroll
+        for (int u = 1; u < kMaxParts; ++u)
+          if (u < splits) {
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) a[i].v[k] += o[u].v[k];
+          }
+        s = kMaxParts;
+      }
+      for (; s < splits; ++s) {
         const Pack<VEC> o = load_pack<VEC>(y + (int64_t)s * stride + base + col[i]);
 #pragma unroll
         for (int k = 0; k < VEC; ++k) a[i].v[k] += o.v[k];
@@ -420,7 +449,7 @@ extern "C" int b200f_sublayer_end(const float* y, int splits, int64_t split_stri
   B200_REQUIRE((x_in || y) && (!y || norm_w) && (!y2 || (y && w1 && w2)) && (x_out || x_out_t) && (!coef || planes == 0 || hist), B200_E_NULL,
                "sublayer_end: null pointer");
   SublayerEnd p{y, splits, split_stride, y2, splits2, split_stride2, w1, w2, x_in, norm_w, add, x_out, hist, planes, plane_stride, coef, hist_out,
-                final_w, width, t_pitch, eps};
+                final_w, width, t_pitch, eps, (int)weights_settled((cudaStream_t)s)};
   return dtype == B200F_BF16 ? sublayer_end_typed<bf16>(p, x_out_t, rows, (cudaStream_t)s)
                              : sublayer_end_typed<float>(p, x_out_t, rows, (cudaStream_t)s);
 }

@@ -34,6 +34,7 @@ struct PrepareParams {
   float eps;
   int heads, dim, rot_dim, kv_rank, head_pitch, qn_pitch, lat_pitch;
   int64_t cache_rows;
+  int early;              // the step's inputs are settled
 };
 
 // First and second half of a rotated pair; the two kernels below round in the same places.
@@ -102,12 +103,20 @@ latent_prepare_vec_kernel(const PrepareParams p, T* __restrict__ qn, T* __restri
   __shared__ float scratch[32];
   __shared__ __align__(16) float latent[4 * kPrepareThreads];
   pdl_launch_dependents();
-  pdl_wait();
   const int64_t t = blockIdx.x;
   const int tid = threadIdx.x;
   const float* src = p.qd + t * p.qd_pitch;
+  // Settled: position, place and gain are read before the wait, the position's rotation is on its way into L2.
+  if (!p.early) pdl_wait();
   const int pos = min(max(p.positions[t], 0), p.max_pos - 1);
   const float* cs = p.rot_dims ? p.rope + (int64_t)pos * p.rot_dims : nullptr;
+  const int64_t loc = p.dkv_norm ? p.out_loc[t] : 0;
+  float4 w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (p.dkv_norm && 4 * tid < p.kv_rank) w = *reinterpret_cast<const float4*>(p.dkv_norm + 4 * tid);
+  if (p.early) {
+    if (32 * tid < p.rot_dims) prefetch_l2(cs + 32 * tid);
+    pdl_wait();
+  }
   const int half = p.rot_dims >> 1;
   // columns i .. i + 3 of a rotated vector
   auto rotated4 = [&](const float* v, int i) {
@@ -143,11 +152,9 @@ latent_prepare_vec_kernel(const PrepareParams p, T* __restrict__ qn, T* __restri
   for (int i = tid; i < p.kv_rank; i += kPrepareThreads) ss = fmaf(latent[i], latent[i], ss);
   ss = block_sum(ss, scratch);
   const float inv = 1.0f / sqrtf(ss / (float)p.kv_rank + p.eps);
-  const int64_t loc = p.out_loc[t];
   if (loc < 0 || loc >= p.cache_rows) return;
   T* row = cache + loc * p.lat_pitch;
   if (own) {
-    const float4 w = *reinterpret_cast<const float4*>(p.dkv_norm + 4 * tid);
     store4(row + 4 * tid, make_float4(x.x * inv * w.x, x.y * inv * w.y, x.z * inv * w.z, x.w * inv * w.w));
   }
   for (int i = 4 * tid; i < p.rot_dim; i += 4 * kPrepareThreads) store4(row + p.kv_rank + i, rotated4(src + d0 + p.kv_rank, i));
@@ -165,6 +172,7 @@ struct AttnParams {
   int splits;
   float* ws;                       // splits > 1: [splits][tokens * heads][kv_rank], then [splits][tokens * heads][2]
   int head_groups, heads_per_cta, tokens_per_cta;
+  int early;                       // a decode step whose inputs and earlier keys are settled
 };
 
 __device__ __forceinline__ int first_key(int pos, int window) { return window > 0 ? max(pos - window + 1, 0) : 0; }
@@ -533,10 +541,12 @@ latent_attn_mma_kernel(const AttnParams p, const bf16* __restrict__ q_lat, const
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // A decode step's key is in the last tile: the copying warp fetches the others before its wait, if they are settled.
+  const bool ahead = kCopyWarp && p.early && warp == WARPS;
   for (int r = warp; r < STAGES * NK; r += S::kThreads / 32)                        // columns behind a row's copied part stay zero
     for (int c = p.lat_pitch + lane; c < d16; c += 32) ks[r * ld + c] = __float2bfloat16_rn(0.0f);
   __syncthreads();
-  pdl_wait();
+  if (!ahead) pdl_wait();
   const int start = p.seq_start ? p.seq_start[seq] : seq;
   const int count = p.seq_start ? p.seq_start[seq + 1] - start : 1;
   const int tok0 = q_tile * p.tokens_per_cta;
@@ -575,7 +585,10 @@ latent_attn_mma_kernel(const AttnParams p, const bf16* __restrict__ q_lat, const
   if (kCopyWarp) {
     if (warp == WARPS) {
       look_up(tile0);
-      for (int tile = tile0; tile < tile1 && ok; ++tile) ok = copy_tile(tile);
+      for (int tile = tile0; tile < tile1 && ok; ++tile) {
+        if (ahead && tile == all_tiles - 1) pdl_wait();
+        ok = copy_tile(tile);
+      }
       return;
     }
   } else if (warp == 0) {
@@ -601,7 +614,8 @@ latent_attn_mma_kernel(const AttnParams p, const bf16* __restrict__ q_lat, const
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int col = (k_lo + i) * 16 + 8 * (j >> 1) + 2 * (lane & 3);
-        qf[i][j] = (i < k_n && live[j & 1] && col < p.lat_pitch) ? __ldg(reinterpret_cast<const unsigned*>(src[j & 1] + col)) : 0u;
+        qf[i][j] = (i < k_n && live[j & 1] && col < p.lat_pitch) 
+                       ? (kCopyWarp ? (unsigned)fresh1(reinterpret_cast<const int32_t*>(src[j & 1] + col)) : __ldg(reinterpret_cast<const unsigned*>(src[j & 1] + col))) : 0u;
       }
   }
   // the rows whose softmax this lane works on (eight lanes per row, four keys each), and the keys they may see
@@ -871,7 +885,7 @@ extern "C" int b200f_latent_prepare(const float* qd, int splits, int64_t split_s
   if (tokens == 0) return B200_OK;
   B200_REQUIRE(qd && positions && qn && q_lat && (!rot_dims || rope) && (!dkv_norm || (cache && out_loc)), B200_E_NULL, "latent_prepare: null pointer");
   PrepareParams p{qd, splits, split_stride, qd_pitch, positions, out_loc, rope, rot_dims, max_pos, dkv_norm, eps, heads, dim, rot_dim,
-                  kv_rank, head_pitch, qn_pitch, lat_pitch, cache_rows};
+                  kv_rank, head_pitch, qn_pitch, lat_pitch, cache_rows, (int)weights_settled((cudaStream_t)s)};
   const bool vec = dim % 4 == 0 && rot_dim % 4 == 0 && rot_dims % 8 == 0 && kv_rank % 4 == 0 && kv_rank <= 4 * kPrepareThreads && head_pitch % 4 == 0 &&
                    qn_pitch % 4 == 0 && lat_pitch % 4 == 0 && qd_pitch % 4 == 0 && (splits == 1 || split_stride % 4 == 0) && (int64_t)heads * head_pitch < (1ll << 31) &&
                    aligned16(qd) && aligned16(rope) && aligned16(dkv_norm) && aligned16(qn) && aligned16(q_lat) && aligned16(cache);
@@ -919,7 +933,7 @@ extern "C" int b200f_latent_attn(const void* q_lat, const void* cache, const int
   B200_REQUIRE(q_lat && cache && page_table && kv_lens && sink && out && (key_splits == 1 || ws), B200_E_NULL, "latent_attn: null pointer");
   cudaStream_t st = (cudaStream_t)s;
   AttnParams p{page_table, table_pitch, kv_lens, seq_start, sink, tokens, heads, kv_rank, rot_dim, lat_pitch, out_pitch, window,
-               scale * kLog2e, key_splits, ws, 1, heads, 1};
+               scale * kLog2e, key_splits, ws, 1, heads, 1, weights_settled((cudaStream_t)s) && !seq_start};
   const AttnPlan pl = (dtype == B200F_BF16 && !simple && lat_pitch % 8 == 0 && out_pitch % 2 == 0 && aligned16(q_lat) && aligned16(cache))
                           ? plan_attn(max_q, heads, kv_rank, rot_dim) : AttnPlan{0, 0, 0, 0, 0, 0};
   // 32-bit prompts: whole float4 columns, up to 768 of them for the output (accumulators), 32 rows and keys in shared memory

@@ -235,6 +235,7 @@ struct MemoryParams {
   float* out;                          // [tokens][heads * vdim]
   float* den;                          // EXP: [tokens][heads]
   int warps;
+  int early;                           // decode: inputs and states of the step are settled
 };
 
 constexpr int kStageTokens = 16;
@@ -1255,9 +1256,16 @@ delta_inverse_kernel(const MemoryParams p, const bf16* __restrict__ rows, bf16* 
 
 // ---------------------------------------------------------------------------------------------------
 // Decode: a CTA per (sequence, head, slice of VQ column quads); 256 / VQ row groups, R rows per thread in registers.
+// (stays on its side of the wait, and marks the line as read once)
+__device__ __forceinline__ float4 fresh_state(const float* p) {
+  float4 v;
+  asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  return v;
+}
+
 template <typename T, int KIND, int R>
 __global__ void __launch_bounds__(256)
-memory_step_kernel(const MemoryParams p, const T* __restrict__ rows, int vq) {
+memory_step_kernel(const MemoryParams p, const T* rows, int vq) {
   __shared__ float qs[512], ks[512], scratch[32];
   __shared__ float4 red[256];
   pdl_launch_dependents();
@@ -1265,7 +1273,7 @@ memory_step_kernel(const MemoryParams p, const T* __restrict__ rows, int vq) {
   const int slice = blockIdx.x, h = blockIdx.y, seq = blockIdx.z;
   const int vp = pad8i(p.vdim), hq = pad8i(p.dim), c = (slice * vq + tx) * 4;
   const int qh = h / (p.heads / p.qk_heads);
-  pdl_wait();
+  if (!p.early) pdl_wait();        // settled: the state, most of what there is to read, comes while the kernels in front still run
   const int64_t slot_head = (int64_t)p.slots[seq] * p.heads + h;
   const bool has_state = p.positions[seq] > 0;
   float* st = p.state + slot_head * p.dim * vp + c;
@@ -1273,8 +1281,9 @@ memory_step_kernel(const MemoryParams p, const T* __restrict__ rows, int vq) {
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const int n = ty + i * rg;
-    S[i] = (has_state && n < p.dim && c < vp) ? __ldcs(reinterpret_cast<const float4*>(st + (int64_t)n * vp)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    S[i] = (has_state && n < p.dim && c < vp) ? fresh_state(st + (int64_t)n * vp) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
+  if (p.early) pdl_wait();
   const T* row = rows + (int64_t)seq * p.row_pitch;
   float sq = 0.0f, sk = 0.0f;
   for (int i = tid; i < rg * R; i += 256) {
@@ -1660,7 +1669,7 @@ extern "C" int b200f_memory_scan(const void* rows, int dtype, int64_t row_pitch,
   B200_REQUIRE(aligned16(rows) && aligned16(gates) && aligned16(state) && row_pitch % 8 == 0 && q_off % 8 == 0 && k_off % 8 == 0 && v_off % 8 == 0,
                B200_E_ALIGN, "memory_scan: rows and heads must start on 16-byte boundaries");
   MemoryParams p{row_pitch, q_off, k_off, v_off, qk_heads, heads, dim, vdim, reinterpret_cast<float4*>(gates), q_scale, skip, state, norm_state,
-                 slots, positions, seq_start, out, den, 0};
+                 slots, positions, seq_start, out, den, 0, weights_settled((cudaStream_t)s) && !seq_start};
   if (seq_start && !simple && chunks_fit(dtype, dim, vdim, max_q)) {
     B200_REQUIRE(kind != B200F_MEMORY_DELTA || (ws && aligned16(ws)), B200_E_NULL, "memory_scan: no workspace");
     const bf16* r = (const bf16*)rows;

@@ -20,6 +20,7 @@ struct MinGruParams {
   const int32_t *slots, *positions, *seq_start;
   int width;
   int64_t out_pitch;
+  int early;           // decode: the step's inputs and states are settled, they are read before the wait
 };
 
 // (1 - z, z * candidate) of one token.
@@ -94,15 +95,18 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 mingru_step_kernel(const MinGruParams p, T* __restrict__ out) {
   pdl_launch_dependents();
-  pdl_wait();
+  if (!p.early) pdl_wait();
   const int c = blockIdx.x * 256 + threadIdx.x, seq = blockIdx.y;
   if (c >= p.width) return;
   const float* src = p.zug + (int64_t)seq * 3 * p.width + c;
   float* st = p.state + (int64_t)p.slots[seq] * p.width + c;
-  const float zp = part_sum(src, p.splits, p.split_stride) + p.bias_z[c];
-  const float up = part_sum(src + p.width, p.splits, p.split_stride) + p.bias_u[c];
+  const float bz = p.bias_z[c], bu = p.bias_u[c];
+  float s = *st;
+  if (p.positions[seq] <= 0) s = 0.0f;
+  if (p.early) pdl_wait();
+  const float zp = part_sum(src, p.splits, p.split_stride) + bz;
+  const float up = part_sum(src + p.width, p.splits, p.split_stride) + bu;
   const float g = part_sum(src + 2 * p.width, p.splits, p.split_stride);
-  float s = p.positions[seq] > 0 ? *st : 0.0f;
   float a, b;
   mingru_gate(zp, up, &a, &b);
   s = fmaf(a, s, b);
@@ -132,7 +136,7 @@ extern "C" int b200f_mingru(const float* zug, int splits, int64_t split_stride, 
                B200_E_SHAPE, "mingru: tokens=%lld batch=%d width=%d splits=%d", (long long)tokens, batch, width, splits);
   if (tokens == 0 || batch == 0) return B200_OK;
   B200_REQUIRE(zug && bias_z && bias_u && state && slots && positions && out, B200_E_NULL, "mingru: null pointer");
-  MinGruParams p{zug, splits, split_stride, bias_z, bias_u, state, slots, positions, seq_start, width, out_pitch};
+  MinGruParams p{zug, splits, split_stride, bias_z, bias_u, state, slots, positions, seq_start, width, out_pitch, (int)weights_settled((cudaStream_t)s)};
   return dtype == B200F_BF16 ? mingru_typed<bf16>(p, (bf16*)out, tokens, batch, (cudaStream_t)s)
                              : mingru_typed<float>(p, (float*)out, tokens, batch, (cudaStream_t)s);
 }

@@ -117,11 +117,10 @@ class Engine:
             if picks != list(range(base)):
                 logits = logits[torch.tensor(picks, device=self.device)] if picks else None
         else:
-            dev = host.pin_memory().to(self.device, non_blocking=True)
-            batch.input_ids, batch.positions, batch.out_loc = dev[0], dev[1], dev[2]
-            # (from pinned memory as well: a copy from pageable memory would wait for everything issued before it, and the GPU then
+            # (one copy, from pinned memory: one from pageable memory would wait for everything issued before it, and the GPU then
             # idles while this step's launches are issued: 8186 prompt tokens 17.8 -> 17.1 ms a step)
-            batch.logit_rows = torch.tensor(picks, dtype=torch.int64).pin_memory().to(self.device, non_blocking=True)
+            dev = torch.cat([host.flatten(), torch.tensor(picks, dtype=torch.int32)]).pin_memory().to(self.device, non_blocking=True)
+            batch.input_ids, batch.positions, batch.out_loc, batch.logit_rows = dev.split([base, base, base, len(picks)])
             self.backend.prepare_metadata(batch)
             with self.ctx.forward_batch(batch):
                 logits = self.model.forward() if picks else self._forward_without_logits()

@@ -100,7 +100,7 @@ class CacheManager:
             return
         rows = sorted(self._dirty)
         self._dirty.clear()
-        at, src = torch.tensor(rows), self._host[rows]
-        if self.page_table.is_cuda:                        # (pinned: copies from pageable memory wait for the stream)
-            at, src = (t.pin_memory().to(self.page_table.device, non_blocking=True) for t in (at, src))
-        self.page_table.index_copy_(0, at, src)
+        new = torch.cat([torch.tensor(rows, dtype=torch.int32)[:, None], self._host[rows]], dim=1)
+        if self.page_table.is_cuda:                        # (pinned: a copy from pageable memory waits for the stream)
+            new = new.pin_memory().to(self.page_table.device, non_blocking=True)
+        self.page_table[new[:, 0]] = new[:, 1:]
