@@ -323,6 +323,8 @@ B200_API int b200_gemm_w8a8_absmax(const int8_t* x8, const int8_t* w8, const int
  *                             b200_silu_mul_q15_tail: b200_silu_mul_q15 with codes on such a gate_up result (it zeroes them again).
  *   b200_gemm_w8a8_acc_ws     leaves the exact accumulators in zero_ws; exactly one of the two calls below must then
  *                             consume them (they zero the buffer again) before zero_ws is reused.
+ *   b200_gemm_pending_pays    1 where a linear of these sizes is better left pending: decode sizes, and prompts of fewer 256 x 256 tiles
+ *                             than there are pairs of SMs.
  *   b200_rmsnorm_q15_pending  b200_rmsnorm_q15 with x = the Q15.16 result of that linear, computed on the fly from
  *                             (acc, x_absmax int32 [rows], w_mul, w_shift int32 [hidden]): the same bits as
  *                             b200_gemm_w8a8_absmax followed by b200_rmsnorm_q15, in two launches instead of four.
@@ -330,6 +332,7 @@ B200_API int b200_gemm_w8a8_absmax(const int8_t* x8, const int8_t* w8, const int
  *                             * 128], q | k | v heads side by side).
  * No reference counterpart: the reference materialises every linear's output (layers/quantization/w8a8_int8.py:242-286)
  * before RMSNorm (models/integer/qwen3_integer.py:62-80) or q/k-norm + RoPE (models/utils_integer.py:209-227) read it. */
+B200_API int b200_gemm_pending_pays(int64_t m, int64_t n);
 B200_API int b200_gemm_w8a8_absmax_tail(const int8_t* x8, const int8_t* w8, const int32_t* x_absmax, const int32_t* w_mul,
                                         const int32_t* w_shift, int32_t* out_q15, int32_t* zero_ws, int64_t* tail_col0, int64_t m, int64_t n,
                                         int64_t k, b200_stream_t s);

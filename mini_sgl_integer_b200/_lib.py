@@ -50,6 +50,7 @@ SIGNATURES: dict[str, list] = {
     "b200_gemm_w8a8_absmax": [P, P, P, P, P, P, P, L, L, L, P],
     "b200_gemm_w8a8_reduce_peers": [P, P, P, I, L, L, L, P],
     "b200_gemm_w8a8_absmax_ws": [P, P, P, P, P, P, P, L, L, L, P],
+    "b200_gemm_pending_pays": [L, L],
     "b200_gemm_w8a8_absmax_tail": [P, P, P, P, P, P, P, P, L, L, L, P],
     "b200_silu_mul_q15_tail": [P, P, P, P, P, L, P, P, P, L, I, I, P],
     "b200_gemm_w8a8_acc_ws": [P, P, P, L, L, L, P],

@@ -1095,8 +1095,23 @@ static int launch_gemm_2sm_ws(const CUtensorMap& mw, const CUtensorMap& mx, cons
 // tiles, 35.8 with two tiles in two parts).  Below, it depends on the shape (split, whole): 1000 x 2048 with 16, 32, 36 and 40 k-blocks
 // 16.5, 13.8; 19.0, 18.4; 19.7, 19.6; 20.3, 20.7; 333 x 4096 with 16, 24 and 40 14.3, 13.5; 15.5, 15.9; 18.0, 20.6; where four parts fit
 // (one_wave, see lone_prompt) from 20 on: 300 x 1024 with 16, 20 and 32 10.8, 12.8; 11.1, 13.9; 12.0, 17.3.
-static int prompt_tiles(GemmParams* p, int w_blocks, int num_kb, int pairs, bool one_wave) {
+//
+// A pending linear has neither the clearing nor the requantising kernel behind it, and its tiles no requantisation in their epilogues: there
+// tiles are as wide as they get, and K is split where that shortens the CTA pairs' longest run of k-blocks (a part more counts as two: its
+// sums are added in memory).  Materialised and pending, 333 tokens: 6144 x 4096 19.1, 14.7 us; 4096 x 4096 18.4, 11.8; 4096 x 12288 27.1, 20.8;
+// 2048 x 2048 13.3, 8.0; 700 tokens: 6144 x 4096 24.9, 20.4; 4096 x 4096 23.5, 15.6.
+static int prompt_tiles(GemmParams* p, int w_blocks, int num_kb, int pairs, bool one_wave, bool pending) {
   const int fewest = (p->M + 255) / 256;
+  if (pending) {
+    p->tok_tile = ((p->M + fewest - 1) / fewest + 31) / 32 * 32;
+    p->tok_tiles = (p->M + p->tok_tile - 1) / p->tok_tile;
+    int best = 1, cost = 1 << 30;
+    for (int s = 1; s <= 4 && (s == 1 || num_kb / s >= 4); ++s) {
+      const int per = (num_kb + s - 1) / s, c = (w_blocks * p->tok_tiles * s + pairs - 1) / pairs * per + 2 * s;
+      if ((s - 1) * per < num_kb && c <= cost) { best = s; cost = c; }
+    }
+    return best;
+  }
   int tiles = fewest, splits = 1;
   if (num_kb >= (one_wave ? 20 : 40)) splits = pairs / (w_blocks * fewest) < 4 ? pairs / (w_blocks * fewest) : 4;
   while (splits > 1 && (splits - 1) * ((num_kb + splits - 1) / splits) >= num_kb) --splits;     // no empty part
@@ -1111,6 +1126,7 @@ static int prompt_tiles(GemmParams* p, int w_blocks, int num_kb, int pairs, bool
 // Prompts that stay on single CTAs with narrow tiles of 128 tokens: where all tiles of 32 weight rows run at once and K is too short to be
 // split (300 x 512: 6.0 us with 1 k-block, 10.2 with 16, 14.6 with 32; on pairs 9.2, 13.4, 18.2 whole and 11.2 in four parts), and, with K short, where a
 // pair's second half would have no weight rows (15000 x 128 with 1 and 16 k-blocks: 10.1, 16.3 us; on pairs 15.3, 19.9; with 32: 26.2, 25.2).
+static bool is_few_tiles(int64_t m, int64_t n) { return m > 256 && (m + 255) / 256 * ((n + 255) / 256) < sm_count() / 2; }
 static bool lone_prompt(int64_t m, int64_t n, int num_kb, bool one_wave) { return (one_wave && num_kb < 20) || (n <= kBM && num_kb <= 16); }
 
 static bool pair_ws_enabled() {
@@ -1165,7 +1181,7 @@ static int gemm_impl(const int8_t* x8, const int8_t* w8, const int32_t* x_absmax
   // several token tiles, see prompt_tiles.
   const int pairs = sm_count() / 2;
   const bool one_wave = (m + kBM - 1) / kBM * ((n + 31) / 32) <= sm_count();
-  const bool few_tiles = m > 256 && (m + 255) / 256 * ((n + 255) / 256) < pairs;
+  const bool few_tiles = is_few_tiles(m, n);
   const bool prompt_ws = few_tiles && !lone_prompt(m, n, num_kb, one_wave);
   const bool pair_ws = prompt_ws || (m >= pair_min && m <= 256 && pair_ws_enabled());
   const int block_rows = pair_ws ? 2 * kBM : kBM, units = pair_ws ? pairs : sm_count();
@@ -1180,7 +1196,7 @@ static int gemm_impl(const int8_t* x8, const int8_t* w8, const int32_t* x_absmax
     splits = splits < 1 ? 1 : (splits > 8 ? 8 : splits);
     while (splits > 1 && num_kb / splits < 4) --splits;
     while (splits > 1 && (splits - 1) * ((num_kb + splits - 1) / splits) >= num_kb) --splits;   // no empty part
-    if (prompt_ws) splits = prompt_tiles(&p, w_blocks, num_kb, pairs, one_wave);
+    if (prompt_ws) splits = prompt_tiles(&p, w_blocks, num_kb, pairs, one_wave, zero_ws && !out_q15);
     p.splits = splits;
     p.full_blocks = splits > 1 && !prompt_ws ? w_blocks - split_blocks : 0;
     const int64_t col0 = (int64_t)p.full_blocks * block_rows;     // first column that parts are added into
@@ -1263,6 +1279,8 @@ extern "C" int b200_gemm_w8a8_absmax_tail(const int8_t* x8, const int8_t* w8, co
   *tail_col0 = n;
   return gemm_impl(x8, w8, x_absmax, nullptr, nullptr, w_mul, w_shift, out_q15, nullptr, m, n, k, s, zero_ws, tail_col0);
 }
+
+extern "C" int b200_gemm_pending_pays(int64_t m, int64_t n) { return (m > 0 && m <= 256) || (n > 0 && is_few_tiles(m, n)); }
 
 extern "C" int b200_gemm_w8a8_acc_ws(const int8_t* x8, const int8_t* w8, int32_t* zero_ws, int64_t m, int64_t n, int64_t k,
                                      b200_stream_t s) {

@@ -5,6 +5,8 @@ in a workspace and the consumer (add + RMSNorm + quant, or the q/k/v preparation
 while it loads them - the same bits as the materialised Q15.16 tensor of ``apply_weights_q15``
 (layers/quantization/w8a8_int8.py:242-286), two launches fewer per linear.
 
+A prompt of few tiles gains as well: its sums are split over the SMs, and neither the clearing of the sums nor their requantisation is a kernel.
+
 The workspace protocol: a buffer is all zero whenever no linear is pending in it.  The GEMM adds its split-K parts
 into it (no clearing launch), the consumer zeroes every element it reads.  Buffers are kept per (device, width)
 and shared by the linears of that width; calls on one stream follow each other, so at most one linear is pending
@@ -18,9 +20,9 @@ from typing import Optional
 
 import torch
 
-from .._lib import call, ptr, stream
+from .._lib import call, ptr, query, stream
 
-__all__ = ["PendingLinear", "TailLinear", "zero_workspace", "workspace_scope", "reset_workspaces", "PENDING_MAX_ROWS"]
+__all__ = ["PendingLinear", "TailLinear", "leaves_pending", "zero_workspace", "workspace_scope", "reset_workspaces", "PENDING_MAX_ROWS"]
 
 PENDING_MAX_ROWS = 256          # the GEMM splits K (and needs a zeroed buffer) up to this many token rows
 TAIL_MAX_ROWS = 64              # up to here the activation finishes the split columns of gate_up
@@ -46,15 +48,21 @@ class workspace_scope:
 
 
 def zero_workspace(device: torch.device, rows: int, n: int) -> torch.Tensor:
-    """An all-zero int32 [rows, n] view of the buffer kept for (device, n, scope); grows (zeroed) when rows exceed it."""
+    """An all-zero int32 [rows, n] view of the buffer kept for (device, n, scope, rows up to 256 or the next power of two): a buffer is never
+    replaced, since a captured graph may hold it."""
     index = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
-    key = (index, n, _scope[0])
+    cap = max(PENDING_MAX_ROWS, 1 << (rows - 1).bit_length())
+    key = (index, n, _scope[0], cap)
     buf = _workspaces.get(key)
-    if buf is None or buf.shape[0] < rows:
-        cap = max(rows, PENDING_MAX_ROWS)
-        buf = torch.zeros((cap, n), dtype=torch.int32, device=device)
-        _workspaces[key] = buf
+    if buf is None:
+        buf = _workspaces[key] = torch.zeros((cap, n), dtype=torch.int32, device=device)
     return buf[:rows]
+
+
+def leaves_pending(rows: int, n: int) -> bool:
+    """Whether a linear to ``n`` channels is better finished by its consumer (b200_gemm_pending_pays).  Beyond decode sizes only where there are
+    few tiles, less than 5 M sums, so the workspaces stay small."""
+    return query("b200_gemm_pending_pays", rows, n) == 1
 
 
 def reset_workspaces() -> None:

@@ -17,7 +17,7 @@ import torch
 
 from ..attention import Int8PagedKVCache, NewTokens, decode_attention_int8_paged, extend_attention_int8_paged, qkv_rope_quant_store
 from ..kernel import fixed_point as fp
-from ..kernel.pending import PENDING_MAX_ROWS, TAIL_MAX_ROWS, PendingLinear
+from ..kernel.pending import PENDING_MAX_ROWS, TAIL_MAX_ROWS, PendingLinear, leaves_pending
 from ..distributed import DistributedCommunicator
 from .tp_linear import PeerReduceBuffers, TpExchange, row_parallel_q15, row_parallel_q15_fused
 from .w8a8_int8 import W8A8Int8LinearMethod
@@ -112,7 +112,7 @@ class Qwen3DecoderLayerInteger:
                     trace: Optional[dict] = None, defer_down: bool = False, new: Optional[NewTokens] = None):
         """Returns (x_out, residual_out), both Q15.16 int32 [tokens, hidden].
 
-        At decode sizes on one GPU the qkv and o projections are left pending (kernel/pending.py) and finished by
+        At decode sizes and for prompts of few tiles on one GPU the qkv and o projections are left pending (kernel/pending.py) and finished by
         the kernels that read them; with ``defer_down`` the down projection is returned pending too, for the next
         layer's (or the final) add + RMSNorm + quant, and ``x_q15`` may be such a pending linear.  ``new``: what the
         step's layers share about its new tokens (attention.new_tokens)."""
@@ -123,12 +123,13 @@ class Qwen3DecoderLayerInteger:
         w, m = self.w, self.method
         T = x_q15.shape[0]
         tp = self.comm.size > 1 or (self.exchange is not None and self.exchange.size > 1)
-        defer = trace is None and not tp and 0 < T <= PENDING_MAX_ROWS and _PENDING_ON
+        alone = trace is None and not tp and T > 0 and _PENDING_ON
+        defer = lambda l: alone and leaves_pending(T, l.weight.shape[0])
         # input_layernorm (+ residual add) -> int8 codes for qkv_proj
         codes, _, absmax, res, _ = fp.fused_add_rmsnorm_quant(x_q15, residual_q15, w["input_norm"])
         residual = res if residual_q15 is not None else x_q15
         t["ln1_codes"], t["ln1_absmax"] = codes, absmax
-        qkv = m.apply_pending(w["qkv"], codes, absmax) if defer else m.apply_quantised(w["qkv"], codes, absmax)
+        qkv = m.apply_pending(w["qkv"], codes, absmax) if defer(w["qkv"]) else m.apply_quantised(w["qkv"], codes, absmax)
         t["qkv"] = qkv
         qd, kd = self.hq * 128, self.hk * 128
         if trace is None:
@@ -160,7 +161,7 @@ class Qwen3DecoderLayerInteger:
             rowp = lambda l, x: row_parallel_q15(m, l, x, self.comm)
         if tp:
             o = rowp(w["o"], attn.view(T, qd))
-        elif defer and getattr(w["o"], "input_scale", None) is None:
+        elif getattr(w["o"], "input_scale", None) is None and defer(w["o"]):
             a_codes, _, a_absmax = fp.per_token_quant_int8_from_q15(attn.view(T, qd), return_absmax=True)
             o = m.apply_pending(w["o"], a_codes, a_absmax)
         else:
@@ -169,14 +170,14 @@ class Qwen3DecoderLayerInteger:
         # post_attention_layernorm (+ residual add) -> codes for gate_up_proj
         codes, _, absmax, residual, _ = fp.fused_add_rmsnorm_quant(o, residual, w["post_norm"])
         t["ln2_codes"], t["res2"] = codes, residual
-        if defer and _GATE_UP_SILU_ON and self.hadamard_block in (0, 128) and m.can_fuse_gate_up_silu(w["gate_up"], T):
+        if alone and T <= PENDING_MAX_ROWS and _GATE_UP_SILU_ON and self.hadamard_block in (0, 128) and m.can_fuse_gate_up_silu(w["gate_up"], T):
             # decode sizes on one GPU: SiLU(gate) * up in the gate_up GEMM's epilogue, then rotation + quant
             act = m.apply_gate_up_silu(w["gate_up"], codes, absmax)
             codes, _, absmax = fp.fwht_quant_q15(act, self.hadamard_block)
             down = (m.apply_pending if defer_down else m.apply_quantised)(w["down"], codes, absmax)
             return down, residual
         # (more rows are faster with the requantisation in a kernel of its own: a step of 256 rows 9.19 ms, 9.33 without)
-        tail = defer and T <= TAIL_MAX_ROWS and self.inter % 128 == 0 and self.hadamard_block in (0, 128)
+        tail = alone and T <= TAIL_MAX_ROWS and self.inter % 128 == 0 and self.hadamard_block in (0, 128)
         gate_up = m.apply_tail(w["gate_up"], codes, absmax) if tail else m.apply_quantised(w["gate_up"], codes, absmax)
         t["gate_up"] = gate_up
         if tp:   # the token's absmax spans all ranks' columns: rotate locally, agree on the scale, then quantise
@@ -184,6 +185,6 @@ class Qwen3DecoderLayerInteger:
         else:
             codes, _, absmax, _ = fp.silu_mul_fwht_quant(gate_up, self.hadamard_block)
             t["act_codes"], t["act_absmax"] = codes, absmax
-            down = (m.apply_pending if defer and defer_down else m.apply_quantised)(w["down"], codes, absmax)
+            down = (m.apply_pending if defer_down and defer(w["down"]) else m.apply_quantised)(w["down"], codes, absmax)
         t["down"] = down
         return down, residual

@@ -97,3 +97,25 @@ def test_a_step_that_reads_ahead_gives_the_bits_of_one_that_does_not(requests):
             logits = model.method.apply_quantised(model.lm_head, codes, absmax)
         out.append([logits] + [t.clone() for i in range(3) for t in (pool.k_cache(i), pool.v_cache(i), pool.meta(i))])
     assert all(torch.equal(a, b) for a, b in zip(*out)) and _workspaces_zero()
+
+
+# One more row than a decode batch, one to four parts of K, several token tiles, single CTAs (a short K), and too many tiles to be left pending
+@pytest.mark.parametrize("m,n,k,pays", [(257, 2048, 512, True), (333, 4096, 4096, True), (333, 6144, 4096, True), (700, 3072, 2048, True), (1025, 1024, 4096, True),
+                                        (2000, 128, 1024, True), (300, 1028, 128, True), (600, 8192, 512, False)])
+def test_prompts_of_few_tiles_are_left_pending(m, n, k, pays):
+    from mini_sgl_integer_b200.kernel import fixed_point as fp
+    from mini_sgl_integer_b200.kernel.pending import leaves_pending
+    from mini_sgl_integer_b200.layers.w8a8_int8 import W8A8Int8LinearMethod
+    codes, absmax, w8, wm, ws, acc, q15 = _linear_case(m + n, m, n, k)
+    assert leaves_pending(m, n) == pays
+    layer, method = _layer(w8, wm, ws), W8A8Int8LinearMethod()
+    rng = np.random.default_rng(m)
+    res, gain = rng.integers(-(2**18), 2**18, (m, n)).astype(np.int32), rng.integers(2**13, 2**15, n).astype(np.int32)
+    want, want_res = ofp.fused_add_rmsnorm_v2(res, q15, gain)
+    for _ in range(2):
+        pending = method.apply_pending(layer, d(codes), d(absmax))
+        np.testing.assert_array_equal(pending.acc.cpu().numpy(), acc)
+        got = fp.fused_add_rmsnorm_quant(pending, d(res), d(gain))
+        np.testing.assert_array_equal(got[0].cpu().numpy(), ofp.per_token_quant_from_q15(want)[0])
+        np.testing.assert_array_equal(got[3].cpu().numpy(), want_res)
+        assert _workspaces_zero()
