@@ -69,10 +69,25 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
   return warp_sum(lane < nw ? scratch[lane] : 0.0f);
 }
 
-// Sum over the parts of a split linear, in order.  The linears of this library give at most kMaxParts, whose loads are all in flight
-// together: in a loop of unknown length they were two or three memory latencies, one after the other.
-constexpr int kMaxParts = 6;
+// Sum over the parts of a split linear, in order.
 __device__ __forceinline__ float part_sum(const float* p, int splits, int64_t stride) {
+  float v = p[0];
+  for (int s = 1; s < splits; ++s) v += p[(int64_t)s * stride];
+  return v;
+}
+__device__ __forceinline__ float4 part_sum4(const float* p, int splits, int64_t stride) {
+  float4 v = *reinterpret_cast<const float4*>(p);
+  for (int s = 1; s < splits; ++s) {
+    const float4 o = *reinterpret_cast<const float4*>(p + (int64_t)s * stride);
+    v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+  }
+  return v;
+}
+// The same sums with all parts in flight together, for kernels of few rows: in a loop of unknown length they are two or three memory
+// latencies, one after the other.  (The registers would cost kernels of many rows their occupancy: latent_prepare of 8186 tokens 90 -> 154 us.)
+// The linears of this library give at most kMaxParts.
+constexpr int kMaxParts = 6;
+__device__ __forceinline__ float part_sum_few(const float* p, int splits, int64_t stride) {
   float v = p[0];
   if (splits > 1) {
     float o[kMaxParts];
@@ -85,7 +100,7 @@ __device__ __forceinline__ float part_sum(const float* p, int splits, int64_t st
   }
   return v;
 }
-__device__ __forceinline__ float4 part_sum4(const float* p, int splits, int64_t stride) {
+__device__ __forceinline__ float4 part_sum4_few(const float* p, int splits, int64_t stride) {
   float4 v = *reinterpret_cast<const float4*>(p);
   if (splits > 1) {
     float4 o[kMaxParts];

@@ -111,7 +111,7 @@ __device__ __forceinline__ void store_pack(bf16* p, const Pack<VEC>& a) {
   }
 }
 
-template <typename T, int VEC, int NV, bool EARLY>
+template <typename T, int VEC, int NV, bool EARLY, bool PARTS = false>
 __global__ void sublayer_end_kernel(const SublayerEnd p, T* __restrict__ x_out_t) {
   __shared__ float scratch[32];
   pdl_launch_dependents();
@@ -192,7 +192,7 @@ __global__ void sublayer_end_kernel(const SublayerEnd p, T* __restrict__ x_out_t
       if (col[i] >= p.width) continue;
       a[i] = load_pack<VEC>(y + base + col[i]);
       int s = 1;
-      if (EARLY && splits > 1) {                     // (part_sum explains why)
+      if (PARTS && splits > 1) {                     // (part_sum_few explains why)
         Pack<VEC> o[kMaxParts];
 #pragma unroll
         for (int u = 1; u < kMaxParts; ++u)
@@ -318,11 +318,11 @@ xielu_kernel(const float* __restrict__ y, int splits, int64_t split_stride, T* _
   const float* src = y + row * n + c;
   T* dst = out + row * out_pitch + c;
   if (vec) {
-    float4 v = part_sum4(src, splits, split_stride);
+    float4 v = part_sum4_few(src, splits, split_stride);
     v.x = xielu_f32(v.x, a, b); v.y = xielu_f32(v.y, a, b); v.z = xielu_f32(v.z, a, b); v.w = xielu_f32(v.w, a, b);
     store4(dst, v);
   } else {
-    for (int k = 0; k < 4 && c + k < n; ++k) dst[k] = from_f32<T>(xielu_f32(part_sum(src + k, splits, split_stride), a, b));
+    for (int k = 0; k < 4 && c + k < n; ++k) dst[k] = from_f32<T>(xielu_f32(part_sum_few(src + k, splits, split_stride), a, b));
   }
 }
 
@@ -339,11 +339,11 @@ gated_silu_kernel(const float* __restrict__ y, int splits, int64_t split_stride,
   const float* src = y + row * y_pitch + (c >> 4) * 32 + (c & 15);
   T* dst = out + row * out_pitch + c;
   if (vec) {
-    const float4 g = part_sum4(src, splits, split_stride), u = part_sum4(src + 16, splits, split_stride);
+    const float4 g = part_sum4_few(src, splits, split_stride), u = part_sum4_few(src + 16, splits, split_stride);
     store4(dst, make_float4(silu_f32(g.x) * u.x, silu_f32(g.y) * u.y, silu_f32(g.z) * u.z, silu_f32(g.w) * u.w));
   } else {
     for (int k = 0; k < 4 && c + k < n; ++k)
-      dst[k] = from_f32<T>(silu_f32(part_sum(src + k, splits, split_stride)) * part_sum(src + 16 + k, splits, split_stride));
+      dst[k] = from_f32<T>(silu_f32(part_sum_few(src + k, splits, split_stride)) * part_sum_few(src + 16 + k, splits, split_stride));
   }
 }
 
@@ -392,7 +392,10 @@ static int launch_sublayer_end(const SublayerEnd& p, T* x_out_t, int64_t rows, c
   // up to four rows per SM, if so many CTAs of the early form's registers are resident (2048 columns: three; 592 rows of them take 5.9 us
   // early and 4.6 late, 400 rows 3.8 and 4.5)
   const bool few = rows <= 592 && rows * threads <= 444 * 256;
-  if (nv <= 1 && few) launch_pdl(sublayer_end_kernel<T, VEC, 1, true>, grid, block, 0, st, p, x_out_t);
+  const bool parts = p.splits > 1 || p.splits2 > 1;         // (a decode step: more registers than 444 CTAs have, but no more than 256 rows)
+  if (nv <= 1 && few && parts) launch_pdl(sublayer_end_kernel<T, VEC, 1, true, true>, grid, block, 0, st, p, x_out_t);
+  else if (nv <= 2 && few && parts) launch_pdl(sublayer_end_kernel<T, VEC, 2, true, true>, grid, block, 0, st, p, x_out_t);
+  else if (nv <= 1 && few) launch_pdl(sublayer_end_kernel<T, VEC, 1, true>, grid, block, 0, st, p, x_out_t);
   else if (nv <= 2 && few) launch_pdl(sublayer_end_kernel<T, VEC, 2, true>, grid, block, 0, st, p, x_out_t);
   else if (nv <= 1) launch_pdl(sublayer_end_kernel<T, VEC, 1, false>, grid, block, 0, st, p, x_out_t);
   else if (nv <= 2) launch_pdl(sublayer_end_kernel<T, VEC, 2, false>, grid, block, 0, st, p, x_out_t);

@@ -97,7 +97,8 @@ latent_prepare_kernel(const PrepareParams p, T* __restrict__ qn, T* __restrict__
 // columns, with the launch: 8186 tokens 123 -> 94 us (88 without that order); 256 tokens in four parts 29.5 -> 18.4; one token in six
 // parts 29.4 -> 17.1.
 constexpr int kPrepareThreads = 256;
-template <typename T>
+// PARTS: of several parts, a decode step.
+template <typename T, bool PARTS>
 __global__ void __launch_bounds__(kPrepareThreads)
 latent_prepare_vec_kernel(const PrepareParams p, T* __restrict__ qn, T* __restrict__ q_lat, T* __restrict__ cache) {
   __shared__ float scratch[32];
@@ -118,12 +119,13 @@ latent_prepare_vec_kernel(const PrepareParams p, T* __restrict__ qn, T* __restri
     pdl_wait();
   }
   const int half = p.rot_dims >> 1;
+  auto sum4 = [&](const float* v) { return PARTS ? part_sum4_few(v, p.splits, p.split_stride) : *reinterpret_cast<const float4*>(v); };
   // columns i .. i + 3 of a rotated vector
   auto rotated4 = [&](const float* v, int i) {
-    const float4 a = part_sum4(v + i, p.splits, p.split_stride);
+    const float4 a = sum4(v + i);
     if (i >= p.rot_dims) return a;
     const bool low = i < half;
-    const float4 o = part_sum4(v + (low ? i + half : i - half), p.splits, p.split_stride);
+    const float4 o = sum4(v + (low ? i + half : i - half));
     const float4 c = *reinterpret_cast<const float4*>(cs + (low ? i : i - half)), s = *reinterpret_cast<const float4*>(cs + half + (low ? i : i - half));
     return low ? make_float4(turn_low(a.x, o.x, c.x, s.x), turn_low(a.y, o.y, c.y, s.y), turn_low(a.z, o.z, c.z, s.z), turn_low(a.w, o.w, c.w, s.w))
                : make_float4(turn_high(a.x, o.x, c.x, s.x), turn_high(a.y, o.y, c.y, s.y), turn_high(a.z, o.z, c.z, s.z), turn_high(a.w, o.w, c.w, s.w));
@@ -132,13 +134,13 @@ latent_prepare_vec_kernel(const PrepareParams p, T* __restrict__ qn, T* __restri
   const int64_t d0 = (int64_t)p.heads * p.head_pitch;
   const bool own = p.dkv_norm && 4 * tid < p.kv_rank;
   float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  if (own) x = part_sum4(src + d0 + 4 * tid, p.splits, p.split_stride);
+  if (own) x = sum4(src + d0 + 4 * tid);
   *reinterpret_cast<float4*>(latent + 4 * tid) = x;
 #pragma unroll 2
   for (int i = tid; i < p.heads * per; i += kPrepareThreads) {
     const int h = i / per, c = i - h * per;
     const float* q = src + (int64_t)h * p.head_pitch;
-    if (c < d4) store4(qn + (t * p.heads + h) * p.qn_pitch + 4 * c, part_sum4(q + 4 * c, p.splits, p.split_stride));
+    if (c < d4) store4(qn + (t * p.heads + h) * p.qn_pitch + 4 * c, sum4(q + 4 * c));
     else store4(q_lat + (t * p.heads + h) * p.lat_pitch + p.kv_rank + 4 * (c - d4), rotated4(q + p.dim, 4 * (c - d4)));
   }
   if (p.lat_pitch > lat)
@@ -890,10 +892,12 @@ extern "C" int b200f_latent_prepare(const float* qd, int splits, int64_t split_s
                    qn_pitch % 4 == 0 && lat_pitch % 4 == 0 && qd_pitch % 4 == 0 && (splits == 1 || split_stride % 4 == 0) && (int64_t)heads * head_pitch < (1ll << 31) &&
                    aligned16(qd) && aligned16(rope) && aligned16(dkv_norm) && aligned16(qn) && aligned16(q_lat) && aligned16(cache);
   if (vec) {
-    if (dtype == B200F_BF16)
-      launch_pdl(latent_prepare_vec_kernel<bf16>, dim3((unsigned)tokens), dim3(kPrepareThreads), 0, (cudaStream_t)s, p, (bf16*)qn, (bf16*)q_lat, (bf16*)cache);
-    else
-      launch_pdl(latent_prepare_vec_kernel<float>, dim3((unsigned)tokens), dim3(kPrepareThreads), 0, (cudaStream_t)s, p, (float*)qn, (float*)q_lat, (float*)cache);
+    const dim3 grid((unsigned)tokens), block(kPrepareThreads);
+    cudaStream_t st = (cudaStream_t)s;
+    if (dtype == B200F_BF16 && splits > 1) launch_pdl(latent_prepare_vec_kernel<bf16, true>, grid, block, 0, st, p, (bf16*)qn, (bf16*)q_lat, (bf16*)cache);
+    else if (dtype == B200F_BF16) launch_pdl(latent_prepare_vec_kernel<bf16, false>, grid, block, 0, st, p, (bf16*)qn, (bf16*)q_lat, (bf16*)cache);
+    else if (splits > 1) launch_pdl(latent_prepare_vec_kernel<float, true>, grid, block, 0, st, p, (float*)qn, (float*)q_lat, (float*)cache);
+    else launch_pdl(latent_prepare_vec_kernel<float, false>, grid, block, 0, st, p, (float*)qn, (float*)q_lat, (float*)cache);
     return check_launch("latent_prepare");
   }
   if (dtype == B200F_BF16)

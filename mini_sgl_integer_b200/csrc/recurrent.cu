@@ -104,9 +104,9 @@ mingru_step_kernel(const MinGruParams p, T* __restrict__ out) {
   float s = *st;
   if (p.positions[seq] <= 0) s = 0.0f;
   if (p.early) pdl_wait();
-  const float zp = part_sum(src, p.splits, p.split_stride) + bz;
-  const float up = part_sum(src + p.width, p.splits, p.split_stride) + bu;
-  const float g = part_sum(src + 2 * p.width, p.splits, p.split_stride);
+  const float zp = part_sum_few(src, p.splits, p.split_stride) + bz;
+  const float up = part_sum_few(src + p.width, p.splits, p.split_stride) + bu;
+  const float g = part_sum_few(src + 2 * p.width, p.splits, p.split_stride);
   float a, b;
   mingru_gate(zp, up, &a, &b);
   s = fmaf(a, s, b);
