@@ -474,6 +474,29 @@ B200_API int b200_tp_set_timeout_us(int64_t microseconds);    /* synchronises wi
  * Synchronises with the device.  No counterpart in the reference. */
 B200_API int b200_gemm_status(int* out_host, int reset);
 
+/* ---- All layers of a step on one GPU, and the final norm: what Qwen3DecoderLayerInteger.forward_q15 launches (models/integer/qwen3_integer.py:62-123), in
+ * one call.  Every member is eight bytes; pointers are device pointers.  Workspaces as for the pending linears above: ws_qkv
+ * [tokens, (q_heads + 2 kv_heads) * 128] and ws_hidden [tokens, hidden] where b200_gemm_pending_pays (else NULL), ws_gate_up [tokens, 2 inter] up to 256 tokens.
+ * scratch: b200_qwen3_scratch_bytes, 256-byte aligned.  q_lens NULL: a decode step (one token for each of `batch` sequences, b200_attn_decode), else
+ * prompts (b200_attn_prefill; longest: most new tokens of one).  launches (host memory): entry points called. */
+typedef struct { const int8_t* weight; const int32_t *mul, *shift; } b200_linear;
+typedef struct {
+  b200_linear qkv, o, gate_up, down;
+  const int32_t *input_norm, *post_norm, *q_norm, *k_norm;
+  int8_t *k_codes, *v_codes;
+  int32_t* meta;
+} b200_qwen3_layer;
+typedef struct {
+  int64_t tokens, layers, hidden, q_heads, kv_heads, inter, hadamard_block, num_pages, max_pos, table_pitch, batch, max_kv_len, longest, tail_rows;
+  const int32_t *x, *positions, *out_loc, *cos_sin, *page_table, *kv_lens, *row_order, *q_lens, *q_start, *final_norm;
+  int32_t *ws_qkv, *ws_hidden, *ws_gate_up;
+  void* scratch;
+  int8_t* codes;
+  int32_t* absmax;
+} b200_qwen3_step;
+B200_API int64_t b200_qwen3_scratch_bytes(int64_t tokens, int64_t hidden, int64_t q_heads, int64_t kv_heads, int64_t inter);
+B200_API int b200_qwen3_layers(const b200_qwen3_step* step, const b200_qwen3_layer* layers, int64_t* launches, b200_stream_t s);
+
 /* on != 0: from here on, until it is called with 0, the calling thread's launches use weights that no kernel of this library writes,
  * and its GEMMs of decode size may read them while the kernels in front of them still run.  The next launch is made
  * in full stream order, so that whatever wrote the weights earlier in the stream has completed; launches of other streams

@@ -60,6 +60,8 @@ SIGNATURES: dict[str, list] = {
     "b200_qkv_prepare_pending": [P, P, P, P, P, P, I, P, P, P, P, P, P, P, P, P, L, I, I, L, I, P],
     "b200_gemm_status": [P, I],
     "b200_settled_weights": [I],
+    "b200_qwen3_scratch_bytes": [L, L, L, L, L],
+    "b200_qwen3_layers": [P, P, P, P],
     "b200_quant_given_absmax_q15": [P, P, P, L, I, P],
     "b200_requant_q15": [P, P, P, P, P, P, L, L, P],
     "b200_attn_decode": [P, P, P, P, P, P, P, L, P, P, P, P, P, I, I, I, L, I, I, P],
@@ -110,7 +112,7 @@ FLOAT_SIGNATURES: dict[str, list] = {
     "b200f_argmax": [P, L, L, L, P, P],
 }
 _SHARED = ("b200_last_error_string", "b200_decode_prepare")      # in every library
-_RESTYPES = {"b200_last_error_string": c_char_p, "b200_attn_workspace_bytes": ctypes.c_size_t,
+_RESTYPES = {"b200_last_error_string": c_char_p, "b200_attn_workspace_bytes": ctypes.c_size_t, "b200_qwen3_scratch_bytes": ctypes.c_int64,
              "b200_tp_block_bytes": ctypes.c_size_t, "b200f_latent_attn_ws_floats": ctypes.c_size_t, "b200f_gemm_f32_ws_bytes": ctypes.c_int64,
              "b200f_grouped_attn_ws_floats": ctypes.c_size_t, "b200f_memory_scan_ws_bytes": ctypes.c_size_t}
 
@@ -182,6 +184,12 @@ def call(name: str, *args) -> None:
     if rc != 0:
         msg = lib.b200_last_error_string().decode("utf-8", "replace")
         raise B200Error(name, rc, msg)
+
+
+def count_calls(more: int) -> None:
+    """Entry points that native code has called in the place of ``call``."""
+    global CALLS
+    CALLS += more
 
 
 def query(name: str, *args) -> int:

@@ -20,7 +20,7 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 INCLUDE = os.path.join(os.path.dirname(PKG_DIR), "include")
 LIBRARIES = {
     "int": ("libb200int.so", ["runtime.cu", "api.cu", "batch_ops.cu", "rowops.cu", "attn.cu", "attn_split.cu", "attn_prefill.cu",
-                              "gemm.cu", "model_ops.cu", "tp.cu"]),
+                              "gemm.cu", "model_ops.cu", "qwen3_layers.cu", "tp.cu"]),
     "float": ("libb200float.so", ["runtime.cu", "batch_ops.cu", "float_gemm.cu", "float_gemm32.cu", "float_rows.cu", "recurrent.cu", "latent_attn.cu", "matrix_memory.cu",
                                   "grouped_attn.cu"]),
 }

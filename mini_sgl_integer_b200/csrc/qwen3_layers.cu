@@ -1,0 +1,136 @@
+// All layers of an integer step, launched from native code: the sequence of entry points that Qwen3DecoderLayerInteger.forward_q15 goes
+// through on one GPU, with the final norm behind it.  Host code only.
+//
+// A step outside a CUDA graph is eleven launches a layer.  From Python each cost 13 - 17 us with its checks and allocations, from here about four, most
+// of them in the CUDA runtime; a short prompt is bound by that (1.4B shapes, 64 tokens, 24 layers: 4.5 -> 2.0 ms).
+#include "common.cuh"
+
+using namespace b200;
+
+namespace {
+
+// Pieces of the caller's scratch area, 256-byte aligned.
+struct Arena {
+  char* base;
+  int64_t used;
+  template <typename T>
+  T* take(int64_t count) {
+    T* p = reinterpret_cast<T*>(base + used);
+    used += (count * (int64_t)sizeof(T) + 255) / 256 * 256;
+    return p;
+  }
+};
+
+struct Scratch {
+  int8_t *codes, *q8, *attn_codes, *act_codes;
+  int32_t *absmax, *attn_absmax, *act_absmax, *q_mul, *q_shift, *residual[2], *attn, *wide, *narrow;
+  float* scale;
+};
+
+// `wide` holds the qkv output, then gate_up (the first is used up by then); `narrow` the o, then the down output.
+int64_t lay_out(Scratch* s, char* base, int64_t T, int64_t hidden, int64_t q_heads, int64_t kv_heads, int64_t inter) {
+  Arena a{base, 0};
+  const int64_t qd = q_heads * 128, qkv = (q_heads + 2 * kv_heads) * 128;
+  s->codes = a.take<int8_t>(T * hidden);
+  s->q8 = a.take<int8_t>(T * qd);
+  s->attn_codes = a.take<int8_t>(T * qd);
+  s->act_codes = a.take<int8_t>(T * inter);
+  s->absmax = a.take<int32_t>(T);
+  s->attn_absmax = a.take<int32_t>(T);
+  s->act_absmax = a.take<int32_t>(T);
+  s->scale = a.take<float>(T);
+  s->q_mul = a.take<int32_t>(T * q_heads);
+  s->q_shift = a.take<int32_t>(T * q_heads);
+  s->residual[0] = a.take<int32_t>(T * hidden);
+  s->residual[1] = a.take<int32_t>(T * hidden);
+  s->attn = a.take<int32_t>(T * qd);
+  s->wide = a.take<int32_t>(T * (qkv > 2 * inter ? qkv : 2 * inter));
+  s->narrow = a.take<int32_t>(T * hidden);
+  return a.used;
+}
+
+}  // namespace
+
+extern "C" int64_t b200_qwen3_scratch_bytes(int64_t tokens, int64_t hidden, int64_t q_heads, int64_t kv_heads, int64_t inter) {
+  Scratch s;
+  return tokens > 0 && hidden > 0 && q_heads > 0 && kv_heads > 0 && inter > 0 ? lay_out(&s, nullptr, tokens, hidden, q_heads, kv_heads, inter) : 0;
+}
+
+extern "C" int b200_qwen3_layers(const b200_qwen3_step* p, const b200_qwen3_layer* layers, int64_t* launches, b200_stream_t st) {
+  B200_REQUIRE(p && layers && launches, B200_E_NULL, "qwen3_layers: null pointer");
+  B200_REQUIRE(p->tokens > 0 && p->layers > 0 && p->hidden > 0 && p->inter > 0 && p->q_heads > 0 && p->kv_heads > 0 && p->batch > 0, B200_E_SHAPE,
+               "qwen3_layers: tokens=%lld layers=%lld hidden=%lld inter=%lld", (long long)p->tokens, (long long)p->layers, (long long)p->hidden, (long long)p->inter);
+  B200_REQUIRE(p->x && p->scratch && p->final_norm && p->codes && p->absmax, B200_E_NULL, "qwen3_layers: null pointer");
+  const int64_t T = p->tokens, H = p->hidden, qd = p->q_heads * 128, kd = p->kv_heads * 128, qkv = qd + 2 * kd, inter = p->inter;
+  const int hidden = (int)H, hq = (int)p->q_heads, hk = (int)p->kv_heads;
+  Scratch s;
+  lay_out(&s, reinterpret_cast<char*>(p->scratch), T, H, p->q_heads, p->kv_heads, inter);
+  int64_t count = 0;
+  int rc = B200_OK;
+#define B200_STEP(call)              \
+  do {                               \
+    ++count;                         \
+    rc = (call);                     \
+    if (rc != B200_OK) return rc;    \
+  } while (0)
+  // out = requantised x8 w^T: decode sizes add split parts into the kept workspace
+  auto linear = [&](const b200_linear& l, const int8_t* x8, const int32_t* x_absmax, int32_t* out, int32_t* ws, int64_t n, int64_t k) {
+    return T <= 256 && ws && l.shift ? b200_gemm_w8a8_absmax_ws(x8, l.weight, x_absmax, l.mul, l.shift, out, ws, T, n, k, st)
+                                     : b200_gemm_w8a8_absmax(x8, l.weight, x_absmax, l.mul, l.shift, out, nullptr, T, n, k, st);
+  };
+  const int32_t* residual = nullptr;
+  int flip = 0;
+  // residual += the linear that stands in `narrow` or, pending, in its workspace; norm -> codes
+  auto norm = [&](const b200_linear* l, const int32_t* l_absmax, const int32_t* gain, int8_t* codes, int32_t* absmax) {
+    int32_t* next = s.residual[flip];
+    if (!l) {                                        // in front of the first layer: the embedding itself
+      residual = p->x;
+      return b200_rmsnorm_q15(p->x, nullptr, gain, nullptr, nullptr, codes, s.scale, absmax, T, hidden, st);
+    }
+    const int32_t* old = residual;
+    residual = next;
+    flip ^= 1;
+    return p->ws_hidden ? b200_rmsnorm_q15_pending(p->ws_hidden, l_absmax, l->mul, l->shift, old, gain, next, nullptr, codes, s.scale, absmax, T, hidden, st)
+                        : b200_rmsnorm_q15(s.narrow, old, gain, next, nullptr, codes, s.scale, absmax, T, hidden, st);
+  };
+  const b200_linear* before = nullptr;
+  for (int64_t i = 0; i < p->layers; ++i) {
+    const b200_qwen3_layer& l = layers[i];
+    B200_STEP(norm(before, s.act_absmax, l.input_norm, s.codes, s.absmax));
+    if (p->ws_qkv) {
+      B200_STEP(b200_gemm_w8a8_acc_ws(s.codes, l.qkv.weight, p->ws_qkv, T, qkv, H, st));
+      B200_STEP(b200_qkv_prepare_pending(p->positions, p->ws_qkv, s.absmax, l.qkv.mul, l.qkv.shift, p->cos_sin, (int)p->max_pos, l.q_norm, l.k_norm,
+                                         p->out_loc, l.k_codes, l.v_codes, l.meta, s.q8, s.q_mul, s.q_shift, T, hq, hk, p->num_pages, 1, st));
+    } else {
+      B200_STEP(linear(l.qkv, s.codes, s.absmax, s.wide, nullptr, qkv, H));
+      B200_STEP(b200_qkv_prepare_q15(p->positions, s.wide, qkv, s.wide + qd, qkv, s.wide + qd + kd, qkv, p->cos_sin, (int)p->max_pos, l.q_norm, l.k_norm,
+                                     p->out_loc, l.k_codes, l.v_codes, l.meta, s.q8, s.q_mul, s.q_shift, T, hq, hk, p->num_pages, 1, st));
+    }
+    if (p->q_lens)
+      B200_STEP(b200_attn_prefill(s.q8, s.q_mul, s.q_shift, l.k_codes, l.v_codes, l.meta, p->page_table, p->table_pitch, p->kv_lens, p->q_lens, p->q_start,
+                                  s.attn, nullptr, nullptr, (int)p->batch, (int)p->longest, hq, hk, p->num_pages, (int)p->max_kv_len, st));
+    else
+      B200_STEP(b200_attn_decode(s.q8, s.q_mul, s.q_shift, l.k_codes, l.v_codes, l.meta, p->page_table, p->table_pitch, p->kv_lens, p->row_order, s.attn,
+                                 nullptr, nullptr, (int)p->batch, hq, hk, p->num_pages, (int)p->max_kv_len, 0, st));
+    B200_STEP(b200_per_token_quant_q15(s.attn, s.attn_codes, s.scale, s.attn_absmax, T, (int)qd, st));
+    if (p->ws_hidden) B200_STEP(b200_gemm_w8a8_acc_ws(s.attn_codes, l.o.weight, p->ws_hidden, T, H, qd, st));
+    else B200_STEP(linear(l.o, s.attn_codes, s.attn_absmax, s.narrow, nullptr, H, qd));
+    B200_STEP(norm(&l.o, s.attn_absmax, l.post_norm, s.codes, s.absmax));
+    if (p->ws_gate_up && p->tail_rows >= T && inter % 128 == 0) {
+      int64_t col0 = 2 * inter;
+      B200_STEP(b200_gemm_w8a8_absmax_tail(s.codes, l.gate_up.weight, s.absmax, l.gate_up.mul, l.gate_up.shift, s.wide, p->ws_gate_up, &col0, T, 2 * inter, H, st));
+      B200_STEP(b200_silu_mul_q15_tail(s.wide, p->ws_gate_up, s.absmax, l.gate_up.mul, l.gate_up.shift, col0, s.act_codes, s.scale, s.act_absmax, T, (int)inter,
+                                       (int)p->hadamard_block, st));
+    } else {
+      B200_STEP(linear(l.gate_up, s.codes, s.absmax, s.wide, p->ws_gate_up, 2 * inter, H));
+      B200_STEP(b200_silu_mul_q15(s.wide, nullptr, s.act_codes, s.scale, s.act_absmax, T, (int)inter, (int)p->hadamard_block, st));
+    }
+    if (p->ws_hidden) B200_STEP(b200_gemm_w8a8_acc_ws(s.act_codes, l.down.weight, p->ws_hidden, T, H, inter, st));
+    else B200_STEP(linear(l.down, s.act_codes, s.act_absmax, s.narrow, nullptr, H, inter));
+    before = &l.down;
+  }
+  B200_STEP(norm(before, s.act_absmax, p->final_norm, p->codes, p->absmax));
+#undef B200_STEP
+  *launches = count;
+  return B200_OK;
+}

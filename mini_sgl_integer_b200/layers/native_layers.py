@@ -1,0 +1,97 @@
+"""The layers of an integer step from native code (b200_qwen3_layers): the kernels that Qwen3DecoderLayerInteger.forward_q15 launches one by one,
+in one call for all layers."""
+from __future__ import annotations
+
+import ctypes
+from array import array
+from typing import Optional, Tuple
+
+import torch
+
+from .._lib import call, count_calls, i32, query, stream
+from ..attention import Int8PagedKVCache, NewTokens
+from ..attention.ops import _cluster_fits
+from ..kernel.pending import PENDING_MAX_ROWS, TAIL_MAX_ROWS, leaves_pending, zero_workspace
+from . import decoder_layer
+from .w8a8_int8 import W8A8Int8LinearMethod
+
+
+def _plain(t: Optional[torch.Tensor], dtype: torch.dtype, shape: tuple, device: torch.device) -> bool:
+    return t is not None and t.dtype is dtype and t.shape == shape and t.is_contiguous() and t.device == device
+
+
+def layer_pointers(model, T: int, dev: torch.device) -> Optional[array]:
+    """What run_layers needs of the model (Qwen3ModelInteger); None where its layers need what only their own forward has: several ranks,
+    static activation scales, other layouts.  Apart, because it is best done before the step's one wait for the device."""
+    cfg = model.cfg
+    H, hq, hk, inter = cfg.hidden, cfg.num_qo_heads, cfg.num_kv_heads, cfg.inter
+    if T == 0 or not model.layers or model.comm.size > 1 or model.exchange is not None or not decoder_layer._PENDING_ON or decoder_layer._GATE_UP_SILU_ON:
+        return None
+    if cfg.hadamard_block not in (0, 128) or inter % 128 or cfg.head_dim != 128:
+        return None
+    linears = (("qkv", (hq + 2 * hk) * 128, H), ("o", H, hq * 128), ("gate_up", 2 * inter, H), ("down", H, inter))
+    pool, shape = model.pool, (hq, hk, H, inter, cfg.hadamard_block)
+    if type(pool) is not Int8PagedKVCache or pool.kv_heads != hk or pool._k.device != dev:
+        return None
+    caches = [(c.data_ptr(), c.stride(0) * c.element_size()) for c in (pool._k, pool._v, pool._meta)]
+    pointers = array("Q")
+    for layer in model.layers:
+        w = layer.w
+        if type(layer) is not decoder_layer.Qwen3DecoderLayerInteger or layer.peer_buffers is not None or layer.pool is not pool or \
+                layer.cache is not model.cache or type(layer.method) is not W8A8Int8LinearMethod or \
+                (layer.hq, layer.hk, layer.hidden, layer.inter, layer.hadamard_block) != shape:
+            return None
+        for name, rows, k in linears:
+            l = w[name]
+            mul, shift = getattr(l, "weight_mul", None), getattr(l, "weight_shift", None)
+            if mul is None or not _plain(l.weight, torch.int8, (rows, k), dev) or not _plain(mul, torch.int32, (rows,), dev):
+                return None
+            if (shift is not None and not _plain(shift, torch.int32, (rows,), dev)) or (name == "o" and getattr(l, "input_scale", None) is not None):
+                return None
+            pointers.extend((l.weight.data_ptr(), mul.data_ptr(), 0 if shift is None else shift.data_ptr()))
+        for name, size in (("input_norm", H), ("post_norm", H), ("q_norm", 128), ("k_norm", 128)):
+            g = w.get(name)
+            if g is None and size == 128:
+                pointers.append(0)
+            elif _plain(g, torch.int32, (size,), dev):
+                pointers.append(g.data_ptr())
+            else:
+                return None
+        if not 0 <= layer.layer_id < pool.num_layers:
+            return None
+        pointers.extend([at + layer.layer_id * step for at, step in caches])
+    if not _plain(model.w["final_norm"], torch.int32, (H,), dev) or not _plain(model.cache, torch.int32, (model.cache.shape[0], 128), dev):
+        return None
+    return pointers
+
+
+def run_layers(model, pointers: Optional[array], x: torch.Tensor, batch, new: Optional[NewTokens]) -> Optional[Tuple[torch.Tensor, torch.Tensor]]:
+    """The final norm's codes and absmax for the embedding ``x``; None without ``pointers`` (layer_pointers), and where the batch needs the layers' own
+    forward: other layouts, contexts beyond the cluster kernel."""
+    if pointers is None:
+        return None
+    cfg, T, dev, pool = model.cfg, x.shape[0], x.device, model.pool
+    H, hq, hk, inter = cfg.hidden, cfg.num_qo_heads, cfg.num_kv_heads, cfg.inter
+    positions, out_loc, table, kv_lens, order = i32(batch.positions), i32(batch.out_loc), i32(batch.page_table), i32(batch.kv_lens), i32(batch.row_order)
+    n = kv_lens.shape[0]
+    given = [positions, out_loc, table, kv_lens] + ([] if order is None else [order])
+    if not _plain(x, torch.int32, (T, H), dev) or any(t.device != dev for t in given) or \
+            table.ndim != 2 or table.shape[0] != n or positions.numel() != T or out_loc.numel() != T:
+        return None
+    if (batch.q_lens is None) != (new is None) or (new is None and (n != T or not _cluster_fits(hq // hk, batch.max_kv_len))):
+        return None
+    if new is not None and (new.rows != T or new.q_lens.shape[0] != n or new.q_lens.device != dev):
+        return None
+    final, cos_sin = model.w["final_norm"], model.cache
+    workspace = lambda width, wanted: zero_workspace(dev, T, width) if wanted else None
+    ws = [workspace((hq + 2 * hk) * 128, leaves_pending(T, (hq + 2 * hk) * 128)), workspace(H, leaves_pending(T, H)), workspace(2 * inter, T <= PENDING_MAX_ROWS)]
+    scratch = torch.empty(query("b200_qwen3_scratch_bytes", T, H, hq, hk, inter), dtype=torch.uint8, device=dev)
+    codes, absmax = torch.empty((T, H), dtype=torch.int8, device=dev), torch.empty((T, 1), dtype=torch.int32, device=dev)
+    step = array("Q", (T, len(model.layers), H, hq, hk, inter, cfg.hadamard_block, pool.num_pages, cos_sin.shape[0], table.stride(0), n, int(batch.max_kv_len),
+                       0 if new is None else min(new.longest, T), TAIL_MAX_ROWS))
+    step.extend(0 if t is None else t.data_ptr() for t in (x, positions, out_loc, cos_sin, table, kv_lens, order, None if new is None else new.q_lens,
+                                                           None if new is None else new.q_start, final, *ws, scratch, codes, absmax))
+    launches = ctypes.c_int64(0)
+    call("b200_qwen3_layers", step.buffer_info()[0], pointers.buffer_info()[0], ctypes.addressof(launches), stream())
+    count_calls(launches.value - 1)
+    return codes, absmax

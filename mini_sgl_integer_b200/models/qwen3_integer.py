@@ -19,6 +19,7 @@ from ..attention import Int8PagedKVCache, new_tokens
 from ..distributed import DistributedCommunicator
 from ..kernel import fixed_point as fp
 from ..layers.decoder_layer import AttnBatch, Qwen3DecoderLayerInteger, _Linear
+from ..layers.native_layers import layer_pointers, run_layers
 from ..layers.tp_linear import TpExchange
 from ..layers.w8a8_int8 import W8A8Int8LinearMethod
 
@@ -174,6 +175,7 @@ class Qwen3ModelInteger:
         if self.comm.size > 1 and not self.embed_replicated:
             x = self.comm.all_reduce(x)
         T = x.shape[0]
+        pointers = layer_pointers(self, T, x.device)
         new = new_tokens(batch.q_lens, T) if batch.q_lens is not None and self.layers else None
         if self.exchange is not None and self.exchange.size > 1 and self.exchange.fits(T, self.cfg.hidden) and self.layers:
             # tensor parallel on an exchange block: the rows of the residual stream have owners, and every row-split
@@ -185,6 +187,9 @@ class Qwen3ModelInteger:
                 nw = self.layers[i + 1].w["input_norm"] if i + 1 < len(self.layers) else self.w["final_norm"]
                 codes, absmax = layer.forward_codes(codes, absmax, residual, batch, nw, new=new)
             return codes, absmax
+        done = run_layers(self, pointers, x, batch, new)
+        if done is not None:
+            return done
         residual = None
         for layer in self.layers:
             x, residual = layer.forward_q15(x, residual, batch, defer_down=True, new=new)

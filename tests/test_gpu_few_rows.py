@@ -119,3 +119,46 @@ def test_prompts_of_few_tiles_are_left_pending(m, n, k, pays):
         np.testing.assert_array_equal(got[0].cpu().numpy(), ofp.per_token_quant_from_q15(want)[0])
         np.testing.assert_array_equal(got[3].cpu().numpy(), want_res)
         assert _workspaces_zero()
+
+
+# One to 256 decoding requests (pending linears, the activation's tail), prompts of few tiles and of many; no shifts, no q/k norms
+@pytest.mark.parametrize("lens,decode", [([40], True), ([5, 64, 33] * 9, True), ([17] * 200, True), ([3], False), ([100, 1, 60], False), ([300, 90], False), ([900, 1200], False)])
+@pytest.mark.parametrize("plain", [True, False])
+def test_layers_from_native_code_give_the_bits_of_their_own_forward(lens, decode, plain, monkeypatch):
+    from mini_sgl_integer_b200 import _lib
+    from mini_sgl_integer_b200.attention import Int8PagedKVCache
+    from mini_sgl_integer_b200.layers.decoder_layer import AttnBatch
+    from mini_sgl_integer_b200.models import Qwen3ForCausalLMInteger, Qwen3IntegerConfig, qwen3_integer, random_weights
+    cfg = Qwen3IntegerConfig(3, 2304, 8, 2, 1280, 1000, max_pos=2048)
+    weights = random_weights(cfg, 5, generate_on_device=True, qk_norm=plain)
+    if not plain:
+        weights["layers"][1]["gate_up"].weight_shift = weights["layers"][2]["o"].weight_shift = None
+    g = torch.Generator(device="cuda").manual_seed(7)
+    n, pitch = len(lens), -(-max(lens) // 16)
+    table = torch.randperm(n * pitch, device="cuda", generator=g).to(torch.int32).view(n, pitch)
+    kv = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    seq = torch.arange(n, device="cuda") if decode else torch.repeat_interleave(torch.arange(n, device="cuda"), kv.long())
+    pos = kv.long() - 1 if decode else torch.cat([torch.arange(k, device="cuda") for k in lens])
+    loc = (table[seq, pos // 16] * 16 + pos % 16).to(torch.int32)
+    ids = torch.randint(0, 1000, (len(pos),), device="cuda", generator=g, dtype=torch.int32)
+    batch = AttnBatch(pos.to(torch.int32), loc, table, kv, None if decode else kv, max(lens))
+    out, calls = [], []
+    for native in (True, False):
+        pool = Int8PagedKVCache(2, 3, 128, n * pitch, "cuda")
+        for i in range(3):
+            gi = torch.Generator(device="cuda").manual_seed(i)
+            for c in (pool.k_cache(i), pool.v_cache(i)):
+                c.copy_(torch.randint(-127, 128, c.shape, dtype=torch.int8, device="cuda", generator=gi))
+            meta = pool.meta(i)
+            meta[:, :, :32], meta[:, :, 32:40] = 2**30 + 12345, 0x24242424
+        model = Qwen3ForCausalLMInteger(cfg, weights, pool)
+        run = qwen3_integer.run_layers
+        took = []
+        monkeypatch.setattr(qwen3_integer, "run_layers", (lambda *a: took.append(run(*a)) or took[-1]) if native else (lambda *a: None))
+        before = _lib.CALLS
+        logits = model.forward(ids, batch)
+        calls.append(_lib.CALLS - before)
+        monkeypatch.setattr(qwen3_integer, "run_layers", run)
+        assert not native or took[0] is not None
+        out.append([logits] + [t.clone() for i in range(3) for t in (pool.k_cache(i), pool.v_cache(i), pool.meta(i))])
+    assert all(torch.equal(a, b) for a, b in zip(*out)) and _workspaces_zero() and calls[0] == calls[1]
