@@ -235,6 +235,223 @@ qkv_prepare_kernel(const int32_t* __restrict__ positions, const int32_t* __restr
   }
 }
 
+// Many rows: eight lanes per (token, head), 16 values each (elements 4l .. 4l + 3 of every 32), four rows in a warp.  What bounds it is
+// issue, and a third of the instructions of a warp per row were the row's own scalars (absmax to scale, inverse root, reciprocal, place, the
+// division by the head count), computed by 32 lanes alike: here by eight.  The butterfly keeps four of its seven stages within a lane.  q and k rows
+// come first, then v rows, so that a warp has one kind.  8244 tokens x 48 heads
+// 199 -> 141 us (242 -> 176 in a prefill, its rows cold); 333 tokens 10.2 -> 8.4; 256 tokens even, and fewer are too few warps: 50 tokens
+// 3.8 -> 4.9 (so the line of qkv_rows_pay).  Rows of a pending linear, of which there are few, keep a warp each: 333 tokens 14.1 us in a
+// prompt, 17.7 in this form.
+struct QkvRows {
+  const int32_t *positions, *q, *k, *v;
+  int64_t q_pitch, k_pitch, v_pitch;
+  const int32_t *cos_sin, *q_norm, *k_norm, *out_loc;
+  int8_t *k_codes, *v_codes, *q8;
+  int32_t *meta, *q_mul, *q_shift;
+  int64_t tokens, num_pages;
+  int q_heads, kv_heads, max_pos, with_fwht;
+  bool wide;                  // q and k rows, gains, cos and sin on 16 bytes (they need only 8)
+};
+
+__device__ __forceinline__ int4 load4(const int32_t* p, bool wide) {
+  if (wide) return *reinterpret_cast<const int4*>(p);
+  const int2 a = *reinterpret_cast<const int2*>(p), b = *reinterpret_cast<const int2*>(p + 2);
+  return make_int4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ int max8(int v) {       // over a row's eight lanes
+#pragma unroll
+  for (int bit = 1; bit < 8; bit <<= 1) v = max(v, __shfl_xor_sync(FULL_MASK, v, bit));
+  return v;
+}
+__device__ __forceinline__ int absmax16(const int (&x)[16]) {
+  int m = 0;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) m = max(m, abs_wrap(x[i]));
+  return max8(m);
+}
+// The row's codes, four to a word; the choice of the arithmetic is the whole warp's.
+template <bool CLAMP>
+__device__ __forceinline__ void quant16(const int (&x)[16], int m, bool fast, unsigned (&w)[4]) {
+  const float mf = __int2float_rn(m), y = __frcp_rn(mf);
+  if (__all_sync(FULL_MASK, fast && m < (1 << 22))) {
+    const float y127 = __fmul_rn(127.0f, y);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = quant4_bytes_fast_small<CLAMP>(make_int4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]), mf, y127);
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    w[i] = pack4(quant_code_fast(x[4 * i], mf, y), quant_code_fast(x[4 * i + 1], mf, y), quant_code_fast(x[4 * i + 2], mf, y),
+                 quant_code_fast(x[4 * i + 3], mf, y));
+}
+
+__global__ void __launch_bounds__(256)
+qkv_prepare_rows_kernel(const QkvRows p) {
+  pdl_launch_dependents();
+  const int l = threadIdx.x & 7;
+  const unsigned qk = (unsigned)(p.q_heads + p.kv_heads);
+  const unsigned qk_rows = (unsigned)p.tokens * qk, v_rows = (unsigned)p.tokens * (unsigned)p.kv_heads;
+  const unsigned warp = blockIdx.x * 8u + (threadIdx.x >> 5), qk_warps = (qk_rows + 3) >> 2;
+  const bool is_v = warp >= qk_warps;
+  const unsigned row = 4 * (is_v ? warp - qk_warps : warp) + ((threadIdx.x >> 3) & 3), per = is_v ? (unsigned)p.kv_heads : qk;
+  const bool active = row < (is_v ? v_rows : qk_rows);
+  if (!__any_sync(FULL_MASK, active)) return;
+  const unsigned t = active ? row / per : 0, h = active ? row - t * per : 0;
+  const bool is_q = !is_v && h < (unsigned)p.q_heads;
+  const unsigned hh = is_q || is_v ? h : h - (unsigned)p.q_heads;
+  pdl_wait();
+  const int64_t loc = p.out_loc[t];
+  const int64_t pid = loc >> 4;
+  const int tok = (int)(loc & 15);
+  const bool stored = active && (is_q || (loc >= 0 && pid < p.num_pages));   // out-of-pool locations are dropped, never written
+  int x[16];
+  {
+    const int32_t* src = (is_q ? p.q + t * p.q_pitch : is_v ? p.v + t * p.v_pitch : p.k + t * p.k_pitch) + (int64_t)hh * kD + 4 * l;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      int4 a = make_int4(0, 0, 0, 0);
+      if (active) a = load4(src + 32 * i, p.wide || is_v);
+      x[4 * i] = a.x; x[4 * i + 1] = a.y; x[4 * i + 2] = a.z; x[4 * i + 3] = a.w;
+    }
+  }
+  int m = absmax16(x);
+  bool plain = false;
+  if (!is_v) {
+    const int32_t* nw = is_q ? p.q_norm : p.k_norm;
+    if (__any_sync(FULL_MASK, nw != nullptr)) {        // per-head fixed-point RMSNorm over the 128 values
+      const NormRow nr = norm_row_from_absmax(m);
+      unsigned long long sq = 0;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) sq += (unsigned)norm_normalised_sq(x[i], nr.p);
+#pragma unroll
+      for (int bit = 1; bit < 8; bit <<= 1) sq += __shfl_xor_sync(FULL_MASK, sq, bit);
+      const int inv = norm_inv_sqrt((long long)sq, 128, g_inv_sqrt_lut);
+      const bool high = __all_sync(FULL_MASK, nr.p >= 14);
+      if (nw != nullptr) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int4 w = load4(nw + 32 * i + 4 * l, p.wide);
+          if (high) {
+            x[4 * i] = norm_apply_high(x[4 * i], inv, w.x, nr.p - 14);
+            x[4 * i + 1] = norm_apply_high(x[4 * i + 1], inv, w.y, nr.p - 14);
+            x[4 * i + 2] = norm_apply_high(x[4 * i + 2], inv, w.z, nr.p - 14);
+            x[4 * i + 3] = norm_apply_high(x[4 * i + 3], inv, w.w, nr.p - 14);
+          } else {
+            x[4 * i] = nr.zero ? 0 : norm_apply(x[4 * i], inv, w.x, nr.p);
+            x[4 * i + 1] = nr.zero ? 0 : norm_apply(x[4 * i + 1], inv, w.y, nr.p);
+            x[4 * i + 2] = nr.zero ? 0 : norm_apply(x[4 * i + 2], inv, w.z, nr.p);
+            x[4 * i + 3] = nr.zero ? 0 : norm_apply(x[4 * i + 3], inv, w.w, nr.p);
+          }
+        }
+      }
+    }
+    // (rope_row_vals explains the two forms: plain where nothing can saturate)
+    const int32_t* cs = p.cos_sin + (int64_t)max(0, min(p.max_pos - 1, p.positions[t])) * 128 + 4 * l;
+    int c[8], s[8];
+    unsigned unit = 0, top = 0;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int4 a = load4(cs + 32 * i, p.wide), b = load4(cs + 64 + 32 * i, p.wide);
+      c[4 * i] = a.x; c[4 * i + 1] = a.y; c[4 * i + 2] = a.z; c[4 * i + 3] = a.w;
+      s[4 * i] = b.x; s[4 * i + 1] = b.y; s[4 * i + 2] = b.z; s[4 * i + 3] = b.w;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) unit = max(unit, max(abs_u(c[i]), abs_u(s[i])));
+#pragma unroll
+    for (int i = 0; i < 16; ++i) top = max(top, abs_u(x[i]));
+    plain = __all_sync(FULL_MASK, unit <= 32768u && top < (1u << 22));
+    if (plain) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int lo = x[i], hi = x[8 + i];
+        x[i] = rsr15_small((long long)lo * c[i] - (long long)hi * s[i]);
+        x[8 + i] = rsr15_small((long long)lo * s[i] + (long long)hi * c[i]);
+      }
+      if (p.with_fwht) {
+#pragma unroll
+        for (int bit = 1; bit < 16; bit <<= 1)
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if (!(i & bit)) {
+              const int a = x[i], b = x[i | bit];
+              x[i] = a + b;
+              x[i | bit] = a - b;
+            }
+#pragma unroll
+        for (int bit = 1; bit < 8; bit <<= 1) {
+          const int sign = (l & bit) ? -1 : 1;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) x[i] = __shfl_xor_sync(FULL_MASK, x[i], bit) + sign * x[i];
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = fwht_scale128(x[i]);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int lo = x[i], hi = x[8 + i];
+        x[i] = sat32(rsr15((long long)lo * c[i] - (long long)hi * s[i]));
+        x[8 + i] = sat32(rsr15((long long)lo * s[i] + (long long)hi * c[i]));
+      }
+      if (p.with_fwht) {       // saturating, so in the order of the distances: 1, 2, then 4, 8, 16, then 32, 64
+        auto within = [&](int bit) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if (!(i & bit)) {
+              const int a = x[i], b = x[i | bit];
+              x[i] = add_sat(a, b);
+              x[i | bit] = sub_sat(a, b);
+            }
+        };
+        within(1);
+        within(2);
+#pragma unroll 1
+        for (int bit = 1; bit < 8; bit <<= 1)
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const int o = __shfl_xor_sync(FULL_MASK, x[i], bit);
+            x[i] = (l & bit) ? sub_sat(o, x[i]) : add_sat(x[i], o);
+          }
+        within(4);
+        within(8);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = fwht_scale(x[i], 2896);
+      }
+    }
+    m = absmax16(x);
+  }
+  m = max(1, m);
+  unsigned w[4];
+  if (is_v) quant16<true>(x, m, true, w);
+  else quant16<false>(x, m, plain, w);           // (values that did not saturate are not -2^31)
+  int mul, shift;
+  absmax_to_ms_dev(m, &mul, &shift);
+  if (!stored) return;
+  if (is_q) {
+    const int64_t at = (int64_t)t * p.q_heads + hh;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<unsigned*>(p.q8 + at * kD + 32 * i + 4 * l) = w[i];
+    if (l == 0) { p.q_mul[at] = mul; p.q_shift[at] = shift; }
+    return;
+  }
+  const int64_t chunk = pid * p.kv_heads + hh;
+  if (is_v) {
+    int8_t* vdst = p.v_codes + chunk * (kD * kPage);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) vdst[v_chunk_offset(32 * i + 4 * l + e, tok)] = (int8_t)((w[i] >> (8 * e)) & 0xff);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<unsigned*>(p.k_codes + (chunk * kPage + tok) * kD + 32 * i + 4 * l) = w[i];
+  }
+  if (l == 0) {
+    int32_t* mt = p.meta + chunk * kMetaWords + (is_v ? 16 : 0);
+    mt[tok] = mul;
+    reinterpret_cast<int8_t*>(p.meta + chunk * kMetaWords + (is_v ? 36 : 32))[tok] = (int8_t)shift;
+  }
+}
+
 // ============================================================================ decode
 struct DecodeParams {
   const int8_t* q;
@@ -869,6 +1086,9 @@ static int store_common(bool quant, const void* k, int64_t k_pitch, const void* 
   return check_launch(name);
 }
 
+// (32-bit row numbers: 2^31 rows would be a terabyte)
+static bool qkv_rows_pay(int64_t rows) { return rows > 83 * 148 && rows < (1ll << 31); }
+
 extern "C" int b200_qkv_prepare_q15(const int32_t* positions, const int32_t* q, int64_t q_pitch, const int32_t* k,
                                     int64_t k_pitch, const int32_t* v, int64_t v_pitch, const int32_t* cos_sin,
                                     int max_pos, const int32_t* q_norm_w, const int32_t* k_norm_w,
@@ -891,6 +1111,14 @@ extern "C" int b200_qkv_prepare_q15(const int32_t* positions, const int32_t* q, 
   const int64_t warps = tokens * (q_heads + 2 * kv_heads);
   const int64_t blocks = (warps + 7) / 8;
   B200_REQUIRE(blocks < (1ll << 31), B200_E_SHAPE, "qkv_prepare_q15: too many rows");
+  if (qkv_rows_pay(warps)) {
+    const bool wide = aligned16(q) && aligned16(k) && aligned16(cos_sin) && aligned16(q_norm_w) && aligned16(k_norm_w) && q_pitch % 4 == 0 && k_pitch % 4 == 0;
+    const QkvRows p = {positions, q, k, v, q_pitch, k_pitch, v_pitch, cos_sin, q_norm_w, k_norm_w, out_loc, k_codes, v_codes, q8, meta, q_mul, q_shift, tokens,
+                       num_pages, q_heads, kv_heads, max_pos, with_fwht, wide};
+    const int64_t qk = tokens * (q_heads + kv_heads), grid = ((qk + 3) / 4 + (tokens * kv_heads + 3) / 4 + 7) / 8;
+    launch_pdl(qkv_prepare_rows_kernel, dim3((unsigned)grid), dim3(256), 0, (cudaStream_t)s, p);
+    return check_launch("qkv_prepare_q15");
+  }
   const PendingLinear none = {nullptr, nullptr, nullptr, nullptr};
   launch_pdl(qkv_prepare_kernel<false, false>, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)s, positions, q, q_pitch, k, k_pitch, v, v_pitch, cos_sin,
                                                                     max_pos, q_norm_w, k_norm_w, out_loc, k_codes, v_codes,

@@ -162,3 +162,35 @@ def test_layers_from_native_code_give_the_bits_of_their_own_forward(lens, decode
         assert not native or took[0] is not None
         out.append([logits] + [t.clone() for i in range(3) for t in (pool.k_cache(i), pool.v_cache(i), pool.meta(i))])
     assert all(torch.equal(a, b) for a, b in zip(*out)) and _workspaces_zero() and calls[0] == calls[1]
+
+
+# Eight lanes a row (more than 12284 rows of q, k and v heads) against a warp a row: head counts that leave warps partly empty, 8-byte constants, one norm,
+# rows of zeros, of every magnitude up to the saturating ones and of -2^31, dropped places
+@pytest.mark.parametrize("tokens,hq,hk", [(3072, 2, 1), (1759, 5, 1), (1367, 7, 1), (1400, 32, 8)])
+@pytest.mark.parametrize("norms,fwht,shift", [("qk", True, 0), ("q", True, 2), ("", True, 2), ("k", False, 0)])
+def test_qkv_rows_of_eight_lanes_have_the_bits_of_rows_of_a_warp(tokens, hq, hk, norms, fwht, shift):
+    from mini_sgl_integer_b200.attention import Int8PagedKVCache, qkv_rope_quant_store
+    g = torch.Generator(device="cuda").manual_seed(tokens + hq)
+    ints = lambda lo, hi, *shape: torch.randint(lo, hi, shape, dtype=torch.int32, device="cuda", generator=g)
+    heads, pages = hq + 2 * hk, tokens // 16 + 2
+    x = ints(-2**31, 2**31 - 1, tokens, heads, 128) >> ints(0, 32, tokens, heads, 1)       # a magnitude per row: warps of small and of large rows, too
+    x[::3] >>= 13
+    x[5, 0], x[6, :], x[7, -1, 9], x[8, hq, 3] = 0, 0, -2**31, -2**31
+    x = x.reshape(tokens, heads * 128)
+    at = lambda t: torch.cat([t.new_zeros(shift), t.reshape(-1)])[shift:].view(t.shape)      # 8 bytes past a 16-byte boundary
+    angle = torch.rand((300, 64), device="cuda", generator=g) * 6.3
+    cache = at(torch.cat([angle.cos(), angle.sin()], 1).mul(32768).round().to(torch.int32))
+    cache[17, 3] = 40000                                                                     # not of a rotation: the general form
+    gains = {n: at(ints(2**11, 2**14, 128)) if n in norms else None for n in "qk"}
+    pos, loc = ints(0, 300, tokens), torch.randperm(pages * 16, device="cuda", generator=g)[:tokens].to(torch.int32)
+    loc[3], loc[4] = -1, pages * 16 + 5
+    pool = [Int8PagedKVCache(hk, 1, 128, pages, "cuda") for _ in range(2)]
+    for c in pool:
+        c.k_cache(0).zero_(), c.v_cache(0).zero_(), c.meta(0).zero_()
+    step = 12284 // heads
+    run = lambda i, rows, src: qkv_rope_quant_store(pos[rows], src, hq, pool[i], 0, loc[rows], cache, gains["q"], gains["k"], with_fwht=fwht)
+    parts = [run(0, slice(a, a + step), x[a:a + step]) for a in range(0, tokens, step)]
+    want = [torch.cat(p) for p in zip(*parts)]
+    got = run(1, slice(0, tokens), x)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    assert all(torch.equal(a, b) for f in ("k_cache", "v_cache", "meta") for a, b in [(getattr(pool[0], f)(0), getattr(pool[1], f)(0))])
