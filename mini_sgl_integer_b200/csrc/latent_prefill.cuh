@@ -1,0 +1,390 @@
+// Latent attention of bf16 prompts on tcgen05 (part of latent_attn.cu, whose status word its waits use).
+//
+// One CTA: 128 query rows (all heads of 128 / heads tokens, which lie side by side) and up to 256 columns of the output.
+// Tensor memory holds the output (256 columns), two tiles of scores (64 keys each) and the weights, which are the second product's
+// A operand from there; shared memory the queries (up to 9 chunks of 64 latent columns) and one or two tiles of 64 keys.  The cache's
+// rows are both operands: K-major with the keys as N for the scores, N-major with the keys as K for the output, from one copy.
+// More than 256 columns of values are CTAs of their own that form the scores again: tensor memory has room for 512 columns of
+// accumulators in all, and 1.5 times the multiply-adds on tcgen05 are still a small part of what mma.sync took.
+// With one tile of keys in shared memory (rank 512) the chunks that this CTA does not need as values are copied and multiplied
+// while the softmax of the tile before is under way and while its own values are copied.
+//
+// Against the mma.sync kernel (64 rows, 32 keys, operands by ldmatrix; still the one for decode steps and split keys), 16 heads:
+//   rank 512, window 1024: 13 prompts of 200 - 1060 tokens 758 -> 321 us (288 TFLOP/s of the latent space), one of 4000 919 -> 347, of 333 55 -> 27,
+//   of 40 18 -> 12;  rank 256, window 512: 482 -> 127, 342 -> 83, 37 -> 19, 15 -> 12.
+// What bounds it: a tile of 64 keys takes 6000 cycles at rank 512, of which the products are 3400 (a 128 x 64 x 16 product reads its operands from shared
+// memory for longer than it multiplies, 75 cycles), the softmax 1450; the rest is the wait for values, whose place in shared memory (222 KB)
+// the product before had.  Eight softmax warps or four: the same.
+#pragma once
+
+#include "umma.cuh"
+
+namespace b200 {
+
+constexpr int kLpKeys = 64, kLpRows = 128, kLpCols = 256, kLpThreads = 320, kLpMaxChunks = 9;
+constexpr int kLpQChunk = kLpRows * 128, kLpKChunk = kLpKeys * 128;      // bytes of 64 columns
+constexpr unsigned kLpScores = 256, kLpWeights = 384;                    // columns of tensor memory behind the output
+constexpr float kLpSlack = 8.0f;     // an output is rescaled only when its row's maximum has grown by more than 2^8 (weights up to 2^8 are as exact)
+
+struct LatentPrefill {
+  const int32_t* page_table;
+  int64_t table_pitch;
+  const int32_t *kv_lens, *seq_start;
+  const float* sink;
+  int heads, kv_rank, out_pitch, window, tokens_per_cta, batch, q_tiles, chunks, halves;
+  float scale2;
+};
+
+// Which prompts come here: more rows than a tile of the mma.sync kernel, whole chunks of values, and keys that are not worth more than four
+// parts.  (20 new tokens behind 1000 keys, rank 512: 37 us in eight parts, 55 here; 160 new tokens 71 in two parts, 56 here; rank 256: 25 in parts, 23 here.)
+static bool lp_takes(int max_q, int heads, int kv_rank, int rot_dim) {
+  return max_q > 1 && (int64_t)max_q * heads > 64 && heads <= kLpRows && kv_rank % 64 == 0 && kv_rank <= 512 &&
+         (kv_rank + rot_dim + 63) / 64 <= kLpMaxChunks;
+}
+static size_t lp_smem(int chunks, int stages) { return (size_t)chunks * (kLpQChunk + stages * kLpKChunk) + 1024 + 208 + 2 * 2 * kLpRows * 4; }
+
+__device__ __forceinline__ void umma_bf16_ss(unsigned d, uint64_t a, uint64_t b, unsigned idesc, unsigned accumulate) {
+  asm volatile(
+      "{\n.reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_bf16_ts(unsigned d, unsigned a, uint64_t b, unsigned idesc, unsigned accumulate) {      // A from tensor memory
+  asm volatile(
+      "{\n.reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+      ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x32(unsigned taddr, const int (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+      ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x32(unsigned taddr, const int (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};"
+      ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
+        "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
+        "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]), "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// N-major operand of 128-byte rows (64 values of N), 128-byte swizzle: eight rows (of K) are one 1024-byte atom, the next eight
+// follow it, the next 64 values of N lie kLpKChunk further.
+__device__ __forceinline__ uint64_t n_major_desc(unsigned addr) { return make_smem_desc(addr) | ((uint64_t)(kLpKChunk >> 4) << 16); }
+
+__device__ __forceinline__ unsigned ld_shared(unsigned at) {
+  unsigned v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_shared(unsigned at, unsigned v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(v) : "memory"); }
+__device__ __forceinline__ void softmax_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ float lp_exp2(float v) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+template <int STAGES>
+__global__ void __launch_bounds__(kLpThreads, 1)
+latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const LatentPrefill p, bf16* __restrict__ out) {
+  extern __shared__ unsigned char lp_raw[];
+  // sequences vary fastest and a sequence's last tiles, which have most keys, come first
+  const int seq = (int)(blockIdx.x % (unsigned)p.batch), rest = (int)(blockIdx.x / (unsigned)p.batch);
+  const int half = rest % p.halves, q_tile = p.q_tiles - 1 - rest / p.halves;
+  pdl_wait();
+  const int start = p.seq_start[seq], count = p.seq_start[seq + 1] - start, tok0 = q_tile * p.tokens_per_cta;
+  if (tok0 >= count) return;
+  const unsigned base = (smem_u32(lp_raw) + 1023u) & ~1023u;
+  const unsigned q_s = base, k_s = q_s + (unsigned)p.chunks * kLpQChunk, bars = k_s + (unsigned)(STAGES * p.chunks) * kLpKChunk;
+  // key tiles are copied in two groups: the chunks that are this CTA's values (released by the second product) and the others
+  const unsigned q_full = bars, full_x = bars + 8, full_v = bars + 40, empty_x = bars + 72, empty_v = bars + 104, s_full = bars + 136, p_full = bars + 152,
+                 pv_done = bars + 160, tmem_slot = bars + 168, odd_slot = bars + 176, bad_slot = bars + 192, max_s = bars + 208;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int v0 = half * (kLpCols / 64), nv = min(kLpCols, p.kv_rank - half * kLpCols) / 64, nx = p.chunks - nv;      // value chunks v0 .. v0 + nv - 1
+  if (threadIdx.x == 0) {
+    mbar_init(q_full, 1);
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(full_x + 8 * s, 1);
+      mbar_init(full_v + 8 * s, 1);
+      mbar_init(empty_x + 8 * s, 1);
+      mbar_init(empty_v + 8 * s, 1);
+    }
+    mbar_init(s_full, 1);
+    mbar_init(s_full + 8, 1);
+    mbar_init(p_full, 8);
+    mbar_init(pv_done, 1);
+    for (int j = 0; j < 4; ++j) st_shared(odd_slot + 4 * j, 0);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 9) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  pdl_launch_dependents();         // (with its columns in hand: a dependent that waits here would hold them)
+  const unsigned tmem = ld_shared(tmem_slot);
+  const int rows = min(p.tokens_per_cta, count - tok0) * p.heads;
+  const int pos0 = p.kv_lens[seq] - count + tok0;                            // position of the tile's first token
+  const int key_lo = p.window > 0 ? max(pos0 - p.window + 1, 0) : 0, key_hi = pos0 + min(p.tokens_per_cta, count - tok0);
+  const int k0 = key_lo & ~15, tiles = key_hi > key_lo ? (key_hi - k0 + kLpKeys - 1) / kLpKeys : 0;      // (0: tokens in front of the first key)
+
+  if (warp == 8) {
+    // copies: lane j the j-th page of a tile; pages behind the last one repeat it
+    const int32_t* pages = p.page_table + (int64_t)seq * p.table_pitch;
+    const int last = (key_hi - 1) >> 4;
+    if (lane == 0 && tiles > 0) {
+      mbar_expect_tx(q_full, (unsigned)p.chunks * kLpQChunk);
+      for (int c = 0; c < p.chunks; ++c) tma_load_2d(q_s + c * kLpQChunk, &map_q, c * 64, (start + tok0) * p.heads, q_full);
+    }
+    bool ok = true;
+    int i = 0;
+    for (; i < tiles && ok; ++i) {
+      const unsigned s = (unsigned)i % STAGES, ph = ((unsigned)i / STAGES) & 1;
+      const int row = lane < 4 ? pages[min((k0 >> 4) + 4 * i + lane, last)] * 16 : 0;
+      const unsigned dst = k_s + s * (unsigned)p.chunks * kLpKChunk + (unsigned)lane * 2048;
+      ok = __all_sync(FULL_MASK, mbar_wait(empty_x + 8 * s, ph ^ 1, 5));
+      if (!ok) break;
+      if (lane == 0) mbar_expect_tx(full_x + 8 * s, (unsigned)nx * kLpKChunk);
+      __syncwarp();
+      if (lane < 4)
+        for (int c = 0; c < p.chunks; ++c)
+          if (c < v0 || c >= v0 + nv) tma_load_2d(dst + c * kLpKChunk, &map_k, c * 64, row, full_x + 8 * s);
+      ok = __all_sync(FULL_MASK, mbar_wait(empty_v + 8 * s, ph ^ 1, 5));
+      if (!ok) break;
+      if (lane == 0) mbar_expect_tx(full_v + 8 * s, (unsigned)nv * kLpKChunk);
+      __syncwarp();
+      if (lane < 4)
+        for (int c = v0; c < v0 + nv; ++c) tma_load_2d(dst + c * kLpKChunk, &map_k, c * 64, row, full_v + 8 * s);
+    }
+    if (tiles > 0) mbar_wait(q_full, 0, 6);       // whatever became of its consumers, this CTA's own copies land before it leaves
+    for (int t = max(0, i - STAGES); t < i + (ok ? 0 : 1); ++t) {
+      mbar_wait(full_x + 8 * ((unsigned)t % STAGES), ((unsigned)t / STAGES) & 1, 6);
+      if (t < i) mbar_wait(full_v + 8 * ((unsigned)t % STAGES), ((unsigned)t / STAGES) & 1, 6);
+    }
+  } else if (warp == 9) {
+    if (lane == 0 && tiles > 0) {
+      const unsigned base_idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(kLpRows >> 4) << 24);      // fp32 += bf16 x bf16
+      const unsigned s_idesc = base_idesc | ((unsigned)(kLpKeys >> 3) << 17), o_idesc = base_idesc | ((unsigned)(nv * 8) << 17) | (1u << 16);
+      bool first = true;
+      // scores of tile i over chunks [lo, hi) of one group
+      auto scores = [&](int i, bool values, int lo, int hi) {
+        const unsigned s = (unsigned)i % STAGES;
+        if (!mbar_wait((values ? full_v : full_x) + 8 * s, ((unsigned)i / STAGES) & 1, 2)) return false;
+        tcgen05_fence_after();
+        const unsigned d = tmem + kLpScores + kLpKeys * (unsigned)(i & 1), ks = k_s + s * (unsigned)p.chunks * kLpKChunk;
+        for (int g = lo; g < hi; ++g) {
+          const int c = values ? v0 + g : g < v0 ? g : g + nv;
+          const uint64_t da = make_smem_desc(q_s + c * kLpQChunk), db = make_smem_desc(ks + c * kLpKChunk);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            umma_bf16_ss(d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), s_idesc, first ? 0u : 1u);
+            first = false;
+          }
+        }
+        if (!values && hi == nx) tcgen05_commit(empty_x + 8 * s);
+        return true;
+      };
+      bool ok = mbar_wait(q_full, 0, 2) && scores(0, false, 0, nx) && scores(0, true, 0, nv);
+      if (ok) tcgen05_commit(s_full);
+      const int nx0 = STAGES > 1 ? nx : (nx + 1) / 2;            // (one tile of keys: the others while its values are copied)
+      for (int i = 0; i < tiles && ok; ++i) {
+        first = true;
+        if (i + 1 < tiles) {
+          ok = scores(i + 1, false, 0, nx0);
+          if (STAGES > 1 && ok) {
+            ok = scores(i + 1, true, 0, nv);
+            if (ok) tcgen05_commit(s_full + 8 * ((i + 1) & 1));
+          }
+        }
+        ok = ok && mbar_wait(p_full, (unsigned)i & 1, 3);
+        if (!ok) break;
+        tcgen05_fence_after();
+        const uint64_t db = n_major_desc(k_s + (((unsigned)i % STAGES) * (unsigned)p.chunks + (unsigned)v0) * kLpKChunk);
+#pragma unroll
+        for (int k = 0; k < kLpKeys / 16; ++k)                     // 16 keys are 2048 bytes of every chunk, 8 columns of weights
+          umma_bf16_ts(tmem, tmem + kLpWeights + 8 * k, db + (uint64_t)(k * (2048 >> 4)), o_idesc, (i > 0 || k > 0) ? 1u : 0u);
+        tcgen05_commit(empty_v + 8 * ((unsigned)i % STAGES));
+        tcgen05_commit(pv_done);
+        if (STAGES == 1 && i + 1 < tiles) {
+          ok = (nx0 == nx || scores(i + 1, false, nx0, nx)) && scores(i + 1, true, 0, nv);
+          if (ok) tcgen05_commit(s_full + 8 * ((i + 1) & 1));
+        }
+      }
+    }
+    __syncwarp();
+  } else {
+    // softmax: two threads per row, 32 of a tile's keys each; they exchange the maximum, and each adds up its own weights
+    const int part = warp >> 2, r = (int)threadIdx.x & (kLpRows - 1), pos = pos0 + r / p.heads;
+    const int vis_hi = r < rows ? pos : -1, vis_lo = p.window > 0 ? pos - p.window + 1 : 0;
+    const unsigned lanes = tmem + ((unsigned)((warp & 3) * 32) << 16);
+    const int cols = nv * 64, pos_last = key_hi - 1;
+    float m = -INFINITY, l = 0.0f;
+    bool ok = true;
+    for (int i = 0; i < tiles; ++i) {
+      if (ok) ok = __all_sync(FULL_MASK, mbar_wait(s_full + 8 * (i & 1), ((unsigned)i >> 1) & 1, 4));       // (after an expired wait only the barriers are kept)
+      tcgen05_fence_after();
+      const int tile0 = k0 + i * kLpKeys, key0 = tile0 + 32 * part;
+      const unsigned slot = odd_slot + 4 * (i & 3), maxima = max_s + (unsigned)(i & 1) * 2 * kLpRows * 4;
+      // every token of the CTA sees every key of the tile
+      const bool whole = tile0 + kLpKeys - 1 <= pos0 && (p.window == 0 || tile0 >= pos_last - p.window + 1);
+      int v[32];
+      tmem_ld_32x32(lanes + kLpScores + kLpKeys * (unsigned)(i & 1) + 32 * part, v);
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      if (whole) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const float t = __int_as_float(v[j]) * p.scale2;
+          v[j] = __float_as_int(t);
+          mx[j & 3] = fmaxf(mx[j & 3], t);
+        }
+      } else {
+        bool odd = false;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const float raw = __int_as_float(v[j]);
+          odd = odd || !(fabsf(raw) < INFINITY);
+          const float t = key0 + j <= vis_hi && key0 + j >= vis_lo ? raw * p.scale2 : -INFINITY;
+          v[j] = __float_as_int(t);
+          mx[j & 3] = fmaxf(mx[j & 3], t);
+        }
+        if (odd && r < rows) st_shared(slot, 1);
+      }
+      const float mine = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      st_shared(maxima + (unsigned)(part * kLpRows + r) * 4, __float_as_uint(mine));
+      softmax_sync();
+      if (threadIdx.x == 0) st_shared(odd_slot + 4 * ((i + 2) & 3), 0);        // (set again no sooner than behind the next tile's barrier)
+      const float top = fmaxf(mine, __uint_as_float(ld_shared(maxima + (unsigned)((part ^ 1) * kLpRows + r) * 4)));
+      const unsigned vs = k_s + (((unsigned)i % STAGES) * (unsigned)p.chunks + (unsigned)v0) * kLpKChunk;
+      if (!whole) {
+        // A weight of 0 does not stop an infinity or a NaN.  Key rows outside the CTA's range may hold anything: zeros; rows of keys that only
+        // some of the CTA's tokens see and that are not finite (their scores are not either): zeros, and the tokens that see them get NaN.
+        int z_lo = key_lo - tile0, z_hi = key_hi - tile0;
+        uint64_t bad = 0;
+        if (ld_shared(slot)) {
+          if (threadIdx.x == 0) st_shared(bad_slot, 0), st_shared(bad_slot + 4, 0);
+          if (ok) ok = __all_sync(FULL_MASK, mbar_wait(full_v + 8 * ((unsigned)i % STAGES), ((unsigned)i / STAGES) & 1, 4));
+          softmax_sync();
+          for (int key = warp * 8; key < warp * 8 + 8; ++key) {
+            bool inf = false;
+            for (int w = lane; w < nv * 32; w += 32) {
+              const unsigned u = ld_shared(vs + (unsigned)(w >> 5) * kLpKChunk + (unsigned)key * 128 + (unsigned)(w & 31) * 4);
+              inf = inf || (u & 0x7f80u) == 0x7f80u || (u & 0x7f800000u) == 0x7f800000u;
+            }
+            if (__any_sync(FULL_MASK, inf) && lane == 0 && key >= z_lo && key < z_hi)
+              asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(bad_slot + 4 * (unsigned)(key >> 5)), "r"(1u << (key & 31)) : "memory");
+          }
+          softmax_sync();
+          bad = ld_shared(bad_slot) | (uint64_t)ld_shared(bad_slot + 4) << 32;
+        }
+        if (z_lo > 0 || z_hi < kLpKeys || bad) {
+          for (int j = (int)threadIdx.x; j < nv * kLpKeys * 8; j += 256) {
+            const int key = (j >> 3) & (kLpKeys - 1);
+            if (key < z_lo || key >= z_hi || (bad >> key & 1)) asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(vs + (unsigned)j * 16), "r"(0) : "memory");
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          for (int key = 0; bad && key < kLpKeys; ++key)
+            if ((bad >> key & 1) && tile0 + key <= vis_hi && tile0 + key >= vis_lo) l = __int_as_float(0x7fffffff);
+        }
+      }
+      const bool grow = top > m + kLpSlack;
+      const float alpha = grow ? lp_exp2(m - top) : 1.0f;
+      if (grow) m = top;
+      const float mu = m == -INFINITY ? 0.0f : m;                              // no visible key so far: every weight is 0
+      float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      int w[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        w[j] = (int)f32_to_bf16x2(lp_exp2(__int_as_float(v[2 * j]) - mu), lp_exp2(__int_as_float(v[2 * j + 1]) - mu));
+        // the weights as they are multiplied: a row that one key decides comes out as that key's values, whatever its weight was rounded to
+        sum[j & 3] += __int_as_float(w[j] << 16) + __int_as_float(w[j] & (int)0xffff0000);
+      }
+      l = fmaf(l, alpha, (sum[0] + sum[1]) + (sum[2] + sum[3]));
+      if (i > 0) {
+        if (ok) ok = __all_sync(FULL_MASK, mbar_wait(pv_done, (unsigned)(i - 1) & 1, 4));
+        tcgen05_fence_after();
+        if (__any_sync(FULL_MASK, grow)) {
+#pragma unroll 1
+          for (int c = 32 * part; c < cols; c += 64) {
+            int o[32];
+            tmem_ld_32x32(lanes + (unsigned)c, o);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) o[j] = __float_as_int(__int_as_float(o[j]) * alpha);
+            tmem_st_32x32(lanes + (unsigned)c, o);
+          }
+        }
+      }
+      tmem_st_32x32(lanes + kLpWeights + 16 * part, w);
+      tmem_st_wait();
+      tcgen05_fence_before();
+      __syncwarp();
+      if (ok && lane == 0) mbar_arrive(p_full);
+    }
+    if (ok && tiles > 0) ok = __all_sync(FULL_MASK, mbar_wait(pv_done, (unsigned)(tiles - 1) & 1, 4));
+    const unsigned sums = max_s + (unsigned)(tiles & 1) * 2 * kLpRows * 4;       // (the half that the last tile's maxima are not in)
+    st_shared(sums + (unsigned)(part * kLpRows + r) * 4, __float_as_uint(l));
+    softmax_sync();
+    if (ok) {
+      tcgen05_fence_after();
+      const int64_t gr = (int64_t)(start + tok0) * p.heads + r;
+      const float sink2 = r < rows ? p.sink[r % p.heads] * 1.4426950408889634f : 0.0f, mf = fmaxf(m, sink2);
+      l = __uint_as_float(ld_shared(sums + (unsigned)r * 4)) + __uint_as_float(ld_shared(sums + (unsigned)(kLpRows + r) * 4));
+      const float e = exp2f(m - mf), inv = e / (l * e + exp2f(sink2 - mf));
+      bf16* dst = out + gr * p.out_pitch + half * kLpCols;
+#pragma unroll 1
+      for (int c = 32 * part; c < cols; c += 64) {
+        int o[32] = {};
+        if (tiles > 0) tmem_ld_32x32(lanes + (unsigned)c, o);
+        if (r < rows) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            unsigned u[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) u[k] = f32_to_bf16x2(__int_as_float(o[8 * j + 2 * k]) * inv, __int_as_float(o[8 * j + 2 * k + 1]) * inv);
+            *reinterpret_cast<uint4*>(dst + c + 8 * j) = make_uint4(u[0], u[1], u[2], u[3]);
+          }
+        }
+      }
+    }
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  if (warp == 9) {
+    tcgen05_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+  }
+}
+
+// ----------------------------------------------------------------------------- host side
+// bf16 [rows, columns] at a pitch, boxes of 64 columns, 128-byte swizzle; columns behind the last read as zeros
+static bool lp_map(CUtensorMap* map, const void* base, int64_t rows, int columns, int pitch, int box_rows) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  const cuuint64_t dims[2] = {(cuuint64_t)columns, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)pitch * 2};
+  const cuuint32_t box[2] = {64, (cuuint32_t)box_rows}, estr[2] = {1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int STAGES>
+static int launch_latent_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const LatentPrefill& p, bf16* out, cudaStream_t st) {
+  const size_t smem = lp_smem(p.chunks, STAGES);
+  cudaError_t e = cudaFuncSetAttribute(latent_prefill_kernel<STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  B200_REQUIRE(e == cudaSuccess, B200_E_CUDA, "latent_attn: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  launch_pdl(latent_prefill_kernel<STAGES>, dim3((unsigned)((int64_t)p.q_tiles * p.halves * p.batch)), dim3(kLpThreads), smem, st, mq, mk, p, out);
+  return check_launch("latent_attn (prompts)");
+}
+
+}  // namespace b200
