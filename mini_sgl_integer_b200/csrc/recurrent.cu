@@ -1,14 +1,13 @@
 // Gated linear recurrence (minGRU) over fp32 state: S_t = (1 - z_t) S_(t-1) + z_t cand_t, the gates independent of the state.
 //
-// Prompts: one CTA per (sequence, 32 channels).  A lane owns a channel, a warp owns kSeg consecutive tokens of the current
-// stretch of kWarps * kSeg tokens.  Every warp composes its tokens' affine maps (A, B): S -> A S + B, the warps exchange the
+// Prompts: one CTA per (sequence, 32 channels).  A lane owns a channel, a warp owns kScanSeg consecutive tokens of the current
+// stretch of WARPS * kScanSeg tokens.  Every warp composes its tokens' affine maps (A, B): S -> A S + B, the warps exchange the
 // pairs through shared memory, and each then replays its tokens from the state in front of them; gates are read once.
 // Decode: one thread per (sequence, channel).
 #include "float_common.cuh"
 
 namespace b200 {
 
-constexpr int kScanWarps = 16;
 constexpr int kScanSeg = 8;
 
 struct MinGruParams {
@@ -31,14 +30,28 @@ __device__ __forceinline__ void mingru_gate(float zp, float up, float* a, float*
   *b = z * cand;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kScanWarps * 32)
-mingru_scan_kernel(const MinGruParams p, T* __restrict__ out) {
-  __shared__ float2 maps[2][kScanWarps][32];
+// ORDERED: the longest of up to 32 sequences first; CTAs of a long one that start last run on alone.  For more CTAs than start together (13 prompts
+// of 200 - 1060 tokens, 3072 channels: 177 -> 157 us; of 630 each 155 -> 159).  WARPS: 16, which suits long sequences (one of 3500 tokens 172 us,
+// 258 with eight), eight where they have up to 64 tokens on average and the other warps of a CTA would only wait (20 of 32 tokens, 1536
+// channels: 21.8 -> 12; 8 of 40, 3072: 17.2 -> 12).  The bits are the same: eight tokens to a map, maps in order.
+template <typename T, int WARPS, bool ORDERED>
+__device__ __forceinline__ void mingru_scan(const MinGruParams& p, T* __restrict__ out) {
+  __shared__ float2 maps[2][WARPS][32];
   pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int seq = blockIdx.y, c = blockIdx.x * 32 + lane;
+  int seq = blockIdx.y;
+  if (ORDERED) {
+    const int n = (int)gridDim.y;
+    const int len = lane < n ? p.seq_start[lane + 1] - p.seq_start[lane] : 0;
+    int rank = lane < n ? 0 : 32;
+    for (int j = 0; j < n; ++j) {
+      const int o = __shfl_sync(FULL_MASK, len, j);
+      rank += o > len || (o == len && j < lane);
+    }
+    seq = __ffs(__ballot_sync(FULL_MASK, rank == (int)blockIdx.y)) - 1;
+  }
+  const int c = blockIdx.x * 32 + lane;
   const bool live = c < p.width;
   const int t0 = p.seq_start[seq], t1 = p.seq_start[seq + 1];
   if (t0 >= t1) return;
@@ -47,7 +60,7 @@ mingru_scan_kernel(const MinGruParams p, T* __restrict__ out) {
   float carry = (live && p.positions[t0] > 0) ? *st : 0.0f;
   const float bz = live ? p.bias_z[c] : 0.0f, bu = live ? p.bias_u[c] : 0.0f;
   int buf = 0;
-  for (int base = t0; base < t1; base += kScanWarps * kScanSeg, buf ^= 1) {
+  for (int base = t0; base < t1; base += WARPS * kScanSeg, buf ^= 1) {
     const int tw = base + warp * kScanSeg;
     float a[kScanSeg], b[kScanSeg], g[kScanSeg];
 #pragma unroll
@@ -77,7 +90,7 @@ mingru_scan_kernel(const MinGruParams p, T* __restrict__ out) {
     __syncthreads();
     float s = carry;
 #pragma unroll
-    for (int w = 0; w < kScanWarps; ++w) {
+    for (int w = 0; w < WARPS; ++w) {
       if (w == warp) s = carry;
       const float2 m = maps[buf][w][lane];
       carry = fmaf(m.x, carry, m.y);
@@ -89,6 +102,22 @@ mingru_scan_kernel(const MinGruParams p, T* __restrict__ out) {
     }
   }
   if (warp == 0 && live) *st = carry;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(16 * 32)
+mingru_scan_kernel(const MinGruParams p, T* __restrict__ out) {
+  mingru_scan<T, 16, false>(p, out);
+}
+template <typename T>
+__global__ void __launch_bounds__(16 * 32)
+mingru_scan_ordered_kernel(const MinGruParams p, T* __restrict__ out) {
+  mingru_scan<T, 16, true>(p, out);
+}
+template <typename T>
+__global__ void __launch_bounds__(8 * 32, 4)
+mingru_scan_short_kernel(const MinGruParams p, T* __restrict__ out) {
+  mingru_scan<T, 8, false>(p, out);
 }
 
 template <typename T>
@@ -116,8 +145,13 @@ mingru_step_kernel(const MinGruParams p, T* __restrict__ out) {
 
 template <typename T>
 static int mingru_typed(const MinGruParams& p, T* out, int64_t tokens, int batch, cudaStream_t st) {
-  if (p.seq_start)
-    launch_pdl(mingru_scan_kernel<T>, dim3((unsigned)((p.width + 31) / 32), (unsigned)batch), dim3(kScanWarps * 32), 0, st, p, out);
+  const dim3 scan((unsigned)((p.width + 31) / 32), (unsigned)batch);
+  if (p.seq_start && tokens <= 64 * (int64_t)batch)
+    launch_pdl(mingru_scan_short_kernel<T>, scan, dim3(8 * 32), 0, st, p, out);
+  else if (p.seq_start && batch > 1 && batch <= 32 && (int64_t)scan.x * scan.y > 2 * 148)
+    launch_pdl(mingru_scan_ordered_kernel<T>, scan, dim3(16 * 32), 0, st, p, out);
+  else if (p.seq_start)
+    launch_pdl(mingru_scan_kernel<T>, scan, dim3(16 * 32), 0, st, p, out);
   else
     launch_pdl(mingru_step_kernel<T>, dim3((unsigned)((p.width + 255) / 256), (unsigned)batch), dim3(256), 0, st, p, out);
   return check_launch("mingru");

@@ -310,6 +310,24 @@ def test_argmax_takes_the_lowest_index_on_ties():
 
 
 # ----------------------------------------------------------------------------- recurrence
+# Sequences taken longest first (2 to 32 of them, more CTAs than start together), sixteen warps or, for 64 tokens on average, eight: each comes out as
+# it does alone
+@pytest.mark.parametrize("lens", [[300, 1, 129, 300, 17], [64, 64], [64, 65], [5, 0, 128, 7], [40, 70] * 16, [40, 90] * 16 + [3]])
+@pytest.mark.parametrize("width", [72, 2410])
+def test_mingru_sequences_give_the_bits_that_they_give_alone(lens, width):
+    g = torch.Generator(device="cuda").manual_seed(len(lens))
+    zug, bias = torch.randn((1, sum(lens), 3 * width), device="cuda", generator=g), torch.randn((2, width), device="cuda", generator=g)
+    start = np.concatenate([[0], np.cumsum(lens)])
+    pos, old = i32(np.concatenate([np.arange(n) + (i % 2) * 9 for i, n in enumerate(lens)])), torch.randn((len(lens), width), device="cuda", generator=g)
+    out, state = torch.empty((sum(lens), width), device="cuda"), old.clone()
+    fo.mingru(zug, bias[0], bias[1], state, i32(range(len(lens))), pos, i32(start), len(lens), out)
+    for i, n in enumerate(lens):
+        at, alone = slice(start[i], start[i] + n), torch.empty((n, width), device="cuda")
+        if n:
+            fo.mingru(zug[:, at].contiguous(), bias[0], bias[1], old, i32([i]), pos[at], i32([0, n]), 1, alone)
+        assert torch.equal(out[at], alone) and torch.equal(state[i], old[i])
+
+
 @pytest.mark.parametrize("dtype", DT)
 @pytest.mark.parametrize("width", [40, 161, 512])
 def test_mingru_prompts_portions_and_steps(dtype, width):
